@@ -1,0 +1,57 @@
+"""The native eager path: inputs the kernels read in place (views of a fused projection) and inputs that have to be
+copied first (misaligned, expanded) give the results of contiguous tensors; autograd's usual guarantees hold."""
+
+import pytest
+import torch
+
+import triton_sigmoid_b200 as m
+
+pytestmark = pytest.mark.gpu
+
+
+def _views(kind, B, T, H, D, dtype):
+    g = torch.Generator(device="cuda").manual_seed(7)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dtype)  # noqa: E731
+    if kind == "fused":            # [B, T, 3, H, D]
+        return rand(B, T, 3, H, D).unbind(2)
+    if kind == "head_major":       # [B, H, T, D] seen as [B, T, H, D]
+        return [rand(B, H, T, D).transpose(1, 2) for _ in range(3)]
+    if kind == "misaligned":       # rows that start off a 16-byte boundary
+        return rand(B, T, H, 3 * D + 2)[..., 1:1 + 3 * D].split(D, dim=-1)
+    return [rand(B, 1, H, D).expand(B, T, H, D) for _ in range(3)]  # "expanded": stride 0 over the tokens
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("kind", ["fused", "head_major", "misaligned", "expanded"])
+@pytest.mark.parametrize("B,T,D", [(1, 1, 64), (2, 130, 64), (2, 129, 128)])
+def test_strided_inputs_match_contiguous_ones(kind, B, T, D, dtype):
+    H = 2
+    views = _views(kind, B, T, H, D, dtype)
+    results = []
+    for prep in (lambda t: t.detach(), lambda t: t.detach().clone(memory_format=torch.contiguous_format)):
+        q, k, v = [prep(t).requires_grad_() for t in views]
+        out = m.sigmoid_attention(q, k, v, is_causal=True)
+        results.append((out.detach(), *torch.autograd.grad(out.sum(), (q, k, v))))  # (an expanded output gradient)
+    (o, dq, dk, dv), ref = results
+    for a, b in zip((o, dk, dv), (ref[0], ref[2], ref[3])):  # computed in one order: bitwise
+        assert torch.equal(a, b)
+    assert torch.allclose(dq.float(), ref[1].float(), rtol=1e-2, atol=1e-4)  # order of the fp32 reductions
+
+
+def test_inputs_changed_in_place_before_backward_are_refused():
+    q, k, v = [torch.randn(1, 64, 2, 64, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+    q.requires_grad_()
+    out = m.sigmoid_attention(q, k, v)
+    k.add_(1.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.sum().backward()
+
+
+def test_second_backward_needs_retain_graph():
+    q = torch.randn(1, 64, 2, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    out = m.sigmoid_attention(q, q, q).sum()
+    first, = torch.autograd.grad(out, q, retain_graph=True)
+    second, = torch.autograd.grad(out, q)
+    assert torch.equal(first, second)
+    with pytest.raises(RuntimeError, match="backward through the graph a second time"):
+        torch.autograd.grad(out, q)

@@ -1,4 +1,4 @@
-"""Locations shared by the build script and the ctypes binding."""
+"""Locations shared by the build script, the ctypes binding and the torch extension."""
 
 import os
 
@@ -7,3 +7,5 @@ ROOT = os.path.dirname(PKG_DIR)
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_DIR = os.path.join(PKG_DIR, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libsigattn_b200.so")
+EXT_NAME = "_sigattn_torch"
+EXT_PATH = os.path.join(LIB_DIR, EXT_NAME + ".so")

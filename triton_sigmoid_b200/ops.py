@@ -21,7 +21,7 @@ from typing import Optional, Tuple
 import torch
 import torch.nn.functional as F
 
-from . import _cabi
+from . import _cabi, _native
 
 _NS = "sigattn_b200"
 _SUPPORTED_DTYPES = (torch.float16, torch.bfloat16, torch.float32)
@@ -62,12 +62,29 @@ def _accurate() -> bool:
 def accurate_sigmoid(enabled: Optional[bool] = True):
     """Within the block, run the tensor-core kernels with the accurate sigmoid (``True``), the default fast
     one (``False``), or whatever the environment says (``None``)."""
-    global _accurate_override
-    prev, _accurate_override = _accurate_override, enabled
+    prev = _accurate_override
+    _set_accurate(enabled)
     try:
         yield
     finally:
-        _accurate_override = prev
+        _set_accurate(prev)
+
+
+def _set_accurate(enabled: Optional[bool]) -> None:
+    global _accurate_override
+    _accurate_override = enabled
+    ext = _native.loaded()
+    if ext is not None:  # (else it is told when it is loaded)
+        ext.set_accurate(_override_code())
+
+
+def _override_code() -> int:
+    return -1 if _accurate_override is None else int(bool(_accurate_override))
+
+
+def _ext():
+    """The native eager host path (csrc/torch_ext.cpp)."""
+    return _native.loaded() or _native.load(_override_code())
 
 
 def _debug_sync() -> bool:
@@ -299,36 +316,17 @@ def _padded_backward(ctx, dO):
 sigmoid_attn_padded_fwd_op.register_autograd(_padded_backward, setup_context=_padded_setup_context)
 
 
-# ----------------------------------------------------------------------------- eager shortcut
-class _EagerSigmoidAttention(torch.autograd.Function):
-    """What the dense and padded ops do, minus the dispatcher: in eager mode the public functions call the
-    library through this plain autograd function, because a `torch.library.custom_op` round trip with its
-    generated autograd wrapper costs about 100 us of host time per forward + backward pair, which is more
-    than the kernels of a short-sequence call take.  Under `torch.compile` the public functions use the
-    registered ops (fake kernels, autograd registration) instead.  `bias` is a [B] tensor, a Python float
-    (one value for the whole call, passed by value) or None (minus the logarithm of each batch element's
-    number of valid keys, computed by the kernels)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, bias, score_mod, seq_lens_q, seq_lens_k, scale, is_causal):
-        bias_t = bias if isinstance(bias, torch.Tensor) else None
-        ctx.save_for_backward(q, k, v, bias_t, score_mod, seq_lens_q, seq_lens_k)
-        ctx.bias_value = None if bias_t is not None else bias
-        ctx.scale, ctx.is_causal = scale, is_causal
-        return _run_fwd(q, k, v, bias, score_mod, seq_lens_q, seq_lens_k, scale, is_causal)
-
-    @staticmethod
-    def backward(ctx, dO):
-        q, k, v, bias_t, score_mod, seq_lens_q, seq_lens_k = ctx.saved_tensors
-        bias = bias_t if bias_t is not None else ctx.bias_value
-        dq, dk, dv = _run_bwd(q, k, v, dO, bias, score_mod, seq_lens_q, seq_lens_k, ctx.scale, ctx.is_causal)
-        return dq, dk, dv, None, None, None, None, None, None
-
-
-def _eager_attention(q, k, v, bias, score_mod, seq_lens_q, seq_lens_k, scale, is_causal):
-    if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
-        return _EagerSigmoidAttention.apply(q, k, v, bias, score_mod, seq_lens_q, seq_lens_k, scale, is_causal)
-    return _run_fwd(q, k, v, bias, score_mod, seq_lens_q, seq_lens_k, scale, is_causal)
+# ----------------------------------------------------------------------------- eager path
+# In eager mode the public functions call the library through csrc/torch_ext.cpp (allocation, parameters, autograd
+# node), not through the ops above: a `torch.library.custom_op` round trip with its generated autograd wrapper costs
+# about 100 us of host time per forward + backward pair, more than the kernels of a short-sequence call take.  Under
+# `torch.compile` the public functions use the registered ops (fake kernels, autograd registration) instead.
+def _eager_attention(q, k, v, bias, score_mod, seq_lens_q, seq_lens_k, cu_q, cu_k, max_q, max_k, scale, is_causal):
+    """The native path for validated inputs that were not plain: `bias` is a Python float (one value for the whole
+    call) or None (minus the logarithm of each batch element's number of valid keys, computed by the kernels)."""
+    _check_kernel_inputs(q, k, v)
+    _, score_mod, seq_lens_q, seq_lens_k = _prep_aux(q, None, score_mod, seq_lens_q, seq_lens_k)
+    return _ext().attention(q, k, v, score_mod, seq_lens_q, seq_lens_k, cu_q, cu_k, max_q, max_k, bias, scale, is_causal)
 
 
 # ----------------------------------------------------------------------------- packed (variable-length) ops
@@ -460,26 +458,6 @@ def _varlen_backward(ctx, dO):
 sigmoid_attn_varlen_fwd_op.register_autograd(_varlen_backward, setup_context=_varlen_setup_context)
 
 
-class _EagerSigmoidAttentionVarlen(torch.autograd.Function):
-    """The packed entry point's counterpart of :class:`_EagerSigmoidAttention` (same reasons, same `bias` forms)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, cu_q, cu_k, max_q, max_k, bias, score_mod, scale, is_causal):
-        bias_t = bias if isinstance(bias, torch.Tensor) else None
-        ctx.save_for_backward(q, k, v, cu_q, cu_k, bias_t, score_mod)
-        ctx.bias_value = None if bias_t is not None else bias
-        ctx.max_q, ctx.max_k, ctx.scale, ctx.is_causal = max_q, max_k, scale, is_causal
-        return _run_varlen_fwd(q, k, v, cu_q, cu_k, max_q, max_k, bias, score_mod, scale, is_causal)
-
-    @staticmethod
-    def backward(ctx, dO):
-        q, k, v, cu_q, cu_k, bias_t, score_mod = ctx.saved_tensors
-        bias = bias_t if bias_t is not None else ctx.bias_value
-        dq, dk, dv = _run_varlen_bwd(q, k, v, dO, cu_q, cu_k, ctx.max_q, ctx.max_k, bias, score_mod, ctx.scale,
-                                     ctx.is_causal)
-        return dq, dk, dv, None, None, None, None, None, None, None, None
-
-
 # ----------------------------------------------------------------------------- public API
 def _validate_qkv(query, key, value):
     if query.dim() != 4 or key.dim() != 4 or value.dim() != 4:
@@ -537,6 +515,11 @@ def sigmoid_attention(
     gradient.  Same contract as the reference's ``sigmoid_attention``
     (``sigmoid_triton_dense.py:761-853``).
     """
+    compiling = torch.compiler.is_compiling()
+    if not compiling and query.is_cuda:  # plain inputs: everything else happens natively
+        out = _ext().dense(query, key, value, is_causal, scale, sigmoid_bias, score_mod)
+        if out is not None:
+            return out
     B, T_q, T_k, T_v, H, D = _validate_qkv(query, key, value)
     if T_q != T_k or T_q != T_v:
         raise ValueError(f"Dense attention requires same sequence length for Q, K, V, got {T_q}, {T_k}, {T_v}")
@@ -552,14 +535,15 @@ def sigmoid_attention(
     query, key, value = (_pad_head_dim(t, Dk).contiguous() for t in (query, key, value))
 
     bias_value = float(sigmoid_bias) if sigmoid_bias is not None else (-math.log(float(T_q)) if T_q > 0 else 0.0)
-    if torch.compiler.is_compiling():
+    if compiling:
         for x in (query, key, value):
             torch._dynamo.mark_static(x, -2)  # heads
             torch._dynamo.mark_static(x, -1)  # head dimension
         bias = torch.full((B,), bias_value, dtype=torch.float32, device=query.device)
         out = sigmoid_attention_fwd_op(query, key, value, bias, score_mod, float(scale), bool(is_causal))
     else:
-        out = _eager_attention(query, key, value, bias_value, score_mod, None, None, float(scale), bool(is_causal))
+        out = _eager_attention(query, key, value, bias_value, score_mod, None, None, None, None, 0, 0, float(scale),
+                               bool(is_causal))
     return out if Dk == D else out[..., :D]
 
 
@@ -583,11 +567,15 @@ def sigmoid_attention_padded(
     Same contract as the reference's ``sigmoid_attention_padded``
     (``sigmoid_triton_padded.py:853-1010``); lengths outside ``[0, T]`` are clamped.
     """
+    compiling = torch.compiler.is_compiling()
+    if not compiling and query.is_cuda:  # plain inputs: everything else happens natively
+        out = _ext().padded(query, key, value, seq_lens_k, seq_lens_q, is_causal, scale, sigmoid_bias, score_mod)
+        if out is not None:
+            return out
     B, T_q, T_k, T_v, H, D = _validate_qkv(query, key, value)
     if T_k != T_v:
         raise ValueError(f"Key and value sequence lengths must match, got K={T_k}, V={T_v}")
 
-    compiling = torch.compiler.is_compiling()
     full_k = seq_lens_k is None
     if seq_lens_k is None:
         if compiling:  # the op's schema wants tensors; the eager path passes "all valid" as a null pointer
@@ -638,7 +626,8 @@ def sigmoid_attention_padded(
         out = sigmoid_attn_padded_fwd_op(query, key, value, seq_lens_k, seq_lens_q, bias, score_mod, float(scale),
                                          bool(is_causal))
     else:
-        out = _eager_attention(query, key, value, bias, score_mod, seq_lens_q, seq_lens_k, float(scale), bool(is_causal))
+        out = _eager_attention(query, key, value, bias, score_mod, seq_lens_q, seq_lens_k, None, None, 0, 0, float(scale),
+                               bool(is_causal))
     return out if Dk == D else out[..., :D]
 
 
@@ -666,6 +655,12 @@ def sigmoid_attention_varlen(
     shape ``[total_k]``), but no padded tile is loaded or stored.  The reference has no such entry
     point; its benchmark feeds this layout to the flash-attention provider it compares with.
     """
+    compiling = torch.compiler.is_compiling()
+    if not compiling and query.is_cuda:  # plain inputs: everything else happens natively
+        out = _ext().varlen(query, key, value, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, is_causal, scale,
+                            sigmoid_bias, score_mod)
+        if out is not None:
+            return out
     if query.dim() != 3 or key.dim() != 3 or value.dim() != 3:
         raise ValueError("Expected query, key, and value to be 3D tensors [total_tokens, H, D]")
     total_q, H, D = query.shape
@@ -693,7 +688,7 @@ def sigmoid_attention_varlen(
     Dk = _kernel_head_dim(D)
     query, key, value = (_pad_head_dim(t, Dk).contiguous() for t in (query, key, value))
 
-    if torch.compiler.is_compiling():
+    if compiling:
         if sigmoid_bias is None:
             lens_k = (cu_seqlens_k[1:] - cu_seqlens_k[:-1]).clamp(min=0, max=int(max_seqlen_k))
             bias = -torch.log(lens_k.float())  # +inf for an empty key set; every probability is masked there anyway
@@ -702,12 +697,8 @@ def sigmoid_attention_varlen(
         out = sigmoid_attn_varlen_fwd_op(query, key, value, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q),
                                          int(max_seqlen_k), bias, score_mod, float(scale), bool(is_causal))
     else:
-        # eager: no dispatcher round trip, the default bias computed by the kernels, an explicit one passed by value
+        # the default bias is computed by the kernels, an explicit one passed by value
         bias = None if sigmoid_bias is None else float(sigmoid_bias)
-        args = (query, key, value, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), bias, score_mod,
-                float(scale), bool(is_causal))
-        if torch.is_grad_enabled() and (query.requires_grad or key.requires_grad or value.requires_grad):
-            out = _EagerSigmoidAttentionVarlen.apply(*args)
-        else:
-            out = _run_varlen_fwd(*args)
+        out = _eager_attention(query, key, value, bias, score_mod, None, None, cu_seqlens_q, cu_seqlens_k,
+                               int(max_seqlen_q), int(max_seqlen_k), float(scale), bool(is_causal))
     return out if Dk == D else out[..., :D]
