@@ -9,10 +9,24 @@
 // (src/triton_sigmoid/sigmoid_triton_dense.py:23-154, 162-467), so nothing is accumulated
 // across CTAs and the results are run-to-run deterministic.
 //
-// Tiles are 64 x 64; 256 threads as a 16 x 16 grid, thread (ty, tx) owning rows ty + 16 a and
-// columns tx + 16 c of every product (a stride of 16 keeps the shared-memory reads of a warp on
-// distinct banks).  Rows beyond a valid length are zero in shared memory whatever global memory
-// holds, masked probabilities are exactly zero.
+// All three have one structure.  A CTA keeps kRows = 16 kR rows of the stationary side in shared memory and streams
+// tiles of 64 rows of the other side past them.  Its kR x kC warps split a 64-column score tile into 16-row by
+// 64 / kC-column parts; a thread owns 8 rows and every 16th column.  Both products of a step are register-blocked:
+//   scores       s[row][col]  = sum_d A[row][d] B[col][d]   16-byte reads along d on both sides, two partial sums per
+//                               score (even and odd d) so that every pair of FMAs is one packed instruction
+//   accumulation acc[row][d] += W[row][col] X[col][d]       W = P or dS from shared memory, 16-byte reads along col
+// so that a step of 4 in the contraction costs a thread 12 shared-memory reads for 128 FMAs (kC = 1), half of what the
+// shared memory delivers in that time.  What is left is latency (2 - 3 warps per scheduler) and the elementwise step:
+// B=4 T=2048 H=8 D=64 takes 0.82 ms forward and 2.78 ms backward, 42 and 43 TFLOP/s of products done against 25 and 28
+// for 4 x 4 blocks of scalar FMAs with two __syncthreads more per tile (1.37 and 4.31 ms).  W rows are produced and
+// read by the warps of one row group only: a __syncwarp (kC = 1) or a barrier of those kC warps orders them.  Tiles
+// arrive by cp.async, each while the product that does not need it runs.
+//
+// Two shapes: 64 rows per CTA (kR = 4, kC = D / 64) for throughput, and 16 rows (kR = 1, kC = 4) when the larger tiles
+// would not fill the chip: four times as many CTAs and four times the threads per row.
+//
+// Rows beyond a valid length are zero in shared memory whatever global memory holds, masked probabilities are exactly
+// zero.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -40,94 +54,214 @@ struct F32Params {
   int causal;
 };
 
-constexpr int kF32Tile = 64;
-constexpr int kF32Threads = 256;
+constexpr int kF32Cols = 64;  // rows of a streamed tile
 
-template <int D>
-struct F32Smem {
-  static constexpr int kRow = D + 4;             // floats per tile row (padding keeps float4 reads conflict-free)
-  static constexpr int kTileFloats = kF32Tile * kRow;
-  static constexpr int kPRow = kF32Tile + 1;
-  static constexpr int kPFloats = kF32Tile * kPRow;
-  static constexpr int kFwdBytes = (3 * kTileFloats + kPFloats) * 4;        // Q K V | P
-  static constexpr int kDkdvBytes = (4 * kTileFloats + 2 * kPFloats) * 4;   // K V Q dO | P dS
-  static constexpr int kDqBytes = (4 * kTileFloats + kPFloats) * 4;         // Q dO K V | dS
+template <int D, int kR, int kC>
+struct F32Shape {
+  static constexpr int kRows = 16 * kR;
+  static constexpr int kThreads = 32 * kR * kC;
+  static constexpr int kNC = 4 / kC;              // score columns per thread
+  static constexpr int kNX = D / (16 * kC);       // accumulator columns per thread (contiguous, in vectors of kVX)
+  static constexpr int kVX = kNX < 4 ? kNX : 4;
+  static constexpr int kRow = D + 4;              // floats per tile row: 8 consecutive rows start in 8 different 16-byte bank groups
+  static constexpr int kWRow = kF32Cols + 16;     // the two rows a warp writes at a time lie half the banks apart
+  static constexpr int kStatFloats = kRows * kRow;
+  static constexpr int kTileFloats = kF32Cols * kRow;
+  static constexpr int kWFloats = kRows * kWRow;
+  static constexpr int kFwdBytes = (kStatFloats + 2 * kTileFloats + kWFloats) * 4;       // Q | K V | P
+  static constexpr int kDkdvBytes = (2 * kStatFloats + 2 * kTileFloats + 2 * kWFloats) * 4;  // K V | Q dO | P dS
+  static constexpr int kDqBytes = (2 * kStatFloats + 2 * kTileFloats + kWFloats) * 4;    // Q dO | K V | dS
 };
 
-// Rows [row0, row0 + 64) of a (token, head-dim) slab into shared memory; rows at or beyond `limit` are zero.
-template <int D>
-__device__ __forceinline__ void f32_load_tile(float* dst, const float* src, int64_t stride_t, int row0, int limit) {
-  constexpr int kRow = F32Smem<D>::kRow;
-  for (int i = threadIdx.x; i < kF32Tile * (D / 4); i += kF32Threads) {
-    const int r = i / (D / 4), c = i % (D / 4);
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row0 + r < limit) v = *reinterpret_cast<const float4*>(src + (int64_t)(row0 + r) * stride_t + 4 * c);
-    *reinterpret_cast<float4*>(dst + r * kRow + 4 * c) = v;
+__device__ __forceinline__ void f32_cp16(float* dst, const float* src, bool live) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void f32_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void f32_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
+
+// Rows [row0, row0 + kN) of a (token, head-dim) slab into shared memory; rows at or beyond `limit` are zero.
+template <int D, int kN, int kThreads>
+__device__ __forceinline__ void f32_load_rows(float* dst, const float* src, int64_t stride_t, int row0, int limit) {
+  constexpr int kRow = D + 4, kChunks = D / 4;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < kN * kChunks; i += kThreads) {
+    const int r = i / kChunks, c = i % kChunks;
+    const bool live = row0 + r < limit;
+    f32_cp16(dst + r * kRow + 4 * c, live ? src + (int64_t)(row0 + r) * stride_t + 4 * c : src, live);
   }
 }
 
-// acc[a][c] = sum_d A[ty + 16 a][d] * B[tx + 16 c][d]   (both tiles row-major over d)
-template <int D>
-__device__ __forceinline__ void f32_dot_rows(const float* A, const float* Bt, int ty, int tx, float (&acc)[4][4]) {
-  constexpr int kRow = F32Smem<D>::kRow;
+// Where this thread sits: rows row0 + 2 a (a < 8), score columns col0 + 16 c, accumulator columns x0 + ...
+template <typename S>
+struct F32Thread {
+  int row0, col0, x0, group;
+  __device__ __forceinline__ F32Thread(int kR_) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cg = warp / kR_;
+    group = warp % kR_;
+    row0 = 16 * group + (lane >> 4);
+    col0 = cg * 16 * S::kNC + (lane & 15);
+    x0 = cg * 16 * S::kNX + (lane & 15) * S::kVX;
+  }
+};
+
+// The kC warps of one row group have written W and may read each other's part.
+template <int kC>
+__device__ __forceinline__ void f32_group_sync(int group) {
+  if constexpr (kC == 1) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(32 * kC) : "memory");
+}
+
+// s[a][c] = sum_d A[row0 + 2 a][d] * B[col0 + 16 c][d]
+template <int D, int kNC>
+__device__ __forceinline__ void f32_scores(const float* A, const float* B, int row0, int col0, float (&s)[8][kNC]) {
+  constexpr int kRow = D + 4;
+  float2 acc[8][kNC];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < 8; ++a)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) acc[a][c] = 0.f;
+    for (int c = 0; c < kNC; ++c) acc[a][c] = make_float2(0.f, 0.f);
+  const float* ap = A + row0 * kRow;
+  const float* bp = B + col0 * kRow;
 #pragma unroll 4
   for (int d = 0; d < D; d += 4) {
-    float4 av[4], bv[4];
+    float4 b[kNC];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) av[a] = *reinterpret_cast<const float4*>(A + (ty + 16 * a) * kRow + d);
+    for (int c = 0; c < kNC; ++c) b[c] = *reinterpret_cast<const float4*>(bp + 16 * c * kRow + d);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) bv[c] = *reinterpret_cast<const float4*>(Bt + (tx + 16 * c) * kRow + d);
+    for (int a = 0; a < 8; a += 2) {
+      const float4 x = *reinterpret_cast<const float4*>(ap + 2 * a * kRow + d);
+      const float4 y = *reinterpret_cast<const float4*>(ap + (2 * a + 2) * kRow + d);
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        acc[a][c] = fmaf(av[a].x, bv[c].x, acc[a][c]);
-        acc[a][c] = fmaf(av[a].y, bv[c].y, acc[a][c]);
-        acc[a][c] = fmaf(av[a].z, bv[c].z, acc[a][c]);
-        acc[a][c] = fmaf(av[a].w, bv[c].w, acc[a][c]);
+      for (int c = 0; c < kNC; ++c) {
+        acc[a][c] = __ffma2_rn(make_float2(x.x, x.y), make_float2(b[c].x, b[c].y), acc[a][c]);
+        acc[a + 1][c] = __ffma2_rn(make_float2(y.x, y.y), make_float2(b[c].x, b[c].y), acc[a + 1][c]);
       }
+#pragma unroll
+      for (int c = 0; c < kNC; ++c) {
+        acc[a][c] = __ffma2_rn(make_float2(x.z, x.w), make_float2(b[c].z, b[c].w), acc[a][c]);
+        acc[a + 1][c] = __ffma2_rn(make_float2(y.z, y.w), make_float2(b[c].z, b[c].w), acc[a + 1][c]);
+      }
+    }
   }
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int c = 0; c < kNC; ++c) s[a][c] = acc[a][c].x + acc[a][c].y;
 }
 
-// acc[a][c] += sum_j W[j-or-row index] * X[j][tx + 16 c]:
-// kTransposed = false: W row-major [row][j], rows ty + 16 a     (O += P V,  dQ += dS K)
-// kTransposed = true : W row-major [j][col], columns ty + 16 a  (dV += P^T dO, dK += dS^T Q)
-template <int D, bool kTransposed>
-__device__ __forceinline__ void f32_accumulate(const float* W, const float* X, int ty, int tx, float (&acc)[4][D / 16]) {
-  constexpr int kRow = F32Smem<D>::kRow;
-  constexpr int kPRow = F32Smem<D>::kPRow;
+// acc[a][x] += sum_j W[row0 + 2 a][j] * X[j][x0 + ...], j over the 64 rows of a tile
+template <int D, int kNX>
+__device__ __forceinline__ void f32_accumulate(const float* W, const float* X, int row0, int x0, float (&acc)[8][kNX]) {
+  constexpr int kRow = D + 4, kWRow = kF32Cols + 16;
+  constexpr int kVX = kNX < 4 ? kNX : 4;
+  const float* wp = W + row0 * kWRow;
+  const float* xp = X + x0;
 #pragma unroll 4
-  for (int j = 0; j < kF32Tile; ++j) {
-    float w[4], x[D / 16];
+  for (int j = 0; j < kF32Cols; j += 4) {
+    float x[4][kNX];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) w[a] = kTransposed ? W[j * kPRow + ty + 16 * a] : W[(ty + 16 * a) * kPRow + j];
+    for (int jj = 0; jj < 4; ++jj)
 #pragma unroll
-    for (int c = 0; c < D / 16; ++c) x[c] = X[j * kRow + tx + 16 * c];
+      for (int v = 0; v < kNX / kVX; ++v) {
+        const float* src = xp + (j + jj) * kRow + 64 * v;
+        if constexpr (kVX == 4) *reinterpret_cast<float4*>(&x[jj][4 * v]) = *reinterpret_cast<const float4*>(src);
+        else if constexpr (kVX == 2) *reinterpret_cast<float2*>(&x[jj][0]) = *reinterpret_cast<const float2*>(src);
+        else x[jj][0] = *src;
+      }
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 8; a += 2) {
+      const float4 w0 = *reinterpret_cast<const float4*>(wp + 2 * a * kWRow + j);
+      const float4 w1 = *reinterpret_cast<const float4*>(wp + (2 * a + 2) * kWRow + j);
+      const float w[2][4] = {{w0.x, w0.y, w0.z, w0.w}, {w1.x, w1.y, w1.z, w1.w}};
 #pragma unroll
-      for (int c = 0; c < D / 16; ++c) acc[a][c] = fmaf(w[a], x[c], acc[a][c]);
+      for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float wv = w[r][jj];
+          if constexpr (kNX == 1) {
+            acc[a + r][0] = fmaf(wv, x[jj][0], acc[a + r][0]);
+          } else {
+#pragma unroll
+            for (int c = 0; c < kNX; c += 2) {
+              const float2 t = __ffma2_rn(make_float2(wv, wv), make_float2(x[jj][c], x[jj][c + 1]),
+                                          make_float2(acc[a + r][c], acc[a + r][c + 1]));
+              acc[a + r][c] = t.x;
+              acc[a + r][c + 1] = t.y;
+            }
+          }
+        }
+    }
   }
 }
 
-__device__ __forceinline__ float f32_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
+// Rows row0 + 2 a (of the tensor: first + that) below `limit`, times mul; rows at or beyond `live` are zero.
+template <int kNX>
+__device__ __forceinline__ void f32_store_rows(float* base, int64_t stride_t, int first, int row0, int x0, int limit, int live,
+                                               float mul, const float (&acc)[8][kNX]) {
+  constexpr int kVX = kNX < 4 ? kNX : 4;
+#pragma unroll
+  for (int a = 0; a < 8; ++a) {
+    const int i = first + row0 + 2 * a;
+    if (i >= limit) continue;
+    const float m = i < live ? mul : 0.f;
+#pragma unroll
+    for (int v = 0; v < kNX / kVX; ++v) {
+      float* dst = base + (int64_t)i * stride_t + x0 + 64 * v;
+      if constexpr (kVX == 4) {
+        float4 w = make_float4(acc[a][4 * v] * m, acc[a][4 * v + 1] * m, acc[a][4 * v + 2] * m, acc[a][4 * v + 3] * m);
+        if (i >= live) w = make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4*>(dst) = w;
+      } else if constexpr (kVX == 2) {
+        float2 w = make_float2(acc[a][0] * m, acc[a][1] * m);
+        if (i >= live) w = make_float2(0.f, 0.f);
+        *reinterpret_cast<float2*>(dst) = w;
+      } else {
+        *dst = i >= live ? 0.f : acc[a][0] * m;
+      }
+    }
+  }
+}
+
+// With t = e^-|x| in (0, 1]: sigmoid = (x < 0 ? t : 1) / (1 + t).  The divisor lies in [1, 2], so its reciprocal is the
+// hardware's approximation and one Newton-Raphson step, with no special cases (and no branches, which a general
+// division brings along: they cost a quarter of the elementwise step here).
+__device__ __forceinline__ float f32_sigmoid(float x) {
+  const float t = expf(-fabsf(x));
+  const float y = 1.0f + t;
+  float r = rcp_approx(y);
+  r = fmaf(r, fmaf(-y, r, 1.0f), r);
+  return x < 0.f ? t * r : r;
+}
 
 struct F32Item {
   int b, h, Lq, Lk;
+  int tile;          // row tile of the stationary side
   int bc;            // batch coordinate for the strides (0 when packed)
   int tq0, tk0;      // first row of the sequence in the token dimension (0 unless packed)
   int row_lim;       // query rows below this are written (Tq; packed: Lq)
   int key_lim;       // key rows below this are written / have a score_mod entry (Tk; packed: Lk)
   int64_t sm_off;    // offset of the sequence's first key in score_mod
 };
-__device__ __forceinline__ F32Item f32_item(const F32Params& p) {
+// One CTA per (batch, head, row tile).  Without a causal mask the tiles of one head are neighbours in launch order
+// (they read the same streamed side); with one, all heads' heaviest tiles come first (late query tiles, early key
+// tiles), so that the light ones fill the last wave.
+__device__ __forceinline__ F32Item f32_item(const F32Params& p, int n_tiles, bool late_heavy) {
   F32Item it;
-  it.h = blockIdx.y;
-  it.b = blockIdx.z;
+  const unsigned int n_bh = (unsigned int)(p.B * p.H);
+  unsigned int bh;
+  if (p.causal) {
+    bh = blockIdx.x % n_bh;
+    it.tile = (int)(blockIdx.x / n_bh);
+    if (late_heavy) it.tile = n_tiles - 1 - it.tile;
+  } else {
+    bh = blockIdx.x / n_tiles;
+    it.tile = (int)(blockIdx.x % n_tiles);
+  }
+  it.b = (int)(bh / p.H);
+  it.h = (int)(bh % p.H);
   it.Lq = p.Tq;
   it.Lk = p.Tk;
   if (p.lens_q) it.Lq = min(max(p.lens_q[it.b], 0), p.Tq);
@@ -150,102 +284,112 @@ __device__ __forceinline__ F32Item f32_item(const F32Params& p) {
   return it;
 }
 
+// Probabilities of a thread's part of a score tile, in place.  i0 / j0: its first query and key; (di, dj) from one row a
+// to the next, (ci, cj) from one column c to the next.
+template <int kNC, bool kMask>
+__device__ __forceinline__ void f32_probs_of(const F32Params& p, const F32Item& it, float (&s)[8][kNC], int i0, int j0, int di,
+                                             int dj, int ci, int cj, float bias, const float* sm) {
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int c = 0; c < kNC; ++c) {
+      const int i = i0 + a * di + c * ci, j = j0 + a * dj + c * cj;
+      float x = s[a][c] * p.scale + bias;
+      if (sm) x += (!kMask || j < it.key_lim) ? sm[j] : 0.f;
+      float pr = f32_sigmoid(x);
+      if constexpr (kMask) pr = (i < it.Lq && j < it.Lk && (!p.causal || j <= i)) ? pr : 0.f;
+      s[a][c] = pr;
+    }
+}
+template <int kNC>
+__device__ __forceinline__ void f32_probs(const F32Params& p, const F32Item& it, float (&s)[8][kNC], bool all_visible, int i0,
+                                          int j0, int di, int dj, int ci, int cj, float bias, const float* sm) {
+  if (all_visible) f32_probs_of<kNC, false>(p, it, s, i0, j0, di, dj, ci, cj, bias, sm);
+  else f32_probs_of<kNC, true>(p, it, s, i0, j0, di, dj, ci, cj, bias, sm);
+}
+// Every (query, key) pair of the tile [q0, q0 + nq) x [k0, k0 + nk) is visible.
+__device__ __forceinline__ bool f32_all_visible(const F32Params& p, const F32Item& it, int q0, int nq, int k0, int nk) {
+  return q0 + nq <= it.Lq && k0 + nk <= it.Lk && (!p.causal || k0 + nk - 1 <= q0);
+}
+
+// dS from P and dP; a masked element (P exactly 0) stays 0 whatever dP is.
+__device__ __forceinline__ float f32_ds(float pr, float dp) { return pr != 0.f ? pr * (1.0f - pr) * dp : 0.f; }
+
 // ---------------------------------------------------------------- forward
-template <int D>
-__global__ void __launch_bounds__(kF32Threads) sigattn_fwd_f32_kernel(const F32Params p) {
-  using L = F32Smem<D>;
+template <int D, int kR, int kC>
+__global__ void __launch_bounds__(32 * kR * kC, D == 64 && kR == 4 ? 3 : 1) sigattn_fwd_f32_kernel(const F32Params p, const int n_tiles) {
+  using S = F32Shape<D, kR, kC>;
   extern __shared__ float4 f32_smem4[];
   float* Qs = reinterpret_cast<float*>(f32_smem4);
-  float* Ks = Qs + L::kTileFloats;
-  float* Vs = Ks + L::kTileFloats;
-  float* Ps = Vs + L::kTileFloats;
-  const F32Item it = f32_item(p);
-  const int q0 = blockIdx.x * kF32Tile;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  float* Ks = Qs + S::kStatFloats;
+  float* Vs = Ks + S::kTileFloats;
+  float* Ps = Vs + S::kTileFloats;
+  const F32Item it = f32_item(p, n_tiles, true);
+  const F32Thread<S> th(kR);
+  const int q0 = it.tile * S::kRows;
   const float* qb = p.q + (int64_t)it.bc * p.q_sb + (int64_t)it.h * p.q_sh + (int64_t)it.tq0 * p.q_st;
   const float* kb = p.k + (int64_t)it.bc * p.k_sb + (int64_t)it.h * p.k_sh + (int64_t)it.tk0 * p.k_st;
   const float* vb = p.v + (int64_t)it.bc * p.v_sb + (int64_t)it.h * p.v_sh + (int64_t)it.tk0 * p.v_st;
   const float bias = item_bias(p.bias, p.bias_scalar, it.b, it.Lk);
   const float* sm = p.score_mod ? p.score_mod + it.sm_off : nullptr;
 
-  float o[4][D / 16];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int c = 0; c < D / 16; ++c) o[a][c] = 0.f;
-
+  float o[8][S::kNX] = {};
   int kv_end = (q0 < it.Lq) ? it.Lk : 0;
-  if (p.causal) kv_end = min(kv_end, q0 + kF32Tile);
-  if (kv_end > 0) f32_load_tile<D>(Qs, qb, p.q_st, q0, it.Lq);
-  for (int k0 = 0; k0 < kv_end; k0 += kF32Tile) {
-    __syncthreads();  // the previous tile's K, V and P are no longer read
-    f32_load_tile<D>(Ks, kb, p.k_st, k0, it.Lk);
-    f32_load_tile<D>(Vs, vb, p.v_st, k0, it.Lk);
+  if (p.causal) kv_end = min(kv_end, q0 + S::kRows);
+  if (kv_end > 0) {
+    f32_load_rows<D, S::kRows, S::kThreads>(Qs, qb, p.q_st, q0, it.Lq);
+    f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, 0, it.Lk);
+    f32_commit();
+    f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, 0, it.Lk);
+    f32_commit();
+    f32_wait<1>();
     __syncthreads();
-    float s[4][4];
-    f32_dot_rows<D>(Qs, Ks, ty, tx, s);
+  }
+  for (int k0 = 0; k0 < kv_end; k0 += kF32Cols) {
+    const bool more = k0 + kF32Cols < kv_end;
+    {
+      float s[8][S::kNC];
+      f32_scores<D, S::kNC>(Qs, Ks, th.row0, th.col0, s);
+      f32_probs<S::kNC>(p, it, s, f32_all_visible(p, it, q0, S::kRows, k0, kF32Cols), q0 + th.row0, k0 + th.col0, 2, 0, 0, 16,
+                        bias, sm);
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < 8; ++a)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int i = q0 + ty + 16 * a, j = k0 + tx + 16 * c;
-        const bool visible = i < it.Lq && j < it.Lk && (!p.causal || j <= i);
-        float x = s[a][c] * p.scale + bias;
-        if (sm && j < it.key_lim) x += sm[j];
-        Ps[(ty + 16 * a) * L::kPRow + tx + 16 * c] = visible ? f32_sigmoid(x) : 0.f;
-      }
-    __syncthreads();
-    f32_accumulate<D, false>(Ps, Vs, ty, tx, o);
+        for (int c = 0; c < S::kNC; ++c) Ps[(th.row0 + 2 * a) * S::kWRow + th.col0 + 16 * c] = s[a][c];
+    }
+    f32_wait<0>();
+    __syncthreads();  // V has arrived, P is complete, K is no longer read
+    if (more) {
+      f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, k0 + kF32Cols, it.Lk);
+      f32_commit();
+    }
+    f32_accumulate<D, S::kNX>(Ps, Vs, th.row0, th.x0, o);
+    f32_wait<0>();
+    __syncthreads();  // the next K has arrived, V and P are no longer read
+    if (more) {
+      f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, k0 + kF32Cols, it.Lk);
+      f32_commit();
+    }
   }
   float* ob = p.o + (int64_t)it.bc * p.o_sb + (int64_t)it.h * p.o_sh + (int64_t)it.tq0 * p.o_st;
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int i = q0 + ty + 16 * a;
-    if (i < it.row_lim) {
-#pragma unroll
-      for (int c = 0; c < D / 16; ++c) ob[(int64_t)i * p.o_st + tx + 16 * c] = (i < it.Lq) ? o[a][c] : 0.f;
-    }
-  }
-}
-
-// P and dS of one 64 x 64 tile pair into shared memory (rows = queries, columns = keys).
-// Qs, dOs: query tile; Ks, Vs: key tile.  Ps may be nullptr when only dS is wanted.
-template <int D>
-__device__ __forceinline__ void f32_p_and_ds(const F32Params& p, const F32Item& it, const float* Qs, const float* dOs,
-                                             const float* Ks, const float* Vs, float* Ps, float* dSs, int q0, int k0,
-                                             float bias, const float* sm, int ty, int tx) {
-  using L = F32Smem<D>;
-  float s[4][4], dp[4][4];
-  f32_dot_rows<D>(Qs, Ks, ty, tx, s);
-  f32_dot_rows<D>(dOs, Vs, ty, tx, dp);
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int i = q0 + ty + 16 * a, j = k0 + tx + 16 * c;
-      const bool visible = i < it.Lq && j < it.Lk && (!p.causal || j <= i);
-      float x = s[a][c] * p.scale + bias;
-      if (sm && j < it.key_lim) x += sm[j];
-      const float pr = visible ? f32_sigmoid(x) : 0.f;
-      if (Ps) Ps[(ty + 16 * a) * L::kPRow + tx + 16 * c] = pr;
-      dSs[(ty + 16 * a) * L::kPRow + tx + 16 * c] = visible ? pr * (1.0f - pr) * dp[a][c] : 0.f;
-    }
+  f32_store_rows<S::kNX>(ob, p.o_st, q0, th.row0, th.x0, it.row_lim, it.Lq, 1.0f, o);
 }
 
 // ---------------------------------------------------------------- backward: dK, dV of one key tile
-template <int D>
-__global__ void __launch_bounds__(kF32Threads) sigattn_bwd_dkdv_f32_kernel(const F32Params p) {
-  using L = F32Smem<D>;
+// Score tiles are transposed here (rows = keys), so that P^T and dS^T are row-private like P in the forward.
+template <int D, int kR, int kC>
+__global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(const F32Params p, const int n_tiles) {
+  using S = F32Shape<D, kR, kC>;
   extern __shared__ float4 f32_smem4[];
   float* Ks = reinterpret_cast<float*>(f32_smem4);
-  float* Vs = Ks + L::kTileFloats;
-  float* Qs = Vs + L::kTileFloats;
-  float* dOs = Qs + L::kTileFloats;
-  float* Ps = dOs + L::kTileFloats;
-  float* dSs = Ps + L::kPFloats;
-  const F32Item it = f32_item(p);
-  const int k0 = blockIdx.x * kF32Tile;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  float* Vs = Ks + S::kStatFloats;
+  float* Qs = Vs + S::kStatFloats;
+  float* dOs = Qs + S::kTileFloats;
+  float* Ps = dOs + S::kTileFloats;
+  float* dSs = Ps + S::kWFloats;
+  const F32Item it = f32_item(p, n_tiles, false);
+  const F32Thread<S> th(kR);
+  const int k0 = it.tile * S::kRows;
   const float* qb = p.q + (int64_t)it.bc * p.q_sb + (int64_t)it.h * p.q_sh + (int64_t)it.tq0 * p.q_st;
   const float* kb = p.k + (int64_t)it.bc * p.k_sb + (int64_t)it.h * p.k_sh + (int64_t)it.tk0 * p.k_st;
   const float* vb = p.v + (int64_t)it.bc * p.v_sb + (int64_t)it.h * p.v_sh + (int64_t)it.tk0 * p.v_st;
@@ -253,57 +397,74 @@ __global__ void __launch_bounds__(kF32Threads) sigattn_bwd_dkdv_f32_kernel(const
   const float bias = item_bias(p.bias, p.bias_scalar, it.b, it.Lk);
   const float* sm = p.score_mod ? p.score_mod + it.sm_off : nullptr;
 
-  float dk[4][D / 16], dv[4][D / 16];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int c = 0; c < D / 16; ++c) dk[a][c] = dv[a][c] = 0.f;
-
+  float dk[8][S::kNX] = {}, dv[8][S::kNX] = {};
   const int q_end = (k0 < it.Lk) ? it.Lq : 0;
-  const int q_begin = p.causal ? (k0 / kF32Tile) * kF32Tile : 0;  // earlier query tiles see none of these keys
+  const int q_begin = p.causal ? (k0 / kF32Cols) * kF32Cols : 0;  // earlier query tiles see none of these keys
   if (q_begin < q_end) {
-    f32_load_tile<D>(Ks, kb, p.k_st, k0, it.Lk);
-    f32_load_tile<D>(Vs, vb, p.v_st, k0, it.Lk);
+    f32_load_rows<D, S::kRows, S::kThreads>(Ks, kb, p.k_st, k0, it.Lk);
+    f32_load_rows<D, S::kRows, S::kThreads>(Vs, vb, p.v_st, k0, it.Lk);
+    f32_load_rows<D, kF32Cols, S::kThreads>(Qs, qb, p.q_st, q_begin, it.Lq);
+    f32_commit();
+    f32_load_rows<D, kF32Cols, S::kThreads>(dOs, dob, p.do_st, q_begin, it.Lq);
+    f32_commit();
+    f32_wait<1>();
+    __syncthreads();
   }
-  for (int q0 = q_begin; q0 < q_end; q0 += kF32Tile) {
-    __syncthreads();
-    f32_load_tile<D>(Qs, qb, p.q_st, q0, it.Lq);
-    f32_load_tile<D>(dOs, dob, p.do_st, q0, it.Lq);
-    __syncthreads();
-    f32_p_and_ds<D>(p, it, Qs, dOs, Ks, Vs, Ps, dSs, q0, k0, bias, sm, ty, tx);
-    __syncthreads();
-    f32_accumulate<D, true>(Ps, dOs, ty, tx, dv);
-    f32_accumulate<D, true>(dSs, Qs, ty, tx, dk);
+  for (int q0 = q_begin; q0 < q_end; q0 += kF32Cols) {
+    const bool more = q0 + kF32Cols < q_end;
+    {
+      float pr[8][S::kNC];
+      f32_scores<D, S::kNC>(Ks, Qs, th.row0, th.col0, pr);
+      f32_probs<S::kNC>(p, it, pr, f32_all_visible(p, it, q0, kF32Cols, k0, S::kRows), q0 + th.col0, k0 + th.row0, 0, 2, 16, 0,
+                        bias, sm);
+#pragma unroll
+      for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int c = 0; c < S::kNC; ++c) Ps[(th.row0 + 2 * a) * S::kWRow + th.col0 + 16 * c] = pr[a][c];
+      f32_wait<0>();
+      __syncthreads();  // dO has arrived
+      float dp[8][S::kNC];
+      f32_scores<D, S::kNC>(Vs, dOs, th.row0, th.col0, dp);
+#pragma unroll
+      for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int c = 0; c < S::kNC; ++c)
+          dSs[(th.row0 + 2 * a) * S::kWRow + th.col0 + 16 * c] = f32_ds(pr[a][c], dp[a][c]);
+    }
+    f32_group_sync<kC>(th.group);
+    f32_accumulate<D, S::kNX>(dSs, Qs, th.row0, th.x0, dk);
+    __syncthreads();  // Q is no longer read
+    if (more) {
+      f32_load_rows<D, kF32Cols, S::kThreads>(Qs, qb, p.q_st, q0 + kF32Cols, it.Lq);
+      f32_commit();
+    }
+    f32_accumulate<D, S::kNX>(Ps, dOs, th.row0, th.x0, dv);
+    f32_wait<0>();
+    __syncthreads();  // the next Q has arrived, dO, P and dS are no longer read
+    if (more) {
+      f32_load_rows<D, kF32Cols, S::kThreads>(dOs, dob, p.do_st, q0 + kF32Cols, it.Lq);
+      f32_commit();
+    }
   }
   float* dkb = p.dk + (int64_t)it.bc * p.dk_sb + (int64_t)it.h * p.dk_sh + (int64_t)it.tk0 * p.dk_st;
   float* dvb = p.dv + (int64_t)it.bc * p.dv_sb + (int64_t)it.h * p.dv_sh + (int64_t)it.tk0 * p.dv_st;
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int j = k0 + ty + 16 * a;
-    if (j < it.key_lim) {
-      const bool live = j < it.Lk;
-#pragma unroll
-      for (int c = 0; c < D / 16; ++c) {
-        dkb[(int64_t)j * p.dk_st + tx + 16 * c] = live ? dk[a][c] * p.scale : 0.f;
-        dvb[(int64_t)j * p.dv_st + tx + 16 * c] = live ? dv[a][c] : 0.f;
-      }
-    }
-  }
+  f32_store_rows<S::kNX>(dkb, p.dk_st, k0, th.row0, th.x0, it.key_lim, it.Lk, p.scale, dk);
+  f32_store_rows<S::kNX>(dvb, p.dv_st, k0, th.row0, th.x0, it.key_lim, it.Lk, 1.0f, dv);
 }
 
 // ---------------------------------------------------------------- backward: dQ of one query tile
-template <int D>
-__global__ void __launch_bounds__(kF32Threads) sigattn_bwd_dq_f32_kernel(const F32Params p) {
-  using L = F32Smem<D>;
+template <int D, int kR, int kC>
+__global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dq_f32_kernel(const F32Params p, const int n_tiles) {
+  using S = F32Shape<D, kR, kC>;
   extern __shared__ float4 f32_smem4[];
   float* Qs = reinterpret_cast<float*>(f32_smem4);
-  float* dOs = Qs + L::kTileFloats;
-  float* Ks = dOs + L::kTileFloats;
-  float* Vs = Ks + L::kTileFloats;
-  float* dSs = Vs + L::kTileFloats;
-  const F32Item it = f32_item(p);
-  const int q0 = blockIdx.x * kF32Tile;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  float* dOs = Qs + S::kStatFloats;
+  float* Ks = dOs + S::kStatFloats;
+  float* Vs = Ks + S::kTileFloats;
+  float* dSs = Vs + S::kTileFloats;
+  const F32Item it = f32_item(p, n_tiles, true);
+  const F32Thread<S> th(kR);
+  const int q0 = it.tile * S::kRows;
   const float* qb = p.q + (int64_t)it.bc * p.q_sb + (int64_t)it.h * p.q_sh + (int64_t)it.tq0 * p.q_st;
   const float* kb = p.k + (int64_t)it.bc * p.k_sb + (int64_t)it.h * p.k_sh + (int64_t)it.tk0 * p.k_st;
   const float* vb = p.v + (int64_t)it.bc * p.v_sb + (int64_t)it.h * p.v_sh + (int64_t)it.tk0 * p.v_st;
@@ -311,36 +472,50 @@ __global__ void __launch_bounds__(kF32Threads) sigattn_bwd_dq_f32_kernel(const F
   const float bias = item_bias(p.bias, p.bias_scalar, it.b, it.Lk);
   const float* sm = p.score_mod ? p.score_mod + it.sm_off : nullptr;
 
-  float dq[4][D / 16];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int c = 0; c < D / 16; ++c) dq[a][c] = 0.f;
-
+  float dq[8][S::kNX] = {};
   int kv_end = (q0 < it.Lq) ? it.Lk : 0;
-  if (p.causal) kv_end = min(kv_end, q0 + kF32Tile);
+  if (p.causal) kv_end = min(kv_end, q0 + S::kRows);
   if (kv_end > 0) {
-    f32_load_tile<D>(Qs, qb, p.q_st, q0, it.Lq);
-    f32_load_tile<D>(dOs, dob, p.do_st, q0, it.Lq);
+    f32_load_rows<D, S::kRows, S::kThreads>(Qs, qb, p.q_st, q0, it.Lq);
+    f32_load_rows<D, S::kRows, S::kThreads>(dOs, dob, p.do_st, q0, it.Lq);
+    f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, 0, it.Lk);
+    f32_commit();
+    f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, 0, it.Lk);
+    f32_commit();
+    f32_wait<1>();
+    __syncthreads();
   }
-  for (int k0 = 0; k0 < kv_end; k0 += kF32Tile) {
-    __syncthreads();
-    f32_load_tile<D>(Ks, kb, p.k_st, k0, it.Lk);
-    f32_load_tile<D>(Vs, vb, p.v_st, k0, it.Lk);
-    __syncthreads();
-    f32_p_and_ds<D>(p, it, Qs, dOs, Ks, Vs, nullptr, dSs, q0, k0, bias, sm, ty, tx);
-    __syncthreads();
-    f32_accumulate<D, false>(dSs, Ks, ty, tx, dq);
-  }
-  float* dqb = p.dq + (int64_t)it.bc * p.dq_sb + (int64_t)it.h * p.dq_sh + (int64_t)it.tq0 * p.dq_st;
+  for (int k0 = 0; k0 < kv_end; k0 += kF32Cols) {
+    const bool more = k0 + kF32Cols < kv_end;
+    {
+      float dp[8][S::kNC];
+      f32_scores<D, S::kNC>(dOs, Vs, th.row0, th.col0, dp);
+      f32_wait<0>();
+      __syncthreads();  // K has arrived, V is no longer read
+      if (more) {
+        f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, k0 + kF32Cols, it.Lk);
+        f32_commit();
+      }
+      float s[8][S::kNC];
+      f32_scores<D, S::kNC>(Qs, Ks, th.row0, th.col0, s);
+      f32_probs<S::kNC>(p, it, s, f32_all_visible(p, it, q0, S::kRows, k0, kF32Cols), q0 + th.row0, k0 + th.col0, 2, 0, 0, 16,
+                        bias, sm);
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int i = q0 + ty + 16 * a;
-    if (i < it.row_lim) {
+      for (int a = 0; a < 8; ++a)
 #pragma unroll
-      for (int c = 0; c < D / 16; ++c) dqb[(int64_t)i * p.dq_st + tx + 16 * c] = (i < it.Lq) ? dq[a][c] * p.scale : 0.f;
+        for (int c = 0; c < S::kNC; ++c) dSs[(th.row0 + 2 * a) * S::kWRow + th.col0 + 16 * c] = f32_ds(s[a][c], dp[a][c]);
+    }
+    f32_group_sync<kC>(th.group);
+    f32_accumulate<D, S::kNX>(dSs, Ks, th.row0, th.x0, dq);
+    f32_wait<0>();
+    __syncthreads();  // the next V has arrived, K and dS are no longer read
+    if (more) {
+      f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, k0 + kF32Cols, it.Lk);
+      f32_commit();
     }
   }
+  float* dqb = p.dq + (int64_t)it.bc * p.dq_sb + (int64_t)it.h * p.dq_sh + (int64_t)it.tq0 * p.dq_st;
+  f32_store_rows<S::kNX>(dqb, p.dq_st, q0, th.row0, th.x0, it.row_lim, it.Lq, p.scale, dq);
 }
 
 }  // namespace sigattn
