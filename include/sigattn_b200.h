@@ -29,7 +29,7 @@
  *    is launched until sigattn_device_status() has been called (which reports and clears the failure).
  *  - Return value 0 = launched; negative = rejected before any launch, with a message
  *    available from sigattn_last_error() on the calling thread.
- *  - Supported: dtype fp16 / bf16 / fp32, D in {64, 128}, 1 <= H, B, Tq, Tk (zero-sized problems
+ *  - Supported: dtype fp16 / bf16 / fp32, D in {64, 128} (narrower heads through head_cols), 1 <= H, B, Tq, Tk (zero-sized problems
  *    return 0 without launching).
  */
 #ifndef SIGATTN_B200_H_
@@ -85,7 +85,9 @@ typedef struct SigAttnParams {
   float scale;           /* multiplies Q K^T */
   float bias_scalar;     /* used for every batch when `bias` is NULL */
   int32_t device;        /* CUDA device ordinal the pointers live on */
-  int32_t reserved0;
+  int32_t head_cols;     /* columns the tensors really have, 0 = D.  A multiple of 8 (fp32: 4), at most D: heads
+                            narrower than 64 or 128 run without being padded in memory (the kernels read the
+                            missing columns as zeros and do not write them) */
 
   const void *q, *k, *v; /* (B,Tq,H,D), (B,Tk,H,D), (B,Tk,H,D) */
   void *o;               /* forward output (B,Tq,H,D); unused by backward */

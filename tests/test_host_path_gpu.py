@@ -55,3 +55,26 @@ def test_second_backward_needs_retain_graph():
     assert torch.equal(first, second)
     with pytest.raises(RuntimeError, match="backward through the graph a second time"):
         torch.autograd.grad(out, q)
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("dtype,dims", [(torch.bfloat16, (8, 24, 56, 72, 120)), (torch.float32, (4, 20, 60, 68, 124))])
+def test_narrow_heads_match_zero_extended_ones(monkeypatch, dtype, dims, split):
+    """Head dimensions below the kernels' 64 / 128 are read and written in place; padding them in memory gives the same."""
+    if split:
+        monkeypatch.setenv("SIGATTN_B200_BWD_SPLIT", "1")
+    B, T, H = 2, 300, 3
+    lens = torch.tensor([300, 131], dtype=torch.int32, device="cuda")
+    for D in dims:
+        g = torch.Generator(device="cuda").manual_seed(D)
+        narrow = [torch.randn(B, T, H, D, device="cuda", generator=g).to(dtype) for _ in range(4)]
+        wide = [torch.nn.functional.pad(t, (0, (64 if D <= 64 else 128) - D)) for t in narrow]
+        res = []
+        for q, k, v, do in (narrow, wide):
+            q, k, v = [t.detach().requires_grad_() for t in (q, k, v)]
+            out = m.sigmoid_attention_padded(q, k, v, seq_lens_k=lens, seq_lens_q=lens, is_causal=True, scale=0.3)
+            res.append([t[..., :D] for t in (out.detach(), *torch.autograd.grad(out, (q, k, v), do))])
+        for i, (a, b) in enumerate(zip(*res)):
+            assert a.shape == narrow[0].shape
+            # one order of operations except for dQ, whose fp32 reductions have none
+            assert torch.equal(a, b) if i != 1 else torch.allclose(a.float(), b.float(), rtol=1e-2, atol=1e-4), (D, i)

@@ -50,7 +50,7 @@ class SigAttnParams(ctypes.Structure):
         ("scale", ctypes.c_float),
         ("bias_scalar", ctypes.c_float),
         ("device", ctypes.c_int32),
-        ("reserved0", ctypes.c_int32),
+        ("head_cols", ctypes.c_int32),
         ("q", ctypes.c_void_p),
         ("k", ctypes.c_void_p),
         ("v", ctypes.c_void_p),

@@ -77,6 +77,7 @@ struct BwdParams {
   float scale;
   float bias_scalar;
   int B, H, Tq, Tk;
+  int d_cols;   // columns of the tensors in memory (<= D; the rest reads as zeros and is not written)
   int causal;
   int n_kvblk;  // ceil(Tk / 128)
   int n_items;  // B * H * n_kvblk
@@ -633,7 +634,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
             const int r8 = 8 * i + (lane >> 2);
             const uint4 x = *reinterpret_cast<const uint4*>(patch + r8 * L::kDqPatchRow + 16 * (lane & 3));
             const int krow = it.kv0 + quarter * 32 + r8;
-            if (krow < it.key_lim) *reinterpret_cast<uint4*>(out + 2 * (int64_t)krow * out_st) = x;
+            if (krow < it.key_lim && 32 * half + 8 * (lane & 3) < p.d_cols) *reinterpret_cast<uint4*>(out + 2 * (int64_t)krow * out_st) = x;
           }
           __syncwarp();  // the patch is rewritten by the next pass / the next item's first dQ tile
         }
@@ -947,7 +948,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         constexpr int kChunksPerRow = D * 2 / 16;
         for (int i = threadIdx.x; i < kBwdTileKV * kChunksPerRow; i += kBwdComputeWarps * 32) {
           const int row = kv0 + i / kChunksPerRow;
-          if (row < it.key_lim) {
+          if (row < it.key_lim && 8 * (i % kChunksPerRow) < p.d_cols) {
             *reinterpret_cast<uint4*>(dk_base + 2 * (int64_t)row * p.dk_st + 16 * (i % kChunksPerRow)) = make_uint4(0, 0, 0, 0);
             *reinterpret_cast<uint4*>(dv_base + 2 * (int64_t)row * p.dv_st + 16 * (i % kChunksPerRow)) = make_uint4(0, 0, 0, 0);
           }
@@ -1099,7 +1100,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
             const int r = 8 * i + (lane >> 2);  // row within the quarter (quarter * 32 is a multiple of 8: same swizzle phase)
             const uint4 x = *reinterpret_cast<const uint4*>(ds_gen + r * 128 + (((chunk0 + c) ^ (uint32_t)(r & 7)) << 4));
             const int krow = kv0 + quarter * 32 + r;
-            if (krow < it.key_lim) *reinterpret_cast<uint4*>(out_base + 2 * (int64_t)krow * out_st + 16 * c) = x;
+            if (krow < it.key_lim && col0 + 8 * c < p.d_cols) *reinterpret_cast<uint4*>(out_base + 2 * (int64_t)krow * out_st + 16 * c) = x;
           }
           __syncwarp();  // phase B of the next item rewrites these slots
         } else {
@@ -1108,7 +1109,8 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
 #pragma unroll
             for (int c = 0; c < D / 64; ++c) {
 #pragma unroll
-              for (int q4 = 0; q4 < 4; ++q4) *reinterpret_cast<uint4*>(out_row + 64 * c + 16 * q4) = w[c][q4];
+              for (int q4 = 0; q4 < 4; ++q4)
+                if (col0 + 32 * c + 8 * q4 < p.d_cols) *reinterpret_cast<uint4*>(out_row + 64 * c + 16 * q4) = w[c][q4];
             }
           }
         }
@@ -1148,6 +1150,7 @@ struct DqConvertParams {
   void* dq;
   int64_t sb, st, sh;
   int B, T, H;
+  int d_cols;  // columns of dQ (the accumulator has D)
   float scale;
 };
 
@@ -1158,6 +1161,7 @@ __global__ void __launch_bounds__(256) sigattn_dq_convert_kernel(const DqConvert
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     const int c = (int)(i % kChunks);
+    if (8 * c >= p.d_cols) continue;
     long long r = i / kChunks;
     const int h = (int)(r % p.H);
     r /= p.H;

@@ -46,6 +46,7 @@ struct BwdStreamParams {
   float scale;
   float bias_scalar;
   int B, H, Tr, Tc;  // extents of the stationary and the streamed side
+  int d_cols;        // columns of the tensors in memory (<= D)
   int Tk;            // key extent (row length of score_mod)
   int causal;
   int n_rblk;   // ceil(Tr / 128)
@@ -574,7 +575,8 @@ sigattn_bwd_stream_kernel(const __grid_constant__ CUtensorMap r1_map, const __gr
         // nothing on the streamed side sees this tile: its gradients are zero
         if (row < it.row_lim) {
 #pragma unroll
-          for (int c = 0; c < kCols / 8; ++c) *reinterpret_cast<uint4*>(out_row + 16 * c) = make_uint4(0, 0, 0, 0);
+          for (int c = 0; c < kCols / 8; ++c)
+            if (col_first + 8 * c < p.d_cols) *reinterpret_cast<uint4*>(out_row + 16 * c) = make_uint4(0, 0, 0, 0);
         }
       } else {
         ok = mbar_wait_warp(bar(L::kAccFull), (uint32_t)act & 1u, abort_flag, kSiteBase + 15);
@@ -606,7 +608,8 @@ sigattn_bwd_stream_kernel(const __grid_constant__ CUtensorMap r1_map, const __gr
         if (lane == 0) mbar_arrive(bar(L::kAccEmpty));
         if (row < it.row_lim) {
 #pragma unroll
-          for (int c = 0; c < kCols / 8; ++c) *reinterpret_cast<uint4*>(out_row + 16 * c) = w[c];
+          for (int c = 0; c < kCols / 8; ++c)
+            if (col_first + 8 * c < p.d_cols) *reinterpret_cast<uint4*>(out_row + 16 * c) = w[c];
         }
       }
       __syncwarp();

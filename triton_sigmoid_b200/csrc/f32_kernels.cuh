@@ -51,6 +51,7 @@ struct F32Params {
   float scale;
   float bias_scalar;
   int B, H, Tq, Tk;
+  int d_cols;  // columns of the tensors in memory (<= D; the rest reads as zeros and is not written)
   int causal;
 };
 
@@ -83,12 +84,13 @@ __device__ __forceinline__ void f32_wait() { asm volatile("cp.async.wait_group %
 
 // Rows [row0, row0 + kN) of a (token, head-dim) slab into shared memory; rows at or beyond `limit` are zero.
 template <int D, int kN, int kThreads>
-__device__ __forceinline__ void f32_load_rows(float* dst, const float* src, int64_t stride_t, int row0, int limit) {
+__device__ __forceinline__ void f32_load_rows(float* dst, const float* src, int64_t stride_t, int row0, int limit,
+                                              int d_cols) {
   constexpr int kRow = D + 4, kChunks = D / 4;
 #pragma unroll 4
   for (int i = threadIdx.x; i < kN * kChunks; i += kThreads) {
     const int r = i / kChunks, c = i % kChunks;
-    const bool live = row0 + r < limit;
+    const bool live = row0 + r < limit && 4 * c < d_cols;
     f32_cp16(dst + r * kRow + 4 * c, live ? src + (int64_t)(row0 + r) * stride_t + 4 * c : src, live);
   }
 }
@@ -116,7 +118,8 @@ __device__ __forceinline__ void f32_group_sync(int group) {
 
 // s[a][c] = sum_d A[row0 + 2 a][d] * B[col0 + 16 c][d]
 template <int D, int kNC>
-__device__ __forceinline__ void f32_scores(const float* A, const float* B, int row0, int col0, float (&s)[8][kNC]) {
+__device__ __forceinline__ void f32_scores(const float* A, const float* B, int row0, int col0, int d_cols,
+                                           float (&s)[8][kNC]) {
   constexpr int kRow = D + 4;
   float2 acc[8][kNC];
 #pragma unroll
@@ -125,8 +128,11 @@ __device__ __forceinline__ void f32_scores(const float* A, const float* B, int r
     for (int c = 0; c < kNC; ++c) acc[a][c] = make_float2(0.f, 0.f);
   const float* ap = A + row0 * kRow;
   const float* bp = B + col0 * kRow;
-#pragma unroll 4
-  for (int d = 0; d < D; d += 4) {
+  // (columns from d_cols to the next multiple of 16 are zero in shared memory)
+#pragma unroll 1
+  for (int d16 = 0; d16 < d_cols; d16 += 16)
+#pragma unroll
+  for (int d = d16; d < d16 + 16; d += 4) {
     float4 b[kNC];
 #pragma unroll
     for (int c = 0; c < kNC; ++c) b[c] = *reinterpret_cast<const float4*>(bp + 16 * c * kRow + d);
@@ -200,7 +206,7 @@ __device__ __forceinline__ void f32_accumulate(const float* W, const float* X, i
 // Rows row0 + 2 a (of the tensor: first + that) below `limit`, times mul; rows at or beyond `live` are zero.
 template <int kNX>
 __device__ __forceinline__ void f32_store_rows(float* base, int64_t stride_t, int first, int row0, int x0, int limit, int live,
-                                               float mul, const float (&acc)[8][kNX]) {
+                                               int d_cols, float mul, const float (&acc)[8][kNX]) {
   constexpr int kVX = kNX < 4 ? kNX : 4;
 #pragma unroll
   for (int a = 0; a < 8; ++a) {
@@ -209,6 +215,7 @@ __device__ __forceinline__ void f32_store_rows(float* base, int64_t stride_t, in
     const float m = i < live ? mul : 0.f;
 #pragma unroll
     for (int v = 0; v < kNX / kVX; ++v) {
+      if (x0 + 64 * v >= d_cols) continue;
       float* dst = base + (int64_t)i * stride_t + x0 + 64 * v;
       if constexpr (kVX == 4) {
         float4 w = make_float4(acc[a][4 * v] * m, acc[a][4 * v + 1] * m, acc[a][4 * v + 2] * m, acc[a][4 * v + 3] * m);
@@ -337,10 +344,10 @@ __global__ void __launch_bounds__(32 * kR * kC, D == 64 && kR == 4 ? 3 : 1) siga
   int kv_end = (q0 < it.Lq) ? it.Lk : 0;
   if (p.causal) kv_end = min(kv_end, q0 + S::kRows);
   if (kv_end > 0) {
-    f32_load_rows<D, S::kRows, S::kThreads>(Qs, qb, p.q_st, q0, it.Lq);
-    f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, 0, it.Lk);
+    f32_load_rows<D, S::kRows, S::kThreads>(Qs, qb, p.q_st, q0, it.Lq, p.d_cols);
+    f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, 0, it.Lk, p.d_cols);
     f32_commit();
-    f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, 0, it.Lk);
+    f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, 0, it.Lk, p.d_cols);
     f32_commit();
     f32_wait<1>();
     __syncthreads();
@@ -349,7 +356,7 @@ __global__ void __launch_bounds__(32 * kR * kC, D == 64 && kR == 4 ? 3 : 1) siga
     const bool more = k0 + kF32Cols < kv_end;
     {
       float s[8][S::kNC];
-      f32_scores<D, S::kNC>(Qs, Ks, th.row0, th.col0, s);
+      f32_scores<D, S::kNC>(Qs, Ks, th.row0, th.col0, p.d_cols, s);
       f32_probs<S::kNC>(p, it, s, f32_all_visible(p, it, q0, S::kRows, k0, kF32Cols), q0 + th.row0, k0 + th.col0, 2, 0, 0, 16,
                         bias, sm);
 #pragma unroll
@@ -360,19 +367,19 @@ __global__ void __launch_bounds__(32 * kR * kC, D == 64 && kR == 4 ? 3 : 1) siga
     f32_wait<0>();
     __syncthreads();  // V has arrived, P is complete, K is no longer read
     if (more) {
-      f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, k0 + kF32Cols, it.Lk);
+      f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, k0 + kF32Cols, it.Lk, p.d_cols);
       f32_commit();
     }
     f32_accumulate<D, S::kNX>(Ps, Vs, th.row0, th.x0, o);
     f32_wait<0>();
     __syncthreads();  // the next K has arrived, V and P are no longer read
     if (more) {
-      f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, k0 + kF32Cols, it.Lk);
+      f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, k0 + kF32Cols, it.Lk, p.d_cols);
       f32_commit();
     }
   }
   float* ob = p.o + (int64_t)it.bc * p.o_sb + (int64_t)it.h * p.o_sh + (int64_t)it.tq0 * p.o_st;
-  f32_store_rows<S::kNX>(ob, p.o_st, q0, th.row0, th.x0, it.row_lim, it.Lq, 1.0f, o);
+  f32_store_rows<S::kNX>(ob, p.o_st, q0, th.row0, th.x0, it.row_lim, it.Lq, p.d_cols, 1.0f, o);
 }
 
 // ---------------------------------------------------------------- backward: dK, dV of one key tile
@@ -401,11 +408,11 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(cons
   const int q_end = (k0 < it.Lk) ? it.Lq : 0;
   const int q_begin = p.causal ? (k0 / kF32Cols) * kF32Cols : 0;  // earlier query tiles see none of these keys
   if (q_begin < q_end) {
-    f32_load_rows<D, S::kRows, S::kThreads>(Ks, kb, p.k_st, k0, it.Lk);
-    f32_load_rows<D, S::kRows, S::kThreads>(Vs, vb, p.v_st, k0, it.Lk);
-    f32_load_rows<D, kF32Cols, S::kThreads>(Qs, qb, p.q_st, q_begin, it.Lq);
+    f32_load_rows<D, S::kRows, S::kThreads>(Ks, kb, p.k_st, k0, it.Lk, p.d_cols);
+    f32_load_rows<D, S::kRows, S::kThreads>(Vs, vb, p.v_st, k0, it.Lk, p.d_cols);
+    f32_load_rows<D, kF32Cols, S::kThreads>(Qs, qb, p.q_st, q_begin, it.Lq, p.d_cols);
     f32_commit();
-    f32_load_rows<D, kF32Cols, S::kThreads>(dOs, dob, p.do_st, q_begin, it.Lq);
+    f32_load_rows<D, kF32Cols, S::kThreads>(dOs, dob, p.do_st, q_begin, it.Lq, p.d_cols);
     f32_commit();
     f32_wait<1>();
     __syncthreads();
@@ -414,7 +421,7 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(cons
     const bool more = q0 + kF32Cols < q_end;
     {
       float pr[8][S::kNC];
-      f32_scores<D, S::kNC>(Ks, Qs, th.row0, th.col0, pr);
+      f32_scores<D, S::kNC>(Ks, Qs, th.row0, th.col0, p.d_cols, pr);
       f32_probs<S::kNC>(p, it, pr, f32_all_visible(p, it, q0, kF32Cols, k0, S::kRows), q0 + th.col0, k0 + th.row0, 0, 2, 16, 0,
                         bias, sm);
 #pragma unroll
@@ -424,7 +431,7 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(cons
       f32_wait<0>();
       __syncthreads();  // dO has arrived
       float dp[8][S::kNC];
-      f32_scores<D, S::kNC>(Vs, dOs, th.row0, th.col0, dp);
+      f32_scores<D, S::kNC>(Vs, dOs, th.row0, th.col0, p.d_cols, dp);
 #pragma unroll
       for (int a = 0; a < 8; ++a)
 #pragma unroll
@@ -435,21 +442,21 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(cons
     f32_accumulate<D, S::kNX>(dSs, Qs, th.row0, th.x0, dk);
     __syncthreads();  // Q is no longer read
     if (more) {
-      f32_load_rows<D, kF32Cols, S::kThreads>(Qs, qb, p.q_st, q0 + kF32Cols, it.Lq);
+      f32_load_rows<D, kF32Cols, S::kThreads>(Qs, qb, p.q_st, q0 + kF32Cols, it.Lq, p.d_cols);
       f32_commit();
     }
     f32_accumulate<D, S::kNX>(Ps, dOs, th.row0, th.x0, dv);
     f32_wait<0>();
     __syncthreads();  // the next Q has arrived, dO, P and dS are no longer read
     if (more) {
-      f32_load_rows<D, kF32Cols, S::kThreads>(dOs, dob, p.do_st, q0 + kF32Cols, it.Lq);
+      f32_load_rows<D, kF32Cols, S::kThreads>(dOs, dob, p.do_st, q0 + kF32Cols, it.Lq, p.d_cols);
       f32_commit();
     }
   }
   float* dkb = p.dk + (int64_t)it.bc * p.dk_sb + (int64_t)it.h * p.dk_sh + (int64_t)it.tk0 * p.dk_st;
   float* dvb = p.dv + (int64_t)it.bc * p.dv_sb + (int64_t)it.h * p.dv_sh + (int64_t)it.tk0 * p.dv_st;
-  f32_store_rows<S::kNX>(dkb, p.dk_st, k0, th.row0, th.x0, it.key_lim, it.Lk, p.scale, dk);
-  f32_store_rows<S::kNX>(dvb, p.dv_st, k0, th.row0, th.x0, it.key_lim, it.Lk, 1.0f, dv);
+  f32_store_rows<S::kNX>(dkb, p.dk_st, k0, th.row0, th.x0, it.key_lim, it.Lk, p.d_cols, p.scale, dk);
+  f32_store_rows<S::kNX>(dvb, p.dv_st, k0, th.row0, th.x0, it.key_lim, it.Lk, p.d_cols, 1.0f, dv);
 }
 
 // ---------------------------------------------------------------- backward: dQ of one query tile
@@ -476,11 +483,11 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dq_f32_kernel(const 
   int kv_end = (q0 < it.Lq) ? it.Lk : 0;
   if (p.causal) kv_end = min(kv_end, q0 + S::kRows);
   if (kv_end > 0) {
-    f32_load_rows<D, S::kRows, S::kThreads>(Qs, qb, p.q_st, q0, it.Lq);
-    f32_load_rows<D, S::kRows, S::kThreads>(dOs, dob, p.do_st, q0, it.Lq);
-    f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, 0, it.Lk);
+    f32_load_rows<D, S::kRows, S::kThreads>(Qs, qb, p.q_st, q0, it.Lq, p.d_cols);
+    f32_load_rows<D, S::kRows, S::kThreads>(dOs, dob, p.do_st, q0, it.Lq, p.d_cols);
+    f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, 0, it.Lk, p.d_cols);
     f32_commit();
-    f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, 0, it.Lk);
+    f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, 0, it.Lk, p.d_cols);
     f32_commit();
     f32_wait<1>();
     __syncthreads();
@@ -489,15 +496,15 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dq_f32_kernel(const 
     const bool more = k0 + kF32Cols < kv_end;
     {
       float dp[8][S::kNC];
-      f32_scores<D, S::kNC>(dOs, Vs, th.row0, th.col0, dp);
+      f32_scores<D, S::kNC>(dOs, Vs, th.row0, th.col0, p.d_cols, dp);
       f32_wait<0>();
       __syncthreads();  // K has arrived, V is no longer read
       if (more) {
-        f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, k0 + kF32Cols, it.Lk);
+        f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, k0 + kF32Cols, it.Lk, p.d_cols);
         f32_commit();
       }
       float s[8][S::kNC];
-      f32_scores<D, S::kNC>(Qs, Ks, th.row0, th.col0, s);
+      f32_scores<D, S::kNC>(Qs, Ks, th.row0, th.col0, p.d_cols, s);
       f32_probs<S::kNC>(p, it, s, f32_all_visible(p, it, q0, S::kRows, k0, kF32Cols), q0 + th.row0, k0 + th.col0, 2, 0, 0, 16,
                         bias, sm);
 #pragma unroll
@@ -510,12 +517,12 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dq_f32_kernel(const 
     f32_wait<0>();
     __syncthreads();  // the next V has arrived, K and dS are no longer read
     if (more) {
-      f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, k0 + kF32Cols, it.Lk);
+      f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, k0 + kF32Cols, it.Lk, p.d_cols);
       f32_commit();
     }
   }
   float* dqb = p.dq + (int64_t)it.bc * p.dq_sb + (int64_t)it.h * p.dq_sh + (int64_t)it.tq0 * p.dq_st;
-  f32_store_rows<S::kNX>(dqb, p.dq_st, q0, th.row0, th.x0, it.row_lim, it.Lq, p.scale, dq);
+  f32_store_rows<S::kNX>(dqb, p.dq_st, q0, th.row0, th.x0, it.row_lim, it.Lq, p.d_cols, p.scale, dq);
 }
 
 }  // namespace sigattn

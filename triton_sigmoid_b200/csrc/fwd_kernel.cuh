@@ -58,6 +58,7 @@ struct FwdParams {
   float scale;
   float bias_scalar;
   int B, H, Tq, Tk;
+  int d_cols;   // columns of the tensors in memory (<= D; the rest reads as zeros and is not written)
   int causal;
   int n_qblk;   // ceil(Tq / 256)
   int n_items;  // B * H * n_qblk
@@ -481,7 +482,8 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         for (int s = 0; s < 2; ++s) {
           const bool has_o = (s == 0 ? it.n0 : it.n1) > 0;  // else the tile is entirely padding: zero rows
           // this lane's rows of the tile are sub_row, sub_row + 4, ...; row 4 i + sub_row may be written if 4 i < rows_left
-          const int rows_left = it.row_lim - (it.q0 + 128 * s + 32 * (warp & 3) + sub_row);
+          int rows_left = it.row_lim - (it.q0 + 128 * s + 32 * (warp & 3) + sub_row);
+          if (8 * ch >= p.d_cols) rows_left = 0;
           uint8_t* o_ptr = o_base + 2 * (int64_t)(128 * s) * p.o_st;
           const uint8_t* st_ptr = stage + 4096 * s + sub_row * 128;
 #pragma unroll
@@ -541,9 +543,10 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         }
         __syncwarp();
         // this lane's rows of the tile are (lane >> 4), (lane >> 4) + 2, ...; row 2 i + (lane >> 4) may be written if 2 i < rows_left
-        const int rows_left = it.row_lim - (it.q0 + 128 * s + 32 * (warp & 3) + (lane >> 4));
-        uint8_t* o_ptr = o_base + 2 * (int64_t)(128 * s) * p.o_st;
         const int ch = lane & 15;
+        int rows_left = it.row_lim - (it.q0 + 128 * s + 32 * (warp & 3) + (lane >> 4));
+        if (8 * ch >= p.d_cols) rows_left = 0;
+        uint8_t* o_ptr = o_base + 2 * (int64_t)(128 * s) * p.o_st;
 #pragma unroll 4
         for (int i = 0; i < 16; ++i) {
           const int r = 2 * i + (lane >> 4);

@@ -111,6 +111,9 @@ int check_common(const SigAttnParams* p, bool backward) {
   if (p->dtype != SIGATTN_FP16 && p->dtype != SIGATTN_BF16 && p->dtype != SIGATTN_FP32)
     return fail(-2, "unsupported dtype %d (fp16=0, bf16=1, fp32=2)", p->dtype);
   if (p->D != 64 && p->D != 128) return fail(-2, "unsupported head dimension %d (64 or 128)", p->D);
+  const int per16 = p->dtype == SIGATTN_FP32 ? 4 : 8;
+  if (p->head_cols < 0 || p->head_cols > p->D || p->head_cols % per16 != 0)
+    return fail(-2, "head_cols %d must be 0 or a multiple of %d up to D = %d", p->head_cols, per16, p->D);
   if (p->B < 0 || p->H < 0 || p->Tq < 0 || p->Tk < 0) return fail(-2, "negative extent");
   if (p->H > 65535 || p->B > 65535) return fail(-2, "B and H must not exceed 65535");
   const bool packed = p->cu_seqlens_q || p->cu_seqlens_k;
@@ -125,6 +128,9 @@ int check_common(const SigAttnParams* p, bool backward) {
   if (backward && (!p->dout || !p->dq || !p->dk || !p->dv)) return fail(-1, "dout, dq, dk, dv must not be NULL");
   return 0;
 }
+
+// Columns of the tensors in memory (the kernels' head dimension D is 64 or 128).
+int head_cols(const SigAttnParams* p) { return p->head_cols > 0 ? p->head_cols : p->D; }
 
 bool is_contiguous(const int64_t* s, int T, int H, int D) {
   return s[2] == D && s[1] == (int64_t)H * D && s[0] == (int64_t)T * H * D;
@@ -326,6 +332,7 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
   fp.H = p->H;
   fp.Tq = p->Tq;
   fp.Tk = p->Tk;
+  fp.d_cols = head_cols(p);
   fp.causal = (p->flags & SIGATTN_CAUSAL) ? 1 : 0;
   fp.n_qblk = (p->Tq + kFwdBlockM - 1) / kFwdBlockM;
   const int64_t n_items = (int64_t)fp.n_qblk * p->H * p->B;
@@ -376,6 +383,7 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
   bp.bias_scalar = p->bias_scalar;
   if (p->flags & SIGATTN_BIAS_NEG_LOG_LK) { bp.bias = nullptr; bp.bias_scalar = nanf(""); }  // see item_bias()
   bp.B = p->B; bp.H = p->H; bp.Tq = p->Tq; bp.Tk = p->Tk;
+  bp.d_cols = head_cols(p);
   bp.causal = (p->flags & SIGATTN_CAUSAL) ? 1 : 0;
   bp.n_kvblk = (p->Tk + kBwdTileKV - 1) / kBwdTileKV;
   const int64_t n_items = (int64_t)bp.n_kvblk * p->H * p->B;
@@ -406,6 +414,7 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
     cp.dq = p->dq;
     cp.sb = p->dq_strides[0]; cp.st = p->dq_strides[1]; cp.sh = p->dq_strides[2];
     cp.B = ex.B; cp.T = ex.Tq; cp.H = p->H;
+    cp.d_cols = head_cols(p);
     cp.scale = p->scale;
     const long long chunks = (long long)ex.B * ex.Tq * p->H * (D / 8);
     const int threads = 256;
@@ -444,6 +453,7 @@ int launch_bwd_stream_mode(const SigAttnParams* p, const CUtensorMap& r1, const 
   bp.bias_scalar = p->bias_scalar;
   if (p->flags & SIGATTN_BIAS_NEG_LOG_LK) { bp.bias = nullptr; bp.bias_scalar = nanf(""); }  // see item_bias()
   bp.B = p->B; bp.H = p->H; bp.Tk = p->Tk;
+  bp.d_cols = head_cols(p);
   bp.causal = (p->flags & SIGATTN_CAUSAL) ? 1 : 0;
   bp.n_rblk = (bp.Tr + kBsTile - 1) / kBsTile;
   const int64_t n_items = (int64_t)bp.n_rblk * p->H * p->B;
@@ -557,6 +567,7 @@ int launch_f32_d(const SigAttnParams* p, bool backward) {
   fp.bias_scalar = p->bias_scalar;
   if (p->flags & SIGATTN_BIAS_NEG_LOG_LK) { fp.bias = nullptr; fp.bias_scalar = nanf(""); }  // see item_bias()
   fp.B = p->B; fp.H = p->H; fp.Tq = p->Tq; fp.Tk = p->Tk;
+  fp.d_cols = head_cols(p);
   fp.causal = (p->flags & SIGATTN_CAUSAL) ? 1 : 0;
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   FwdDeviceInfo info;
@@ -681,13 +692,13 @@ int sigattn_fwd(const SigAttnParams* p) {
   if (ex.Tq == 0 || p->Tq == 0) return 0;
   if (ex.Tk == 0 || p->Tk == 0) {  // no keys at all: the output is all zeros
     const Strides3 os = map_strides(p->o_strides, ex.Tq, ex.packed);
-    return zero_fill(p->o, os.s, ex.B, ex.Tq, p->H, p->D, p->dtype, static_cast<cudaStream_t>(p->stream), "o");
+    return zero_fill(p->o, os.s, ex.B, ex.Tq, p->H, head_cols(p), p->dtype, static_cast<cudaStream_t>(p->stream), "o");
   }
   if (p->dtype == SIGATTN_FP32) return launch_f32(p, false);
   CUtensorMap qm, km, vm;
-  if ((rc = make_map(&qm, p->q, p->dtype, ex.B, ex.Tq, p->H, p->D, map_strides(p->q_strides, ex.Tq, ex.packed).s, 128, "q"))) return rc;
-  if ((rc = make_map(&km, p->k, p->dtype, ex.B, ex.Tk, p->H, p->D, map_strides(p->k_strides, ex.Tk, ex.packed).s, 128, "k"))) return rc;
-  if ((rc = make_map(&vm, p->v, p->dtype, ex.B, ex.Tk, p->H, p->D, map_strides(p->v_strides, ex.Tk, ex.packed).s, 128, "v"))) return rc;
+  if ((rc = make_map(&qm, p->q, p->dtype, ex.B, ex.Tq, p->H, head_cols(p), map_strides(p->q_strides, ex.Tq, ex.packed).s, 128, "q"))) return rc;
+  if ((rc = make_map(&km, p->k, p->dtype, ex.B, ex.Tk, p->H, head_cols(p), map_strides(p->k_strides, ex.Tk, ex.packed).s, 128, "k"))) return rc;
+  if ((rc = make_map(&vm, p->v, p->dtype, ex.B, ex.Tk, p->H, head_cols(p), map_strides(p->v_strides, ex.Tk, ex.packed).s, 128, "v"))) return rc;
   if ((reinterpret_cast<uintptr_t>(p->o) & 15u) != 0) return fail(-3, "o: base pointer must be 16-byte aligned");
   for (int i = ex.packed ? 1 : 0; i < 3; ++i)
     if (p->o_strides[i] % 8 != 0) return fail(-3, "o: strides must be multiples of 8 elements");
@@ -723,16 +734,16 @@ int sigattn_bwd(const SigAttnParams* p) {
   if (ex.Tq == 0 || ex.Tk == 0 || p->Tq == 0 || p->Tk == 0) {
     // no query or no key: every gradient is zero
     cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-    if ((rc = zero_fill(p->dq, map_strides(p->dq_strides, ex.Tq, ex.packed).s, ex.B, ex.Tq, p->H, p->D, p->dtype, stream, "dq"))) return rc;
-    if ((rc = zero_fill(p->dk, map_strides(p->dk_strides, ex.Tk, ex.packed).s, ex.B, ex.Tk, p->H, p->D, p->dtype, stream, "dk"))) return rc;
-    return zero_fill(p->dv, map_strides(p->dv_strides, ex.Tk, ex.packed).s, ex.B, ex.Tk, p->H, p->D, p->dtype, stream, "dv");
+    if ((rc = zero_fill(p->dq, map_strides(p->dq_strides, ex.Tq, ex.packed).s, ex.B, ex.Tq, p->H, head_cols(p), p->dtype, stream, "dq"))) return rc;
+    if ((rc = zero_fill(p->dk, map_strides(p->dk_strides, ex.Tk, ex.packed).s, ex.B, ex.Tk, p->H, head_cols(p), p->dtype, stream, "dk"))) return rc;
+    return zero_fill(p->dv, map_strides(p->dv_strides, ex.Tk, ex.packed).s, ex.B, ex.Tk, p->H, head_cols(p), p->dtype, stream, "dv");
   }
   if (p->dtype == SIGATTN_FP32) return launch_f32(p, true);
   CUtensorMap qm, km, vm, dom;
-  if ((rc = make_map(&qm, p->q, p->dtype, ex.B, ex.Tq, p->H, p->D, map_strides(p->q_strides, ex.Tq, ex.packed).s, 128, "q"))) return rc;
-  if ((rc = make_map(&km, p->k, p->dtype, ex.B, ex.Tk, p->H, p->D, map_strides(p->k_strides, ex.Tk, ex.packed).s, 128, "k"))) return rc;
-  if ((rc = make_map(&vm, p->v, p->dtype, ex.B, ex.Tk, p->H, p->D, map_strides(p->v_strides, ex.Tk, ex.packed).s, 128, "v"))) return rc;
-  if ((rc = make_map(&dom, p->dout, p->dtype, ex.B, ex.Tq, p->H, p->D, map_strides(p->do_strides, ex.Tq, ex.packed).s, 128, "dout"))) return rc;
+  if ((rc = make_map(&qm, p->q, p->dtype, ex.B, ex.Tq, p->H, head_cols(p), map_strides(p->q_strides, ex.Tq, ex.packed).s, 128, "q"))) return rc;
+  if ((rc = make_map(&km, p->k, p->dtype, ex.B, ex.Tk, p->H, head_cols(p), map_strides(p->k_strides, ex.Tk, ex.packed).s, 128, "k"))) return rc;
+  if ((rc = make_map(&vm, p->v, p->dtype, ex.B, ex.Tk, p->H, head_cols(p), map_strides(p->v_strides, ex.Tk, ex.packed).s, 128, "v"))) return rc;
+  if ((rc = make_map(&dom, p->dout, p->dtype, ex.B, ex.Tq, p->H, head_cols(p), map_strides(p->do_strides, ex.Tq, ex.packed).s, 128, "dout"))) return rc;
   const void* outs[3] = {p->dq, p->dk, p->dv};
   const int64_t* ostr[3] = {p->dq_strides, p->dk_strides, p->dv_strides};
   for (int t = 0; t < 3; ++t) {

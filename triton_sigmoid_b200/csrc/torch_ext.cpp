@@ -105,6 +105,9 @@ void fill_strides(int64_t* out, const Tensor& t) {
 
 Tensor new_like(const Tensor& t) { return at::detail::empty_cuda(t.sizes(), t.scalar_type(), t.device(), std::nullopt); }
 
+// The kernels' head dimension for tensors of D columns (the missing columns read as zeros).
+int kernel_head_dim(int64_t D) { return D <= 64 ? 64 : 128; }
+
 void fill_common(SigAttnParams& p, const Tensors& t, const Call& c) {
   std::memset(&p, 0, sizeof(p));
   p.struct_bytes = sizeof(p);
@@ -114,7 +117,8 @@ void fill_common(SigAttnParams& p, const Tensors& t, const Call& c) {
   const bool packed = t.cu_q.defined();
   const int64_t n = t.q.dim();
   p.H = (int32_t)t.q.size(n - 2);
-  p.D = (int32_t)t.q.size(n - 1);
+  p.head_cols = (int32_t)t.q.size(n - 1);
+  p.D = kernel_head_dim(p.head_cols);
   if (packed) {
     p.B = (int32_t)t.cu_q.numel() - 1;
     p.Tq = (int32_t)c.max_q;
@@ -204,7 +208,7 @@ void run_backward(const Tensors& t, const Call& c, const Tensor& grad, Tensor& d
   if (env_true("SIGATTN_B200_BWD_SPLIT")) {
     p.flags |= SIGATTN_BWD_SPLIT;
   } else if (p.dtype != SIGATTN_FP32) {
-    const int64_t elems = std::max<int64_t>(dq.numel(), 4);
+    const int64_t elems = std::max<int64_t>(dq.numel() / p.head_cols * p.D, 4);
     ws = at::detail::empty_cuda({elems}, at::kFloat, t.q.device(), std::nullopt);
     p.workspace = ws.mutable_data_ptr();
     p.workspace_bytes = (size_t)elems * sizeof(float);
@@ -304,12 +308,13 @@ bool get_number(PyObject* o, double* v, bool* given) {
   *v = PyFloat_AsDouble(o);
   return !PyErr_Occurred();
 }
-// Same device, one supported dtype, a head dimension the kernels take as it is.
+// Same device, one supported dtype, a head dimension whose rows are whole 16-byte pieces.
 bool qkv_ok(const Tensors& t) {
   int code;
   const auto dt = t.q.scalar_type();
   const int64_t D = t.q.size(t.q.dim() - 1);
-  return dtype_code(dt, &code) && t.k.scalar_type() == dt && t.v.scalar_type() == dt && (D == 64 || D == 128) &&
+  return dtype_code(dt, &code) && t.k.scalar_type() == dt && t.v.scalar_type() == dt && D > 0 && D <= 128 &&
+         D % (16 / (int64_t)t.q.element_size()) == 0 &&
          t.k.device() == t.q.device() && t.v.device() == t.q.device() && is_b200(t.q.get_device());
 }
 
