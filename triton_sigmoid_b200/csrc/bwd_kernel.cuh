@@ -15,39 +15,24 @@
 //   dV_j += P^T  dO_i           (TMEM x smem -> TMEM)
 //   dK_j += dS^T Q_i            (TMEM x smem -> TMEM)
 //   dQ_i  = dS K_j              (smem x smem -> TMEM), then added into an fp32 accumulator in
-//                                global memory.  The L2 performs such reductions at full speed
-//                                only when a request covers consecutive addresses, and a warp
-//                                that reads dQ with query rows on the TMEM lanes would scatter
-//                                32 lanes over 32 rows.  So:
-//                                D = 128: the transposed product dQ^T = K^T dS^T is computed
-//                                  instead; the head dimension lies on the lanes and one
-//                                  red.global.add.f32 per query covers a full 128-byte line;
-//                                D = 64: the transposed product would have M = 64 and idle half of
-//                                  the tensor core and half of the lanes, so dQ is kept as it is and
-//                                  each warp takes full 128-byte half rows of every second query row,
-//                                  regrouped through a private shared-memory patch so that eight
-//                                  lanes cover a line, and adds them with red.global.add.v4.f32
-//                                  (the reduction traffic, not the math, is what bounds this case).
+//                                global memory by bulk reductions out of shared memory (see acc_piece)
 //
-// Warp roles (20 warps; 28 at D = 64):
+// Warp roles (28 warps):
 //   warps 0-15  compute: warp w owns TMEM lanes (key rows) 32 (w & 3) .. +31 and the query
-//               columns 32 (w >> 2) .. +31 of every tile; at D = 128 the same warps drain dQ
+//               columns 32 (w >> 2) .. +31 of every tile
 //   warp  16    item scheduler + TMA producer (also clears padded rows of tiles that straddle a valid length)
 //   warp  17    tcgen05 issuer A: S^T and dP^T; owns the TMEM allocation
 //   warp  18    tcgen05 issuer B: dV, dK, dQ
 //   warp  19    idle
-//   warps 20-27 D = 64 only: dQ drain.  The reductions into the fp32 accumulator are slow to issue (the
-//               L2 serves a warp's reductions one 128-byte line at a time), and while the compute warps
-//               issued them themselves (29 % of their time, measured) the MUFU unit and the tensor pipe
-//               stood idle and the next tile's scores, which reuse the dQ columns, were late.  Eight
-//               warps that do nothing else take dQ out of TMEM as soon as it is complete (freeing the
-//               columns at once) and feed the reductions while the compute warps are two phases ahead.
-//               They also take the epilogue (dK_j, dV_j) of short items, see kDrainEpilogueMaxTiles.
-//               Registers are re-balanced with setmaxnreg (compute 80, role warps 72, drain warps 56 per thread);
-//               to fit, the compute warps do not keep P in registers between their two phases but read its
-//               16-bit copy back from TMEM.
-//               (No room for this at D = 128: the drain needs its whole tile in registers or shared
-//               memory before it can release the columns, and neither has any left there.)
+//   warps 20-27 dQ drain: take finished dQ tiles out of TMEM (freeing the columns at once) and feed the reductions
+//               while the compute warps are on the next tile.  At D = 64 they also take the epilogue (dK_j, dV_j) of
+//               short items, see kDrainEpilogueMaxTiles.
+//               Registers are re-balanced with setmaxnreg.  To fit, the compute warps of D = 64 do not keep P in
+//               registers between their two phases but read its 16-bit copy back from TMEM.
+// What bounds it (timeline of one SM, B=4 T=4096 H=16): D = 128 shared memory - the operands of S, dP and dQ, which
+// saturate its 128 bytes per clock while they run, the tiles coming in, dS, and dQ going out: 3800 of a tile's 4200
+// clocks (1.70 -> 1.42 ms for the backward when the drain moved from the compute warps to these); D = 64 the two phases
+// of the compute warps with the barriers between them, 2900 clocks (0.85 -> 0.77 ms).
 // Two issuing warps, because one warp's instruction stream (waits, 32 MMAs, commits per tile
 // pair) is a serial chain that otherwise bounds the kernel.  Everything the two exchange goes
 // through mbarriers: "S columns free" after dV, "dP columns free" after dK.
@@ -60,7 +45,10 @@
 namespace sigattn {
 
 struct BwdParams {
-  float* dq_acc;  // [B, Tq, H, D] fp32, zero-filled before the launch
+  // fp32, zero-filled before the launch: one region of (rows of the sequence) x D floats per batch element and head,
+  // see acc_piece()
+  float* dq_acc;
+  int64_t acc_sb, acc_sh;  // floats from one batch element / head to the next (packed: acc_sb = 0)
   void* dk;
   void* dv;
   int64_t dk_sb, dk_st, dk_sh;
@@ -68,8 +56,8 @@ struct BwdParams {
   const int* lens_q;
   const int* lens_k;
   // Packed (variable-length) layout: sequence b occupies rows cu_q[b] .. cu_q[b+1]-1 of a (total, H, D)
-  // tensor (likewise cu_k for keys / values); Tq, Tk are then upper bounds of the lengths and dq_acc is
-  // [total queries, H, D].  nullptr = (B, T, H, D).
+  // tensor (likewise cu_k for keys / values); Tq, Tk are then upper bounds of the lengths and dq_acc has
+  // one region per head and sequence.  nullptr = (B, T, H, D).
   const int* cu_q;
   const int* cu_k;
   const float* bias;
@@ -96,15 +84,17 @@ constexpr int kBwdDrainWarps = 8;
 // this many query tiles, so that the compute warps go straight on to the next item; for longer items, whose
 // epilogue is a small share, the compute warps do it themselves (the drain warps, busy with it, would fall
 // behind with the next item's dQ tiles: measured -1.5 % at 32 tiles per item, +7 % at 4).
-constexpr int kDrainEpilogueMaxTiles = 8;    // D = 64 only
+// (D = 128: the compute warps always do; the drain warps have no shared memory to turn rows in.)
+template <int D> constexpr int kDrainEpilogueMaxTiles = (D == 64) ? 8 : 0;
 constexpr int kBwdFirstDrainWarp = 20;
-template <int D> constexpr int kBwdThreads = (D == 64) ? (kBwdFirstDrainWarp + kBwdDrainWarps) * 32 : 20 * 32;
+constexpr int kBwdThreads = (kBwdFirstDrainWarp + kBwdDrainWarps) * 32;
 constexpr int kBwdTileKV = 128;
 constexpr int kBwdTileQ = 128;
 
 template <int D>
 struct BwdSmem {
-  static constexpr int kStages = 2;
+  static constexpr int kStages = 2;                      // Q tiles
+  static constexpr int kDoStages = (D == 64) ? 2 : 1;      // dO tiles (one at D = 128: the room goes to the drain's patches)
   static constexpr int kTileBytes = 128 * D * 2;
   // K_j / V_j buffers: two at D = 64 (the next item's are loaded while this item still computes), one at
   // D = 128 (no room for more)
@@ -113,21 +103,21 @@ struct BwdSmem {
   static constexpr int kVOff = kKOff + kKvBufs * kTileBytes;
   static constexpr int kQOff = kVOff + kKvBufs * kTileBytes;
   static constexpr int kDoOff = kQOff + kStages * kTileBytes;
-  static constexpr int kDsOff = kDoOff + kStages * kTileBytes;
+  static constexpr int kDsOff = kDoOff + kDoStages * kTileBytes;
   static constexpr int kDsBytes = 128 * 128 * 2;
-  // D = 64 only: a private patch of 32 rows x 128 bytes per drain warp, used to regroup dQ rows so
-  // that eight adjacent lanes add the 128 bytes of one row (16 bytes of padding per row keep the
-  // 16-byte accesses of different rows off each other's banks)
-  static constexpr int kDqPatchRow = 128 + 16;
+  // a private 4 KB patch per drain warp: 32 query rows x 32 head columns of dQ on their way to the accumulator; at
+  // D = 64 also 32 rows x 64 bytes of dK / dV in the epilogue of short items, turned there so that four adjacent lanes
+  // write one row (16 bytes of padding per row keep the 16-byte accesses of different rows off each other's banks)
+  static constexpr int kPatchRow = 64 + 16;
   static constexpr int kDqPatchOff = kDsOff + kDsBytes;
-  static constexpr int kDqPatchBytes = (D == 64) ? 32 * kDqPatchRow : 0;
+  static constexpr int kDqPatchBytes = 4096;
   static constexpr int kBarOff = kDqPatchOff + kBwdDrainWarps * kDqPatchBytes;
   static constexpr int kKvFull = 0;                   // [2] per K/V buffer
   static constexpr int kQFull = 2;                    // [2]
   static constexpr int kQEmpty = kQFull + kStages;    // [2]  both issuers release a stage
-  static constexpr int kDoFull = kQEmpty + kStages;   // [2]
-  static constexpr int kDoEmpty = kDoFull + kStages;  // [2]
-  static constexpr int kSFull = kDoEmpty + kStages;   // [2] S^T written (per S buffer)
+  static constexpr int kDoFull = kQEmpty + kStages;     // [kDoStages]
+  static constexpr int kDoEmpty = kDoFull + kDoStages;  // [kDoStages]
+  static constexpr int kSFull = kDoEmpty + kDoStages;   // [2] S^T written (per S buffer)
   static constexpr int kDpFull = kSFull + 2;          // dP^T written
   static constexpr int kPReady = kDpFull + 1;         // [2] P^T in TMEM (16 warps; per S buffer)
   static constexpr int kDsReady = kPReady + 2;        // dS^T in TMEM and shared memory (16 warps)
@@ -148,104 +138,91 @@ struct BwdSmem {
   static constexpr int kDynBytes = kTotal + 1024;
 };
 
-// Phase A of one tile for one thread: 32 scores of its key row -> probabilities (kept in pv[]
-// for phase B) and their 16-bit packing written over the first 16 of the 32 columns read.
+// The two phases of one tile for one thread (its key row, 32 query columns) in the D = 128 kernel.
+//
+// Phase A: scores -> probabilities, kept in registers for phase B; their 16-bit packing is written over the first 16
+// of the 32 columns read (the operand of dV).  Both phases move 16 columns at a time, so that besides the 32
+// probabilities only few registers are live.
 // q0 = query index of the first column; valid queries for this key row are [q_lo, q_hi).
 template <bool kBF16, bool kMask, bool kAccurate>
 __device__ __forceinline__ void bwd_phase_a(uint32_t s_addr, float c1, float c0, int q0, int q_lo, int q_hi,
-                                            float (&pv)[32]) {
-  uint32_t r[32];
-  tmem_ld32_sync(s_addr, r);
-  uint32_t pk[16];
-  float2 t[16];
+                                            float2 (&pv)[16]) {
   // unmasked tiles work on logits shifted up by kDeepShift (see sigmoid2_from_shifted_log2_deep)
   const float c0s = (kMask || kAccurate) ? c0 : c0 + kDeepShift;
+  {
+    uint32_t r[32];
+    tmem_ld32_sync(s_addr, r);
 #pragma unroll
-  for (int i = 0; i < 16; ++i)
-    t[i] = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), make_float2(c1, c1),
-                      make_float2(c0s, c0s));
+    for (int i = 0; i < 16; ++i)
+      pv[i] = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), make_float2(c1, c1),
+                         make_float2(c0s, c0s));
+  }
+  // f(logits) -> probabilities, in place; eight pairs at a time leave for TMEM
+  auto emit = [&](auto f) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t pk[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float2 pe = f(pv[8 * h + i]);
+        if constexpr (kMask) {
+          const int q = q0 + 16 * h + 2 * i;
+          pe.x = (q >= q_lo && q < q_hi) ? pe.x : 0.0f;
+          pe.y = (q + 1 >= q_lo && q + 1 < q_hi) ? pe.y : 0.0f;
+        }
+        pv[8 * h + i] = pe;
+        pk[i] = pack2<kBF16>(pe.x, pe.y);
+      }
+      tmem_st8(s_addr + 8 * h, pk);
+    }
+  };
   if constexpr (kAccurate) {
     // exponential and reciprocal both on the special-function unit (see sigmoid2_accurate_from_log2)
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float2 pe = sigmoid2_accurate_from_log2(t[i]);
-      if constexpr (kMask) {
-        const int q = q0 + 2 * i;
-        pe.x = (q >= q_lo && q < q_hi) ? pe.x : 0.0f;
-        pe.y = (q + 1 >= q_lo && q + 1 < q_hi) ? pe.y : 0.0f;
-      }
-      pv[2 * i] = pe.x;
-      pv[2 * i + 1] = pe.y;
-      pk[i] = pack2<kBF16>(pe.x, pe.y);
-    }
-  } else
-  // all logits far below zero (the usual case under the default bias): short series, no compare / select per element
-  if (!kMask && warp_all_negative(t)) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float2 pe = sigmoid2_from_shifted_log2_deep<kBF16>(t[i]);
-      pv[2 * i] = pe.x;
-      pv[2 * i + 1] = pe.y;
-      pk[i] = pack2<kBF16>(pe.x, pe.y);
-    }
+    emit([](float2 x) { return sigmoid2_accurate_from_log2(x); });
+  } else if (!kMask && warp_all_negative(pv)) {
+    // all logits far below zero (the usual case under the default bias): short series, no compare / select per element
+    emit([](float2 x) { return sigmoid2_from_shifted_log2_deep<kBF16>(x); });
   } else {
     bool all_neg = false;
     if constexpr (!kMask) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) t[i] = __fadd2_rn(t[i], make_float2(-kDeepShift, -kDeepShift));
-      all_neg = warp_all_negative(t);  // negative but not far below zero: full polynomial, still no select
+      for (int i = 0; i < 16; ++i) pv[i] = __fadd2_rn(pv[i], make_float2(-kDeepShift, -kDeepShift));
+      all_neg = warp_all_negative(pv);  // negative but not far below zero: full polynomial, still no select
     }
-    if (all_neg) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float2 pe = sigmoid2_from_log2_neg<kBF16>(t[i]);
-        pv[2 * i] = pe.x;
-        pv[2 * i + 1] = pe.y;
-        pk[i] = pack2<kBF16>(pe.x, pe.y);
-      }
-    } else
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float2 pe = sigmoid2_from_log2<kBF16>(t[i]);
-      if constexpr (kMask) {
-        const int q = q0 + 2 * i;
-        pe.x = (q >= q_lo && q < q_hi) ? pe.x : 0.0f;
-        pe.y = (q + 1 >= q_lo && q + 1 < q_hi) ? pe.y : 0.0f;
-      }
-      pv[2 * i] = pe.x;
-      pv[2 * i + 1] = pe.y;
-      pk[i] = pack2<kBF16>(pe.x, pe.y);
-    }
+    if (all_neg) emit([](float2 x) { return sigmoid2_from_log2_neg<kBF16>(x); });
+    else         emit([](float2 x) { return sigmoid2_from_log2<kBF16>(x); });
   }
-  tmem_st16(s_addr, pk);
 }
 
 // Phase B: dS = P (1 - P) dP for the same 32 columns; 16-bit dS^T goes to TMEM (over the first
 // 16 dP columns read) and to the swizzled shared-memory copy the dQ GEMM reads.
 template <bool kBF16, bool kMask>
 __device__ __forceinline__ void bwd_phase_b(uint32_t dp_addr, uint32_t ds_line, uint32_t chunk0, uint32_t sw,
-                                            const float (&pv)[32]) {
-  uint32_t r[32];
-  tmem_ld32_sync(dp_addr, r);
-  uint32_t pk[16];
+                                            const float2 (&pv)[16]) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const float2 pp = make_float2(pv[2 * i], pv[2 * i + 1]);
-    const float2 w = __ffma2_rn(make_float2(-pp.x, -pp.y), pp, pp);  // P - P^2
-    float2 d = __fmul2_rn(w, make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
-    if constexpr (kMask) {
-      d.x = (pp.x != 0.0f) ? d.x : 0.0f;  // masked elements have P exactly 0; keeps NaN/Inf padding out
-      d.y = (pp.y != 0.0f) ? d.y : 0.0f;
+  for (int h = 0; h < 2; ++h) {
+    uint32_t r[16], pk[8];
+    tmem_ld16(dp_addr + 16 * h, r);
+    tmem_ld_wait_for(r);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float2 pp = pv[8 * h + i];
+      const float2 w = __ffma2_rn(make_float2(-pp.x, -pp.y), pp, pp);  // P - P^2
+      float2 d = __fmul2_rn(w, make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
+      if constexpr (kMask) {
+        d.x = (pp.x != 0.0f) ? d.x : 0.0f;  // masked elements have P exactly 0; keeps NaN/Inf padding out
+        d.y = (pp.y != 0.0f) ? d.y : 0.0f;
+      }
+      pk[i] = pack2<kBF16>(d.x, d.y);
     }
-    pk[i] = pack2<kBF16>(d.x, d.y);
-  }
-  tmem_st16(dp_addr, pk);
+    tmem_st8(dp_addr + 8 * h, pk);
 #pragma unroll
-  for (int m = 0; m < 4; ++m) {
-    const uint32_t chunk = (chunk0 + m) ^ sw;  // 128-byte swizzle: 16-byte chunk index XOR (row & 7)
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(ds_line + chunk * 16), "r"(pk[4 * m]),
-                 "r"(pk[4 * m + 1]), "r"(pk[4 * m + 2]), "r"(pk[4 * m + 3])
-                 : "memory");
+    for (int m = 0; m < 2; ++m) {
+      const uint32_t chunk = (chunk0 + 2 * h + m) ^ sw;  // 128-byte swizzle: 16-byte chunk index XOR (row & 7)
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(ds_line + chunk * 16), "r"(pk[4 * m]),
+                   "r"(pk[4 * m + 1]), "r"(pk[4 * m + 2]), "r"(pk[4 * m + 3])
+                   : "memory");
+    }
   }
 }
 
@@ -339,6 +316,15 @@ __device__ __forceinline__ void bwd_phase_b16(uint32_t p_addr, uint32_t dp_addr,
   }
 }
 
+// The fp32 dQ accumulator.  Each (batch element, head) has a region of its rows x D floats.  A quarter (32 rows, fewer
+// at the region's end) of query tile i starts at (128 i + 32 quarter) D and holds [D / 32][8][rows][4] floats: blocks of
+// 32 columns, in them the four-column pieces, in those the rows.  That is the order in which a drain warp, one query row
+// per lane, writes 32 columns to shared memory without bank conflicts, and one bulk reduction adds the 4 KB to global
+// memory.  (Reductions issued lane by lane, red.global.add, reach the same 5.8 TB/s of the L2, but they wait for it in
+// the load/store queue of the SM, and every barrier and shared-memory access of the other warps waits behind them: 250
+// to 450 clocks per barrier in a timeline of one SM.)
+__device__ __forceinline__ int acc_piece(int rows, int c4, int row) { return ((c4 * rows) + row) * 4; }
+
 // One work item.  The producer warp decodes it once (integer divisions, length and bias loads from global
 // memory) and publishes the record through shared memory; every other role reads it from there.
 struct BwdItem {
@@ -346,7 +332,7 @@ struct BwdItem {
   int bc;               // batch coordinate of the tensor maps and strides (0 when packed)
   int tq0, tk0;         // first row of the sequence in the token dimension (0 unless packed)
   int key_lim;          // key rows below this exist in this sequence's tensors (Tk; packed: Lk)
-  int64_t acc_row0;     // first row of the sequence in the dQ accumulator
+  int64_t acc_base;     // start of the (batch element, head) in the dQ accumulator, in floats
   int Lq, Lk;
   int i_begin, n_q;     // first query tile that sees this key tile, number of query tiles
   bool ragged_kv;       // the key tile straddles Lk
@@ -356,7 +342,7 @@ struct BwdItem {
 // record layout in shared memory: 16 ints, [0] = item index (-1: no more work)
 __device__ __forceinline__ void bwd_publish_item(volatile int* rec, int item, const BwdItem& it) {
   rec[1] = it.b; rec[2] = it.h; rec[3] = it.kv0; rec[4] = it.bc; rec[5] = it.tq0; rec[6] = it.tk0; rec[7] = it.key_lim;
-  rec[8] = (int)(uint32_t)((uint64_t)it.acc_row0 & 0xffffffffull); rec[9] = (int)(uint32_t)((uint64_t)it.acc_row0 >> 32);
+  rec[8] = (int)(uint32_t)((uint64_t)it.acc_base & 0xffffffffull); rec[9] = (int)(uint32_t)((uint64_t)it.acc_base >> 32);
   rec[10] = it.Lq; rec[11] = it.Lk; rec[12] = it.i_begin; rec[13] = it.n_q;
   rec[14] = (it.ragged_kv ? 1 : 0) | (it.ragged_last_q ? 2 : 0); rec[15] = __float_as_int(it.bias);
   rec[0] = item;
@@ -364,12 +350,13 @@ __device__ __forceinline__ void bwd_publish_item(volatile int* rec, int item, co
 __device__ __forceinline__ BwdItem bwd_load_item(const volatile int* rec) {
   BwdItem it;
   it.b = rec[1]; it.h = rec[2]; it.kv0 = rec[3]; it.bc = rec[4]; it.tq0 = rec[5]; it.tk0 = rec[6]; it.key_lim = rec[7];
-  it.acc_row0 = (int64_t)(((uint64_t)(uint32_t)rec[9] << 32) | (uint64_t)(uint32_t)rec[8]);
+  it.acc_base = (int64_t)(((uint64_t)(uint32_t)rec[9] << 32) | (uint64_t)(uint32_t)rec[8]);
   it.Lq = rec[10]; it.Lk = rec[11]; it.i_begin = rec[12]; it.n_q = rec[13];
   const int fl = rec[14];
   it.ragged_kv = (fl & 1) != 0; it.ragged_last_q = (fl & 2) != 0; it.bias = __int_as_float(rec[15]);
   return it;
 }
+template <int D>
 __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item) {
   BwdItem it;
   // Groups of `group` (batch, head) pairs: within a group every pair's key tile 0 comes first, then
@@ -391,7 +378,6 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item)
   it.bc = it.b;
   it.tq0 = it.tk0 = 0;
   it.key_lim = p.Tk;
-  it.acc_row0 = (int64_t)it.b * p.Tq;
   if (p.cu_q) {
     it.tq0 = p.cu_q[it.b];
     it.tk0 = p.cu_k[it.b];
@@ -399,8 +385,8 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item)
     it.Lk = min(max(p.cu_k[it.b + 1] - it.tk0, 0), p.Tk);
     it.bc = 0;
     it.key_lim = it.Lk;
-    it.acc_row0 = it.tq0;
   }
+  it.acc_base = (int64_t)it.bc * p.acc_sb + (int64_t)it.h * p.acc_sh + (int64_t)it.tq0 * D;
   const int i_end = (it.Lq + kBwdTileQ - 1) / kBwdTileQ;
   it.i_begin = p.causal ? j : 0;  // query tiles that can see this key tile (top-left aligned)
   it.n_q = (it.kv0 < it.Lk) ? max(i_end - it.i_begin, 0) : 0;
@@ -411,7 +397,7 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item)
 }
 
 template <int D, bool kBF16, bool kAccurate>
-__global__ void __launch_bounds__(kBwdThreads<D>, 1)
+__global__ void __launch_bounds__(kBwdThreads, 1)
 sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                    const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap do_map,
                    const BwdParams p) {
@@ -421,10 +407,9 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   // TMEM plan.  D = 64: two S^T buffers (tiles alternate), so that the scores of the next tile are
   // computed while this one is still being processed; dQ_i is written over the S^T buffer of its
   // own tile once dV has read P^T from it:   S0 0 | S1 128 | dP 256 | dV 384 | dK 448.
-  // D = 128: no room for that: one S^T buffer, dQ^T over the dP^T columns:  S 0 | dP 128 | dV 256 | dK 384.
+  // D = 128: no room for that: one S^T buffer, dQ over the dP^T columns:  S 0 | dP 128 | dV 256 | dK 384.
   // Column group c keeps its 16-bit P^T in S columns 32c + [0,16), dS^T likewise in the dP columns.
   constexpr bool kTwoS = (D == 64);
-  constexpr bool kDqT = (D == 128);         // dQ^T (head dimension on lanes) instead of dQ
   constexpr uint32_t kColS = 0;
   constexpr uint32_t kColDp = kTwoS ? 256 : 128;
   constexpr uint32_t kColDv = kTwoS ? 384 : 256;
@@ -435,12 +420,14 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   // index and parity of the per-S-buffer barriers for tile g
   auto sbuf = [](int g) -> int { return kTwoS ? (g & 1) : 0; };
   auto spar = [](int g) -> uint32_t { return kTwoS ? (uint32_t)(g >> 1) & 1u : (uint32_t)g & 1u; };
-  // where dQ (or dQ^T) of tile g is written
+  // stage of dO of tile g and the parity of that stage's "full" barrier
+  auto do_stage = [](int g) -> int { return L::kDoStages == 2 ? (g & 1) : 0; };
+  auto do_par = [](int g) -> uint32_t { return L::kDoStages == 2 ? (uint32_t)(g >> 1) & 1u : (uint32_t)g & 1u; };
+  // where dQ of tile g is written
   auto dq_col = [&](int g) -> uint32_t { return kTwoS ? kColS + 128u * (uint32_t)(g & 1) : kColDp; };
   constexpr int kSiteBase = 0x20000;
-  constexpr bool kDrainWarps = kTwoS;  // dedicated dQ drain warps (see the file header)
   // compute warps, the two issuing warps and the drain warps read the item ring
-  constexpr int kItemReaders = kBwdComputeWarps + 2 + (kDrainWarps ? kBwdDrainWarps : 0);
+  constexpr int kItemReaders = kBwdComputeWarps + 2 + kBwdDrainWarps;
 
   extern __shared__ uint8_t smem_dyn[];
   const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
@@ -469,6 +456,8 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     for (int i = 0; i < L::kStages; ++i) {
       mbar_init(bar(L::kQFull + i), 1);
       mbar_init(bar(L::kQEmpty + i), 2);   // S^T (issuer A) and dK (issuer B) both read Q_i
+    }
+    for (int i = 0; i < L::kDoStages; ++i) {
       mbar_init(bar(L::kDoFull + i), 1);
       mbar_init(bar(L::kDoEmpty + i), 2);  // dP^T (issuer A) and dV (issuer B) both read dO_i
     }
@@ -482,8 +471,8 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     mbar_init(bar(L::kDpFree), 1);
     mbar_init(bar(L::kDqFull + 0), 1);
     mbar_init(bar(L::kDqFull + 1), 1);
-    mbar_init(bar(L::kDqEmpty + 0), kDrainWarps ? kBwdDrainWarps : kBwdComputeWarps);
-    mbar_init(bar(L::kDqEmpty + 1), kDrainWarps ? kBwdDrainWarps : kBwdComputeWarps);
+    mbar_init(bar(L::kDqEmpty + 0), kBwdDrainWarps);
+    mbar_init(bar(L::kDqEmpty + 1), kBwdDrainWarps);
     mbar_init(bar(L::kDkvFull), 1);
     mbar_init(bar(L::kDkvEmpty + 0), kBwdComputeWarps);
     mbar_init(bar(L::kDkvEmpty + 1), kBwdDrainWarps);
@@ -520,23 +509,29 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     return item;
   };
 
-  if constexpr (kDrainWarps) {
-    // 896 threads get 72 registers each at launch.  Each aligned group of four warps executes one
-    // instruction; the counts add up to exactly what the CTA holds (512 x 80 + 128 x 72 + 256 x 56).
-    // (The issuing warps are the ones that must not spill: their instruction stream is the critical chain.)
+  // 896 threads get 72 registers each at launch.  Each aligned group of four warps executes one
+  // instruction; the counts add up to exactly what the CTA holds:
+  //   D = 64:  compute 80, role 72 (the issuing warps must not spill: their instruction stream is the critical
+  //            chain), drain 56 (512 x 80 + 128 x 72 + 256 x 56);
+  //   D = 128: compute 72, role 56, drain 80 (a dQ tile goes from the drain warps' registers, 64 per thread, to the
+  //            accumulator in two steps, so that its TMEM columns are free for the next dP at once; 512 x 72 + 128 x 56 + 256 x 80).
+  if constexpr (D == 64) {
     if (warp < kBwdComputeWarps)         setmaxnreg_inc<80>();
     else if (warp >= kBwdFirstDrainWarp) setmaxnreg_dec<56>();
+  } else {
+    if (warp >= kBwdFirstDrainWarp)      setmaxnreg_inc<80>();
+    else if (warp >= kBwdComputeWarps)   setmaxnreg_dec<56>();
   }
 
-  if (kDrainWarps && warp >= kBwdFirstDrainWarp) {
-    // ============================================================ dQ drain (D = 64)
-    // Warp d = warp - 20: lane quarter d & 3 (32 query rows), head columns [32 (d >> 2), +32) = one 128-byte
-    // line of the accumulator per row.  Per tile: wait for the dQ product, move the 32 x 32 block through
-    // registers into the warp's shared-memory patch, release the TMEM columns, then add the rows into the
-    // accumulator with red.global.add.v4.f32, eight adjacent lanes per line.
-    if constexpr (kDrainWarps) {
+  if (warp >= kBwdFirstDrainWarp) {
+    // ============================================================ dQ drain
+    // Warp d = warp - 20: lane quarter d & 3 (32 query rows, one per lane), half of the head columns d >> 2.  Per tile:
+    // wait for the dQ product, take the block into registers, release the TMEM columns, then add it into the
+    // accumulator (see acc_tile).
+    {
       const int dw = warp - kBwdFirstDrainWarp;
       const int quarter = dw & 3, half = dw >> 2;
+      constexpr int kCols = D / 2;  // head columns per warp
       const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
       uint8_t* patch = smem_gen + L::kDqPatchOff + dw * L::kDqPatchBytes;
       int g = 0;
@@ -547,39 +542,39 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         const int item = read_item(k, it);
         if (item < 0) break;
         if (it.n_q == 0) continue;
-        for (int t = 0; t < it.n_q && ok; ++t) {
+        const int row_lim = p.cu_q ? it.Lq : p.Tq;
+        for (int t = 0; t < it.n_q; ++t) {
           const int gt = g + t;
           ok = mbar_wait_warp(bar(L::kDqFull + sbuf(gt)), spar(gt), abort_flag, kSiteBase + 14);
           if (!ok) break;
           tc_fence_after_sync();
-          const uint32_t addr = tmem + lane_addr + dq_col(gt) + 32u * (uint32_t)half;
-          uint4* mine = reinterpret_cast<uint4*>(patch + lane * L::kDqPatchRow);
+          const uint32_t addr = tmem + lane_addr + dq_col(gt) + (uint32_t)(kCols * half);
+          uint32_t r[kCols / 32][32];
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            uint32_t r[16];
-            tmem_ld(addr + 16 * u, r);
-            tmem_ld_wait_for(r);
+          for (int c = 0; c < kCols / 32; ++c) tmem_ld32(addr + 32 * c, r[c]);
 #pragma unroll
-            for (int m = 0; m < 4; ++m) mine[4 * u + m] = make_uint4(r[4 * m], r[4 * m + 1], r[4 * m + 2], r[4 * m + 3]);
-          }
+          for (int c = 0; c < kCols / 32; ++c) tmem_ld_wait_for(r[c]);
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(L::kDqEmpty + sbuf(gt)));  // the TMEM columns are free again
-          const int q_tile = (it.i_begin + t) * kBwdTileQ + quarter * 32;
-          const int slot = lane >> 3, chunk = lane & 7;  // patch row within a group of four, 16-byte chunk of the row
+          const int row0 = (it.i_begin + t) * kBwdTileQ + quarter * 32;
+          const int rows = min(row_lim - row0, 32);  // rows at or beyond Lq hold zeros, which do no harm
+          if (rows <= 0) continue;
+          float* dst = p.dq_acc + it.acc_base + (int64_t)row0 * D + (kCols / 32) * half * (rows * 32);
 #pragma unroll
-          for (int kq = 0; kq < 8; ++kq) {
-            const int prow = 4 * kq + slot;
-            const int q = q_tile + prow;
-            const uint4 w = *reinterpret_cast<const uint4*>(patch + prow * L::kDqPatchRow + chunk * 16);
-            if (q < it.Lq) {  // queries at or beyond Lq get no gradient
-              float* dst = p.dq_acc + ((it.acc_row0 + q) * p.H + it.h) * D + 32 * half + 4 * chunk;
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(__uint_as_float(w.x)),
-                           "f"(__uint_as_float(w.y)), "f"(__uint_as_float(w.z)), "f"(__uint_as_float(w.w))
-                           : "memory");
+          for (int c = 0; c < kCols / 32; ++c) {
+            if (lane == 0) bulk_wait_read();  // the patch's previous content has been read
+            __syncwarp();
+            if (lane < rows) {
+#pragma unroll
+              for (int c4 = 0; c4 < 8; ++c4)
+                reinterpret_cast<uint4*>(patch)[acc_piece(rows, c4, lane) / 4] =
+                    make_uint4(r[c][4 * c4], r[c][4 * c4 + 1], r[c][4 * c4 + 2], r[c][4 * c4 + 3]);
             }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) bulk_reduce_add_f32(dst + c * (rows * 32), smem_u32(patch), (uint32_t)rows * 128u);
           }
-          __syncwarp();  // the patch is rewritten at the next tile
         }
         if (!ok) break;
         g += it.n_q;
@@ -588,20 +583,19 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         // lanes cover a row's 64 bytes and an instruction 8 rows; a lane writing its own row would touch 32
         // lines per instruction, which the load/store unit takes one at a time) and out to global memory,
         // while the compute warps are already on the next item's first tiles.
-        if (it.n_q > kDrainEpilogueMaxTiles) {
-          ++act;  // the compute warps' business
-          continue;
-        }
-        ok = mbar_wait_warp(bar(L::kDkvFull), (uint32_t)act & 1u, abort_flag, kSiteBase + 15);
-        if (!ok) break;
         ++act;
+        if (it.n_q > kDrainEpilogueMaxTiles<D>) continue;  // the compute warps' business
+        if constexpr (D == 64) {
+        if (lane == 0) bulk_wait_read();  // the patch is about to be rewritten
+        ok = mbar_wait_warp(bar(L::kDkvFull), (uint32_t)(act - 1) & 1u, abort_flag, kSiteBase + 15);
+        if (!ok) break;
         tc_fence_after_sync();
         const bool row_ok = it.kv0 + quarter * 32 + lane < it.Lk;  // padded key rows get zero gradients
 #pragma unroll
         for (int which = 0; which < 2; ++which) {  // 0: dV, 1: dK
           const uint32_t acc_addr = tmem + lane_addr + (which ? kColDk : kColDv) + 32u * (uint32_t)half;
           const float mul = which ? p.scale : 1.0f;
-          uint4* mine = reinterpret_cast<uint4*>(patch + lane * L::kDqPatchRow);
+          uint4* mine = reinterpret_cast<uint4*>(patch + lane * L::kPatchRow);
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
             uint32_t r[16];
@@ -632,16 +626,17 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int r8 = 8 * i + (lane >> 2);
-            const uint4 x = *reinterpret_cast<const uint4*>(patch + r8 * L::kDqPatchRow + 16 * (lane & 3));
+            const uint4 x = *reinterpret_cast<const uint4*>(patch + r8 * L::kPatchRow + 16 * (lane & 3));
             const int krow = it.kv0 + quarter * 32 + r8;
             if (krow < it.key_lim && 32 * half + 8 * (lane & 3) < p.d_cols) *reinterpret_cast<uint4*>(out + 2 * (int64_t)krow * out_st) = x;
           }
-          __syncwarp();  // the patch is rewritten by the next pass / the next item's first dQ tile
+          __syncwarp();  // the patch is rewritten by the next pass
+        }
         }
       }
+      if (lane == 0) bulk_wait_all();  // every reduction has been performed when the kernel ends
     }
-  } else
-  if (warp == kBwdProducerWarp) {
+  } else if (warp == kBwdProducerWarp) {
     // ============================================================ item scheduler + TMA producer
     // Rows beyond the valid lengths may hold anything (NaN included).  Masked probabilities are
     // exactly zero, but 0 * NaN is NaN inside an MMA, so the padded rows of every tile that is
@@ -669,7 +664,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       }
       item = __shfl_sync(0xffffffffu, item, 0);
       BwdItem it = {};
-      if (item >= 0) it = bwd_decode_item(p, item);
+      if (item >= 0) it = bwd_decode_item<D>(p, item);
       if (lane == 0) {
         if (item >= 0) bwd_publish_item(item_ring + 16 * slot, item, it);
         else item_ring[16 * slot] = -1;
@@ -691,13 +686,15 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           for (int c = 0; c < D / 64; ++c)
             tma_load_4d(smem_base + L::kQOff + st * kTileBytes + c * 16384, &q_map, bar(L::kQFull + st), c * 64, it.h, it.tq0 + qrow, it.bc);
         }
-        ok = mbar_wait_warp(bar(L::kDoEmpty + st), ph ^ 1u, abort_flag, kSiteBase + 2);
+        const int dst = do_stage(gt);
+        const uint32_t dph = do_par(gt);
+        ok = mbar_wait_warp(bar(L::kDoEmpty + dst), dph ^ 1u, abort_flag, kSiteBase + 2);
         if (!ok) break;
         if (lane == 0) {
-          mbar_expect_tx(bar(L::kDoFull + st), kTileBytes);
+          mbar_expect_tx(bar(L::kDoFull + dst), kTileBytes);
 #pragma unroll
           for (int c = 0; c < D / 64; ++c)
-            tma_load_4d(smem_base + L::kDoOff + st * kTileBytes + c * 16384, &do_map, bar(L::kDoFull + st), c * 64, it.h, it.tq0 + qrow, it.bc);
+            tma_load_4d(smem_base + L::kDoOff + dst * kTileBytes + c * 16384, &do_map, bar(L::kDoFull + dst), c * 64, it.h, it.tq0 + qrow, it.bc);
         }
         if (t == 0) {
           // K_j, V_j of this item into buffer kb, once the products of the item that used it last have
@@ -725,10 +722,10 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         }
         if (qrow + kBwdTileQ > it.Lq) {
           ok = mbar_wait_warp(bar(L::kQFull + st), ph, abort_flag, kSiteBase + 18);
-          ok = ok && mbar_wait_warp(bar(L::kDoFull + st), ph, abort_flag, kSiteBase + 19);
+          ok = ok && mbar_wait_warp(bar(L::kDoFull + dst), dph, abort_flag, kSiteBase + 19);
           if (!ok) break;
           zero_rows(smem_gen + L::kQOff + st * kTileBytes, it.Lq - qrow);
-          zero_rows(smem_gen + L::kDoOff + st * kTileBytes, it.Lq - qrow);
+          zero_rows(smem_gen + L::kDoOff + dst * kTileBytes, it.Lq - qrow);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(L::kQdoFix + st));
@@ -796,17 +793,17 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         issue(kColS + 128u * (uint32_t)sbuf(gt), k_lo + kv_off, q_lo0 + (uint32_t)st * kStageStep);
         mma_commit(leader, bar(L::kSFull + sbuf(gt)));
         mma_commit(leader, bar(L::kQEmpty + st));
-        ok = mbar_wait_warp(bar(L::kDoFull + st), ph, abort_flag, kSiteBase + 6);
+        ok = mbar_wait_warp(bar(L::kDoFull + do_stage(gt)), do_par(gt), abort_flag, kSiteBase + 6);
         if (gt > 0) {
           // the dP columns hold dS^T of the previous tile (read by dK) and, when dQ shares them,
           // the previous dQ tile until it has been drained
-          ok = ok && mbar_wait_warp(bar(kDqT ? L::kDqEmpty : L::kDpFree), prev, abort_flag, kSiteBase + 7);
+          ok = ok && mbar_wait_warp(bar(kTwoS ? L::kDpFree : L::kDqEmpty), prev, abort_flag, kSiteBase + 7);
         }
         if (!ok) break;
         tc_fence_after_sync();
-        issue(kColDp, v_lo + kv_off, do_lo0 + (uint32_t)st * kStageStep);
+        issue(kColDp, v_lo + kv_off, do_lo0 + (uint32_t)do_stage(gt) * kStageStep);
         mma_commit(leader, bar(L::kDpFull));
-        mma_commit(leader, bar(L::kDoEmpty + st));
+        mma_commit(leader, bar(L::kDoEmpty + do_stage(gt)));
       }
       if (!ok) break;
       mma_commit(leader, bar(L::kKvEmpty + kb));  // this warp's products no longer read K_j, V_j once they complete
@@ -817,8 +814,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     // ============================================================ issuer B: dV, dK, dQ
     const bool leader = elect_one();
     constexpr uint32_t idesc_acc = make_idesc(128, D, kBF16, false, true);  // A in TMEM, B rows = contraction
-    // dQ (M = queries, N = D) or dQ^T (M = D, N = queries): both operands rows = contraction
-    constexpr uint32_t idesc_dq = kDqT ? make_idesc(D, 128, kBF16, true, true) : make_idesc(128, D, kBF16, true, true);
+    constexpr uint32_t idesc_dq = make_idesc(128, D, kBF16, true, true);  // dQ: both operands rows = contraction
     constexpr uint32_t kStageStep = kTileBytes >> 4;
     // operands whose rows are the contraction index; the next 64-column block lies 16 KB further
     const uint64_t k_mn = smem_desc_sw128(smem_base + L::kKOff, 16384, 1024);
@@ -856,7 +852,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         ok = mbar_wait_warp(bar(L::kDkvEmpty + prev_kind), (empty_par >> prev_kind) & 1u, abort_flag, kSiteBase + 33);
         empty_par ^= 1u << prev_kind;
       }
-      prev_kind = (kDrainWarps && it.n_q <= kDrainEpilogueMaxTiles) ? 1 : 0;
+      prev_kind = it.n_q <= kDrainEpilogueMaxTiles<D> ? 1 : 0;
       for (int t = 0; t < it.n_q && ok; ++t) {
         const int gt = g + t;
         const int st = gt & 1;
@@ -866,13 +862,13 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         // product is the first of this warp's to read dO_i and waits for that tile itself - without it a row
         // of the stage could still hold the tile of two steps earlier (seen once in some hundred runs on one
         // shape, as dV rows carrying dO of query q - 256 instead of q).
-        ok = mbar_wait_warp(bar(L::kDoFull + st), (uint32_t)(gt >> 1) & 1u, abort_flag, kSiteBase + 22);
+        ok = mbar_wait_warp(bar(L::kDoFull + do_stage(gt)), do_par(gt), abort_flag, kSiteBase + 22);
         ok = ok && mbar_wait_warp(bar(L::kPReady + sbuf(gt)), spar(gt), abort_flag, kSiteBase + 8);
         if (!ok) break;
         tc_fence_after_sync();
-        issue_acc(kColDv, kColS + 128u * (uint32_t)sbuf(gt), do_lo0 + (uint32_t)st * kStageStep, acc0);
+        issue_acc(kColDv, kColS + 128u * (uint32_t)sbuf(gt), do_lo0 + (uint32_t)do_stage(gt) * kStageStep, acc0);
         if (!kTwoS) mma_commit(leader, bar(L::kSFree));
-        mma_commit(leader, bar(L::kDoEmpty + st));
+        mma_commit(leader, bar(L::kDoEmpty + do_stage(gt)));
         // dK += dS^T Q  (no wait for Q_i of this warp's own: dS exists only because S^T = K Q^T was computed
         // from the landed tile, so its arrival precedes the barrier below)
         ok = mbar_wait_warp(bar(L::kDsReady), par, abort_flag, kSiteBase + 9);
@@ -890,7 +886,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           mma_commit(leader, bar(L::kDqFull + sbuf(gt)));
         }
         issue_acc(kColDk, kColDp, q_lo0 + (uint32_t)st * kStageStep, acc0);
-        if (!kDqT) mma_commit(leader, bar(L::kDpFree));
+        if (kTwoS) mma_commit(leader, bar(L::kDpFree));
         mma_commit(leader, bar(L::kQEmpty + st));
         // dK_j, dV_j are complete with the last tile's dK: the epilogue need not wait for its dQ
         if (t == it.n_q - 1) mma_commit(leader, bar(L::kDkvFull));
@@ -902,7 +898,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
 #pragma unroll
           for (int kk = 0; kk < kBwdTileKV / 16; ++kk) {
             const uint64_t kd = make_desc(k_lo + kv_off + kk * (2048 >> 4), hi), dsd = make_desc(ds_lo + kk * (2048 >> 4), hi);
-            mma_ss(leader, tmem + dq_col(gt), kDqT ? kd : dsd, kDqT ? dsd : kd, idesc_dq, kk > 0);
+            mma_ss(leader, tmem + dq_col(gt), dsd, kd, idesc_dq, kk > 0);
           }
           mma_commit(leader, bar(L::kDqFull + sbuf(gt)));
         }
@@ -926,9 +922,6 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     const uint32_t ds_line = smem_base + L::kDsOff + (cg >> 1) * 16384 + lane_row * 128;
     const uint32_t chunk0 = (uint32_t)(cg & 1) * 4;
     const uint32_t sw = (uint32_t)(lane_row & 7);
-    // D = 128: lane l of quarter k holds d = 32 k + l of dQ^T; this warp takes query columns 32 cg ..
-    // D = 64:  this thread holds query row `lane_row`, head columns 16 cg .. 16 cg + 15 of dQ
-    const uint32_t dq_off = tmem + lane_addr + (kDqT ? 32 : 16) * cg;
     int g = 0;    // query tiles processed so far (all items)
     int act = 0;  // items with work so far
     bool ok = true;
@@ -960,33 +953,6 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       c0 *= kLog2e;
       const bool row_ok = kv < Lk;
 
-      // ---- dQ drain (see the file header); t = index within the item of the query tile whose dQ is complete
-      // ---- dQ^T drain by the compute warps themselves (D = 128; at D = 64 the drain warps do it): lane l of
-      // quarter k holds d = 32 k + l, this warp takes query columns 32 cg ..; one red.global.add.f32 per
-      // query covers a full 128-byte line.  t = index within the item of the query tile whose dQ is complete
-      auto drain_dq = [&](int t) {
-        const int gt = g + t;
-        ok = mbar_wait_warp(bar(L::kDqFull + sbuf(gt)), spar(gt), abort_flag, kSiteBase + 14);
-        const uint32_t dq_addr = dq_off + dq_col(gt);
-        if (!ok) return;
-        tc_fence_after_sync();
-        const int q_tile = (i_begin + t) * kBwdTileQ;
-        uint32_t r[32];
-        tmem_ld32_sync(dq_addr, r);
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(L::kDqEmpty + sbuf(gt)));  // the TMEM columns are free again
-        const int q_first = q_tile + 32 * cg;
-        float* dst = p.dq_acc + ((it.acc_row0 + q_first) * p.H + h) * D + lane_row;
-        const int64_t row_stride = (int64_t)p.H * D;
-        const int n_live = min(32, Lq - q_first);  // queries at or beyond Lq get no gradient
-#pragma unroll
-        for (int v = 0; v < 32; ++v) {
-          if (v < n_live)
-            asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + v * row_stride), "f"(__uint_as_float(r[v])) : "memory");
-        }
-      };
-
       for (int t = 0; t < n_q; ++t) {
         const int gt = g + t;
         const int q0 = (i_begin + t) * kBwdTileQ + 32 * cg;  // first query index of my columns
@@ -995,12 +961,12 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         const int q_hi = row_ok ? Lq : 0;
         // warp-uniform on purpose: the two instantiations contain warp-collective TMEM accesses
         const bool need_mask = it.ragged_kv || (q0 + 32 > Lq) || (p.causal && q0 < kv0 + kBwdTileKV - 1);
-        float pv[32];
+        float2 pv[16];  // D = 128 only: the probabilities of this tile
         ok = mbar_wait_warp(bar(L::kSFull + sbuf(gt)), spar(gt), abort_flag, kSiteBase + 12);
         const uint32_t s_addr = s_addr0 + 128u * (uint32_t)sbuf(gt);
         if (!ok) break;
         tc_fence_after_sync();
-        if constexpr (kDrainWarps) {
+        if constexpr (D == 64) {
           if (need_mask) bwd_phase_a16<kBF16, true, kAccurate>(s_addr, c1, c0, q0, q_lo, q_hi);
           else           bwd_phase_a16<kBF16, false, kAccurate>(s_addr, c1, c0, q0, q_lo, q_hi);
         } else {
@@ -1012,22 +978,13 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(L::kPReady + sbuf(gt)));
 
-        if constexpr (kDrainWarps) {
-          // the dQ product of the previous tile (of this or the previous item) reads the shared-memory copy
-          // of dS until it is complete; phase B below rewrites that copy
-          if (gt > 0) ok = mbar_wait_warp(bar(L::kDqFull + sbuf(gt - 1)), spar(gt - 1), abort_flag, kSiteBase + 16);
-          if (!ok) break;
-        } else if (t > 0) {
-          // dQ of the previous tile is complete by now (or soon): drain it while dP^T is computed.
-          // Its completion also means the dQ GEMM no longer reads the shared-memory copy of dS.
-          drain_dq(t - 1);
-          if (!ok) break;
-        }
-
+        // (Phase B rewrites the shared-memory copy of dS, which the dQ product of the previous tile reads.  That
+        // product is complete when dP^T of this tile is: issuer A started the latter only after the previous tile's
+        // dK (D = 64), which its issuer committed after dQ, or after its dQ had been drained (D = 128).)
         ok = mbar_wait_warp(bar(L::kDpFull), (uint32_t)gt & 1u, abort_flag, kSiteBase + 13);
         if (!ok) break;
         tc_fence_after_sync();
-        if constexpr (kDrainWarps) {
+        if constexpr (D == 64) {
           if (need_mask) bwd_phase_b16<kBF16, true>(s_addr, dp_addr, ds_line, chunk0, sw);
           else           bwd_phase_b16<kBF16, false>(s_addr, dp_addr, ds_line, chunk0, sw);
         } else {
@@ -1044,9 +1001,9 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
 
       // ------------------------------------------------------------ epilogue of the item
       // (before the drain of the last dQ tile, whose product is still running); short items' at D = 64 is the
-      // drain warps' (kDrainEpilogueMaxTiles): nothing of the accumulators is needed here then
+      // drain warps' (kDrainEpilogueMaxTiles<D>): nothing of the accumulators is needed here then
       // column groups 0,1 store dV, groups 2,3 store dK (each half of the head dimension)
-      if (kDrainWarps && n_q <= kDrainEpilogueMaxTiles) {
+      if (n_q <= kDrainEpilogueMaxTiles<D>) {
         // (no arrival either: each of the two hand-back barriers is arrived on only by the warps that read the
         // accumulators of that item - a group that runs ahead must not add arrivals to a phase that still
         // waits for the other group's)
@@ -1116,10 +1073,6 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         }
       }
       }
-      if constexpr (!kDrainWarps) {
-        drain_dq(n_q - 1);
-        if (!ok) break;
-      }
       g += n_q;
       ++act;
     }
@@ -1144,39 +1097,60 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   }
 }
 
-// dQ = scale * accumulator, cast to the 16-bit type.  acc is [B, T, H, D] contiguous fp32.
+// dQ = scale * accumulator, cast to the 16-bit type.  One block per (batch element, head, query tile): the accumulator's
+// pieces in as they lie, turned through shared memory, whole rows out.
 struct DqConvertParams {
   const float* acc;
+  int64_t acc_sb, acc_sh;
   void* dq;
   int64_t sb, st, sh;
-  int B, T, H;
+  const int* lens_q;
+  const int* cu_q;
+  int n_tiles, T, H;
   int d_cols;  // columns of dQ (the accumulator has D)
   float scale;
 };
 
 template <int D, bool kBF16>
 __global__ void __launch_bounds__(256) sigattn_dq_convert_kernel(const DqConvertParams p) {
-  constexpr int kChunks = D / 8;  // 8 elements (16 bytes out, 32 bytes in) per chunk
-  const long long total = (long long)p.B * p.T * p.H * kChunks;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % kChunks);
-    if (8 * c >= p.d_cols) continue;
-    long long r = i / kChunks;
-    const int h = (int)(r % p.H);
-    r /= p.H;
-    const int t = (int)(r % p.T);
-    const int b = (int)(r / p.T);
-    const float4 a0 = __ldg(reinterpret_cast<const float4*>(p.acc) + 2 * i);
-    const float4 a1 = __ldg(reinterpret_cast<const float4*>(p.acc) + 2 * i + 1);
-    uint4 w;
-    w.x = pack2<kBF16>(a0.x * p.scale, a0.y * p.scale);
-    w.y = pack2<kBF16>(a0.z * p.scale, a0.w * p.scale);
-    w.z = pack2<kBF16>(a1.x * p.scale, a1.y * p.scale);
-    w.w = pack2<kBF16>(a1.z * p.scale, a1.w * p.scale);
-    uint8_t* dst = reinterpret_cast<uint8_t*>(p.dq) + 2 * ((int64_t)b * p.sb + (int64_t)t * p.st + (int64_t)h * p.sh) + 16 * c;
-    *reinterpret_cast<uint4*>(dst) = w;
+  constexpr int kRowBytes = 2 * D + 16;
+  __shared__ __align__(16) uint8_t tile[128 * kRowBytes];
+  const int i = (int)(blockIdx.x % (unsigned)p.n_tiles);
+  const int bh = (int)(blockIdx.x / (unsigned)p.n_tiles);
+  const int b = bh / p.H, h = bh - b * p.H;
+  int tq0 = 0, limit = p.T, bc = b;
+  if (p.cu_q) {
+    tq0 = p.cu_q[b];
+    limit = min(max(p.cu_q[b + 1] - tq0, 0), p.T);
+    bc = 0;
   }
+  const int rows = min(limit - 128 * i, 128);
+  if (rows <= 0) return;
+  const int live = (p.lens_q ? min(max(p.lens_q[b], 0), p.T) : limit) - 128 * i;  // rows beyond get no gradient
+  const int r = threadIdx.x & 127;
+  if (r < rows) {
+    const int quarter = r >> 5;
+    const int qrows = min(rows - 32 * quarter, 32);
+    const float4* src = reinterpret_cast<const float4*>(p.acc + (int64_t)bc * p.acc_sb + (int64_t)h * p.acc_sh +
+                                                        (int64_t)(tq0 + 128 * i + 32 * quarter) * D);
+#pragma unroll 8
+    for (int c = threadIdx.x >> 7; c < D / 4; c += 2) {
+      const float4 a = __ldg(src + acc_piece(qrows, c, r & 31) / 4);
+      uint2 w;
+      w.x = pack2<kBF16>(a.x * p.scale, a.y * p.scale);
+      w.y = pack2<kBF16>(a.z * p.scale, a.w * p.scale);
+      if (r >= live) w = make_uint2(0u, 0u);
+      *reinterpret_cast<uint2*>(tile + r * kRowBytes + 8 * c) = w;
+    }
+  }
+  __syncthreads();
+  uint8_t* out = reinterpret_cast<uint8_t*>(p.dq) + 2 * ((int64_t)bc * p.sb + (int64_t)h * p.sh + (int64_t)(tq0 + 128 * i) * p.st);
+  constexpr int kLanes = D / 8;  // 16-byte pieces of a row
+  const int piece = threadIdx.x % kLanes;
+  if (8 * piece >= p.d_cols) return;
+  for (int row = threadIdx.x / kLanes; row < rows; row += 256 / kLanes)
+    *reinterpret_cast<uint4*>(out + 2 * (int64_t)row * p.st + 16 * piece) =
+        *reinterpret_cast<const uint4*>(tile + row * kRowBytes + 16 * piece);
 }
 
 }  // namespace sigattn

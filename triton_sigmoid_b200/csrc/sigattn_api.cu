@@ -369,6 +369,8 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
 
   BwdParams bp;
   bp.dq_acc = dq_acc;
+  bp.acc_sh = (int64_t)ex.Tq * D;
+  bp.acc_sb = (int64_t)p->H * bp.acc_sh;
   bp.dk = p->dk;
   bp.dv = p->dv;
   bp.dk_sb = p->dk_strides[0]; bp.dk_st = p->dk_strides[1]; bp.dk_sh = p->dk_strides[2];
@@ -403,7 +405,7 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
     // persistent: one CTA per SM (the kernel's shared memory allows no more), fewer when there are fewer items
     dim3 grid((unsigned int)std::min<int64_t>(n_items, info.n_sm));
     if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
-    kernel<<<grid, kBwdThreads<D>, smem, stream>>>(qm, km, vm, dom, bp);
+    kernel<<<grid, kBwdThreads, smem, stream>>>(qm, km, vm, dom, bp);
     SIG_CUDA(cudaGetLastError());
     if (p->ev_main_stop) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_stop), stream));
   }
@@ -411,16 +413,17 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
     // dQ = scale * accumulator, rounded to the 16-bit type
     DqConvertParams cp;
     cp.acc = dq_acc;
+    cp.acc_sb = bp.acc_sb; cp.acc_sh = bp.acc_sh;
     cp.dq = p->dq;
     cp.sb = p->dq_strides[0]; cp.st = p->dq_strides[1]; cp.sh = p->dq_strides[2];
-    cp.B = ex.B; cp.T = ex.Tq; cp.H = p->H;
+    cp.lens_q = p->seq_lens_q;
+    cp.cu_q = p->cu_seqlens_q;
+    cp.n_tiles = (p->Tq + 127) / 128; cp.T = p->Tq; cp.H = p->H;
     cp.d_cols = head_cols(p);
     cp.scale = p->scale;
-    const long long chunks = (long long)ex.B * ex.Tq * p->H * (D / 8);
-    const int threads = 256;
-    const long long blocks_ll = (chunks + threads - 1) / threads;
-    const int blocks = (int)(blocks_ll > 148LL * 64 ? 148LL * 64 : blocks_ll);
-    sigattn_dq_convert_kernel<D, kBF16><<<blocks, threads, 0, stream>>>(cp);
+    const int64_t blocks = (int64_t)p->B * p->H * cp.n_tiles;
+    if (blocks > INT32_MAX) return fail(-2, "too many (batch, head, query tile) items: %lld", (long long)blocks);
+    sigattn_dq_convert_kernel<D, kBF16><<<(unsigned int)blocks, 256, 0, stream>>>(cp);
     SIG_CUDA(cudaGetLastError());
   }
   return 0;
