@@ -117,7 +117,11 @@ struct FwdSmem {
   static constexpr int kItemEmpty = kItemFull + 2;    // [2] item index read by every consumer warp
   static constexpr int kNumBars = kItemEmpty + 2;
   static constexpr int kMiscOff = kBarOff + 8 * kNumBars;  // tmem base (u32), abort flag (int), 2 x item record (16 int each)
-  static constexpr int kTotal = kMiscOff + 16 + 2 * 64;
+  // D = 64: per-key terms (score_mod) of the chunk a sigmoid warp is on, see fwd_add_score_mod
+  static constexpr int kModFloats = (D == 64) ? 32 : 0;
+  static constexpr int kModOff = (kMiscOff + 16 + 2 * 64 + 15) & ~15;  // read 16 bytes at a time
+  static_assert(kModOff % 16 == 0 && kKOff % 16 == 0, "16-byte accesses");
+  static constexpr int kTotal = kModOff + kFwdSigmoidWarps * kModFloats * 4;
   static constexpr int kDynBytes = kTotal + 1024;  // slack to align the base to 1024 bytes
 };
 
@@ -151,36 +155,52 @@ struct FwdCursor {
 };
 
 // 32 score columns of one TMEM lane (this thread's query row), already in registers -> logits in the
-// base-2 domain, t = (scale * s + bias (+ score_mod[key])) * log2(e).  Chunks that need no element
+// base-2 domain, t = (scale * s + bias) * log2(e).  Chunks that need no element
 // predicate work on logits shifted up by kDeepShift (see sigmoid2_from_shifted_log2_deep).
-// col0 = key index of the first column.
-template <bool kScoreMod, bool kMask, bool kAccurate>
-__device__ __forceinline__ void fwd_chunk_logits(const uint32_t (&r)[32], float2 (&t)[16], float c1, float c0, int col0,
-                                                 const float* sm_row, int Tk) {
-  constexpr int kCh = 32;
+template <bool kMask, bool kAccurate>
+__device__ __forceinline__ void fwd_chunk_logits(const uint32_t (&r)[32], float2 (&t)[16], float c1, float c0) {
   constexpr bool kShift = !kMask && !kAccurate;
   const float c0s = kShift ? c0 + kDeepShift : c0;
 #pragma unroll
-  for (int i = 0; i < kCh / 2; ++i) {
+  for (int i = 0; i < 16; ++i) {
     t[i] = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), make_float2(c1, c1),
                       make_float2(c0s, c0s));
   }
-  if constexpr (kScoreMod) {
-    // per-key additive bias: the same value for every lane (row), read through the read-only path
-    if (col0 + kCh <= Tk && (reinterpret_cast<uintptr_t>(sm_row + col0) & 15u) == 0) {
+}
+
+// Adds the per-key terms, D = 64: `mod` is this lane's, of the chunk's column `lane`, times log2(e).  Every lane needs all
+// 32, so they go through the warp's own patch of shared memory and come back as broadcasts.  The lane's term was loaded
+// while the job before was computed: read from global memory here, 16 bytes by 16 bytes, the loads' latency stood in the
+// chain of every job (B=8 H=8, 64 queries on 4096 keys: 98 us, 47 without the term, 80 this way).
+__device__ __forceinline__ void fwd_add_score_mod(float2 (&t)[16], float mod, float* patch) {
+  __syncwarp();  // the patch's previous content has been read
+  patch[threadIdx.x & 31] = mod;
+  __syncwarp();
 #pragma unroll
-      for (int i = 0; i < kCh / 4; ++i) {
-        const float4 m = __ldg(reinterpret_cast<const float4*>(sm_row + col0) + i);
-        t[2 * i] = __ffma2_rn(make_float2(m.x, m.y), make_float2(kLog2e, kLog2e), t[2 * i]);
-        t[2 * i + 1] = __ffma2_rn(make_float2(m.z, m.w), make_float2(kLog2e, kLog2e), t[2 * i + 1]);
-      }
-    } else {
+  for (int i = 0; i < 8; ++i) {
+    const float4 m = reinterpret_cast<const float4*>(patch)[i];
+    t[2 * i] = __fadd2_rn(t[2 * i], make_float2(m.x, m.y));
+    t[2 * i + 1] = __fadd2_rn(t[2 * i + 1], make_float2(m.z, m.w));
+  }
+}
+
+// D = 128: from global memory.  Twice the warps work on a job there, and cover the latency (the same problem: 55 us, 49
+// without the term; shared memory has room for 16 terms per warp, and two rounds through those took 59 us).
+// col0 = key index of the first column.
+__device__ __forceinline__ void fwd_add_score_mod(float2 (&t)[16], int col0, const float* sm_row, int Tk) {
+  if (col0 + 32 <= Tk && (reinterpret_cast<uintptr_t>(sm_row + col0) & 15u) == 0) {
 #pragma unroll
-      for (int i = 0; i < kCh / 2; ++i) {
-        const int col = col0 + 2 * i;
-        t[i].x = fmaf(col < Tk ? __ldg(sm_row + col) : 0.0f, kLog2e, t[i].x);
-        t[i].y = fmaf(col + 1 < Tk ? __ldg(sm_row + col + 1) : 0.0f, kLog2e, t[i].y);
-      }
+    for (int i = 0; i < 8; ++i) {
+      const float4 m = __ldg(reinterpret_cast<const float4*>(sm_row + col0) + i);
+      t[2 * i] = __ffma2_rn(make_float2(m.x, m.y), make_float2(kLog2e, kLog2e), t[2 * i]);
+      t[2 * i + 1] = __ffma2_rn(make_float2(m.z, m.w), make_float2(kLog2e, kLog2e), t[2 * i + 1]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int col = col0 + 2 * i;
+      t[i].x = fmaf(col < Tk ? __ldg(sm_row + col) : 0.0f, kLog2e, t[i].x);
+      t[i].y = fmaf(col + 1 < Tk ? __ldg(sm_row + col + 1) : 0.0f, kLog2e, t[i].y);
     }
   }
 }
@@ -238,12 +258,13 @@ __device__ __forceinline__ void fwd_chunk_probs(uint32_t s_addr, float2 (&t)[16]
   tmem_st(s_addr, pk);
 }
 
-// Both steps for a chunk whose scores are in registers.
-template <bool kBF16, bool kScoreMod, bool kMask, bool kAccurate>
+// All steps for a chunk whose scores are in registers.  mod_args: those of fwd_add_score_mod after the logits.
+template <bool kBF16, bool kScoreMod, bool kMask, bool kAccurate, typename... ModArgs>
 __device__ __forceinline__ void fwd_sigmoid_chunk(uint32_t s_addr, const uint32_t (&r)[32], float c1, float c0, int col0,
-                                                  int lim, const float* sm_row, int Tk) {
+                                                  int lim, ModArgs... mod_args) {
   float2 t[16];
-  fwd_chunk_logits<kScoreMod, kMask, kAccurate>(r, t, c1, c0, col0, sm_row, Tk);
+  fwd_chunk_logits<kMask, kAccurate>(r, t, c1, c0);
+  if constexpr (kScoreMod) fwd_add_score_mod(t, mod_args...);
   fwd_chunk_probs<kBF16, kMask, kAccurate>(s_addr, t, col0, lim);
 }
 
@@ -767,6 +788,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     int buf = 0;          // 16 warps per job: S buffer of the next job
     uint32_t bph = 0u;    //                   and the parity of that buffer's barriers
     int jobs_base = 0;    // 8 warps per job: jobs of all earlier items, position of this item's first job in the S ring
+    float* mod_patch = reinterpret_cast<float*>(smem_gen + L::kModOff) + L::kModFloats * warp;
     bool ok = true;
 
     for (int k = 0; ok; ++k) {
@@ -824,9 +846,9 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
                 tmem_ld32_sync(s_addr, r);
                 // the predicate code exists only in the instantiation used by boundary chunks
                 if (col0 + 32 > mask_from[s])
-                  fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate>(s_addr, r, c1, c0, col0, lim[s], sm_row, sm_lim);
+                  fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate>(s_addr, r, c1, c0, col0, lim[s], col0, sm_row, sm_lim);
                 else
-                  fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate>(s_addr, r, c1, c0, col0, lim[s], sm_row, sm_lim);
+                  fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate>(s_addr, r, c1, c0, col0, lim[s], col0, sm_row, sm_lim);
                 tmem_st_wait();
                 tc_fence_before_sync();
                 __syncwarp();
@@ -853,6 +875,9 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           for (int n = jobs_base; n < jobs_base + n0 + n1 && ok; ++n)
             ok = mbar_wait_warp(bar(L::kSFull + n % kSBufs), (uint32_t)(n / kSBufs) & 1u, abort_flag, kSiteBase + 10 + s);
         }
+        auto load_mod = [&](int key) -> float { return key < sm_lim ? __ldg(sm_row + key) * kLog2e : 0.0f; };
+        float mod[2] = {0.0f, 0.0f};  // this lane's terms of the two chunks, loaded one key tile ahead
+        if constexpr (kScoreMod) { mod[0] = load_mod(64 * g + lane); mod[1] = load_mod(64 * g + 32 + lane); }
         for (int j = 0; j < n_mine && ok; ++j) {
           const int n = jobs_base + (s == 0 ? j + min(j, n1) : j + min(j + 1, n0));
           const int jb = n % kSBufs;
@@ -870,9 +895,10 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
             tmem_ld_wait_for(r);
             if (c == 0) tmem_ld(s_addr + 32, rbuf[1]);
             if (col0 + 32 * c + 32 > mask_from[s])
-              fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], sm_row, sm_lim);
+              fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], mod[c], mod_patch);
             else
-              fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], sm_row, sm_lim);
+              fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], mod[c], mod_patch);
+            if constexpr (kScoreMod) mod[c] = load_mod((j + 1) * kTileN + 64 * g + 32 * c + lane);
           }
           tmem_st_wait();
           tc_fence_before_sync();
