@@ -1,0 +1,62 @@
+"""Forward with the key range split over a cluster (problems with few items): edges of parts and tiles, against the oracle."""
+
+import pytest
+import torch
+
+import triton_sigmoid_b200 as sa
+from tests.gpu_util import check_against_oracle, make_inputs
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("D", [64, 96, 128])
+@pytest.mark.parametrize("B,H,Tq,Tk,causal", [
+    (2, 2, 64, 512, False),     # one query tile, two parts of two key tiles
+    (1, 3, 1, 1281, False),     # a single query, parts of unequal size, ragged end
+    (3, 1, 128, 4096, False),   # a full query tile, eight parts
+    (2, 3, 129, 1000, False),   # second query tile of one row
+    (1, 2, 700, 700, True),     # causal: parts that only the second query tile sees
+    (1, 1, 1100, 1100, True),
+    (4, 16, 256, 640, False),   # as many items as two parts each have room for
+])
+def test_split_keys(B, H, Tq, Tk, causal, D):
+    dtype = torch.bfloat16 if Tk % 2 else torch.float16
+    q, k, v, do = make_inputs(B, Tq, Tk, H, D, dtype, std=0.7, seed=Tk + D)
+    g = torch.Generator().manual_seed(Tk)
+    lens_k = torch.randint(1, Tk + 1, (B,), generator=g, dtype=torch.int32)
+    lens_k[0] = Tk
+    lens_q = torch.randint(1, Tq + 1, (B,), generator=g, dtype=torch.int32) if B > 2 else torch.full((B,), Tq, dtype=torch.int32)
+    if B > 2:
+        lens_k[1] = 0  # no keys at all: zeros
+        lens_q[2] = 0
+    for b in range(B):
+        k[b, int(lens_k[b]):] = float("nan")
+        v[b, int(lens_k[b]):] = float("nan")
+    mod = 0.5 * torch.randn(B, Tk, generator=g).cuda()
+    ref_k, ref_v = torch.nan_to_num(k), torch.nan_to_num(v)
+    for score_mod in (None, mod):
+        kw = dict(is_causal=causal, sigmoid_bias=-4.0, score_mod=score_mod)
+        lq, lk = lens_q.cuda(), lens_k.cuda()
+        check_against_oracle(lambda a, _k, _v, **x: sa.sigmoid_attention_padded(a, k, v, **x), q, ref_k, ref_v, do, dtype,
+                             lens_q=lq, lens_k=lk, backward=False, **kw)
+        one = sa.sigmoid_attention_padded(q, k, v, seq_lens_k=lk, seq_lens_q=lq, **kw)
+        two = sa.sigmoid_attention_padded(q, k, v, seq_lens_k=lk, seq_lens_q=lq, **kw)
+        assert torch.equal(one, two)  # parts are added in a fixed order
+
+
+def test_split_keys_packed():
+    lens = [700, 1, 513, 1025]
+    cu = torch.tensor([0] + lens).cumsum(0).to(device="cuda", dtype=torch.int32)
+    total, H, D = sum(lens), 2, 64
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = [torch.randn(total, H, D, device="cuda", generator=g).half() for _ in range(3)]
+    mod = 0.5 * torch.randn(total, device="cuda", generator=g)
+    for causal in (False, True):
+        out = sa.sigmoid_attention_varlen(q, k, v, cu, cu, max(lens), max(lens), is_causal=causal, score_mod=mod)
+        for i, n in enumerate(lens):
+            s = slice(int(cu[i]), int(cu[i]) + n)
+            ref = sa.sigmoid_attention_ref(*[t[s].float()[None] for t in (q, k, v)], causal=causal, score_mod=mod[s][None])
+            # one key alone: O = p v up to |v| = 4, whose error is relative: 3.0e-4 (the sigmoid's polynomial) + 4.9e-4 (p in
+            # fp16) + 4.9e-4 (O in fp16) = 1.3e-3, hence the gate of the other parity tests, relative beyond |O| = 1
+            gate = 2e-3 * max(1.0, ref.abs().max().item())
+            assert (out[s].float() - ref[0]).abs().max().item() <= gate

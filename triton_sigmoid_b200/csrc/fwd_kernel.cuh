@@ -35,6 +35,10 @@
 // scores of a later job while the sigmoid warps turn an earlier one into 16-bit P in place
 // (each warp writes P over the start of the columns it has just read) and signal the issuer.
 //
+// Split form (kSplit), for problems with too few items to occupy the SMs: a cluster of p.split CTAs shares one item, each
+// takes a contiguous part of its key tiles, and the partial O, in fp32, are added through distributed shared memory (no
+// workspace, no atomics, a fixed order).  See fwd_split() on the host side for when.
+//
 // Masking: key tiles beyond the causal diagonal or the valid key length are skipped
 // entirely; tiles that straddle either boundary apply an element predicate.
 #pragma once
@@ -63,6 +67,7 @@ struct FwdParams {
   int n_qblk;   // ceil(Tq / 256)
   int n_items;  // B * H * n_qblk
   int group;    // (batch, head) pairs per scheduling group, >= 1 (see fwd_decode_item)
+  int split;    // kSplit: CTAs per cluster = parts of the key range of an item (no tickets then)
   // two counters, zero between launches: [0] items handed out beyond the first per CTA,
   // [1] CTAs that have finished (the last one clears both)
   unsigned int* ticket;
@@ -278,6 +283,7 @@ struct FwdItem {
   int row_lim;        // query rows below this are written (Tq; packed: Lq, the next rows belong to another sequence)
   int key_lim;        // keys below this have a score_mod entry (Tk; packed: Lk)
   int Lq, Lk;
+  int k_first;        // kSplit: first key of this CTA's part; tk0, key_lim, Lk and the tile counts are relative to it (else 0)
   int n0, n1, n_max;  // key tiles of query tile 0 / 1, and the larger of the two
   float bias;         // additive bias of the item's batch element
 };
@@ -285,14 +291,14 @@ struct FwdItem {
 __device__ __forceinline__ void fwd_publish_item(volatile int* rec, int item, const FwdItem& it) {
   rec[1] = it.b; rec[2] = it.h; rec[3] = it.q0; rec[4] = it.bc; rec[5] = it.tq0; rec[6] = it.tk0;
   rec[7] = it.row_lim; rec[8] = it.key_lim; rec[9] = it.Lq; rec[10] = it.Lk; rec[11] = it.n0; rec[12] = it.n1;
-  rec[13] = it.n_max; rec[14] = __float_as_int(it.bias);
+  rec[13] = it.n_max; rec[14] = __float_as_int(it.bias); rec[15] = it.k_first;
   rec[0] = item;
 }
 __device__ __forceinline__ FwdItem fwd_load_item(const volatile int* rec) {
   FwdItem it;
   it.b = rec[1]; it.h = rec[2]; it.q0 = rec[3]; it.bc = rec[4]; it.tq0 = rec[5]; it.tk0 = rec[6];
   it.row_lim = rec[7]; it.key_lim = rec[8]; it.Lq = rec[9]; it.Lk = rec[10]; it.n0 = rec[11]; it.n1 = rec[12];
-  it.n_max = rec[13]; it.bias = __int_as_float(rec[14]);
+  it.n_max = rec[13]; it.bias = __int_as_float(rec[14]); it.k_first = rec[15];
   return it;
 }
 __device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item) {
@@ -340,10 +346,25 @@ __device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item)
   it.n1 = n_kv[1];
   it.n_max = max(it.n0, it.n1);
   it.bias = item_bias(p.bias, p.bias_scalar, it.b, it.Lk);
+  it.k_first = 0;
   return it;
 }
 
-template <int D, bool kBF16, bool kScoreMod, bool kAccurate>
+// kSplit: key tiles [part_begin(r), part_begin(r + 1)) of an item are those of rank r.
+__device__ __forceinline__ int fwd_part_begin(int n_max, int rank, int split) { return n_max * rank / split; }
+// Restricts an item to the part of one rank.
+__device__ __forceinline__ void fwd_take_part(FwdItem& it, int rank, int split) {
+  const int j0 = fwd_part_begin(it.n_max, rank, split), j1 = fwd_part_begin(it.n_max, rank + 1, split);
+  it.k_first = j0 * kTileN;
+  it.tk0 += it.k_first;
+  it.key_lim -= it.k_first;
+  it.Lk -= it.k_first;
+  it.n0 = max(min(it.n0, j1) - j0, 0);
+  it.n1 = max(min(it.n1, j1) - j0, 0);
+  it.n_max = j1 - j0;
+}
+
+template <int D, bool kBF16, bool kScoreMod, bool kAccurate, bool kSplit>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                    const __grid_constant__ CUtensorMap v_map, const FwdParams p) {
@@ -373,7 +394,16 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   const int lane = threadIdx.x & 31;
 
   // a kernel of this library already gave up on a wait: do not pile more work on a sick device
-  if (*reinterpret_cast<volatile int*>(&g_status_word) != 0) return;
+  if constexpr (kSplit) {
+    // (one answer for the CTA; the others of the cluster may get another, and read this one's shared memory)
+    if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) {
+      cluster_sync();
+      cluster_sync();
+      return;
+    }
+  } else if (*reinterpret_cast<volatile int*>(&g_status_word) != 0) {
+    return;
+  }
 
   // ---------------------------------------------------------------- setup
   if (threadIdx.x == 0) {
@@ -431,6 +461,10 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     return item;
   };
 
+  // kSplit, single: no item has a second query tile, so the two groups of sigmoid warps and the two accumulators of
+  // D = 64 take the key tiles alternately instead (job j: group j & 1, O_(j & 1)); the output warps add the two.
+  const bool single = kSplit && D == 64 && p.Tq <= 128;
+
   if (warp >= kFwdOutputWarp0) {
     // ============================================================ output warps: O from TMEM to global memory
     // Four warps, one per TMEM lane quarter (a warp can only read the lanes 32 (warp % 4) ..), one thread
@@ -454,7 +488,33 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         ++act;
         tc_fence_after_sync();
       }
-      if constexpr (D == 64) {
+      if constexpr (kSplit) {
+        // The partial O of this CTA, fp32, over the K / V stages: every tile has been loaded and every product that reads
+        // one is complete.  [tile][row][D], 16-byte pieces swizzled by the row.
+        uint8_t* part = smem_gen + L::kKOff;
+#pragma unroll 1
+        for (int s = 0; s < 2; ++s) {
+          if ((s == 0 ? it.n0 : it.n1) > 0) {
+            uint8_t* row = part + (s * 128 + lane_row) * (4 * D);
+#pragma unroll 1
+            for (int c = 0; c < D / 16; ++c) {
+              uint32_t ra[16], rb[16];
+              tmem_ld16(tmem_lane + kColO + D * s + 16 * c, ra);
+              tmem_ld_wait_for(ra);
+              if (single && it.n0 > 1) {
+                tmem_ld16(tmem_lane + kColO + D + 16 * c, rb);
+                tmem_ld_wait_for(rb);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) ra[i] = __float_as_uint(__uint_as_float(ra[i]) + __uint_as_float(rb[i]));
+              }
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<uint4*>(row + (((4 * c + i) ^ (lane & 7)) << 4)) =
+                    make_uint4(ra[4 * i], ra[4 * i + 1], ra[4 * i + 2], ra[4 * i + 3]);
+            }
+          }
+        }
+      } else if constexpr (D == 64) {
         // The whole item's O goes through shared memory: out of TMEM one row per lane (two 16-column loads in
         // flight at a time), rounded to 16 bits, into this warp's patches (16-byte chunks swizzled by row, so
         // neither side has bank conflicts).  The accumulators are handed back as soon as the last load has
@@ -584,6 +644,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(L::kItemEmpty + islot));
     }
+    if constexpr (kSplit) { cluster_sync(); cluster_sync(); }
   } else if (warp >= kFwdSigmoidWarps) {
   // All four role warps (the idle one included) execute this one instruction: the release is an
   // operation of the whole group of four.
@@ -598,13 +659,19 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       ok = mbar_wait_warp(bar(L::kItemEmpty + slot), ((uint32_t)(k >> 1) & 1u) ^ 1u, abort_flag, kSiteBase + 31);
       if (!ok) break;
       int item = blockIdx.x;  // the first item needs no ticket
-      if (lane == 0 && k > 0) {
-        const unsigned int t = atomicAdd(p.ticket, 1u) + gridDim.x;
-        item = t < (unsigned int)p.n_items ? (int)t : -1;
+      if constexpr (kSplit) {
+        item = k == 0 ? (int)blockIdx.x / p.split : -1;
+      } else {
+        if (lane == 0 && k > 0) {
+          const unsigned int t = atomicAdd(p.ticket, 1u) + gridDim.x;
+          item = t < (unsigned int)p.n_items ? (int)t : -1;
+        }
+        item = __shfl_sync(0xffffffffu, item, 0);
       }
-      item = __shfl_sync(0xffffffffu, item, 0);
       FwdItem it = {};
       if (item >= 0) it = fwd_decode_item(p, item);
+      if constexpr (kSplit)
+        if (item >= 0) fwd_take_part(it, (int)blockIdx.x % p.split, p.split);
       if (lane == 0) {
         if (item >= 0) fwd_publish_item(item_ring + 16 * slot, item, it);
         else item_ring[16 * slot] = -1;
@@ -760,8 +827,8 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         tc_fence_after_sync();
         const uint32_t va = v_lo + (uint32_t)c.st * kStageStep;
         const uint32_t pa = tmem + kColS + 128u * (uint32_t)c.buf;
-        const uint32_t dst = tmem + kColO + (uint32_t)(D * c.s);
-        const uint32_t acc0 = c.j > 0 ? 1u : 0u;
+        const uint32_t dst = tmem + kColO + (uint32_t)(D * (single ? (c.j & 1) : c.s));
+        const uint32_t acc0 = c.j > (single ? 1 : 0) ? 1u : 0u;
 #pragma unroll
         for (int kk = 0; kk < kTileN / 16; ++kk) {
           // P of key columns [32g, 32g+32) sits, 16-bit packed, in buffer columns 32g + [0,16)
@@ -777,6 +844,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       ++act;
     }
   }
+  if constexpr (kSplit) { cluster_sync(); cluster_sync(); }
   }  // role warps
   else {
     // ============================================================ sigmoid warps
@@ -797,7 +865,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       if (!ok) break;
       const int item = item_ring[16 * islot];
       if (item < 0) break;
-      int n0, n1, q0, Lk;
+      int n0, n1, q0, Lk;  // (q0: kSplit: relative to the first key of this CTA's part, as Lk)
       float c0;
       const float* sm_row = nullptr;
       int sm_lim = 0;
@@ -805,11 +873,11 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         const FwdItem it = fwd_load_item(item_ring + 16 * islot);
         n0 = it.n0;
         n1 = it.n1;
-        q0 = it.q0;
+        q0 = it.q0 - (kSplit ? it.k_first : 0);
         Lk = it.Lk;
         c0 = it.bias * kLog2e;
         if constexpr (kScoreMod) {
-          sm_row = p.score_mod + (p.cu_k ? (int64_t)it.tk0 : (int64_t)it.b * p.Tk);
+          sm_row = p.score_mod + (p.cu_k ? (int64_t)it.tk0 : (int64_t)it.b * p.Tk + (kSplit ? it.k_first : 0));
           sm_lim = it.key_lim;
         }
       }
@@ -868,17 +936,22 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         // itself (n1 - n0 is 0 or 1, or n1 = 0: at most two foreign jobs in a row).  A group whose tile has
         // NO job in an item (a query tile beyond the valid length) therefore does not just skip the item: it
         // watches the barrier of every one of its jobs go by.
-        const int s = warp >> 3;
+        const int group = warp >> 3;
+        const int s = single ? 0 : group;
         const int g = (warp >> 2) & 1;
         const int n_mine = s == 0 ? n0 : n1;
+        const int j_first = single ? group : 0, j_step = single ? 2 : 1;
         if (n_mine == 0) {
           for (int n = jobs_base; n < jobs_base + n0 + n1 && ok; ++n)
             ok = mbar_wait_warp(bar(L::kSFull + n % kSBufs), (uint32_t)(n / kSBufs) & 1u, abort_flag, kSiteBase + 10 + s);
         }
         auto load_mod = [&](int key) -> float { return key < sm_lim ? __ldg(sm_row + key) * kLog2e : 0.0f; };
         float mod[2] = {0.0f, 0.0f};  // this lane's terms of the two chunks, loaded one key tile ahead
-        if constexpr (kScoreMod) { mod[0] = load_mod(64 * g + lane); mod[1] = load_mod(64 * g + 32 + lane); }
-        for (int j = 0; j < n_mine && ok; ++j) {
+        if constexpr (kScoreMod) {
+          mod[0] = load_mod(j_first * kTileN + 64 * g + lane);
+          mod[1] = load_mod(j_first * kTileN + 64 * g + 32 + lane);
+        }
+        for (int j = j_first; j < n_mine && ok; j += j_step) {
           const int n = jobs_base + (s == 0 ? j + min(j, n1) : j + min(j + 1, n0));
           const int jb = n % kSBufs;
           ok = mbar_wait_warp(bar(L::kSFull + jb), (uint32_t)(n / kSBufs) & 1u, abort_flag, kSiteBase + 10 + s);
@@ -898,7 +971,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
               fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], mod[c], mod_patch);
             else
               fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], mod[c], mod_patch);
-            if constexpr (kScoreMod) mod[c] = load_mod((j + 1) * kTileN + 64 * g + 32 * c + lane);
+            if constexpr (kScoreMod) mod[c] = load_mod((j + j_step) * kTileN + 64 * g + 32 * c + lane);
           }
           tmem_st_wait();
           tc_fence_before_sync();
@@ -912,6 +985,44 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
 
       // the item's accumulators are the output warps' business; on to the next item
     }
+
+    if constexpr (kSplit) {
+      // ---- the cluster's partial O, added up in the order of the ranks: every rank finishes its share of the rows
+      const int rank = (int)blockIdx.x % p.split;
+      const FwdItem it = fwd_decode_item(p, (int)blockIdx.x / p.split);  // the whole item
+      cluster_sync();
+      constexpr int kPieces = D / 8;  // 8 columns = 16 bytes of O
+      const int share = (p.Tq <= 128 ? 128 : 256) / p.split;
+      for (int i = threadIdx.x; i < share * kPieces; i += kFwdSigmoidWarps * 32) {
+        const int row = rank * share + i / kPieces, piece = i % kPieces;  // row of the item's 256
+        const int n_s = row < 128 ? it.n0 : it.n1;
+        const int qrow = it.q0 + row;
+        if (qrow >= it.row_lim || 8 * piece >= p.d_cols) continue;
+        float acc[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] = 0.0f;
+        if (qrow < it.Lq) {  // rows beyond the valid length are written as zeros
+          const uint32_t at = smem_base + L::kKOff + (uint32_t)row * (4 * D);
+          for (int r = 0; r < p.split; ++r) {
+            if (fwd_part_begin(it.n_max, r, p.split) >= min(n_s, fwd_part_begin(it.n_max, r + 1, p.split))) continue;  // no keys there
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const float4 x = ld_cluster_f4(at + (((2 * piece + h) ^ (row & 7)) << 4), (uint32_t)r);
+              acc[4 * h + 0] += x.x; acc[4 * h + 1] += x.y; acc[4 * h + 2] += x.z; acc[4 * h + 3] += x.w;
+            }
+          }
+        }
+        uint4 w;
+        w.x = pack2<kBF16>(acc[0], acc[1]);
+        w.y = pack2<kBF16>(acc[2], acc[3]);
+        w.z = pack2<kBF16>(acc[4], acc[5]);
+        w.w = pack2<kBF16>(acc[6], acc[7]);
+        *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.o) +
+                                  2 * ((int64_t)it.bc * p.o_sb + (int64_t)it.h * p.o_sh + (int64_t)(it.tq0 + qrow) * p.o_st) +
+                                  16 * piece) = w;
+      }
+      cluster_sync();  // no CTA's shared memory goes away while another reads it
+    }
   }
 
   // ---------------------------------------------------------------- teardown
@@ -921,7 +1032,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     tc_fence_after_sync();
     tmem_dealloc(tmem, kTmemCols);
   }
-  if (threadIdx.x == 0) {
+  if (!kSplit && threadIdx.x == 0) {
     // the last CTA to finish leaves both counters at zero for the next launch that uses them
     __threadfence();
     const unsigned int done = atomicAdd(p.ticket + 1, 1u);
