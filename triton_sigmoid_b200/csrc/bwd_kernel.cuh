@@ -47,6 +47,7 @@ namespace sigattn {
 struct BwdParams {
   // fp32, zero-filled before the launch: one region of (rows of the sequence) x D floats per batch element and head,
   // see acc_piece()
+  // (kByHead: one region per CTA, not filled)
   float* dq_acc;
   int64_t acc_sb, acc_sh;  // floats from one batch element / head to the next (packed: acc_sb = 0)
   void* dk;
@@ -70,6 +71,8 @@ struct BwdParams {
   int n_kvblk;  // ceil(Tk / 128)
   int n_items;  // B * H * n_kvblk
   int group;    // (batch, head) pairs per scheduling group, >= 1 (see bwd_decode_item)
+  void* dq;     // kByHead only (else sigattn_dq_convert_kernel writes dQ)
+  int64_t dq_sb, dq_st, dq_sh;
   // two counters, zero between launches: [0] items handed out beyond the first per CTA,
   // [1] CTAs that have finished (the last one clears both)
   unsigned int* ticket;
@@ -396,7 +399,10 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item)
   return it;
 }
 
-template <int D, bool kBF16, bool kAccurate>
+// kByHead: a CTA takes all key tiles of a (batch element, head), in order, and finishes its dQ itself (see the drain
+// warps), so that the accumulator needs neither the fill nor the conversion pass and stays in the L2.  group is 1 and the
+// tickets count (batch, head) pairs.
+template <int D, bool kBF16, bool kAccurate, bool kByHead>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                    const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap do_map,
@@ -541,8 +547,30 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         BwdItem it;
         const int item = read_item(k, it);
         if (item < 0) break;
-        if (it.n_q == 0) continue;
         const int row_lim = p.cu_q ? it.Lq : p.Tq;
+        // kByHead: the first key tile of a query tile stores its dQ instead of adding it (no fill before the launch), the
+        // last one adds the accumulator to its own and writes the rounded rows (no conversion after it).  All of a
+        // block's traffic is this warp's, so waiting for its own bulk operations orders it.
+        uint8_t* dq_rows = nullptr;  // row 0 of the sequence, this warp's columns
+        int last_j = 0;              // last key tile with keys
+        if constexpr (kByHead) {
+          dq_rows = reinterpret_cast<uint8_t*>(p.dq) +
+                    2 * ((int64_t)it.bc * p.dq_sb + (int64_t)it.h * p.dq_sh + (int64_t)it.tq0 * p.dq_st + kCols * half);
+          last_j = (it.Lk + kBwdTileKV - 1) / kBwdTileKV - 1;
+          if (it.kv0 == 0) {
+            // rows of query tiles that no product is computed for
+            for (int row = it.n_q * kBwdTileQ + quarter * 32 + lane; row < row_lim; row += 128)
+              for (int c = 0; c < kCols && kCols * half + c < p.d_cols; c += 8)
+                *reinterpret_cast<uint4*>(dq_rows + 2 * ((int64_t)row * p.dq_st + c)) = make_uint4(0, 0, 0, 0);
+          } else {
+            if (lane == 0) {
+              bulk_wait_all();  // what earlier key tiles stored and added is in memory
+              fence_proxy_async_global();
+            }
+            __syncwarp();
+          }
+        }
+        if (it.n_q == 0) continue;
         for (int t = 0; t < it.n_q; ++t) {
           const int gt = g + t;
           ok = mbar_wait_warp(bar(L::kDqFull + sbuf(gt)), spar(gt), abort_flag, kSiteBase + 14);
@@ -560,7 +588,45 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           const int row0 = (it.i_begin + t) * kBwdTileQ + quarter * 32;
           const int rows = min(row_lim - row0, 32);  // rows at or beyond Lq hold zeros, which do no harm
           if (rows <= 0) continue;
-          float* dst = p.dq_acc + it.acc_base + (int64_t)row0 * D + (kCols / 32) * half * (rows * 32);
+          float* dst = p.dq_acc + (kByHead ? (int64_t)blockIdx.x * p.acc_sh : it.acc_base) + (int64_t)row0 * D +
+                       (kCols / 32) * half * (rows * 32);
+          const bool store = kByHead && it.kv0 == 0;
+          if (kByHead && it.kv0 == kBwdTileKV * (p.causal ? min(it.i_begin + t, last_j) : last_j)) {
+            const bool live = row0 + lane < it.Lq;
+#pragma unroll
+            for (int c = 0; c < kCols / 32; ++c) {
+              if (lane == 0) bulk_wait_read();
+              __syncwarp();
+              uint4* mine = reinterpret_cast<uint4*>(patch + lane * L::kPatchRow);
+#pragma unroll
+              for (int c8 = 0; c8 < 4; ++c8) {
+                float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+                if (!store && lane < rows) {
+                  a = __ldcg(reinterpret_cast<const float4*>(dst + c * (rows * 32) + acc_piece(rows, 2 * c8, lane)));
+                  b = __ldcg(reinterpret_cast<const float4*>(dst + c * (rows * 32) + acc_piece(rows, 2 * c8 + 1, lane)));
+                }
+                const uint32_t* x = r[c] + 8 * c8;
+                uint4 w;
+                w.x = pack2<kBF16>(p.scale * (a.x + __uint_as_float(x[0])), p.scale * (a.y + __uint_as_float(x[1])));
+                w.y = pack2<kBF16>(p.scale * (a.z + __uint_as_float(x[2])), p.scale * (a.w + __uint_as_float(x[3])));
+                w.z = pack2<kBF16>(p.scale * (b.x + __uint_as_float(x[4])), p.scale * (b.y + __uint_as_float(x[5])));
+                w.w = pack2<kBF16>(p.scale * (b.z + __uint_as_float(x[6])), p.scale * (b.w + __uint_as_float(x[7])));
+                if (!live) w = make_uint4(0, 0, 0, 0);
+                mine[c8] = w;
+              }
+              __syncwarp();
+              // four lanes per row, as in the epilogue below
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int r8 = 8 * i + (lane >> 2);
+                const uint4 w = *reinterpret_cast<const uint4*>(patch + r8 * L::kPatchRow + 16 * (lane & 3));
+                if (r8 < rows && kCols * half + 32 * c + 8 * (lane & 3) < p.d_cols)
+                  *reinterpret_cast<uint4*>(dq_rows + 2 * ((int64_t)(row0 + r8) * p.dq_st + 32 * c + 8 * (lane & 3))) = w;
+              }
+              __syncwarp();
+            }
+            continue;
+          }
 #pragma unroll
           for (int c = 0; c < kCols / 32; ++c) {
             if (lane == 0) bulk_wait_read();  // the patch's previous content has been read
@@ -573,7 +639,10 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
             }
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) bulk_reduce_add_f32(dst + c * (rows * 32), smem_u32(patch), (uint32_t)rows * 128u);
+            if (lane == 0) {
+              if (store) bulk_store(dst + c * (rows * 32), smem_u32(patch), (uint32_t)rows * 128u);
+              else bulk_reduce_add_f32(dst + c * (rows * 32), smem_u32(patch), (uint32_t)rows * 128u);
+            }
           }
         }
         if (!ok) break;
@@ -652,17 +721,28 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     };
     int g = 0;    // query tiles loaded so far (all items)
     int act = 0;  // items with work so far
+    int head = 0, tile = 0;  // kByHead: the pair this CTA is on and its next key tile
     bool ok = true;
     for (int k = 0; ok; ++k) {
       const int slot = k & 1;
       ok = mbar_wait_warp(bar(L::kItemEmpty + slot), ((uint32_t)(k >> 1) & 1u) ^ 1u, abort_flag, kSiteBase + 31);
       if (!ok) break;
       int item = blockIdx.x;  // the first item needs no ticket
-      if (lane == 0 && k > 0) {
-        const unsigned int tk = atomicAdd(p.ticket, 1u) + gridDim.x;
-        item = tk < (unsigned int)p.n_items ? (int)tk : -1;
+      if (kByHead && tile > 0 && tile < p.n_kvblk) {
+        item = head * p.n_kvblk + tile++;
+      } else {
+        const int n_tickets = kByHead ? p.B * p.H : p.n_items;
+        if (lane == 0 && k > 0) {
+          const unsigned int tk = atomicAdd(p.ticket, 1u) + gridDim.x;
+          item = tk < (unsigned int)n_tickets ? (int)tk : -1;
+        }
+        item = __shfl_sync(0xffffffffu, item, 0);
+        if (kByHead && item >= 0) {
+          head = item;
+          tile = 1;
+          item = head * p.n_kvblk;
+        }
       }
-      item = __shfl_sync(0xffffffffu, item, 0);
       BwdItem it = {};
       if (item >= 0) it = bwd_decode_item<D>(p, item);
       if (lane == 0) {

@@ -139,6 +139,13 @@ __device__ __forceinline__ void bulk_reduce_add_f32(float* dst, uint32_t src, ui
                "cp.async.bulk.commit_group;" ::"l"(dst), "r"(src), "r"(bytes)
                : "memory");
 }
+// The same without the addition.
+__device__ __forceinline__ void bulk_store(float* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\t"
+               "cp.async.bulk.commit_group;" ::"l"(dst), "r"(src), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 

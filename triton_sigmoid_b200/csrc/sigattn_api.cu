@@ -386,6 +386,18 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
   return 0;
 }
 
+// Whether the fused backward gives whole (batch element, head) pairs to CTAs (see kByHead): many pairs with short
+// sequences.  The other form fills, reduces into, reads and converts an accumulator of 4 bytes per element of Q, passes
+// over memory that this one saves, but whose share falls with the length, while its CTAs' regions outgrow the L2.  Whole
+// forward + backward, other form -> this one: D = 64 T=128 B=512 H=16 528 -> 480 us, T=256 1138 -> 1010, T=512 3253 -> 3003,
+// T=1024 B=256 5720 -> 5930; causal T=1024 B=256 4030 -> 3700, T=1200 B=100 2527 -> 2392; D = 128 B=128 T=512 1440 -> 1451, causal
+// 1218 -> 1088.  Causal, a region is half as much in use, hence twice the limit.  The pairs must be many, as a CTA's last
+// one ends the launch: 8 per SM (B=80 T=512 H=16: 562 -> 545).  acc_rows: rows of D floats in the caller's accumulator,
+// which the regions must fit (a batch of packed sequences can be shorter than its longest one lets expect).
+bool bwd_by_head(int64_t n_bh, int n_sm, int Tq, int D, bool causal, int64_t acc_rows) {
+  return n_bh >= 8 * (int64_t)n_sm && (int64_t)Tq * D <= (causal ? 98304 : 49152) && (int64_t)n_sm * Tq <= acc_rows;
+}
+
 // The default backward: the fused 5-GEMM kernel with fp32 dQ reductions into a workspace (bwd_kernel.cuh).
 template <int D, bool kBF16, bool kAccurate>
 int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap& km, const CUtensorMap& vm,
@@ -398,12 +410,19 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
     return fail(-4, "backward workspace too small: %zu bytes given, %zu needed", p->workspace_bytes, need);
   if ((reinterpret_cast<uintptr_t>(p->workspace) & 15u) != 0) return fail(-3, "workspace must be 16-byte aligned");
   float* dq_acc = static_cast<float*>(p->workspace);
-  SIG_CUDA(cudaMemsetAsync(dq_acc, 0, need, stream));
+  FwdDeviceInfo info;
+  if (int rc = fwd_device_info(p->device, &info)) return rc;
+  const int64_t n_bh = (int64_t)p->B * p->H;
+  const bool by_head = !kAccurate && bwd_by_head(n_bh, info.n_sm, p->Tq, D, (p->flags & SIGATTN_CAUSAL) != 0,
+                                               (int64_t)ex.B * ex.Tq * p->H);
+  if (!by_head) SIG_CUDA(cudaMemsetAsync(dq_acc, 0, need, stream));
 
   BwdParams bp;
   bp.dq_acc = dq_acc;
-  bp.acc_sh = (int64_t)ex.Tq * D;
+  bp.acc_sh = (int64_t)(by_head ? p->Tq : ex.Tq) * D;
   bp.acc_sb = (int64_t)p->H * bp.acc_sh;
+  bp.dq = p->dq;
+  bp.dq_sb = p->dq_strides[0]; bp.dq_st = p->dq_strides[1]; bp.dq_sh = p->dq_strides[2];
   bp.dk = p->dk;
   bp.dv = p->dv;
   bp.dk_sb = p->dk_strides[0]; bp.dk_st = p->dk_strides[1]; bp.dk_sh = p->dk_strides[2];
@@ -426,23 +445,22 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
   bp.n_items = (int)n_items;
   // Q, dO and the fp32 dQ accumulator of one head; a quarter of the L2 (measured: larger groups cost the
   // reductions their locality, a few heads already balance the CTAs)
-  bp.group = schedule_group(bp.causal != 0, (int64_t)p->B * p->H, (int64_t)p->Tq * D * (2 + 2 + 4), 32ll << 20);
-  FwdDeviceInfo info;
-  if (int rc = fwd_device_info(p->device, &info)) return rc;
+  bp.group = by_head ? 1 : schedule_group(bp.causal != 0, n_bh, (int64_t)p->Tq * D * (2 + 2 + 4), 32ll << 20);
   bp.ticket = next_ticket_pair(info, p->device, stream);
 
   {
-    auto kernel = sigattn_bwd_kernel<D, kBF16, kAccurate>;
+    // (the accurate sigmoid, an option for comparisons, has the general form only)
+    auto kernel = by_head ? sigattn_bwd_kernel<D, kBF16, kAccurate, !kAccurate> : sigattn_bwd_kernel<D, kBF16, kAccurate, false>;
     constexpr int smem = BwdSmem<D>::kDynBytes;
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
     // persistent: one CTA per SM (the kernel's shared memory allows no more), fewer when there are fewer items
-    dim3 grid((unsigned int)std::min<int64_t>(n_items, info.n_sm));
+    dim3 grid((unsigned int)std::min<int64_t>(by_head ? n_bh : n_items, info.n_sm));
     if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
     kernel<<<grid, kBwdThreads, smem, stream>>>(qm, km, vm, dom, bp);
     SIG_CUDA(cudaGetLastError());
     if (p->ev_main_stop) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_stop), stream));
   }
-  {
+  if (!by_head) {
     // dQ = scale * accumulator, rounded to the 16-bit type
     DqConvertParams cp;
     cp.acc = dq_acc;
