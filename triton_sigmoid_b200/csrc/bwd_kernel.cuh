@@ -36,7 +36,7 @@
 // Two issuing warps, because one warp's instruction stream (waits, 32 MMAs, commits per tile
 // pair) is a serial chain that otherwise bounds the kernel.  Everything the two exchange goes
 // through mbarriers: "S columns free" after dV, "dP columns free" after dK.
-// dQ = scale * accumulator is rounded to the 16-bit type by sigattn_dq_convert_kernel.
+// dQ = scale * accumulator is rounded to the 16-bit type by sigattn_dq_convert_kernel; in the kByHead form by the drain warps.
 #pragma once
 
 #include "ptx.cuh"
