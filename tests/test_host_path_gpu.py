@@ -78,3 +78,15 @@ def test_narrow_heads_match_zero_extended_ones(monkeypatch, dtype, dims, split):
             assert a.shape == narrow[0].shape
             # one order of operations except for dQ, whose fp32 reductions have none
             assert torch.equal(a, b) if i != 1 else torch.allclose(a.float(), b.float(), rtol=1e-2, atol=1e-4), (D, i)
+
+
+@pytest.mark.parametrize("D", [64, 30])  # read in place, and through the Python path (zero-extended heads)
+@pytest.mark.parametrize("requires_grad", [False, True])
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_forward_mode_is_refused(which, requires_grad, D):
+    """A tangent cannot be propagated: an output without one would read as a derivative of zero."""
+    args = [torch.randn(1, 64, 2, D, device="cuda", dtype=torch.bfloat16, requires_grad=requires_grad) for _ in range(3)]
+    with torch.autograd.forward_ad.dual_level():
+        args[which] = torch.autograd.forward_ad.make_dual(args[which], torch.ones_like(args[which]))
+        with pytest.raises(NotImplementedError, match="forward-mode"):
+            m.sigmoid_attention(*args)

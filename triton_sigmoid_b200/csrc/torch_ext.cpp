@@ -243,12 +243,18 @@ struct SigmoidAttentionBackward : public torch::autograd::Node {
   }
 };
 
+bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
+
 // Forward, with the autograd node attached when a gradient can be asked for.
 Tensor attention(Tensors t, const Call& c) {
+  const bool grad = at::GradMode::is_enabled() && (t.q.requires_grad() || t.k.requires_grad() || t.v.requires_grad());
+  // There is no forward-mode formula, and the node below knows nothing of tangents: an output without one would read as
+  // a derivative of zero.
+  TORCH_CHECK_NOT_IMPLEMENTED(!has_tangent(t.q) && !has_tangent(t.k) && !has_tangent(t.v) && !(grad && has_tangent(t.score_mod)),
+                              "sigmoid attention has no forward-mode derivative (jvp)");
   t.q = in_place_or_copy(t.q);
   t.k = in_place_or_copy(t.k);
   t.v = in_place_or_copy(t.v);
-  const bool grad = at::GradMode::is_enabled() && (t.q.requires_grad() || t.k.requires_grad() || t.v.requires_grad());
   if (!grad) return run_forward(t, c);
   using torch::autograd::SavedVariable;
   std::shared_ptr<SigmoidAttentionBackward> node(new SigmoidAttentionBackward(), torch::autograd::deleteNode);
