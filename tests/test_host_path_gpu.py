@@ -90,3 +90,63 @@ def test_forward_mode_is_refused(which, requires_grad, D):
         args[which] = torch.autograd.forward_ad.make_dual(args[which], torch.ones_like(args[which]))
         with pytest.raises(NotImplementedError, match="forward-mode"):
             m.sigmoid_attention(*args)
+
+
+def _varlen_call(q, k, v, mod):
+    cu = torch.tensor([0, 70, 130], dtype=torch.int32, device="cuda")
+    return m.sigmoid_attention_varlen(*(t.flatten(0, 1) for t in (q, k, v)), cu, cu, 70, 70, score_mod=mod.flatten())
+
+
+def _padded_call(q, k, v, mod):
+    lens = torch.tensor([65, 40], dtype=torch.int32, device="cuda")
+    return m.sigmoid_attention_padded(q, k, v, seq_lens_k=lens, seq_lens_q=lens, is_causal=True, score_mod=mod)
+
+
+_RELAYOUT = {
+    # the same values, every eighth element of a row (the last stride is 8)
+    "last_stride": lambda t: torch.stack([t] + [torch.full_like(t, 3)] * 7, -1)[..., 0],
+    # rows two elements apart from 16-byte boundaries
+    "misaligned": lambda t: torch.nn.functional.pad(t, (2, 0))[..., 2:],
+    "contiguous": lambda t: t.contiguous(),
+}
+
+
+@pytest.mark.parametrize("call", [_padded_call, _varlen_call])
+@pytest.mark.parametrize("how", sorted(_RELAYOUT))
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_saved_tensor_hooks_may_return_any_layout(how, call, dtype):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = [torch.randn(2, 65, 2, 64, device="cuda", generator=g).to(dtype).requires_grad_() for _ in range(3)]
+    mod = torch.randn(2, 65, device="cuda", generator=g)
+    do = torch.randn(*call(q, k, v, mod).shape, device="cuda", generator=g).to(dtype)
+    ref = torch.autograd.grad(call(q, k, v, mod), (q, k, v), do)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, _RELAYOUT[how]):
+        out = call(q, k, v, mod)
+    got = torch.autograd.grad(out, (q, k, v), do)
+    for name, a, b in zip("qkv", got, ref):  # one key tile per (head, query tile): dQ has one order too
+        assert torch.equal(a, b), name
+
+
+def test_saved_tensor_hooks_that_change_what_was_saved_are_refused():
+    """Another type, size or device than the forward had: an error, before a kernel gets a pointer."""
+    q = torch.randn(2, 65, 2, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    mod = torch.zeros(2, 65, device="cuda")
+    for unpack in (lambda t: t.half(), lambda t: t.cpu(), lambda t: t[..., :1]):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: unpack(t) if t.dim() == 4 else t):
+            out = m.sigmoid_attention(q, q, q, score_mod=mod)
+        with pytest.raises(RuntimeError, match="sigmoid attention backward: query must be"):
+            out.sum().backward()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t if t.dim() == 4 else t[:1]):
+        out = m.sigmoid_attention(q, q, q, score_mod=mod)
+    with pytest.raises(RuntimeError, match="score_mod must have 130 entries"):
+        out.sum().backward()
+
+
+def test_gradient_with_the_negative_bit():
+    """A view whose values are the negated memory, with no strides to give it away."""
+    q = torch.randn(2, 65, 2, 64, device="cuda", requires_grad=True)
+    do = torch._neg_view(torch.randn(2, 65, 2, 64, device="cuda"))
+    assert do.is_neg()
+    got, = torch.autograd.grad(m.sigmoid_attention(q, q, q), q, do)
+    ref, = torch.autograd.grad(m.sigmoid_attention(q, q, q), q, do.clone())
+    assert torch.equal(got, ref)

@@ -180,7 +180,7 @@ Tensor run_forward(const Tensors& t, const Call& c) {
   return out;
 }
 
-void run_backward(const Tensors& t, const Call& c, const Tensor& grad, Tensor& dq, Tensor& dk, Tensor& dv) {
+void run_backward(const Tensors& t, const Call& c, const Tensor& dout, Tensor& dq, Tensor& dk, Tensor& dv) {
   dq = new_like(t.q);
   dk = new_like(t.k);
   dv = new_like(t.v);
@@ -193,7 +193,6 @@ void run_backward(const Tensors& t, const Call& c, const Tensor& grad, Tensor& d
   } else if (dq.numel() == 0 && dk.numel() == 0) {
     return;
   }
-  const Tensor dout = in_place_or_copy(grad);
   SigAttnParams p;
   fill_common(p, t, c);
   p.dout = dout.const_data_ptr();
@@ -216,9 +215,27 @@ void run_backward(const Tensors& t, const Call& c, const Tensor& grad, Tensor& d
   launch(g_abi.bwd, p, "sigattn_bwd", {&dq, &dk, &dv});
 }
 
+// What autograd (the output's gradient) or a saved-tensor hook hands to the backward may have any strides, and from a
+// hook any type, size and device: checked and laid out again before a kernel gets the pointer.
+Tensor taken(const Tensor& given, const char* name, at::IntArrayRef sizes, const Tensor& like) {
+  const Tensor t = given.resolve_neg();
+  TORCH_CHECK(t.layout() == at::kStrided && t.device() == like.device() && t.scalar_type() == like.scalar_type() && t.sizes() == sizes,
+              "sigmoid attention backward: ", name, " must be a ", like.scalar_type(), " tensor of shape ", sizes, " on ", like.device(),
+              ", got ", t.scalar_type(), " ", t.sizes(), " on ", t.device());
+  return in_place_or_copy(t);
+}
+// The same for the per-key term, lengths and offsets (vectors of n values, or undefined).
+Tensor taken_vector(const Tensor& given, const char* name, int64_t n, at::ScalarType type, const Tensor& like) {
+  if (!given.defined()) return given;
+  TORCH_CHECK(given.numel() == n, "sigmoid attention backward: ", name, " must have ", n, " entries, got ", given.numel());
+  return given.to(like.device(), type).contiguous();
+}
+
 struct SigmoidAttentionBackward : public torch::autograd::Node {
   torch::autograd::SavedVariable q, k, v, score_mod, lens_q, lens_k, cu_q, cu_k;
   Call call;
+  at::DimVector q_sizes, k_sizes;
+  int64_t n_offsets = 0;  // entries of cu_q, cu_k
 
   std::string name() const override { return "SigmoidAttentionBackward"; }
   void release_variables() override {
@@ -228,17 +245,19 @@ struct SigmoidAttentionBackward : public torch::autograd::Node {
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
+    const Tensor& grad = grads[0];  // (the engine has checked its type and device)
+    const bool packed = n_offsets > 0;
     Tensors t;
-    t.q = q.unpack();
-    t.k = k.unpack();
-    t.v = v.unpack();
-    t.score_mod = score_mod.unpack();
-    t.lens_q = lens_q.unpack();
-    t.lens_k = lens_k.unpack();
-    t.cu_q = cu_q.unpack();
-    t.cu_k = cu_k.unpack();
+    t.q = taken(q.unpack(), "query", q_sizes, grad);
+    t.k = taken(k.unpack(), "key", k_sizes, grad);
+    t.v = taken(v.unpack(), "value", k_sizes, grad);
+    t.score_mod = taken_vector(score_mod.unpack(), "score_mod", packed ? k_sizes[0] : k_sizes[0] * k_sizes[1], at::kFloat, grad);
+    t.lens_q = taken_vector(lens_q.unpack(), "seq_lens_q", q_sizes[0], at::kInt, grad);
+    t.lens_k = taken_vector(lens_k.unpack(), "seq_lens_k", q_sizes[0], at::kInt, grad);
+    t.cu_q = taken_vector(cu_q.unpack(), "cu_seqlens_q", n_offsets, at::kInt, grad);
+    t.cu_k = taken_vector(cu_k.unpack(), "cu_seqlens_k", n_offsets, at::kInt, grad);
     Tensor dq, dk, dv;
-    run_backward(t, call, grads[0], dq, dk, dv);
+    run_backward(t, call, taken(grad, "grad", q_sizes, grad), dq, dk, dv);
     return {dq, dk, dv};
   }
 };
@@ -268,6 +287,9 @@ Tensor attention(Tensors t, const Call& c) {
   node->cu_q = SavedVariable(t.cu_q, false);
   node->cu_k = SavedVariable(t.cu_k, false);
   node->call = c;
+  node->q_sizes = t.q.sizes();
+  node->k_sizes = t.k.sizes();
+  node->n_offsets = t.cu_q.defined() ? t.cu_q.numel() : 0;
   Tensor out = run_forward(t, c);
   torch::autograd::set_history(out, node);
   return out;
