@@ -150,3 +150,15 @@ def test_gradient_with_the_negative_bit():
     got, = torch.autograd.grad(m.sigmoid_attention(q, q, q), q, do)
     ref, = torch.autograd.grad(m.sigmoid_attention(q, q, q), q, do.clone())
     assert torch.equal(got, ref)
+
+
+def test_second_derivatives_are_refused():
+    """create_graph is fine as long as nobody differentiates the gradients; then it is an error, not a missing term."""
+    q, k, v = [torch.randn(2, 65, 2, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3)]
+    plain = torch.autograd.grad(m.sigmoid_attention(q, k, v).float().square().sum(), (q, k, v))
+    grads = torch.autograd.grad(m.sigmoid_attention(q, k, v).float().square().sum(), (q, k, v), create_graph=True)
+    for a, b in zip(grads, plain):
+        assert torch.equal(a, b)
+    for g in grads:
+        with pytest.raises(RuntimeError, match="differentiate sigmoid attention twice"):
+            (g.float().sum() + q.float().sum()).backward(retain_graph=True)

@@ -16,6 +16,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/grad_mode.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -258,7 +259,14 @@ struct SigmoidAttentionBackward : public torch::autograd::Node {
     t.cu_k = taken_vector(cu_k.unpack(), "cu_seqlens_k", n_offsets, at::kInt, grad);
     Tensor dq, dk, dv;
     run_backward(t, call, taken(grad, "grad", q_sizes, grad), dq, dk, dv);
-    return {dq, dk, dv};
+    torch::autograd::variable_list out{dq, dk, dv};
+    if (!at::GradMode::is_enabled()) return out;
+    // create_graph: the gradients depend on q, k, v and grad in ways that have no formula here.  Left without a history
+    // they would count as constants, and a second derivative would lack their part without a word.
+    for (Tensor& g : out) g.set_requires_grad(true);
+    auto once = std::make_shared<torch::autograd::DelayedError>("trying to differentiate sigmoid attention twice: its backward has no derivative",
+                                                                (int64_t)out.size());
+    return (*once)(std::move(out));
   }
 };
 
