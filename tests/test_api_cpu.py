@@ -148,3 +148,22 @@ def test_torch_reference_matches_oracle():
     a = m.sigmoid_attention_ref(q, k, v, seq_lens_k=lens, seq_lens_q=lens, causal=True)
     b = orc.sigattn_forward(q, k, v, seq_lens_k=lens, seq_lens_q=lens, is_causal=True)
     assert (a - b).abs().max() < 2e-5
+
+
+def test_recording_modes_see_the_registered_ops():
+    """A graph recorded through a dispatch mode holds the attention as an op of its inputs, not its result as a constant."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+
+    lens, cu = torch.tensor([20, 32]), torch.tensor([0, 32, 64], dtype=torch.int32)
+    for D in (64, 30):
+        q, k, v = _qkv(D=D)
+        for op, args, fn in (
+            ("sigmoid_attention_fwd", (q, k, v), lambda q, k, v: m.sigmoid_attention(q, k, v)),
+            ("sigmoid_attn_padded_fwd", (q, k, v, lens), lambda q, k, v, lens: m.sigmoid_attention_padded(q, k, v, lens)),
+            ("sigmoid_attn_varlen_fwd", tuple(t.flatten(0, 1) for t in (q, k, v)) + (cu, cu),
+             lambda q, k, v, cu_q, cu_k: m.sigmoid_attention_varlen(q, k, v, cu_q, cu_k, 32, 32)),
+        ):
+            nodes = list(make_fx(fn, tracing_mode="fake")(*args).graph.nodes)
+            assert any(op in str(n.target) for n in nodes if n.op == "call_function"), (op, D)
+            assert not any(n.op == "get_attr" for n in nodes)
+            assert nodes[-1].args[0].meta["val"].shape == args[0].shape

@@ -74,3 +74,36 @@ def test_varlen_compiled_matches_eager():
     ref = m.sigmoid_attention_varlen(q, k, v, cu, cu, max(lens), max(lens), is_causal=True)
     ref.backward(do)
     assert torch.equal(out, ref) and torch.equal(gk, k.grad)
+
+
+@pytest.mark.parametrize("requires_grad", [False, True])
+def test_jit_trace_records_the_call(requires_grad):
+    """The traced module computes from its inputs (not the traced call's result as a constant), gradients included."""
+    for D in (64, 32):
+        q, k, v, do = make_inputs(2, 130, 130, 2, D, torch.float16, std=0.5, seed=1, requires_grad=requires_grad)
+        traced = torch.jit.trace(lambda a, b, c: m.sigmoid_attention(a, b, c, is_causal=True), (q, k, v))
+        q, k, v, do = make_inputs(2, 130, 130, 2, D, torch.float16, std=0.5, seed=2, requires_grad=requires_grad)
+        out, ref = traced(q, k, v), m.sigmoid_attention(q, k, v, is_causal=True)
+        assert torch.equal(out, ref) and out.requires_grad == requires_grad
+        if requires_grad:
+            got, want = (torch.autograd.grad(o, (q, k, v), do) for o in (out, ref))
+            assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+            assert torch.allclose(got[0].float(), want[0].float(), atol=1e-3, rtol=1e-2)  # order of the fp32 reductions
+
+
+def test_dispatch_modes_see_the_call():
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Log(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    q, k, v, do = make_inputs(2, 130, 130, 2, 64, torch.bfloat16, seed=1, requires_grad=True)
+    with Log() as log:
+        log.seen = []
+        out = m.sigmoid_attention(q, k, v)
+        torch.autograd.grad(out, (q, k, v), do)
+    assert "sigattn_b200.sigmoid_attention_fwd.default" in log.seen
+    assert "sigattn_b200.sigmoid_attention_bwd.default" in log.seen
+    assert torch.equal(out, m.sigmoid_attention(q, k, v))

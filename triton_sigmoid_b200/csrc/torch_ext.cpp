@@ -12,8 +12,10 @@
 // are normalised.
 #include <Python.h>
 
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
@@ -322,6 +324,10 @@ bool plain(const Tensor& t) {
          !t.key_set().has_any(c10::DispatchKeySet({DispatchKey::Negative, DispatchKey::Python, DispatchKey::Functionalize}));
 }
 
+// A Python dispatch mode is active (fake tensors, make_fx, operator counters, selective checkpointing) or torch.jit.trace
+// is recording: what happens here would escape them, the caller takes the registered ops.
+bool observed() { return c10::impl::TorchDispatchModeTLS::any_modes_set() || at::tracer::impl::is_dispatch_enabled(); }
+
 // Argument readers: false = not plain, the caller answers None.
 bool get_tensor(PyObject* o, Tensor* t) {
   if (!THPVariable_CheckExact(o)) return false;
@@ -381,6 +387,7 @@ bool nargs_ok(Py_ssize_t n, Py_ssize_t want, const char* name) {
 PyObject* py_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!nargs_ok(n, 7, "dense")) return nullptr;
+  if (observed()) Py_RETURN_NONE;
   Tensors t;
   Call c;
   if (!get_tensor(a[0], &t.q) || !get_tensor(a[1], &t.k) || !get_tensor(a[2], &t.v)) Py_RETURN_NONE;
@@ -404,6 +411,7 @@ PyObject* py_dense(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_padded(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!nargs_ok(n, 9, "padded")) return nullptr;
+  if (observed()) Py_RETURN_NONE;
   Tensors t;
   Call c;
   if (!get_tensor(a[0], &t.q) || !get_tensor(a[1], &t.k) || !get_tensor(a[2], &t.v)) Py_RETURN_NONE;
@@ -431,6 +439,7 @@ PyObject* py_padded(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_varlen(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!nargs_ok(n, 11, "varlen")) return nullptr;
+  if (observed()) Py_RETURN_NONE;
   Tensors t;
   Call c;
   if (!get_tensor(a[0], &t.q) || !get_tensor(a[1], &t.k) || !get_tensor(a[2], &t.v) || !get_tensor(a[3], &t.cu_q)) Py_RETURN_NONE;

@@ -320,7 +320,20 @@ sigmoid_attn_padded_fwd_op.register_autograd(_padded_backward, setup_context=_pa
 # In eager mode the public functions call the library through csrc/torch_ext.cpp (allocation, parameters, autograd
 # node), not through the ops above: a `torch.library.custom_op` round trip with its generated autograd wrapper costs
 # about 100 us of host time per forward + backward pair, more than the kernels of a short-sequence call take.  Under
-# `torch.compile` the public functions use the registered ops (fake kernels, autograd registration) instead.
+# `torch.compile` the public functions use the registered ops (fake kernels, autograd registration) instead, and so
+# they do while something else records the operators that run.
+def _observed() -> bool:
+    """A dispatch mode (fake tensors, ``make_fx``, operator counters, selective checkpointing) is active or
+    ``torch.jit.trace`` is recording: neither would see the native path."""
+    return torch._C._len_torch_dispatch_stack() > 0 or torch._C._get_tracing_state() is not None
+
+
+def _mark_heads_static(*tensors: torch.Tensor) -> None:
+    for x in tensors:
+        torch._dynamo.mark_static(x, -2)  # heads
+        torch._dynamo.mark_static(x, -1)  # head dimension
+
+
 def _eager_attention(q, k, v, bias, score_mod, seq_lens_q, seq_lens_k, cu_q, cu_k, max_q, max_k, scale, is_causal):
     """The native path for validated inputs that were not plain: `bias` is a Python float (one value for the whole
     call) or None (minus the logarithm of each batch element's number of valid keys, computed by the kernels)."""
@@ -535,10 +548,9 @@ def sigmoid_attention(
     query, key, value = (_pad_head_dim(t, Dk).contiguous() for t in (query, key, value))
 
     bias_value = float(sigmoid_bias) if sigmoid_bias is not None else (-math.log(float(T_q)) if T_q > 0 else 0.0)
-    if compiling:
-        for x in (query, key, value):
-            torch._dynamo.mark_static(x, -2)  # heads
-            torch._dynamo.mark_static(x, -1)  # head dimension
+    if compiling or _observed():
+        if compiling:
+            _mark_heads_static(query, key, value)
         bias = torch.full((B,), bias_value, dtype=torch.float32, device=query.device)
         out = sigmoid_attention_fwd_op(query, key, value, bias, score_mod, float(scale), bool(is_causal))
     else:
@@ -577,8 +589,9 @@ def sigmoid_attention_padded(
         raise ValueError(f"Key and value sequence lengths must match, got K={T_k}, V={T_v}")
 
     full_k = seq_lens_k is None
+    through_ops = compiling or _observed()
     if seq_lens_k is None:
-        if compiling:  # the op's schema wants tensors; the eager path passes "all valid" as a null pointer
+        if through_ops:  # the op's schema wants tensors; the eager path passes "all valid" as a null pointer
             seq_lens_k = torch.full((B,), T_k, dtype=torch.int32, device=query.device)
     else:
         if seq_lens_k.shape != (B,):
@@ -587,7 +600,7 @@ def sigmoid_attention_padded(
             seq_lens_k = seq_lens_k.to(torch.int32)
         seq_lens_k = seq_lens_k.to(query.device).contiguous()
     if seq_lens_q is None:
-        if compiling:
+        if through_ops:
             seq_lens_q = torch.full((B,), T_q, dtype=torch.int32, device=query.device)
     else:
         if seq_lens_q.shape != (B,):
@@ -611,16 +624,15 @@ def sigmoid_attention_padded(
         bias = float(sigmoid_bias)
     elif full_k:
         bias = -math.log(float(T_k)) if T_k > 0 else float("inf")
-    elif compiling:
+    elif through_ops:
         # -log(0) = +inf for an empty key set; every probability is masked there anyway
         bias = -torch.log(seq_lens_k.clamp(min=0, max=T_k).float())
     else:
         bias = None  # the same value, computed by the kernels from the lengths they clamp anyway
 
-    if compiling:
-        for x in (query, key, value):
-            torch._dynamo.mark_static(x, -2)  # heads
-            torch._dynamo.mark_static(x, -1)  # head dimension
+    if through_ops:
+        if compiling:
+            _mark_heads_static(query, key, value)
         if not isinstance(bias, torch.Tensor):
             bias = torch.full((B,), bias, dtype=torch.float32, device=query.device)
         out = sigmoid_attn_padded_fwd_op(query, key, value, seq_lens_k, seq_lens_q, bias, score_mod, float(scale),
@@ -688,7 +700,7 @@ def sigmoid_attention_varlen(
     Dk = _kernel_head_dim(D)
     query, key, value = (_pad_head_dim(t, Dk).contiguous() for t in (query, key, value))
 
-    if compiling:
+    if compiling or _observed():
         if sigmoid_bias is None:
             lens_k = (cu_seqlens_k[1:] - cu_seqlens_k[:-1]).clamp(min=0, max=int(max_seqlen_k))
             bias = -torch.log(lens_k.float())  # +inf for an empty key set; every probability is masked there anyway
