@@ -162,3 +162,10 @@ def test_second_derivatives_are_refused():
     for g in grads:
         with pytest.raises(RuntimeError, match="differentiate sigmoid attention twice"):
             (g.float().sum() + q.float().sum()).backward(retain_graph=True)
+
+
+@pytest.mark.parametrize("name", ["scale", "sigmoid_bias"])
+def test_numbers_beyond_a_float_are_refused(name):
+    q = torch.randn(1, 64, 2, 64, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(OverflowError):
+        m.sigmoid_attention(q, q, q, **{name: 10 ** 400})

@@ -348,7 +348,9 @@ bool get_number(PyObject* o, double* v, bool* given) {
   if (!*given) return true;
   if (!PyFloat_CheckExact(o) && !PyLong_CheckExact(o)) return false;
   *v = PyFloat_AsDouble(o);
-  return !PyErr_Occurred();
+  if (!PyErr_Occurred()) return true;
+  PyErr_Clear();  // an integer beyond a double: not plain, the Python path raises what it is
+  return false;
 }
 // Same device, one supported dtype, a head dimension whose rows are whole 16-byte pieces.
 bool qkv_ok(const Tensors& t) {
