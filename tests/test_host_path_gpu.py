@@ -169,3 +169,18 @@ def test_numbers_beyond_a_float_are_refused(name):
     q = torch.randn(1, 64, 2, 64, device="cuda", dtype=torch.bfloat16)
     with pytest.raises(OverflowError):
         m.sigmoid_attention(q, q, q, **{name: 10 ** 400})
+
+
+def test_an_output_without_a_gradient_gives_zeros():
+    class NoGradient(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            return x.sum()
+
+        @staticmethod
+        def backward(ctx, grad):
+            return None
+
+    qkv = [torch.randn(1, 64, 2, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3)]
+    for g in torch.autograd.grad(NoGradient.apply(m.sigmoid_attention(*qkv)), qkv):
+        assert g.shape == qkv[0].shape and g.abs().sum().item() == 0

@@ -247,7 +247,10 @@ struct SigmoidAttentionBackward : public torch::autograd::Node {
   }
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
-    if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
+    if (!grads[0].defined()) {  // (whoever used the output had no gradient for it: zeros, as for a torch.autograd.Function)
+      const Tensor qs = q.unpack(), ks = k.unpack(), vs = v.unpack();
+      return {at::zeros_like(qs), at::zeros_like(ks), at::zeros_like(vs)};
+    }
     const Tensor& grad = grads[0];  // (the engine has checked its type and device)
     const bool packed = n_offsets > 0;
     Tensors t;
