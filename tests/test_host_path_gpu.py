@@ -184,3 +184,21 @@ def test_an_output_without_a_gradient_gives_zeros():
     qkv = [torch.randn(1, 64, 2, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3)]
     for g in torch.autograd.grad(NoGradient.apply(m.sigmoid_attention(*qkv)), qkv):
         assert g.shape == qkv[0].shape and g.abs().sum().item() == 0
+
+
+@pytest.mark.parametrize("D", [64, 30])
+@pytest.mark.parametrize("requires_grad", [False, True])
+def test_tensor_subclasses_keep_their_type(D, requires_grad):
+    class Tagged(torch.Tensor):
+        pass
+
+    q, k, v = [torch.randn(1, 64, 2, D, device="cuda", dtype=torch.bfloat16, requires_grad=requires_grad) for _ in range(3)]
+    out = m.sigmoid_attention(q.as_subclass(Tagged), k, v)
+    ref = m.sigmoid_attention(q, k, v)
+    assert type(out) is Tagged and type(ref) is torch.Tensor
+    assert type(m.sigmoid_attention(torch.nn.Parameter(q), k, v)) is torch.Tensor
+    assert torch.equal(out.as_subclass(torch.Tensor), ref)
+    if requires_grad:
+        do = torch.randn_like(ref)
+        for a, b in zip(torch.autograd.grad(out, (q, k, v), do), torch.autograd.grad(ref, (q, k, v), do)):
+            assert torch.equal(a.as_subclass(torch.Tensor), b)

@@ -339,7 +339,11 @@ def _eager_attention(q, k, v, bias, score_mod, seq_lens_q, seq_lens_k, cu_q, cu_
     call) or None (minus the logarithm of each batch element's number of valid keys, computed by the kernels)."""
     _check_kernel_inputs(q, k, v)
     _, score_mod, seq_lens_q, seq_lens_k = _prep_aux(q, None, score_mod, seq_lens_q, seq_lens_k)
-    return _ext().attention(q, k, v, score_mod, seq_lens_q, seq_lens_k, cu_q, cu_k, max_q, max_k, bias, scale, is_causal)
+    out = _ext().attention(q, k, v, score_mod, seq_lens_q, seq_lens_k, cu_q, cu_k, max_q, max_k, bias, scale, is_causal)
+    if type(q) not in (torch.Tensor, torch.nn.Parameter):  # a subclass gets what its torch functions give
+        kind = type(q.new_empty(0))
+        out = out if kind is torch.Tensor else out.as_subclass(kind)
+    return out
 
 
 # ----------------------------------------------------------------------------- packed (variable-length) ops
