@@ -202,3 +202,36 @@ def test_tensor_subclasses_keep_their_type(D, requires_grad):
         do = torch.randn_like(ref)
         for a, b in zip(torch.autograd.grad(out, (q, k, v), do), torch.autograd.grad(ref, (q, k, v), do)):
             assert torch.equal(a.as_subclass(torch.Tensor), b)
+
+
+def test_switches_are_read_when_an_op_runs(monkeypatch):
+    """Also by the backward, on autograd's thread, while another thread rewrites the environment."""
+    import os
+    import threading
+
+    q, k, v, do = [torch.randn(2, 700, 2, 64, device="cuda", dtype=torch.bfloat16) for _ in range(4)]
+    leaf = [t.requires_grad_() for t in (q, k, v)]
+    monkeypatch.setenv("SIGATTN_B200_BWD_SPLIT", "1")
+    split = torch.autograd.grad(m.sigmoid_attention(*leaf), leaf, do)
+    monkeypatch.delenv("SIGATTN_B200_BWD_SPLIT")
+    out = m.sigmoid_attention(*leaf)
+    monkeypatch.setenv("SIGATTN_B200_BWD_SPLIT", "1")
+    stop = threading.Event()
+
+    def rewrite():
+        i = 0
+        while not stop.is_set():
+            os.environ[f"SIGATTN_TEST_{i % 50}"] = "x" * (i % 7)
+            i += 1
+
+    other = threading.Thread(target=rewrite)
+    other.start()
+    try:
+        for _ in range(20):
+            for a, b in zip(torch.autograd.grad(out, leaf, do, retain_graph=True), split):
+                assert torch.equal(a, b)  # the split backward is deterministic, dQ included
+    finally:
+        stop.set()
+        other.join()
+        for i in range(50):
+            os.environ.pop(f"SIGATTN_TEST_{i}", None)

@@ -46,7 +46,7 @@ struct Abi {
   int (*device_status)(int) = nullptr;
 } g_abi;
 
-// accurate_sigmoid(): -1 = follow the environment, 0 / 1 = forced.  Read when an op runs, forward or backward.
+// accurate_sigmoid(): -1 = follow the environment, 0 / 1 = forced.
 std::atomic<int> g_accurate_override{-1};
 
 bool env_true(const char* name) {
@@ -56,9 +56,21 @@ bool env_true(const char* name) {
   for (char& c : s) c = (char)std::tolower((unsigned char)c);
   return s == "1" || s == "true" || s == "yes" || s == "on";
 }
-bool accurate_mode() {
+// The run-time switches, read when an op runs.  Only with the GIL: an assignment to os.environ in another Python thread,
+// which holds it too, rewrites the array that getenv() searches.
+struct Switches {
+  bool accurate, split_backward, debug;
+};
+Switches read_switches() {
   const int o = g_accurate_override.load(std::memory_order_relaxed);
-  return o >= 0 ? o != 0 : env_true("TRITON_SIGMOID_ACCURATE");
+  return {o >= 0 ? o != 0 : env_true("TRITON_SIGMOID_ACCURATE"), env_true("SIGATTN_B200_BWD_SPLIT"), env_true("SIGATTN_B200_DEBUG")};
+}
+// On a thread that does not hold it (autograd's).
+Switches read_switches_locked() {
+  const PyGILState_STATE state = PyGILState_Ensure();
+  const Switches s = read_switches();
+  PyGILState_Release(state);
+  return s;
 }
 
 bool dtype_code(at::ScalarType t, int* code) {
@@ -111,7 +123,7 @@ Tensor new_like(const Tensor& t) { return at::detail::empty_cuda(t.sizes(), t.sc
 // The kernels' head dimension for tensors of D columns (the missing columns read as zeros).
 int kernel_head_dim(int64_t D) { return D <= 64 ? 64 : 128; }
 
-void fill_common(SigAttnParams& p, const Tensors& t, const Call& c) {
+void fill_common(SigAttnParams& p, const Tensors& t, const Call& c, const Switches& sw) {
   std::memset(&p, 0, sizeof(p));
   p.struct_bytes = sizeof(p);
   int dt = 0;
@@ -135,7 +147,7 @@ void fill_common(SigAttnParams& p, const Tensors& t, const Call& c) {
     p.Tq = (int32_t)t.q.size(1);
     p.Tk = (int32_t)t.k.size(1);
   }
-  p.flags = (c.causal ? SIGATTN_CAUSAL : 0u) | (accurate_mode() ? SIGATTN_ACCURATE : 0u) |
+  p.flags = (c.causal ? SIGATTN_CAUSAL : 0u) | (sw.accurate ? SIGATTN_ACCURATE : 0u) |
             (c.bias_neg_log_lk ? SIGATTN_BIAS_NEG_LOG_LK : 0u);
   p.scale = c.scale;
   p.bias_scalar = c.bias;
@@ -152,10 +164,10 @@ void fill_common(SigAttnParams& p, const Tensors& t, const Call& c) {
   p.stream = c10::cuda::getCurrentCUDAStream(p.device).stream();
 }
 
-// One C-ABI call.  SIGATTN_B200_DEBUG: outputs are poison-filled beforehand so that unwritten rows show, and the device
+// One C-ABI call.  debug: outputs are poison-filled beforehand so that unwritten rows show, and the device
 // is synchronised and checked after the launch.
-void launch(int (*fn)(const SigAttnParams*), const SigAttnParams& p, const char* what, std::initializer_list<Tensor*> outs) {
-  const bool debug = env_true("SIGATTN_B200_DEBUG");
+void launch(int (*fn)(const SigAttnParams*), const SigAttnParams& p, const char* what, bool debug,
+            std::initializer_list<Tensor*> outs) {
   if (debug && !p.cu_seqlens_q)
     for (Tensor* t : outs) t->fill_(std::nan(""));
   const int rc = fn(&p);
@@ -169,21 +181,21 @@ void launch(int (*fn)(const SigAttnParams*), const SigAttnParams& p, const char*
   }
 }
 
-Tensor run_forward(const Tensors& t, const Call& c) {
+Tensor run_forward(const Tensors& t, const Call& c, const Switches& sw) {
   Tensor out = new_like(t.q);
   if (out.numel() == 0) return out;
   // packed: only rows of the sequences are written; rows between or behind them, and rows of a sequence beyond
   // max_seqlen_q, stay zero (as in the backward)
   if (t.cu_q.defined()) out.zero_();
   SigAttnParams p;
-  fill_common(p, t, c);
+  fill_common(p, t, c, sw);
   p.o = out.mutable_data_ptr();
   fill_strides(p.o_strides, out);
-  launch(g_abi.fwd, p, "sigattn_fwd", {&out});
+  launch(g_abi.fwd, p, "sigattn_fwd", sw.debug, {&out});
   return out;
 }
 
-void run_backward(const Tensors& t, const Call& c, const Tensor& dout, Tensor& dq, Tensor& dk, Tensor& dv) {
+void run_backward(const Tensors& t, const Call& c, const Switches& sw, const Tensor& dout, Tensor& dq, Tensor& dk, Tensor& dv) {
   dq = new_like(t.q);
   dk = new_like(t.k);
   dv = new_like(t.v);
@@ -197,7 +209,7 @@ void run_backward(const Tensors& t, const Call& c, const Tensor& dout, Tensor& d
     return;
   }
   SigAttnParams p;
-  fill_common(p, t, c);
+  fill_common(p, t, c, sw);
   p.dout = dout.const_data_ptr();
   fill_strides(p.do_strides, dout);
   p.dq = dq.mutable_data_ptr();
@@ -207,7 +219,7 @@ void run_backward(const Tensors& t, const Call& c, const Tensor& dout, Tensor& d
   fill_strides(p.dk_strides, dk);
   fill_strides(p.dv_strides, dv);
   Tensor ws;  // the fused backward's fp32 dQ accumulator (kept alive until the launch is queued)
-  if (env_true("SIGATTN_B200_BWD_SPLIT")) {
+  if (sw.split_backward) {
     p.flags |= SIGATTN_BWD_SPLIT;
   } else if (p.dtype != SIGATTN_FP32) {
     const int64_t elems = std::max<int64_t>(dq.numel() / p.head_cols * p.D, 4);
@@ -215,7 +227,7 @@ void run_backward(const Tensors& t, const Call& c, const Tensor& dout, Tensor& d
     p.workspace = ws.mutable_data_ptr();
     p.workspace_bytes = (size_t)elems * sizeof(float);
   }
-  launch(g_abi.bwd, p, "sigattn_bwd", {&dq, &dk, &dv});
+  launch(g_abi.bwd, p, "sigattn_bwd", sw.debug, {&dq, &dk, &dv});
 }
 
 // What autograd (the output's gradient) or a saved-tensor hook hands to the backward may have any strides, and from a
@@ -246,6 +258,7 @@ struct SigmoidAttentionBackward : public torch::autograd::Node {
     for (auto* s : {&q, &k, &v, &score_mod, &lens_q, &lens_k, &cu_q, &cu_k}) s->reset_data();
   }
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    const Switches sw = read_switches_locked();  // (before the lock: nobody waits for the GIL while holding it)
     std::lock_guard<std::mutex> lock(mutex_);
     if (!grads[0].defined()) {  // (whoever used the output had no gradient for it: zeros, as for a torch.autograd.Function)
       const Tensor qs = q.unpack(), ks = k.unpack(), vs = v.unpack();
@@ -263,7 +276,7 @@ struct SigmoidAttentionBackward : public torch::autograd::Node {
     t.cu_q = taken_vector(cu_q.unpack(), "cu_seqlens_q", n_offsets, at::kInt, grad);
     t.cu_k = taken_vector(cu_k.unpack(), "cu_seqlens_k", n_offsets, at::kInt, grad);
     Tensor dq, dk, dv;
-    run_backward(t, call, taken(grad, "grad", q_sizes, grad), dq, dk, dv);
+    run_backward(t, call, sw, taken(grad, "grad", q_sizes, grad), dq, dk, dv);
     torch::autograd::variable_list out{dq, dk, dv};
     if (!at::GradMode::is_enabled()) return out;
     // create_graph: the gradients depend on q, k, v and grad in ways that have no formula here.  Left without a history
@@ -278,7 +291,7 @@ struct SigmoidAttentionBackward : public torch::autograd::Node {
 bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
 
 // Forward, with the autograd node attached when a gradient can be asked for.
-Tensor attention(Tensors t, const Call& c) {
+Tensor attention(Tensors t, const Call& c, const Switches& sw) {
   const bool grad = at::GradMode::is_enabled() && (t.q.requires_grad() || t.k.requires_grad() || t.v.requires_grad());
   // There is no forward-mode formula, and the node below knows nothing of tangents: an output without one would read as
   // a derivative of zero.
@@ -287,7 +300,7 @@ Tensor attention(Tensors t, const Call& c) {
   t.q = in_place_or_copy(t.q);
   t.k = in_place_or_copy(t.k);
   t.v = in_place_or_copy(t.v);
-  if (!grad) return run_forward(t, c);
+  if (!grad) return run_forward(t, c, sw);
   using torch::autograd::SavedVariable;
   std::shared_ptr<SigmoidAttentionBackward> node(new SigmoidAttentionBackward(), torch::autograd::deleteNode);
   node->set_next_edges(torch::autograd::collect_next_edges(t.q, t.k, t.v));
@@ -303,7 +316,7 @@ Tensor attention(Tensors t, const Call& c) {
   node->q_sizes = t.q.sizes();
   node->k_sizes = t.k.sizes();
   node->n_offsets = t.cu_q.defined() ? t.cu_q.numel() : 0;
-  Tensor out = run_forward(t, c);
+  Tensor out = run_forward(t, c, sw);
   torch::autograd::set_history(out, node);
   return out;
 }
@@ -367,11 +380,12 @@ bool qkv_ok(const Tensors& t) {
 
 PyObject* wrap(const Tensors& t, const Call& c) {
   Tensor out;
+  const Switches sw = read_switches();
   {
     // the launch and the allocations need no interpreter; other Python threads may run meanwhile
     PyThreadState* state = PyEval_SaveThread();
     try {
-      out = attention(t, c);
+      out = attention(t, c, sw);
     } catch (...) {
       PyEval_RestoreThread(state);
       throw;
