@@ -4,6 +4,7 @@ against the float64 oracle with the gates of tests/test_f32_gpu.py."""
 import pytest
 import torch
 
+import triton_sigmoid_b200 as sa
 from tests.gpu_util import make_inputs
 from tests.test_f32_gpu import _check
 
@@ -24,3 +25,19 @@ def test_tile_edges(B, H, T, D, causal):
                 t[b, int(lens[b]):] = 1.0e3
     lens = lens.cuda()
     _check(q, k, v, do, lens_q=lens, lens_k=lens, is_causal=causal, score_mod=torch.randn(B, T, device="cuda") * 0.5)
+
+
+@pytest.mark.parametrize("lo,hi", [(-20, -10), (-10, -4), (-4, 0), (0, 8)])
+def test_sigmoid_is_as_accurate_as_the_plain_formula(lo, hi):
+    """One key, one-hot: O is the sigmoid of the query's first column.  Its RMS relative error against float64 is no larger
+    than that of 1 / (1 + exp(-x)) in float32."""
+    T, H = 4096, 16
+    x = torch.linspace(lo, hi, T * H + 2, device="cuda", dtype=torch.float64)[1:-1].float().reshape(T, H)
+    q = torch.zeros(1, T, H, 64, device="cuda")
+    q[0, :, :, 0] = x
+    one = torch.zeros(1, 1, H, 64, device="cuda")
+    one[..., 0] = 1.0
+    out = sa.sigmoid_attention_padded(q, one, one, scale=1.0, sigmoid_bias=0.0)[0, :, :, 0]
+    ref = 1.0 / (1.0 + torch.exp(-x.double()))
+    rms = lambda y: ((y.double() - ref) / ref).square().mean().sqrt().item()  # noqa: E731
+    assert rms(out) <= rms(1.0 / (1.0 + torch.exp(-x)))
