@@ -41,3 +41,22 @@ def test_sigmoid_is_as_accurate_as_the_plain_formula(lo, hi):
     ref = 1.0 / (1.0 + torch.exp(-x.double()))
     rms = lambda y: ((y.double() - ref) / ref).square().mean().sqrt().item()  # noqa: E731
     assert rms(out) <= rms(1.0 / (1.0 + torch.exp(-x)))
+
+
+@pytest.mark.parametrize("H", [1, 80])  # 16-row tiles, 64-row tiles
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_nonfinite_values_pass_through_probabilities_of_zero(bad, causal, H):
+    """dS = P (1 - P) dP of a visible pair is 0 * NaN = NaN also where P has underflowed; of a masked pair it is 0."""
+    T, j = 200, 70
+    q, k, v, do = make_inputs(1, T, T, H, 64, torch.float32, std=0.5, seed=1)
+    v[:, j] = bad
+    do[..., 0] = 1.0  # so that dP is not finite whatever the signs of the other columns
+    do[..., 1:] = 0.0
+    leaf = [t.requires_grad_() for t in (q, k, v)]
+    out = sa.sigmoid_attention(*leaf, is_causal=causal, sigmoid_bias=-1000.0)
+    dq, dk, dv = torch.autograd.grad(out, leaf, do)
+    sees = torch.arange(T, device="cuda") >= (j if causal else 0)  # queries that see key j
+    assert dq[:, sees].isnan().all() and (dq[:, ~sees] == 0).all()
+    at = torch.arange(T, device="cuda") == j
+    assert dk[:, at].isnan().all() and (dk[:, ~at] == 0).all() and (dv == 0).all()

@@ -295,6 +295,9 @@ __device__ __forceinline__ F32Item f32_item(const F32Params& p, int n_tiles, boo
   return it;
 }
 
+__device__ __forceinline__ bool f32_visible(const F32Params& p, const F32Item& it, int i, int j) {
+  return i < it.Lq && j < it.Lk && (!p.causal || j <= i);
+}
 // Probabilities of a thread's part of a score tile, in place.  i0 / j0: its first query and key; (di, dj) from one row a
 // to the next, (ci, cj) from one column c to the next.
 template <int kNC, bool kMask>
@@ -308,7 +311,7 @@ __device__ __forceinline__ void f32_probs_of(const F32Params& p, const F32Item& 
       float x = s[a][c] * p.scale + bias;
       if (sm) x += (!kMask || j < it.key_lim) ? sm[j] : 0.f;
       float pr = f32_sigmoid(x);
-      if constexpr (kMask) pr = (i < it.Lq && j < it.Lk && (!p.causal || j <= i)) ? pr : 0.f;
+      if constexpr (kMask) pr = f32_visible(p, it, i, j) ? pr : 0.f;
       s[a][c] = pr;
     }
 }
@@ -323,8 +326,25 @@ __device__ __forceinline__ bool f32_all_visible(const F32Params& p, const F32Ite
   return q0 + nq <= it.Lq && k0 + nk <= it.Lk && (!p.causal || k0 + nk - 1 <= q0);
 }
 
-// dS from P and dP; a masked element (P exactly 0) stays 0 whatever dP is.
-__device__ __forceinline__ float f32_ds(float pr, float dp) { return pr != 0.f ? pr * (1.0f - pr) * dp : 0.f; }
+// dS from P and dP, in place of dP (positions as for f32_probs).  A masked element is 0 whatever dP is; a visible one
+// passes NaN and infinities on, also where its probability has underflowed to 0.
+template <int kNC, bool kMask>
+__device__ __forceinline__ void f32_ds_of(const F32Params& p, const F32Item& it, const float (&pr)[8][kNC], float (&dp)[8][kNC],
+                                          int i0, int j0, int di, int dj, int ci, int cj) {
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int c = 0; c < kNC; ++c) {
+      const float ds = pr[a][c] * (1.0f - pr[a][c]) * dp[a][c];
+      dp[a][c] = !kMask || f32_visible(p, it, i0 + a * di + c * ci, j0 + a * dj + c * cj) ? ds : 0.f;
+    }
+}
+template <int kNC>
+__device__ __forceinline__ void f32_ds(const F32Params& p, const F32Item& it, const float (&pr)[8][kNC], float (&dp)[8][kNC],
+                                       bool all_visible, int i0, int j0, int di, int dj, int ci, int cj) {
+  if (all_visible) f32_ds_of<kNC, false>(p, it, pr, dp, i0, j0, di, dj, ci, cj);
+  else f32_ds_of<kNC, true>(p, it, pr, dp, i0, j0, di, dj, ci, cj);
+}
 
 // ---------------------------------------------------------------- forward
 template <int D, int kR, int kC>
@@ -426,8 +446,8 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(cons
     {
       float pr[8][S::kNC];
       f32_scores<D, S::kNC>(Ks, Qs, th.row0, th.col0, p.d_cols, pr);
-      f32_probs<S::kNC>(p, it, pr, f32_all_visible(p, it, q0, kF32Cols, k0, S::kRows), q0 + th.col0, k0 + th.row0, 0, 2, 16, 0,
-                        bias, sm);
+      const bool all_visible = f32_all_visible(p, it, q0, kF32Cols, k0, S::kRows);
+      f32_probs<S::kNC>(p, it, pr, all_visible, q0 + th.col0, k0 + th.row0, 0, 2, 16, 0, bias, sm);
 #pragma unroll
       for (int a = 0; a < 8; ++a)
 #pragma unroll
@@ -436,11 +456,11 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(cons
       __syncthreads();  // dO has arrived
       float dp[8][S::kNC];
       f32_scores<D, S::kNC>(Vs, dOs, th.row0, th.col0, p.d_cols, dp);
+      f32_ds<S::kNC>(p, it, pr, dp, all_visible, q0 + th.col0, k0 + th.row0, 0, 2, 16, 0);
 #pragma unroll
       for (int a = 0; a < 8; ++a)
 #pragma unroll
-        for (int c = 0; c < S::kNC; ++c)
-          dSs[(th.row0 + 2 * a) * S::kWRow + th.col0 + 16 * c] = f32_ds(pr[a][c], dp[a][c]);
+        for (int c = 0; c < S::kNC; ++c) dSs[(th.row0 + 2 * a) * S::kWRow + th.col0 + 16 * c] = dp[a][c];
     }
     f32_group_sync<kC>(th.group);
     f32_accumulate<D, S::kNX>(dSs, Qs, th.row0, th.x0, dk);
@@ -509,12 +529,13 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dq_f32_kernel(const 
       }
       float s[8][S::kNC];
       f32_scores<D, S::kNC>(Qs, Ks, th.row0, th.col0, p.d_cols, s);
-      f32_probs<S::kNC>(p, it, s, f32_all_visible(p, it, q0, S::kRows, k0, kF32Cols), q0 + th.row0, k0 + th.col0, 2, 0, 0, 16,
-                        bias, sm);
+      const bool all_visible = f32_all_visible(p, it, q0, S::kRows, k0, kF32Cols);
+      f32_probs<S::kNC>(p, it, s, all_visible, q0 + th.row0, k0 + th.col0, 2, 0, 0, 16, bias, sm);
+      f32_ds<S::kNC>(p, it, s, dp, all_visible, q0 + th.row0, k0 + th.col0, 2, 0, 0, 16);
 #pragma unroll
       for (int a = 0; a < 8; ++a)
 #pragma unroll
-        for (int c = 0; c < S::kNC; ++c) dSs[(th.row0 + 2 * a) * S::kWRow + th.col0 + 16 * c] = f32_ds(s[a][c], dp[a][c]);
+        for (int c = 0; c < S::kNC; ++c) dSs[(th.row0 + 2 * a) * S::kWRow + th.col0 + 16 * c] = dp[a][c];
     }
     f32_group_sync<kC>(th.group);
     f32_accumulate<D, S::kNX>(dSs, Ks, th.row0, th.x0, dq);
