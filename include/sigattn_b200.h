@@ -167,6 +167,20 @@ int sigattn_bwd(const SigAttnParams *p);
 #define SIGATTN_STATIC_SCRATCH_ELEMS (8u * 1024u * 1024u)
 int sigattn_bwd_static_scratch(const SigAttnParams *p);
 
+/* Which form of its kernels a call with these parameters takes on a device of `n_sm` multiprocessors (every form gives the
+ * same results up to the order of fp32 sums).  Looks at extents, dtype and flags only, no pointer is followed and no GPU is
+ * needed: for tests and for explaining a measurement. */
+enum SigAttnForm {
+  SIGATTN_FORM_FWD = 0,         /* persistent */
+  SIGATTN_FORM_FWD_SPLIT = 1,   /* few items: the keys of each are split over a cluster */
+  SIGATTN_FORM_BWD = 2,         /* fused, dQ accumulated over the whole workspace and converted */
+  SIGATTN_FORM_BWD_BY_HEAD = 3, /* fused, a CTA takes whole (batch element, head) pairs */
+  SIGATTN_FORM_BWD_STREAM = 4,  /* SIGATTN_BWD_SPLIT */
+  SIGATTN_FORM_F32_16 = 5,      /* fp32, forward or backward: tiles of 16 rows */
+  SIGATTN_FORM_F32_64 = 6       /* ... of 64 rows */
+};
+int sigattn_form(const SigAttnParams *p, int backward, int n_sm);
+
 /* Bytes of `workspace` sigattn_bwd needs for this problem (fp32 dQ accumulator). */
 size_t sigattn_bwd_workspace_bytes(int32_t B, int32_t Tq, int32_t H, int32_t D);
 

@@ -1,5 +1,7 @@
 """Helpers shared by the GPU parity tests (not collected by pytest)."""
 
+import ctypes
+
 import torch
 
 from oracle import sigattn_oracle as orc
@@ -11,6 +13,23 @@ GRAD_REL_L2 = 1e-2
 
 def rel_l2(got: torch.Tensor, ref: torch.Tensor) -> float:
     return ((got.double() - ref.double()).norm() / (ref.double().norm() + 1e-30)).item()
+
+
+def launch_form(B, H, Tq, Tk, D, dtype, backward, causal=False, accurate=False, packed_rows=0, n_sm=None):
+    """The form of the kernels (`_cabi.FORM_*`) that a call with these extents takes on this device (on one of `n_sm` SMs);
+    packed_rows: total_q of packed sequences, whose longest has Tq rows."""
+    from triton_sigmoid_b200 import _cabi
+
+    p = _cabi.SigAttnParams()
+    p.struct_bytes = ctypes.sizeof(p)
+    p.dtype = (torch.float16, torch.bfloat16, torch.float32).index(dtype)
+    p.B, p.H, p.D, p.head_cols, p.Tq, p.Tk = B, H, 64 if D <= 64 else 128, D, Tq, Tk
+    p.flags = (_cabi.SIGATTN_CAUSAL if causal else 0) | (_cabi.SIGATTN_ACCURATE if accurate else 0)
+    if packed_rows:
+        p.cu_seqlens_q = p.cu_seqlens_k = 16  # (looked at for being there only)
+        p.total_q = p.total_k = packed_rows
+    n_sm = n_sm or torch.cuda.get_device_properties(0).multi_processor_count
+    return _cabi.load().sigattn_form(ctypes.byref(p), int(backward), n_sm)
 
 
 def make_inputs(B, Tq, Tk, H, D, dtype, std=1.0, seed=0, requires_grad=False):

@@ -6,8 +6,10 @@ import os
 import re
 
 import pytest
+import torch
 
 from tests.conftest import ROOT
+from tests.gpu_util import launch_form
 from triton_sigmoid_b200 import _cabi
 from triton_sigmoid_b200.build import LIB_PATH, build
 
@@ -88,6 +90,31 @@ def test_backward_needs_gradient_pointers(lib):
 def test_empty_batch_is_a_no_op(lib):
     assert lib.sigattn_fwd(ctypes.byref(_params(B=0))) == 0
     assert lib.sigattn_last_error() == b""
+
+
+@pytest.mark.parametrize("want,kw", [
+    (_cabi.FORM_FWD, dict(B=4, H=16, Tq=4096, Tk=4096)),
+    (_cabi.FORM_FWD, dict(B=1, H=1, Tq=64, Tk=384)),            # three key tiles: a part would have one
+    (_cabi.FORM_FWD_SPLIT, dict(B=1, H=1, Tq=64, Tk=385)),
+    (_cabi.FORM_FWD_SPLIT, dict(B=4, H=16, Tq=256, Tk=4096)),   # 64 items, two parts each
+    (_cabi.FORM_FWD, dict(B=5, H=13, Tq=256, Tk=4096)),         # 65
+    (_cabi.FORM_BWD, dict(B=4, H=16, Tq=4096, Tk=4096, backward=True)),
+    (_cabi.FORM_BWD, dict(B=1183, H=1, Tq=512, Tk=512, backward=True)),
+    (_cabi.FORM_BWD_BY_HEAD, dict(B=1184, H=1, Tq=512, Tk=512, backward=True)),  # 8 pairs per SM
+    (_cabi.FORM_BWD, dict(B=1184, H=1, Tq=512, Tk=512, backward=True, accurate=True)),
+    (_cabi.FORM_BWD, dict(B=1184, H=1, Tq=1024, Tk=1024, backward=True)),
+    (_cabi.FORM_BWD_BY_HEAD, dict(B=1184, H=1, Tq=1024, Tk=1024, backward=True, causal=True)),
+    (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=512, Tk=512, backward=True, packed_rows=148 * 512 * 4)),
+    (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=512, Tk=512, backward=True, packed_rows=148 * 512 - 1)),
+    (_cabi.FORM_F32_16, dict(B=73, H=1, Tq=64, Tk=64, dtype=torch.float32)),
+    (_cabi.FORM_F32_64, dict(B=74, H=1, Tq=64, Tk=64, dtype=torch.float32, backward=True)),
+])
+def test_form(lib, want, kw):
+    """The rules of the dispatch on 148 SMs."""
+    args = dict(dict(D=64, dtype=torch.float16, backward=False), **kw)
+    assert launch_form(**args, n_sm=148) == want
+    assert lib.sigattn_form(None, 0, 148) < 0 and lib.sigattn_form(ctypes.byref(_params(struct_bytes=8)), 0, 148) < 0
+    assert lib.sigattn_form(ctypes.byref(_params()), 0, 0) < 0
 
 
 def test_documented_reference_side_binding_is_runnable_python():

@@ -5,17 +5,21 @@ import pytest
 import torch
 
 import triton_sigmoid_b200 as sa
-from tests.gpu_util import make_inputs
+from tests.gpu_util import launch_form, make_inputs
 from tests.test_f32_gpu import _check
+from triton_sigmoid_b200._cabi import FORM_F32_16, FORM_F32_64
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("B,H,T", [(1, 1, 15), (1, 2, 17), (1, 1, 81),          # 16-row tiles
-                                   (1, 90, 63), (40, 2, 64), (1, 80, 65), (5, 9, 129)])  # 64-row tiles
-def test_tile_edges(B, H, T, D, causal):
+@pytest.mark.parametrize("B,H,T,form", [(1, 1, 15, FORM_F32_16), (1, 2, 17, FORM_F32_16), (1, 1, 81, FORM_F32_16),
+                                        (1, 90, 63, FORM_F32_64), (40, 2, 64, FORM_F32_64), (1, 80, 65, FORM_F32_64),
+                                        (5, 9, 129, FORM_F32_64)])
+def test_tile_edges(B, H, T, form, D, causal):
+    for backward in (False, True):
+        assert launch_form(B, H, T, T, D, torch.float32, backward, causal) == form
     q, k, v, do = make_inputs(B, T, T, H, D, torch.float32, std=0.5, seed=T + D, requires_grad=True)
     lens = torch.randint(1, T + 1, (B,), generator=torch.Generator().manual_seed(T), dtype=torch.int32)
     lens[0] = T
@@ -49,6 +53,7 @@ def test_sigmoid_is_as_accurate_as_the_plain_formula(lo, hi):
 def test_nonfinite_values_pass_through_probabilities_of_zero(bad, causal, H):
     """dS = P (1 - P) dP of a visible pair is 0 * NaN = NaN also where P has underflowed; of a masked pair it is 0."""
     T, j = 200, 70
+    assert launch_form(1, H, T, T, 64, torch.float32, True, causal) == (FORM_F32_16 if H == 1 else FORM_F32_64)
     q, k, v, do = make_inputs(1, T, T, H, 64, torch.float32, std=0.5, seed=1)
     v[:, j] = bad
     do[..., 0] = 1.0  # so that dP is not finite whatever the signs of the other columns

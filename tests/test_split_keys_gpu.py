@@ -4,7 +4,8 @@ import pytest
 import torch
 
 import triton_sigmoid_b200 as sa
-from tests.gpu_util import check_against_oracle, make_inputs
+from tests.gpu_util import check_against_oracle, launch_form, make_inputs
+from triton_sigmoid_b200._cabi import FORM_FWD_SPLIT
 
 pytestmark = pytest.mark.gpu
 
@@ -21,6 +22,7 @@ pytestmark = pytest.mark.gpu
 ])
 def test_split_keys(B, H, Tq, Tk, causal, D):
     dtype = torch.bfloat16 if Tk % 2 else torch.float16
+    assert launch_form(B, H, Tq, Tk, D, dtype, False, causal) == FORM_FWD_SPLIT
     q, k, v, do = make_inputs(B, Tq, Tk, H, D, dtype, std=0.7, seed=Tk + D)
     g = torch.Generator().manual_seed(Tk)
     lens_k = torch.randint(1, Tk + 1, (B,), generator=g, dtype=torch.int32)
@@ -51,6 +53,7 @@ def test_split_keys_packed():
     g = torch.Generator(device="cuda").manual_seed(5)
     q, k, v = [torch.randn(total, H, D, device="cuda", generator=g).half() for _ in range(3)]
     mod = 0.5 * torch.randn(total, device="cuda", generator=g)
+    assert launch_form(len(lens), H, max(lens), max(lens), D, q.dtype, False, packed_rows=total) == FORM_FWD_SPLIT
     for causal in (False, True):
         out = sa.sigmoid_attention_varlen(q, k, v, cu, cu, max(lens), max(lens), is_causal=causal, score_mod=mod)
         for i, n in enumerate(lens):
@@ -60,3 +63,15 @@ def test_split_keys_packed():
             # fp16) + 4.9e-4 (O in fp16) = 1.3e-3, hence the gate of the other parity tests, relative beyond |O| = 1
             gate = 2e-3 * max(1.0, ref.abs().max().item())
             assert (out[s].float() - ref[0]).abs().max().item() <= gate
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Tq,Tk,causal", [(64, 1281, False), (700, 700, True)])
+def test_split_keys_accurate(Tq, Tk, causal, D):
+    assert launch_form(2, 2, Tq, Tk, D, torch.float16, False, causal, accurate=True) == FORM_FWD_SPLIT
+    q, k, v, do = make_inputs(2, Tq, Tk, 2, D, torch.float16, std=0.7, seed=D)
+    mod = 0.5 * torch.randn(2, Tk, device="cuda")
+    for score_mod in (None, mod):
+        with sa.accurate_sigmoid():
+            check_against_oracle(sa.sigmoid_attention_padded, q, k, v, do, torch.float16, backward=False, is_causal=causal,
+                                 score_mod=score_mod)

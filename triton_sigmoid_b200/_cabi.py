@@ -21,6 +21,8 @@ SIGATTN_BWD_SPLIT = 4
 SIGATTN_BIAS_NEG_LOG_LK = 8
 SIGATTN_STATIC_SCRATCH_ELEMS = 8 * 1024 * 1024
 
+FORM_FWD, FORM_FWD_SPLIT, FORM_BWD, FORM_BWD_BY_HEAD, FORM_BWD_STREAM, FORM_F32_16, FORM_F32_64 = range(7)
+
 Q_ABI_VERSION, Q_SM_ARCH, Q_MAX_HEAD_DIM, Q_PARAMS_SIZE = 0, 1, 2, 3
 
 EXPORTED_SYMBOLS = (
@@ -32,6 +34,7 @@ EXPORTED_SYMBOLS = (
     "sigattn_query",
     "sigattn_device_status",
     "sigattn_selftest_bounded_wait",
+    "sigattn_form",
 )
 
 
@@ -118,6 +121,8 @@ def load() -> ctypes.CDLL:
         lib.sigattn_device_status.restype = ctypes.c_int
         lib.sigattn_selftest_bounded_wait.argtypes = [ctypes.c_int, ctypes.c_int]
         lib.sigattn_selftest_bounded_wait.restype = ctypes.c_int
+        lib.sigattn_form.argtypes = [ctypes.POINTER(SigAttnParams), ctypes.c_int, ctypes.c_int]
+        lib.sigattn_form.restype = ctypes.c_int
         if lib.sigattn_query(Q_PARAMS_SIZE) != ctypes.sizeof(SigAttnParams):
             raise ImportError(
                 f"SigAttnParams layout mismatch: library {lib.sigattn_query(Q_PARAMS_SIZE)} bytes, "

@@ -286,8 +286,12 @@ unsigned int* next_ticket_pair(const FwdDeviceInfo& info, int device, cudaStream
 // within a GPC, whose SM counts are not all multiples of 8: 7/8 of the SMs are counted on).
 // B=8 H=8, 64 queries on 1024 .. 4096 keys: 47 -> 29 us; B=1 T=4096 H=2, D = 64 61 -> 33, D = 128 74 -> 37; B=1 T=1024 H=4
 // 24.6 -> 20.5; with two parts of two tiles, B=1 T=512 H=4, 20 -> 18.4; unchanged beyond 64 items, B=1 T=8192 H=4.
-int fwd_split(int64_t n_items, int Tk, int n_sm) {
-  const int tiles = (Tk + sigattn::kTileN - 1) / sigattn::kTileN;
+int64_t fwd_items(const SigAttnParams* p) {
+  return (int64_t)((p->Tq + sigattn::kFwdBlockM - 1) / sigattn::kFwdBlockM) * p->H * p->B;
+}
+int fwd_split(const SigAttnParams* p, int n_sm) {
+  const int64_t n_items = fwd_items(p);
+  const int tiles = (p->Tk + sigattn::kTileN - 1) / sigattn::kTileN;
   int split = 1;
   while (split < 8 && n_items * split * 2 <= n_sm * 7 / 8 && tiles >= 4 * split) split *= 2;
   return split > 1 ? split : 0;
@@ -318,7 +322,7 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
   fp.d_cols = head_cols(p);
   fp.causal = (p->flags & SIGATTN_CAUSAL) ? 1 : 0;
   fp.n_qblk = (p->Tq + kFwdBlockM - 1) / kFwdBlockM;
-  const int64_t n_items = (int64_t)fp.n_qblk * p->H * p->B;
+  const int64_t n_items = fwd_items(p);
   if (n_items > INT32_MAX) return fail(-2, "too many (batch, head, query block) items: %lld", (long long)n_items);
   fp.n_items = (int)n_items;
   // K and V of one head, half of the L2 for them
@@ -326,7 +330,7 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
   FwdDeviceInfo info;
   if (int rc = fwd_device_info(p->device, &info)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-  fp.split = fwd_split(n_items, p->Tk, info.n_sm);
+  fp.split = fwd_split(p, info.n_sm);
   if (fp.split) {
     auto kernel = sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, true>;
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
@@ -364,10 +368,15 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
 // forward + backward, other form -> this one: D = 64 T=128 B=512 H=16 528 -> 480 us, T=256 1138 -> 1010, T=512 3253 -> 3003,
 // T=1024 B=256 5720 -> 5930; causal T=1024 B=256 4030 -> 3700, T=1200 B=100 2527 -> 2392; D = 128 B=128 T=512 1440 -> 1451, causal
 // 1218 -> 1088.  Causal, a region is half as much in use, hence twice the limit.  The pairs must be many, as a CTA's last
-// one ends the launch: 8 per SM (B=80 T=512 H=16: 562 -> 545).  acc_rows: rows of D floats in the caller's accumulator,
-// which the regions must fit (a batch of packed sequences can be shorter than its longest one lets expect).
-bool bwd_by_head(int64_t n_bh, int n_sm, int Tq, int D, bool causal, int64_t acc_rows) {
-  return n_bh >= 8 * (int64_t)n_sm && (int64_t)Tq * D <= (causal ? 98304 : 49152) && (int64_t)n_sm * Tq <= acc_rows;
+// one ends the launch: 8 per SM (B=80 T=512 H=16: 562 -> 545).  The caller's accumulator must have room for a region per CTA
+// (a batch of packed sequences can be shorter than its longest one lets expect).  The accurate sigmoid, an option for
+// comparisons, has the general form only.
+bool bwd_by_head(const SigAttnParams* p, int n_sm) {
+  const bool causal = (p->flags & SIGATTN_CAUSAL) != 0;
+  const Extents ex = extents(p);
+  const int64_t n_bh = (int64_t)p->B * p->H, acc_rows = (int64_t)ex.B * ex.Tq * p->H;
+  return !(p->flags & SIGATTN_ACCURATE) && n_bh >= 8 * (int64_t)n_sm && (int64_t)p->Tq * p->D <= (causal ? 98304 : 49152) &&
+         (int64_t)n_sm * p->Tq <= acc_rows;
 }
 
 // The default backward: the fused 5-GEMM kernel with fp32 dQ reductions into a workspace (bwd_kernel.cuh).
@@ -385,8 +394,7 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
   FwdDeviceInfo info;
   if (int rc = fwd_device_info(p->device, &info)) return rc;
   const int64_t n_bh = (int64_t)p->B * p->H;
-  const bool by_head = !kAccurate && bwd_by_head(n_bh, info.n_sm, p->Tq, D, (p->flags & SIGATTN_CAUSAL) != 0,
-                                               (int64_t)ex.B * ex.Tq * p->H);
+  const bool by_head = bwd_by_head(p, info.n_sm);
   if (!by_head) SIG_CUDA(cudaMemsetAsync(dq_acc, 0, need, stream));
 
   BwdParams bp;
@@ -421,7 +429,6 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
   bp.ticket = next_ticket_pair(info, p->device, stream);
 
   {
-    // (the accurate sigmoid, an option for comparisons, has the general form only)
     auto kernel = by_head ? sigattn_bwd_kernel<D, kBF16, kAccurate, !kAccurate> : sigattn_bwd_kernel<D, kBF16, kAccurate, false>;
     constexpr int smem = BwdSmem<D>::kDynBytes;
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
@@ -563,6 +570,13 @@ int launch_f32_shape(const SigAttnParams* p, const sigattn::F32Params& fp, bool 
   return 0;
 }
 
+// Rows per CTA: 64 once such tiles occupy half of the SMs; below that 16, with four times the threads per row, which take
+// 1.9 times the SM time per row and a quarter of the latency (B=2 T=256 H=4: 15 against 30 us forward).
+int f32_tile_rows(const SigAttnParams* p, int n_sm) {
+  const int64_t tiles64 = (int64_t)p->B * p->H * ((std::min(p->Tq, p->Tk) + 63) / 64);
+  return 2 * tiles64 >= n_sm ? 64 : 16;
+}
+
 template <int D>
 int launch_f32_d(const SigAttnParams* p, bool backward) {
   using namespace sigattn;
@@ -599,10 +613,7 @@ int launch_f32_d(const SigAttnParams* p, bool backward) {
   FwdDeviceInfo info;
   if (int rc = fwd_device_info(p->device, &info)) return rc;
   if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
-  // 64-row tiles once they occupy half of the SMs; below that, 16-row tiles with four times the threads per row, which
-  // take 1.9 times the SM time per row and a quarter of the latency (B=2 T=256 H=4: 15 against 30 us forward)
-  const int64_t tiles64 = (int64_t)p->B * p->H * ((std::min(p->Tq, p->Tk) + 63) / 64);
-  const int rc = 2 * tiles64 >= info.n_sm ? launch_f32_shape<D, 4, D / 64>(p, fp, backward) : launch_f32_shape<D, 1, 4>(p, fp, backward);
+  const int rc = f32_tile_rows(p, info.n_sm) == 64 ? launch_f32_shape<D, 4, D / 64>(p, fp, backward) : launch_f32_shape<D, 1, 4>(p, fp, backward);
   if (rc) return rc;
   if (p->ev_main_stop) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_stop), stream));
   return 0;
@@ -656,6 +667,17 @@ int sigattn_query(int what) {
     case SIGATTN_Q_PARAMS_SIZE: return (int)sizeof(SigAttnParams);
     default: return -1;
   }
+}
+
+int sigattn_form(const SigAttnParams* p, int backward, int n_sm) {
+  g_err[0] = 0;
+  if (!p) return fail(-1, "params is NULL");
+  if (p->struct_bytes != sizeof(SigAttnParams)) return fail(-1, "struct_bytes %u != sizeof(SigAttnParams) %zu (ABI mismatch)", p->struct_bytes, sizeof(SigAttnParams));
+  if (n_sm < 1) return fail(-2, "n_sm must be positive, got %d", n_sm);
+  if (p->dtype == SIGATTN_FP32) return f32_tile_rows(p, n_sm) == 64 ? SIGATTN_FORM_F32_64 : SIGATTN_FORM_F32_16;
+  if (!backward) return fwd_split(p, n_sm) ? SIGATTN_FORM_FWD_SPLIT : SIGATTN_FORM_FWD;
+  if (p->flags & SIGATTN_BWD_SPLIT) return SIGATTN_FORM_BWD_STREAM;
+  return bwd_by_head(p, n_sm) ? SIGATTN_FORM_BWD_BY_HEAD : SIGATTN_FORM_BWD;
 }
 
 size_t sigattn_bwd_workspace_bytes(int32_t B, int32_t Tq, int32_t H, int32_t D) {
