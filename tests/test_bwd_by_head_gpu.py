@@ -98,9 +98,9 @@ def test_packed(causal):
                 assert torch.equal(a[s], r)
 
 
-def test_packed_batch_too_short_for_the_regions():
-    """Enough pairs, but the accumulator (total_q rows) has no room for a region of the longest sequence per CTA: the
-    general form, with the results of the sequences by themselves."""
+def test_packed_batch_of_mostly_short_sequences():
+    """Enough pairs, but few rows for the longest sequence (the accumulator of total_q rows has no room for a region of it
+    per CTA): the general form, with the results of the sequences by themselves."""
     H, D = 1, 64
     n = _enough(1200, H)
     lens = [16] * n

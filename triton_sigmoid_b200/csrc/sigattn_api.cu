@@ -362,21 +362,34 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
   return 0;
 }
 
-// Whether the fused backward gives whole (batch element, head) pairs to CTAs (see kByHead): many pairs with short
-// sequences.  The other form fills, reduces into, reads and converts an accumulator of 4 bytes per element of Q, passes
-// over memory that this one saves, but whose share falls with the length, while its CTAs' regions outgrow the L2.  Whole
-// forward + backward, other form -> this one: D = 64 T=128 B=512 H=16 528 -> 480 us, T=256 1138 -> 1010, T=512 3253 -> 3003,
-// T=1024 B=256 5720 -> 5930; causal T=1024 B=256 4030 -> 3700, T=1200 B=100 2527 -> 2392; D = 128 B=128 T=512 1440 -> 1451, causal
-// 1218 -> 1088.  Causal, a region is half as much in use, hence twice the limit.  The pairs must be many, as a CTA's last
-// one ends the launch: 8 per SM (B=80 T=512 H=16: 562 -> 545).  The caller's accumulator must have room for a region per CTA
-// (a batch of packed sequences can be shorter than its longest one lets expect).  The accurate sigmoid, an option for
-// comparisons, has the general form only.
+// Whether the fused backward gives whole (batch element, head) pairs to CTAs (see kByHead).  The general form fills, reduces
+// into, reads and converts an accumulator of 4 bytes per element of Q, passes over memory that this one saves; but its items
+// are single key tiles, which balance better, and here the launch ends on somebody's last pair.  So the pairs must be many
+// (8 per SM: B=80 T=512 H=16 562 -> 545 us forward + backward) and short.  Below: the backward alone in this form over the
+// general one, 8 to 40 pairs per SM.
+//  - Tq, as the passes' share falls with it and the CTAs' regions outgrow the L2: D = 64 T=256 0.82 - 0.84, 512 0.91 - 0.97, 640
+//    0.95 - 1.00, 768 0.95 - 1.10, 1024 1.06 - 1.16; D = 128 256 0.82 - 0.86, 384 0.93 - 0.97, 512 0.95 - 1.03.  Causal, a region is
+//    half as much in use: D = 64 1024 0.88 - 0.97, 1280 0.95 - 0.99, 1536 1.03 - 1.06; D = 128 768 0.95 - 1.00.  Ragged batches,
+//    whose general form balances no better and (padded) passes over the padding too, go a little further: D = 64 lengths from
+//    0.4 of 768 0.93 - 0.97, causal 1536 0.96 - 0.99.
+//  - Tk, as a pair of many key tiles is a long chain whose products are what costs: four tiles, or as many as query tiles.
+//    Tq=64 Tk=256 0.94 - 0.96, 512 1.00 - 1.03, 1024 1.03 - 1.06; Tq=256 Tk=512 0.91 - 0.96, 1024 1.00 - 1.08, 2048 1.02 - 1.14, 8192 1.17;
+//    D = 128 Tq=128 Tk=512 0.88 - 0.94, 1024 0.97 - 1.04.  Ragged, lengths from 0.4: Tq=640 Tk=1281 0.97 - 1.01, hence 2.5 times as
+//    many.  (Causal, keys behind the last query have no work: Tq=512 Tk=1024 0.87.)
+//  - packed sequences, on average: a CTA's share of the rows is at least 2.5 of the longest sequence (with 8 pairs per SM, an
+//    average of 0.3 of it; the general form's passes only cover the rows there are).  Some of 768 tokens among many of 128
+//    1.12 - 1.21, of 192 1.02 - 1.05, of 256 0.92 - 1.07; of 512 tokens 1.01 - 1.13, 0.95 - 1.09, 0.91 - 0.98.  This also covers that
+//    the accumulator must have room for a region per CTA.  (Padded, 768 among 96: 0.71 - 0.89.)
+// The accurate sigmoid, an option for comparisons, has the general form only.
 bool bwd_by_head(const SigAttnParams* p, int n_sm) {
-  const bool causal = (p->flags & SIGATTN_CAUSAL) != 0;
+  const bool causal = (p->flags & SIGATTN_CAUSAL) != 0, ragged = p->seq_lens_q || p->seq_lens_k || p->cu_seqlens_q;
   const Extents ex = extents(p);
   const int64_t n_bh = (int64_t)p->B * p->H, acc_rows = (int64_t)ex.B * ex.Tq * p->H;
-  return !(p->flags & SIGATTN_ACCURATE) && n_bh >= 8 * (int64_t)n_sm && (int64_t)p->Tq * p->D <= (causal ? 98304 : 49152) &&
-         (int64_t)n_sm * p->Tq <= acc_rows;
+  const int64_t q_tiles = ((int64_t)p->Tq + 127) / 128, k_tiles = ((int64_t)(causal ? std::min(p->Tk, p->Tq) : p->Tk) + 127) / 128;
+  const int max_q = (p->D == 128 ? 384 : ragged ? 768 : 640) * (causal ? 2 : 1);
+  return !(p->flags & SIGATTN_ACCURATE) && n_bh >= 8 * (int64_t)n_sm && p->Tq <= max_q &&
+         (k_tiles <= std::max<int64_t>(q_tiles, 4) || (ragged && 2 * k_tiles <= 5 * q_tiles)) &&
+         2 * acc_rows >= 5 * (int64_t)n_sm * p->Tq;
 }
 
 // The default backward: the fused 5-GEMM kernel with fp32 dQ reductions into a workspace (bwd_kernel.cuh).
