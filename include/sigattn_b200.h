@@ -73,7 +73,10 @@ enum SigAttnQuery {
   SIGATTN_Q_ABI_VERSION = 0,
   SIGATTN_Q_SM_ARCH = 1,        /* 100: the only architecture the kernels are built for */
   SIGATTN_Q_MAX_HEAD_DIM = 2,   /* 128 */
-  SIGATTN_Q_PARAMS_SIZE = 3     /* sizeof(SigAttnParams), for binding sanity checks */
+  SIGATTN_Q_PARAMS_SIZE = 3,    /* sizeof(SigAttnParams), for binding sanity checks */
+  SIGATTN_Q_HEAD_COLS = 4       /* 1: SigAttnParams.head_cols is obeyed.  Libraries from before that field (same struct size and
+                                 * ABI version, the field reserved) answer -1 and would read narrow rows as D columns wide:
+                                 * ask before setting it */
 };
 
 typedef struct SigAttnParams {

@@ -92,6 +92,23 @@ def test_empty_batch_is_a_no_op(lib):
     assert lib.sigattn_last_error() == b""
 
 
+def test_a_library_without_head_cols_is_told_apart(lib, monkeypatch):
+    """Same struct size and ABI version, but the field was reserved: the binding, which sets it, does not load such a library."""
+    assert lib.sigattn_query(_cabi.Q_HEAD_COLS) == 1
+
+    class Older:
+        def __getattr__(self, name):
+            def fn(what):
+                return ctypes.sizeof(_cabi.SigAttnParams) if what == _cabi.Q_PARAMS_SIZE else -1
+            setattr(self, name, fn)
+            return fn
+
+    monkeypatch.setattr(_cabi, "_lib", None)
+    monkeypatch.setattr(ctypes, "CDLL", lambda path: Older())
+    with pytest.raises(ImportError, match="older than SigAttnParams.head_cols"):
+        _cabi.load()
+
+
 @pytest.mark.parametrize("want,kw", [
     (_cabi.FORM_FWD, dict(B=4, H=16, Tq=4096, Tk=4096)),
     (_cabi.FORM_FWD, dict(B=1, H=1, Tq=64, Tk=384)),            # three key tiles: a part would have one

@@ -23,7 +23,7 @@ SIGATTN_STATIC_SCRATCH_ELEMS = 8 * 1024 * 1024
 
 FORM_FWD, FORM_FWD_SPLIT, FORM_BWD, FORM_BWD_BY_HEAD, FORM_BWD_STREAM, FORM_F32_16, FORM_F32_64 = range(7)
 
-Q_ABI_VERSION, Q_SM_ARCH, Q_MAX_HEAD_DIM, Q_PARAMS_SIZE = 0, 1, 2, 3
+Q_ABI_VERSION, Q_SM_ARCH, Q_MAX_HEAD_DIM, Q_PARAMS_SIZE, Q_HEAD_COLS = range(5)
 
 EXPORTED_SYMBOLS = (
     "sigattn_fwd",
@@ -121,13 +121,15 @@ def load() -> ctypes.CDLL:
         lib.sigattn_device_status.restype = ctypes.c_int
         lib.sigattn_selftest_bounded_wait.argtypes = [ctypes.c_int, ctypes.c_int]
         lib.sigattn_selftest_bounded_wait.restype = ctypes.c_int
-        lib.sigattn_form.argtypes = [ctypes.POINTER(SigAttnParams), ctypes.c_int, ctypes.c_int]
-        lib.sigattn_form.restype = ctypes.c_int
         if lib.sigattn_query(Q_PARAMS_SIZE) != ctypes.sizeof(SigAttnParams):
             raise ImportError(
                 f"SigAttnParams layout mismatch: library {lib.sigattn_query(Q_PARAMS_SIZE)} bytes, "
                 f"binding {ctypes.sizeof(SigAttnParams)} bytes; rebuild the library"
             )
+        if lib.sigattn_query(Q_HEAD_COLS) != 1:
+            raise ImportError(f"{path} is older than SigAttnParams.head_cols, which this binding sets; rebuild the library")
+        lib.sigattn_form.argtypes = [ctypes.POINTER(SigAttnParams), ctypes.c_int, ctypes.c_int]
+        lib.sigattn_form.restype = ctypes.c_int
         _lib = lib
     return _lib
 

@@ -678,6 +678,7 @@ int sigattn_query(int what) {
     case SIGATTN_Q_SM_ARCH: return 100;
     case SIGATTN_Q_MAX_HEAD_DIM: return 128;
     case SIGATTN_Q_PARAMS_SIZE: return (int)sizeof(SigAttnParams);
+    case SIGATTN_Q_HEAD_COLS: return 1;
     default: return -1;
   }
 }
