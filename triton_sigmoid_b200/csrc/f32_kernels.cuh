@@ -234,17 +234,17 @@ __device__ __forceinline__ void f32_store_rows(float* base, int64_t stride_t, in
 
 // With t = e^-|x| in (0, 1]: sigmoid = n / (1 + t), n = x < 0 ? t : 1.  The divisor lies in [1, 2], so the quotient needs no
 // special cases (and no branches, which a general division brings along: they cost a quarter of the elementwise step
-// here): the hardware's approximate reciprocal, and one correction by the remainder.  The divisor enters that with its
-// rounding error, e (exact, Dekker's fast two-sum, as 1 >= t); without it the sum's rounding and the quotient's add up to
-// more than those of 1 / (1 + e^-x).  RMS relative error on [-20, -10], [-10, -4], [-4, 0], [0, 8], in 1e-8: 4.6, 4.7, 4.1, 2.1;
-// 1 / (1 + e^-x) 4.9, 4.7, 4.6, 3.8; without e 5.6, 5.8, 5.1, 3.8.  Below -88, where e^-x overflows, this one stays accurate.
+// here): the hardware's approximate reciprocal gives q, and the remainder n - q (1 + t) corrects it.  The remainder does not
+// use the rounded sum: n - q is exact (n / 2 <= q <= n, Sterbenz), and t q is taken off it with one rounding.  Otherwise the
+// sum's rounding and the quotient's add up to more than those of 1 / (1 + e^-x).  RMS relative error on [-20, -10], [-10, -4],
+// [-4, 0], [0, 8], in 1e-8: 4.6, 4.7, 4.1, 2.1; 1 / (1 + e^-x) 4.9, 4.7, 4.6, 3.8; a plain division by 1 + t 5.6, 5.8, 5.1, 3.8.
+// Below -88, where e^-x overflows, this one stays accurate.
 __device__ __forceinline__ float f32_sigmoid(float x) {
   const float t = expf(-fabsf(x));
-  const float y = 1.0f + t, e = t - (y - 1.0f);
   const float n = x < 0.f ? t : 1.0f;
-  const float r = rcp_approx(y);
+  const float r = rcp_approx(1.0f + t);
   const float q = n * r;
-  return fmaf(fmaf(-e, q, fmaf(-y, q, n)), r, q);
+  return fmaf(fmaf(-q, t, n - q), r, q);
 }
 
 struct F32Item {
