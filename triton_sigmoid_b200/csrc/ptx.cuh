@@ -319,20 +319,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&r)[8]) {
-  asm volatile(
-      "tcgen05.wait::ld.sync.aligned;"
-      : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
-      :
-      : "memory");
-}
 __device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.wait::ld.sync.aligned;"
@@ -382,21 +368,6 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   }
   return r;
-}
-
-// The pair of pack2() back in fp32.
-template <bool kBF16>
-__device__ __forceinline__ float2 unpack2(uint32_t h) {
-  float2 f;
-  if constexpr (kBF16) {
-    f.x = __uint_as_float(h << 16);
-    f.y = __uint_as_float(h & 0xffff0000u);
-  } else {
-    asm("{\n\t.reg .b16 l, u;\n\tmov.b32 {l, u}, %2;\n\tcvt.f32.f16 %0, l;\n\tcvt.f32.f16 %1, u;\n\t}"
-        : "=f"(f.x), "=f"(f.y)
-        : "r"(h));
-  }
-  return f;
 }
 
 }  // namespace sigattn

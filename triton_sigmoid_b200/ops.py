@@ -163,9 +163,6 @@ def _base_params(q, k, v, bias, score_mod, seq_lens_q, seq_lens_k, scale, is_cau
     p.seq_lens_k = seq_lens_k.data_ptr() if seq_lens_k is not None else None
     if isinstance(bias, torch.Tensor):  # one value per batch element
         p.bias, p.bias_scalar = bias.data_ptr(), 0.0
-    elif bias is None:                  # the padded default, -log(valid keys), computed by the kernels
-        p.bias, p.bias_scalar = None, 0.0
-        p.flags |= _cabi.SIGATTN_BIAS_NEG_LOG_LK
     else:                               # one value for the whole call: no device tensor needed
         p.bias, p.bias_scalar = None, float(bias)
     p.score_mod = score_mod.data_ptr() if score_mod is not None else None
@@ -357,20 +354,13 @@ def _varlen_params(q, k, v, cu_q, cu_k, max_q, max_k, bias, score_mod, scale, is
     p.B, p.H, p.D, p.Tq, p.Tk = cu_q.numel() - 1, H, D, int(max_q), int(max_k)
     p.flags = _flags(is_causal)
     p.scale = float(scale)
-    p.bias_scalar = 0.0
     p.device = q.device.index if q.device.index is not None else torch.cuda.current_device()
     p.q, p.k, p.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
     s3 = lambda t: (ctypes.c_int64 * 3)(0, t.stride(0), t.stride(1))
     p.q_strides, p.k_strides, p.v_strides = s3(q), s3(k), s3(v)
     p.cu_seqlens_q, p.cu_seqlens_k = cu_q.data_ptr(), cu_k.data_ptr()
     p.total_q, p.total_k = total_q, k.shape[0]
-    if isinstance(bias, torch.Tensor):
-        p.bias = bias.data_ptr()
-    elif bias is None:  # -log(number of keys of the sequence), computed by the kernels
-        p.bias = None
-        p.flags |= _cabi.SIGATTN_BIAS_NEG_LOG_LK
-    else:
-        p.bias, p.bias_scalar = None, float(bias)
+    p.bias, p.bias_scalar = bias.data_ptr(), 0.0
     p.score_mod = score_mod.data_ptr() if score_mod is not None else None
     p.stream = torch.cuda.current_stream(q.device).cuda_stream
     return p
@@ -507,7 +497,7 @@ def _pad_head_dim(x: torch.Tensor, D_kernel: int) -> torch.Tensor:
 
 
 def _check_dtype(query, key, value):
-    """float16 / bfloat16 run on the tensor cores; float32 runs the exact single-precision
+    """float16 / bfloat16 run on the tensor cores; float32 runs the single-precision
     kernels (slower by design: the reference holds float32 to 1e-5, which tf32 cannot meet)."""
     if query.dtype not in _SUPPORTED_DTYPES:
         raise NotImplementedError(f"unsupported dtype {query.dtype}: use float16, bfloat16 or float32")
