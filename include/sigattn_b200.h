@@ -44,7 +44,7 @@ extern "C" {
 
 #define SIGATTN_ABI_VERSION 2
 
-/* fp16 / bf16: tensor-core kernels.  fp32: exact single-precision kernels on the FMA pipe (the
+/* fp16 / bf16: tensor-core kernels.  fp32: single-precision kernels on the FMA pipe (the
  * reference accepts float32, src/triton_sigmoid/__init__.py:48, and tests it to 1e-5); they need no
  * workspace, and base pointers / strides must be multiples of 16 bytes as for the other types. */
 enum SigAttnDtype { SIGATTN_FP16 = 0, SIGATTN_BF16 = 1, SIGATTN_FP32 = 2 };
@@ -54,7 +54,8 @@ enum SigAttnFlags {
   /* Accurate sigmoid in the tensor-core kernels: exponential and reciprocal both on the special-function
    * unit (relative error ~2^-22) instead of the default one-exponential form with a polynomial
    * reciprocal or a short series.  Counterpart of the reference's TRITON_SIGMOID_ACCURATE switch
-   * (src/triton_sigmoid/kernel_utils.py:190-193, 236-237); slower.  Ignored for fp32 (always exact). */
+   * (src/triton_sigmoid/kernel_utils.py:190-193, 236-237); slower.  Ignored for fp32 (whose sigmoid is good to
+   * about 2^-22 anyway). */
   SIGATTN_ACCURATE = 1u << 1,
   /* Backward only: use the pair of streaming kernels (dK/dV with the keys stationary, then dQ with the
    * queries stationary; 7 GEMMs per tile pair like the reference's split, sigmoid_triton_dense.py:162-467)
@@ -112,7 +113,8 @@ typedef struct SigAttnParams {
 
   /* Optional cudaEvent_t pair (NULL = off), recorded on `stream` immediately before and after
    * the launch of the main attention kernel of the call, so that a caller can time that
-   * kernel alone (the backward call also zero-fills and converts the dQ accumulator). */
+   * kernel alone (the backward call also zero-fills and converts the dQ accumulator, unless it takes
+   * the by-head form, see sigattn_form). */
   void *ev_main_start;
   void *ev_main_stop;
 
@@ -163,8 +165,9 @@ int sigattn_bwd(const SigAttnParams *p);
  *    (negative return, message from sigattn_last_error()) before anything is launched.
  *  - The first call on each device looks up the device address of the array; make that first
  *    call outside any stream capture.
- *  - All calls on one device share the one array.  Each call zero-fills the part it uses on
- *    p->stream before its kernels run, so leftovers of earlier calls never matter; but two calls
+ *  - All calls on one device share the one array.  Each call writes the part it uses on
+ *    p->stream (zero-filled, or stored to, before anything is added or read), so leftovers of earlier
+ *    calls never matter; but two calls
  *    whose GPU work overlaps in time (different streams, no dependency) race on it.  Serialise
  *    them on one stream or with events. */
 #define SIGATTN_STATIC_SCRATCH_ELEMS (8u * 1024u * 1024u)

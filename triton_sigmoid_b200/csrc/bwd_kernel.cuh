@@ -127,7 +127,7 @@ struct BwdSmem {
   static constexpr int kSFree = kDsReady + 1;         // dV has consumed P^T: S columns reusable
   static constexpr int kDpFree = kSFree + 1;          // dK has consumed dS^T: dP columns reusable
   static constexpr int kDqFull = kDpFree + 1;         // [2] dQ tile complete in TMEM
-  static constexpr int kDqEmpty = kDqFull + 2;        // [2] dQ tile read out (16 warps)
+  static constexpr int kDqEmpty = kDqFull + 2;        // [2] dQ tile read out (8 drain warps)
   static constexpr int kDkvFull = kDqEmpty + 2;       // every MMA of the CTA complete
   static constexpr int kKvFix = kDkvFull + 1;         // [2] per K/V buffer: padded rows of K_j zeroed
   static constexpr int kQdoFix = kKvFix + 2;          // [2] per stage: padded rows of the last Q_i / dO_i zeroed
@@ -401,7 +401,9 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item)
 
 // kByHead: a CTA takes all key tiles of a (batch element, head), in order, and finishes its dQ itself (see the drain
 // warps), so that the accumulator needs neither the fill nor the conversion pass and stays in the L2.  group is 1 and the
-// tickets count (batch, head) pairs.
+// tickets count (batch, head) pairs.  (This form spills more: 132 / 188 bytes of stores / loads by -Xptxas -v at D = 64
+// against 68 / 76 in the general one, 208 / 300 against 120 / 188 at D = 128.  All registers of the CTA are handed out, see
+// below; the figures of the rule that chooses the form, bwd_by_head(), include these spills.)
 template <int D, bool kBF16, bool kAccurate, bool kByHead>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
@@ -533,7 +535,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     // ============================================================ dQ drain
     // Warp d = warp - 20: lane quarter d & 3 (32 query rows, one per lane), half of the head columns d >> 2.  Per tile:
     // wait for the dQ product, take the block into registers, release the TMEM columns, then add it into the
-    // accumulator (see acc_tile).
+    // accumulator (see acc_piece).
     {
       const int dw = warp - kBwdFirstDrainWarp;
       const int quarter = dw & 3, half = dw >> 2;

@@ -555,7 +555,7 @@ int static_scratch_ptr(int device, float** out) {
   return 0;
 }
 
-// float32 tensors: the exact FMA-pipe kernels (no tensor maps, no workspace).
+// float32 tensors: the FMA-pipe kernels (no tensor maps, no workspace).
 template <int D, int kR, int kC>
 int launch_f32_shape(const SigAttnParams* p, const sigattn::F32Params& fp, bool backward) {
   using namespace sigattn;
@@ -839,7 +839,7 @@ int sigattn_bwd_static_scratch(const SigAttnParams* p) {
   const Extents ex = extents(p);
   const unsigned long long elems = (unsigned long long)ex.B * (unsigned long long)ex.Tq * (unsigned long long)p->H *
                                    (unsigned long long)p->D;
-  // float32 tensors run the exact kernels, which use no accumulator: no limit applies to them
+  // float32 tensors run kernels of their own, which use no accumulator: no limit applies to them
   if (p->dtype == SIGATTN_FP32) return sigattn_bwd(p);
   if (elems > SIGATTN_STATIC_SCRATCH_ELEMS)
     return fail(-4, "problem too large for the built-in scratch: B*Tq*H*D = %llu elements, limit %u; "
@@ -850,7 +850,7 @@ int sigattn_bwd_static_scratch(const SigAttnParams* p) {
     SIG_CUDA(g.enter(p->device));
     if ((rc = static_scratch_ptr(p->device, &scratch))) return rc;
   }
-  // Same path as sigattn_bwd from here on; it zero-fills the accumulator on p->stream first.
+  // Same path as sigattn_bwd from here on; no form of it reads the accumulator before it has written it.
   SigAttnParams q = *p;
   q.flags &= ~(uint32_t)SIGATTN_BWD_SPLIT;  // the kernel that accumulates dQ in scratch memory
   q.workspace = scratch;
