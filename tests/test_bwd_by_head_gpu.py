@@ -24,7 +24,9 @@ def _enough(B, H):
     (75, 16, 130, 300, False),    # a query tile of two rows, ragged last key tile
     (40, 30, 300, 300, True),     # every query tile has another last key tile
     (75, 16, 400, 150, True),     # query tiles behind the last key tile
-    (75, 16, 100, 400, True),     # key tiles that no query sees
+    (75, 16, 100, 400, True),     # key tiles that no query sees (D = 64: the general form's business, with one query tile)
+    (75, 16, 200, 400, True),
+    (112, 16, 100, 700, False),   # six key tiles, as 12 pairs per SM allow
 ])
 def test_matches_the_general_form(B, H, Tq, Tk, causal, D):
     dtype = torch.bfloat16 if Tq % 2 else torch.float16
@@ -49,7 +51,7 @@ def test_matches_the_general_form(B, H, Tq, Tk, causal, D):
         return torch.autograd.grad(out, leaf, do[s])
 
     step = 20
-    assert launch_form(B, H, Tq, Tk, D, dtype, True, causal) == FORM_BWD_BY_HEAD
+    assert launch_form(B, H, Tq, Tk, D, dtype, True, causal) == (FORM_BWD if (Tq, Tk, D) == (100, 400, 64) else FORM_BWD_BY_HEAD)
     assert launch_form(step, H, Tq, Tk, D, dtype, True, causal) == FORM_BWD
     whole = grads(slice(0, B))
     for b0 in range(0, B, step):

@@ -123,16 +123,18 @@ def test_a_library_without_head_cols_is_told_apart(lib, monkeypatch):
     (_cabi.FORM_BWD_BY_HEAD, dict(B=1184, H=1, Tq=1024, Tk=1024, backward=True, causal=True)),
     (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=512, Tk=512, backward=True, packed_rows=148 * 512 * 4)),
     (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=512, Tk=512, backward=True, packed_rows=148 * 512 * 2)),  # mostly short ones
-    (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=64, Tk=512, backward=True)),
-    (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=64, Tk=513, backward=True)),       # few queries on long contexts
+    (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=64, Tk=1024, backward=True)),  # 8 key tiles, 8.1 pairs per SM
+    (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=64, Tk=1025, backward=True)),          # few queries on long contexts
+    (_cabi.FORM_BWD_BY_HEAD, dict(B=148 * 9, H=1, Tq=64, Tk=1025, backward=True)),
+    (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=200, Tk=2048, backward=True)),
+    (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=200, Tk=2049, backward=True)),
+    (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=200, Tk=512, D=128, backward=True)),
+    (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=200, Tk=513, D=128, backward=True)),
     (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=64, Tk=2 ** 31 - 1, backward=True)),
-    (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=512, Tk=1024, backward=True)),
-    (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=512, Tk=1024, backward=True, causal=True)),  # half of the keys are unseen
-    (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=640, Tk=1281, backward=True, packed_rows=148 * 640 * 4)),
-    (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=640, Tk=1537, backward=True, packed_rows=148 * 640 * 4)),
-    (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=768, Tk=768, backward=True)),
-    (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=768, Tk=768, backward=True, packed_rows=148 * 768 * 4)),
-    (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=1536, Tk=1536, backward=True, causal=True)),
+    (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=200, Tk=8192, backward=True, causal=True)),  # two key tiles have work
+    (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=100, Tk=400, backward=True, causal=True)),           # one has
+    (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=768, Tk=768, backward=True)),
+    (_cabi.FORM_BWD, dict(B=1200, H=1, Tq=769, Tk=769, backward=True)),
     (_cabi.FORM_BWD_BY_HEAD, dict(B=1200, H=1, Tq=768, Tk=768, D=128, backward=True, causal=True)),
     (_cabi.FORM_F32_16, dict(B=73, H=1, Tq=64, Tk=64, dtype=torch.float32)),
     (_cabi.FORM_F32_64, dict(B=74, H=1, Tq=64, Tk=64, dtype=torch.float32, backward=True)),

@@ -364,32 +364,33 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
 
 // Whether the fused backward gives whole (batch element, head) pairs to CTAs (see kByHead).  The general form fills, reduces
 // into, reads and converts an accumulator of 4 bytes per element of Q, passes over memory that this one saves; but its items
-// are single key tiles, which balance better, and here the launch ends on somebody's last pair.  So the pairs must be many
-// (8 per SM: B=80 T=512 H=16 562 -> 545 us forward + backward) and short.  Below: the backward alone in this form over the
-// general one, 8 to 40 pairs per SM.
-//  - Tq, as the passes' share falls with it and the CTAs' regions outgrow the L2: D = 64 T=256 0.82 - 0.84, 512 0.91 - 0.97, 640
-//    0.95 - 1.00, 768 0.95 - 1.10, 1024 1.06 - 1.16; D = 128 256 0.82 - 0.86, 384 0.93 - 0.97, 512 0.95 - 1.03.  Causal, a region is
-//    half as much in use: D = 64 1024 0.88 - 0.97, 1280 0.95 - 0.99, 1536 1.03 - 1.06; D = 128 768 0.95 - 1.00.  Ragged batches,
-//    whose general form balances no better and (padded) passes over the padding too, go a little further: D = 64 lengths from
-//    0.4 of 768 0.93 - 0.97, causal 1536 0.96 - 0.99.
-//  - Tk, as a pair of many key tiles is a long chain whose products are what costs: four tiles, or as many as query tiles.
-//    Tq=64 Tk=256 0.94 - 0.96, 512 1.00 - 1.03, 1024 1.03 - 1.06; Tq=256 Tk=512 0.91 - 0.96, 1024 1.00 - 1.08, 2048 1.02 - 1.14, 8192 1.17;
-//    D = 128 Tq=128 Tk=512 0.88 - 0.94, 1024 0.97 - 1.04.  Ragged, lengths from 0.4: Tq=640 Tk=1281 0.97 - 1.01, hence 2.5 times as
-//    many.  (Causal, keys behind the last query have no work: Tq=512 Tk=1024 0.87.)
+// are single key tiles, which balance better, while here the launch ends on somebody's last pair.  So the pairs must be many
+// (8 per SM: B=80 T=512 H=16 562 -> 545 us forward + backward) and short.  The lines below are from 22,000 random calls (8 to
+// 45 pairs per SM, dense, padded and packed) with both forms forced; figures are the backward alone in this form over the
+// general one, means of a class.  By this rule the form is 0.915 of the general one where it is taken and 1.031 where not.
+//  - Tq, as the passes' share falls with it and the CTAs' regions outgrow the L2.  D = 64, dense: 0.75 - 0.86 up to 384, 0.77 - 0.97
+//    up to 768 (higher at multiples of 128), then 0.86 - 1.06, 1.06 - 1.16 at 1024; causal 0.85 - 0.91 up to 1200, 0.94 - 1.06 up to
+//    1536 and 0.97 beyond.  D = 128 half of these lengths: 0.82 - 0.94 up to 384, 0.95 - 1.03 at 512.
+//  - Tk, as the gain falls with a pair's number of key tiles and the end's share with the pairs per SM: four tiles, or as many as
+//    query tiles, or as many as there are pairs per SM - half as many at D = 128 (0.94 - 1.02 below that, 1.01 - 1.07 above), twice
+//    as many at D = 64 with more than one query tile (0.88 - 0.99, 0.97 - 1.04; one query tile 0.96 - 1.00, 1.00 - 1.02).
+//    Extremes: Tq=64 on 2048 keys 695 -> 757 us, 256 on 8192 2702 -> 3149, 211 on 2088 2604 -> 1916.  Causal, keys behind the last
+//    query have no work (Tq=512 Tk=1024 0.87), but tiles of them pass one after another: D = 64, one query tile, 1.02 - 1.13.
 //  - packed sequences, on average: a CTA's share of the rows is at least 2.5 of the longest sequence (with 8 pairs per SM, an
 //    average of 0.3 of it; the general form's passes only cover the rows there are).  Some of 768 tokens among many of 128
 //    1.12 - 1.21, of 192 1.02 - 1.05, of 256 0.92 - 1.07; of 512 tokens 1.01 - 1.13, 0.95 - 1.09, 0.91 - 0.98.  This also covers that
 //    the accumulator must have room for a region per CTA.  (Padded, 768 among 96: 0.71 - 0.89.)
 // The accurate sigmoid, an option for comparisons, has the general form only.
 bool bwd_by_head(const SigAttnParams* p, int n_sm) {
-  const bool causal = (p->flags & SIGATTN_CAUSAL) != 0, ragged = p->seq_lens_q || p->seq_lens_k || p->cu_seqlens_q;
+  const bool causal = (p->flags & SIGATTN_CAUSAL) != 0, wide = p->D == 128;
   const Extents ex = extents(p);
   const int64_t n_bh = (int64_t)p->B * p->H, acc_rows = (int64_t)ex.B * ex.Tq * p->H;
-  const int64_t q_tiles = ((int64_t)p->Tq + 127) / 128, k_tiles = ((int64_t)(causal ? std::min(p->Tk, p->Tq) : p->Tk) + 127) / 128;
-  const int max_q = (p->D == 128 ? 384 : ragged ? 768 : 640) * (causal ? 2 : 1);
-  return !(p->flags & SIGATTN_ACCURATE) && n_bh >= 8 * (int64_t)n_sm && p->Tq <= max_q &&
-         (k_tiles <= std::max<int64_t>(q_tiles, 4) || (ragged && 2 * k_tiles <= 5 * q_tiles)) &&
-         2 * acc_rows >= 5 * (int64_t)n_sm * p->Tq;
+  const int64_t q_tiles = ((int64_t)p->Tq + 127) / 128, k_tiles = ((int64_t)p->Tk + 127) / 128;
+  const int64_t busy = causal ? std::min(k_tiles, q_tiles) : k_tiles;  // key tiles with work
+  if ((p->flags & SIGATTN_ACCURATE) || n_bh < 8 * (int64_t)n_sm || (int64_t)p->Tq * p->D > (causal ? 98304 : 49152)) return false;
+  if (busy > 4 && busy > q_tiles && 2 * busy * n_sm > n_bh * (wide ? 1 : q_tiles > 1 ? 4 : 2)) return false;
+  if (causal && !wide && q_tiles == 1 && k_tiles > 2) return false;
+  return 2 * acc_rows >= 5 * (int64_t)n_sm * p->Tq;
 }
 
 // The default backward: the fused 5-GEMM kernel with fp32 dQ reductions into a workspace (bwd_kernel.cuh).
