@@ -368,9 +368,10 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
 // (8 per SM: B=80 T=512 H=16 562 -> 545 us forward + backward) and short.  The lines below are from 22,000 random calls (8 to
 // 45 pairs per SM, dense, padded and packed) with both forms forced; figures are the backward alone in this form over the
 // general one, means of a class.  By this rule the form is 0.915 of the general one where it is taken and 1.031 where not.
-//  - Tq, as the passes' share falls with it and the CTAs' regions outgrow the L2.  D = 64, dense: 0.75 - 0.86 up to 384, 0.77 - 0.97
-//    up to 768 (higher at multiples of 128), then 0.86 - 1.06, 1.06 - 1.16 at 1024; causal 0.85 - 0.91 up to 1200, 0.94 - 1.06 up to
-//    1536 and 0.97 beyond.  D = 128 half of these lengths: 0.82 - 0.94 up to 384, 0.95 - 1.03 at 512.
+//  - Tq, as the passes' share falls with it and the CTAs' regions outgrow the L2.  D = 64, dense: 0.75 - 0.83 at 129 to 256, 0.84 -
+//    0.91 up to 512, 0.75 - 0.97 up to 768, 0.87 - 1.00 up to 1000, 1.06 - 1.16 at 1024 - the high ends at multiples of 128, for which
+//    the line is drawn; causal 0.85 - 0.91 up to 1200, 0.94 - 0.97 up to 1536 (there 1.03 - 1.06).  D = 128, half as long: 0.73 - 0.90
+//    up to 384, 0.94 up to 500, 0.95 - 1.03 at 512; causal 0.73 - 0.95 up to 768.
 //  - Tk, as the gain falls with a pair's number of key tiles and the end's share with the pairs per SM: four tiles, or as many as
 //    query tiles, or as many as there are pairs per SM - half as many at D = 128 (0.94 - 1.02 below that, 1.01 - 1.07 above), twice
 //    as many at D = 64 with more than one query tile (0.88 - 0.99, 0.97 - 1.04; one query tile 0.96 - 1.00, 1.00 - 1.02).
