@@ -183,7 +183,8 @@ enum SigAttnForm {
   SIGATTN_FORM_BWD_BY_HEAD = 3, /* fused, a CTA takes whole (batch element, head) pairs */
   SIGATTN_FORM_BWD_STREAM = 4,  /* SIGATTN_BWD_SPLIT */
   SIGATTN_FORM_F32_16 = 5,      /* fp32, forward or backward: tiles of 16 rows */
-  SIGATTN_FORM_F32_64 = 6       /* ... of 64 rows */
+  SIGATTN_FORM_F32_64 = 6,      /* ... of 64 rows */
+  SIGATTN_FORM_F32_TC = 7       /* fp32 on the tensor cores, products of bf16 parts: tiles of 128 rows */
 };
 int sigattn_form(const SigAttnParams *p, int backward, int n_sm);
 

@@ -1,0 +1,113 @@
+"""The float32 kernels on the tensor cores at the edges of their tiles (128 stationary rows, 64 streamed ones), against the
+float64 oracle with the gates of tests/test_f32_gpu.py."""
+
+import pytest
+import torch
+
+import triton_sigmoid_b200 as sa
+from oracle import sigattn_oracle as orc
+from tests.gpu_util import launch_form, make_inputs, rel_l2
+from tests.test_f32_gpu import _check
+from triton_sigmoid_b200._cabi import FORM_F32_TC
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D", [20, 32, 64, 72, 96, 128])
+@pytest.mark.parametrize("T", [256, 257, 319, 385])
+def test_tile_edges(T, D, causal):
+    B, H = 6, 4
+    for backward in (False, True):
+        assert launch_form(B, H, T, T, D, torch.float32, backward, causal) == FORM_F32_TC
+    q, k, v, do = make_inputs(B, T, T, H, D, torch.float32, std=0.5, seed=T + D, requires_grad=True)
+    lens = torch.tensor([T, 128, 129, 63, 1, 0], dtype=torch.int32)
+    with torch.no_grad():  # the oracle multiplies masked zeros with the padding: finite, but nothing a result may hold
+        for t in (q, k, v, do):
+            for b in range(B):
+                t[b, int(lens[b]):] = 1.0e3
+    lens = lens.cuda()
+    _check(q, k, v, do, lens_q=lens, lens_k=lens, is_causal=causal, score_mod=torch.randn(B, T, device="cuda") * 0.5)
+
+
+@pytest.mark.parametrize("Tq,Tk", [(256, 1000), (700, 300)])
+def test_packed_and_cross_lengths(Tq, Tk):
+    """Packed sequences, queries and keys of different lengths, views of a wider tensor; and that a call gives the same bits
+    each time."""
+    H, D = 4, 64
+    lq, lk = [Tq, 130, 1, 0, 64], [Tk, 65, 200, 128, 0]
+    cq, ck = ([0] + torch.tensor(x).cumsum(0).tolist() for x in (lq, lk))
+    g = torch.Generator(device="cuda").manual_seed(Tq)
+    wide = [torch.randn(n, H, D + 32, device="cuda", generator=g) * 0.5 for n in (cq[-1], ck[-1], ck[-1])]
+    q, k, v = (t[..., 16:16 + D].detach().requires_grad_() for t in wide)
+    do = torch.randn(cq[-1], H, D, device="cuda", generator=g) * 0.5
+    cu = [torch.tensor(c, dtype=torch.int32, device="cuda") for c in (cq, ck)]
+
+    def call():
+        out = sa.sigmoid_attention_varlen(q, k, v, *cu, Tq, Tk)
+        return (out.detach(),) + torch.autograd.grad(out, (q, k, v), do)
+
+    got = call()
+    assert all(torch.equal(a, b) for a, b in zip(got, call()))
+    for i in range(len(lq)):
+        if not lq[i] or not lk[i]:
+            continue
+        sl = [t[None, a[i]:a[i + 1]].detach() for t, a in ((q, cq), (k, ck), (v, ck), (do, cq))]
+        ref = (orc.sigattn_forward(*sl[:3], work=torch.float64),) + orc.sigattn_backward(*sl, work=torch.float64)
+        for name, x, a, r in zip(("o", "dq", "dk", "dv"), got, (cq, cq, ck, ck), ref):
+            assert rel_l2(x[a[i]:a[i + 1]].double().cpu(), r[0]) <= 1e-5, (i, name)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf"), 3.4e38])
+def test_values_that_the_parts_cannot_carry(bad, causal, D):
+    """Infinities, NaN and floats beyond the largest bf16 number reach the results as single precision has them."""
+    T, j = 800, 64
+    q, k, v, do = make_inputs(1, T, T, 2, D, torch.float32, std=0.5, seed=1)
+    v[:, j, 0, 0] = bad   # head 0: the value of one key
+    k[:, j, 1] = 0.0
+    k[:, j, 1, 0] = bad   # head 1: the scores of one key (huge, of both signs)
+    q[:, :, 1, 0] = 0.5 * torch.sign(q[:, :, 1, 0]) + q[:, :, 1, 0]
+    out = sa.sigmoid_attention(q, k, v, is_causal=causal, sigmoid_bias=-1.0)
+    with torch.no_grad():
+        x = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) / D ** 0.5 - 1.0
+        p = torch.sigmoid(x)
+        if causal:
+            p = p.masked_fill(torch.ones(T, T, device="cuda").triu(1).bool(), 0.0)
+        w = v.double().clone()
+        w[:, j, 0, 0] = 0.0
+        ref = torch.einsum("bhqk,bkhd->bqhd", p, w)
+        ref[:, :, 0, 0] += torch.where(p[:, 0, :, j] > 0, p[:, 0, :, j] * bad, 0.0)
+    got = out.double()
+    sees = slice(j if causal else 0, None)
+    if bad != bad:
+        assert got[:, sees, 0, 0].isnan().all() and got[:, sees, 1].isnan().all()
+        got[:, sees, 0, 0] = ref[:, sees, 0, 0] = 0.0
+        got[:, sees, 1] = ref[:, sees, 1] = 0.0
+    inf = ref.isinf()
+    assert torch.equal(got[inf], ref[inf])
+    got[inf] = ref[inf] = 0.0
+    assert got.isfinite().all()
+    scale = ref.abs().amax(dim=(0, 1, 3), keepdim=True) if bad != 3.4e38 else ref.abs().clamp(min=1.0)
+    assert ((got - ref).abs() / scale).max().item() <= 1e-5
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_nonfinite_values_pass_through_probabilities_of_zero(bad, causal, D):
+    """As in tests/test_f32_tiles_gpu.py: dS = P (1 - P) dP of a visible pair is NaN also where P has underflowed."""
+    T, j = 800, 70
+    assert launch_form(1, 2, T, T, D, torch.float32, True, causal) == FORM_F32_TC
+    q, k, v, do = make_inputs(1, T, T, 2, D, torch.float32, std=0.5, seed=1)
+    v[:, j] = bad
+    do[..., 0] = 1.0
+    do[..., 1:] = 0.0
+    leaf = [t.requires_grad_() for t in (q, k, v)]
+    out = sa.sigmoid_attention(*leaf, is_causal=causal, sigmoid_bias=-1000.0)
+    dq, dk, dv = torch.autograd.grad(out, leaf, do)
+    sees = torch.arange(T, device="cuda") >= (j if causal else 0)
+    assert dq[:, sees].isnan().all() and (dq[:, ~sees] == 0).all()
+    at = torch.arange(T, device="cuda") == j
+    assert dk[:, at].isnan().all() and (dk[:, ~at] == 0).all() and (dv == 0).all()

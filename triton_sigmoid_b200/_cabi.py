@@ -21,7 +21,7 @@ SIGATTN_BWD_SPLIT = 4
 SIGATTN_BIAS_NEG_LOG_LK = 8
 SIGATTN_STATIC_SCRATCH_ELEMS = 8 * 1024 * 1024
 
-FORM_FWD, FORM_FWD_SPLIT, FORM_BWD, FORM_BWD_BY_HEAD, FORM_BWD_STREAM, FORM_F32_16, FORM_F32_64 = range(7)
+FORM_FWD, FORM_FWD_SPLIT, FORM_BWD, FORM_BWD_BY_HEAD, FORM_BWD_STREAM, FORM_F32_16, FORM_F32_64, FORM_F32_TC = range(8)
 
 Q_ABI_VERSION, Q_SM_ARCH, Q_MAX_HEAD_DIM, Q_PARAMS_SIZE, Q_HEAD_COLS = range(5)
 

@@ -33,6 +33,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ptx.cuh"
+
 namespace sigattn {
 
 struct F32Params {
@@ -115,6 +117,13 @@ template <int kC>
 __device__ __forceinline__ void f32_group_sync(int group) {
   if constexpr (kC == 1) __syncwarp();
   else asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(32 * kC) : "memory");
+}
+
+// The threads that work on one row tile: the whole block (kBar = 0), or the first kThreads threads of a larger one.
+template <int kThreads, int kBar>
+__device__ __forceinline__ void f32_block_sync() {
+  if constexpr (kBar == 0) __syncthreads();
+  else asm volatile("bar.sync %0, %1;" ::"n"(kBar), "n"(kThreads) : "memory");
 }
 
 // s[a][c] = sum_d A[row0 + 2 a][d] * B[col0 + 16 c][d]
@@ -348,19 +357,14 @@ __device__ __forceinline__ void f32_ds(const F32Params& p, const F32Item& it, co
 }
 
 // ---------------------------------------------------------------- forward
-// (Three CTAs per SM at D = 64, kR = 4, at 168 registers and 72 / 88 bytes of spills: 844 us at B=4 T=2048 H=8, 870 with the 222
-// registers and two CTAs that it takes unbounded.)
-template <int D, int kR, int kC>
-__global__ void __launch_bounds__(32 * kR * kC, D == 64 && kR == 4 ? 3 : 1) sigattn_fwd_f32_kernel(const F32Params p, const int n_tiles) {
+template <int D, int kR, int kC, int kBar = 0>
+__device__ __forceinline__ void f32_fwd_rows(const F32Params& p, const F32Item& it, const int q0, float* smem) {
   using S = F32Shape<D, kR, kC>;
-  extern __shared__ float4 f32_smem4[];
-  float* Qs = reinterpret_cast<float*>(f32_smem4);
+  float* Qs = smem;
   float* Ks = Qs + S::kStatFloats;
   float* Vs = Ks + S::kTileFloats;
   float* Ps = Vs + S::kTileFloats;
-  const F32Item it = f32_item(p, n_tiles, true);
   const F32Thread<S> th(kR);
-  const int q0 = it.tile * S::kRows;
   const float* qb = p.q + (int64_t)it.bc * p.q_sb + (int64_t)it.h * p.q_sh + (int64_t)it.tq0 * p.q_st;
   const float* kb = p.k + (int64_t)it.bc * p.k_sb + (int64_t)it.h * p.k_sh + (int64_t)it.tk0 * p.k_st;
   const float* vb = p.v + (int64_t)it.bc * p.v_sb + (int64_t)it.h * p.v_sh + (int64_t)it.tk0 * p.v_st;
@@ -377,7 +381,7 @@ __global__ void __launch_bounds__(32 * kR * kC, D == 64 && kR == 4 ? 3 : 1) siga
     f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, 0, it.Lk, p.d_cols);
     f32_commit();
     f32_wait<1>();
-    __syncthreads();
+    f32_block_sync<S::kThreads, kBar>();
   }
   for (int k0 = 0; k0 < kv_end; k0 += kF32Cols) {
     const bool more = k0 + kF32Cols < kv_end;
@@ -392,14 +396,14 @@ __global__ void __launch_bounds__(32 * kR * kC, D == 64 && kR == 4 ? 3 : 1) siga
         for (int c = 0; c < S::kNC; ++c) Ps[(th.row0 + 2 * a) * S::kWRow + th.col0 + 16 * c] = s[a][c];
     }
     f32_wait<0>();
-    __syncthreads();  // V has arrived, P is complete, K is no longer read
+    f32_block_sync<S::kThreads, kBar>();  // V has arrived, P is complete, K is no longer read
     if (more) {
       f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, k0 + kF32Cols, it.Lk, p.d_cols);
       f32_commit();
     }
     f32_accumulate<D, S::kNX>(Ps, Vs, th.row0, th.x0, o);
     f32_wait<0>();
-    __syncthreads();  // the next K has arrived, V and P are no longer read
+    f32_block_sync<S::kThreads, kBar>();  // the next K has arrived, V and P are no longer read
     if (more) {
       f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, k0 + kF32Cols, it.Lk, p.d_cols);
       f32_commit();
@@ -411,19 +415,16 @@ __global__ void __launch_bounds__(32 * kR * kC, D == 64 && kR == 4 ? 3 : 1) siga
 
 // ---------------------------------------------------------------- backward: dK, dV of one key tile
 // Score tiles are transposed here (rows = keys), so that P^T and dS^T are row-private like P in the forward.
-template <int D, int kR, int kC>
-__global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(const F32Params p, const int n_tiles) {
+template <int D, int kR, int kC, int kBar = 0>
+__device__ __forceinline__ void f32_dkdv_rows(const F32Params& p, const F32Item& it, const int k0, float* smem) {
   using S = F32Shape<D, kR, kC>;
-  extern __shared__ float4 f32_smem4[];
-  float* Ks = reinterpret_cast<float*>(f32_smem4);
+  float* Ks = smem;
   float* Vs = Ks + S::kStatFloats;
   float* Qs = Vs + S::kStatFloats;
   float* dOs = Qs + S::kTileFloats;
   float* Ps = dOs + S::kTileFloats;
   float* dSs = Ps + S::kWFloats;
-  const F32Item it = f32_item(p, n_tiles, false);
   const F32Thread<S> th(kR);
-  const int k0 = it.tile * S::kRows;
   const float* qb = p.q + (int64_t)it.bc * p.q_sb + (int64_t)it.h * p.q_sh + (int64_t)it.tq0 * p.q_st;
   const float* kb = p.k + (int64_t)it.bc * p.k_sb + (int64_t)it.h * p.k_sh + (int64_t)it.tk0 * p.k_st;
   const float* vb = p.v + (int64_t)it.bc * p.v_sb + (int64_t)it.h * p.v_sh + (int64_t)it.tk0 * p.v_st;
@@ -442,7 +443,7 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(cons
     f32_load_rows<D, kF32Cols, S::kThreads>(dOs, dob, p.do_st, q_begin, it.Lq, p.d_cols);
     f32_commit();
     f32_wait<1>();
-    __syncthreads();
+    f32_block_sync<S::kThreads, kBar>();
   }
   for (int q0 = q_begin; q0 < q_end; q0 += kF32Cols) {
     const bool more = q0 + kF32Cols < q_end;
@@ -456,7 +457,7 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(cons
 #pragma unroll
         for (int c = 0; c < S::kNC; ++c) Ps[(th.row0 + 2 * a) * S::kWRow + th.col0 + 16 * c] = pr[a][c];
       f32_wait<0>();
-      __syncthreads();  // dO has arrived
+      f32_block_sync<S::kThreads, kBar>();  // dO has arrived
       float dp[8][S::kNC];
       f32_scores<D, S::kNC>(Vs, dOs, th.row0, th.col0, p.d_cols, dp);
       f32_ds<S::kNC>(p, it, pr, dp, all_visible, q0 + th.col0, k0 + th.row0, 0, 2, 16, 0);
@@ -467,14 +468,14 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(cons
     }
     f32_group_sync<kC>(th.group);
     f32_accumulate<D, S::kNX>(dSs, Qs, th.row0, th.x0, dk);
-    __syncthreads();  // Q is no longer read
+    f32_block_sync<S::kThreads, kBar>();  // Q is no longer read
     if (more) {
       f32_load_rows<D, kF32Cols, S::kThreads>(Qs, qb, p.q_st, q0 + kF32Cols, it.Lq, p.d_cols);
       f32_commit();
     }
     f32_accumulate<D, S::kNX>(Ps, dOs, th.row0, th.x0, dv);
     f32_wait<0>();
-    __syncthreads();  // the next Q has arrived, dO, P and dS are no longer read
+    f32_block_sync<S::kThreads, kBar>();  // the next Q has arrived, dO, P and dS are no longer read
     if (more) {
       f32_load_rows<D, kF32Cols, S::kThreads>(dOs, dob, p.do_st, q0 + kF32Cols, it.Lq, p.d_cols);
       f32_commit();
@@ -487,18 +488,15 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(cons
 }
 
 // ---------------------------------------------------------------- backward: dQ of one query tile
-template <int D, int kR, int kC>
-__global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dq_f32_kernel(const F32Params p, const int n_tiles) {
+template <int D, int kR, int kC, int kBar = 0>
+__device__ __forceinline__ void f32_dq_rows(const F32Params& p, const F32Item& it, const int q0, float* smem) {
   using S = F32Shape<D, kR, kC>;
-  extern __shared__ float4 f32_smem4[];
-  float* Qs = reinterpret_cast<float*>(f32_smem4);
+  float* Qs = smem;
   float* dOs = Qs + S::kStatFloats;
   float* Ks = dOs + S::kStatFloats;
   float* Vs = Ks + S::kTileFloats;
   float* dSs = Vs + S::kTileFloats;
-  const F32Item it = f32_item(p, n_tiles, true);
   const F32Thread<S> th(kR);
-  const int q0 = it.tile * S::kRows;
   const float* qb = p.q + (int64_t)it.bc * p.q_sb + (int64_t)it.h * p.q_sh + (int64_t)it.tq0 * p.q_st;
   const float* kb = p.k + (int64_t)it.bc * p.k_sb + (int64_t)it.h * p.k_sh + (int64_t)it.tk0 * p.k_st;
   const float* vb = p.v + (int64_t)it.bc * p.v_sb + (int64_t)it.h * p.v_sh + (int64_t)it.tk0 * p.v_st;
@@ -517,7 +515,7 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dq_f32_kernel(const 
     f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, 0, it.Lk, p.d_cols);
     f32_commit();
     f32_wait<1>();
-    __syncthreads();
+    f32_block_sync<S::kThreads, kBar>();
   }
   for (int k0 = 0; k0 < kv_end; k0 += kF32Cols) {
     const bool more = k0 + kF32Cols < kv_end;
@@ -525,7 +523,7 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dq_f32_kernel(const 
       float dp[8][S::kNC];
       f32_scores<D, S::kNC>(dOs, Vs, th.row0, th.col0, p.d_cols, dp);
       f32_wait<0>();
-      __syncthreads();  // K has arrived, V is no longer read
+      f32_block_sync<S::kThreads, kBar>();  // K has arrived, V is no longer read
       if (more) {
         f32_load_rows<D, kF32Cols, S::kThreads>(Vs, vb, p.v_st, k0 + kF32Cols, it.Lk, p.d_cols);
         f32_commit();
@@ -543,7 +541,7 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dq_f32_kernel(const 
     f32_group_sync<kC>(th.group);
     f32_accumulate<D, S::kNX>(dSs, Ks, th.row0, th.x0, dq);
     f32_wait<0>();
-    __syncthreads();  // the next V has arrived, K and dS are no longer read
+    f32_block_sync<S::kThreads, kBar>();  // the next V has arrived, K and dS are no longer read
     if (more) {
       f32_load_rows<D, kF32Cols, S::kThreads>(Ks, kb, p.k_st, k0 + kF32Cols, it.Lk, p.d_cols);
       f32_commit();
@@ -551,6 +549,28 @@ __global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dq_f32_kernel(const 
   }
   float* dqb = p.dq + (int64_t)it.bc * p.dq_sb + (int64_t)it.h * p.dq_sh + (int64_t)it.tq0 * p.dq_st;
   f32_store_rows<S::kNX>(dqb, p.dq_st, q0, th.row0, th.x0, it.row_lim, it.Lq, p.d_cols, p.scale, dq);
+}
+
+// ---------------------------------------------------------------- kernels: one row tile per CTA
+// (Three CTAs per SM at D = 64, kR = 4, at 168 registers and 72 / 88 bytes of spills: 844 us at B=4 T=2048 H=8, 870 with the 222
+// registers and two CTAs that it takes unbounded.)
+template <int D, int kR, int kC>
+__global__ void __launch_bounds__(32 * kR * kC, D == 64 && kR == 4 ? 3 : 1) sigattn_fwd_f32_kernel(const F32Params p, const int n_tiles) {
+  extern __shared__ float4 f32_smem4[];
+  const F32Item it = f32_item(p, n_tiles, true);
+  f32_fwd_rows<D, kR, kC>(p, it, it.tile * F32Shape<D, kR, kC>::kRows, reinterpret_cast<float*>(f32_smem4));
+}
+template <int D, int kR, int kC>
+__global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dkdv_f32_kernel(const F32Params p, const int n_tiles) {
+  extern __shared__ float4 f32_smem4[];
+  const F32Item it = f32_item(p, n_tiles, false);
+  f32_dkdv_rows<D, kR, kC>(p, it, it.tile * F32Shape<D, kR, kC>::kRows, reinterpret_cast<float*>(f32_smem4));
+}
+template <int D, int kR, int kC>
+__global__ void __launch_bounds__(32 * kR * kC) sigattn_bwd_dq_f32_kernel(const F32Params p, const int n_tiles) {
+  extern __shared__ float4 f32_smem4[];
+  const F32Item it = f32_item(p, n_tiles, true);
+  f32_dq_rows<D, kR, kC>(p, it, it.tile * F32Shape<D, kR, kC>::kRows, reinterpret_cast<float*>(f32_smem4));
 }
 
 }  // namespace sigattn

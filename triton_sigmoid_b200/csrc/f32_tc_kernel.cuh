@@ -1,0 +1,580 @@
+// fp32 on the tensor cores: forward, dK/dV and dQ of float32 tensors with every product done as six bf16 products.
+//
+// A float is the sum of three bf16 numbers, x = x0 + x1 + x2 (each the rounded remainder of the ones before it; 24 bits
+// and three signs lose nothing but subnormal tails), so x y = x0 y0 + (x0 y1 + x1 y0) + (x0 y2 + x1 y1 + x2 y0) up to terms
+// of 2^-27 |x y|: six products of the bf16 pipe, whose products of 8-bit significands are exact and whose sums are fp32.
+// The small terms go into the accumulator first, and an accumulator takes one tile of 64 streamed rows only: the sums over
+// tiles are made in registers, rounded to nearest, so that the tensor core's own summation never runs over more than
+// 64 terms.
+//
+// B=4 T=2048 H=8 D=64, forward + backward: 1512 us (the FMA kernels 3652, and 1670 at the rate of the FMA pipe alone).
+// Relative error of O, dQ, dK, dV against 64 bits, FMA kernels in brackets: T=256 2.5 - 3.1e-7 (3.4 - 3.6), T=2048 3.1 - 3.8e-7 (8.3 -
+// 8.5), T=32768 causal 4.7 - 5.1e-7 (2.7e-6); D = 128, T=2048 2.0 - 3.0e-7 (8.3 - 8.4), T=16384 4.1 - 4.7e-7 (2.3e-6).  Accumulators
+// kept for 128 or 256 terms would make it 6 and 15e-7, small and large terms in turn 4e-7: the tensor core truncates its sums.
+//
+// One kernel, five modes, one CTA per (batch, head, 128-row tile); R = stationary side, C = streamed side:
+//     kTcFwd   R1 = Q            C1 = K  C2 = V     S = R1 C1^T, P = sigmoid;         out2 = O  += P C2
+//     kTcDkdv  R1 = K  R2 = V    C1 = Q  C2 = dO    S, P, dP = R2 C2^T, dS;           out2 = dV += P C2, out1 = dK += dS C1
+//     kTcDq    R1 = Q  R2 = dO   C1 = K  C2 = V     S, P, dP, dS;                     out1 = dQ += dS C1
+//     kTcDv, kTcDk                                  the two halves of kTcDkdv, for D = 128, where dK and dV together need
+//                                                   more registers and more TMEM than there are
+// A job is the row tile times 64 streamed rows.
+//
+// 24 warps, registers re-split with setmaxnreg:
+//   0-15   compute: 32 rows x 16 columns of a job each (thread = one row): scores out of TMEM, probability (the same
+//          f32_sigmoid as the FMA kernels) or dS, the three bf16 parts back into TMEM as the A operand of the next product,
+//          and the sums over jobs, 1/16 of the output tile per warp
+//   16-19  conversion: the streamed rows from global memory (loads run ahead by one tile), split, into swizzled tiles that
+//          serve as K-major operand (scores) and as MN-major one (outputs); rows beyond the valid length are zero
+//   20     issues every product
+// R1 (and R2 where it fits) is a TMEM operand: a product of 128 x 64 whose A lies in shared memory would read 6 KB in the 32
+// clocks that it takes, half again what shared memory delivers.
+//
+// Values that the split cannot carry (infinities and NaN; finite ones within 2^-9 of the largest float) turn into NaN in
+// every result that they reach.  A CTA that finds an accumulator that is not finite computes its tile again with the FMA
+// code (f32_fwd_rows and so on), which gives what single precision gives.
+#pragma once
+
+#include "f32_kernels.cuh"
+#include "ptx.cuh"
+
+namespace sigattn {
+
+enum TcMode { kTcFwd = 0, kTcDkdv = 1, kTcDq = 2, kTcDv = 3, kTcDk = 4 };
+
+constexpr int kTcRows = 128;
+constexpr int kTcJob = 64;
+constexpr int kTcComputeWarps = 16;
+constexpr int kTcConvWarps = 4;
+constexpr int kTcIssuerWarp = 20;
+constexpr int kTcThreads = 24 * 32;
+
+template <int D, int kMode>
+struct TcShape {
+  static constexpr bool kKeyRows = kMode == kTcDkdv || kMode == kTcDv || kMode == kTcDk;  // R = keys, C = queries
+  static constexpr bool kOut1 = kMode == kTcDkdv || kMode == kTcDq || kMode == kTcDk;      // dP, dS C1
+  static constexpr bool kOut2 = kMode == kTcDkdv || kMode == kTcFwd || kMode == kTcDv;     // P C2
+  static constexpr bool kBoth = kOut1 && kOut2;
+  static_assert(!kBoth || D == 64, "registers and TMEM");
+  static constexpr bool kR2Smem = kBoth || (kOut1 && D == 128);
+  // TMEM: the three parts of R1 (R2), score slots, outputs of one job.
+  // Slot: S in columns [0, 64); P over it (parts 0 and 1 of k-step kk at 16 kk and 16 kk + 8, part 2 at 64 + 8 kk).  With both
+  // outputs, dP / dS have a slot of their own of the same form; with dS alone, dP has columns [64, 128) and part 2 of dS lies
+  // over it at 64 + 16 kk.
+  static constexpr int kPartCols = D / 2;  // columns of one part of a 128 x D operand
+  static constexpr int kR1Col = 0;
+  static constexpr int kR2Col = 3 * kPartCols;
+  static constexpr int kSCol = 3 * kPartCols + (kOut1 && !kR2Smem ? 3 * kPartCols : 0);
+  static constexpr int kSlotCols = kOut2 ? 96 : 128;
+  static constexpr int kSlots = D == 64 ? (kOut1 ? 2 : 3) : (kOut1 ? 1 : 2);
+  static constexpr int kDpCol = kBoth ? kSCol + kSlots * kSlotCols : kSCol + 64;
+  static constexpr int kOutCol = kSCol + kSlots * kSlotCols + (kBoth ? 96 : 0);
+  static constexpr int kOuts = !kOut1 && D == 64 ? 2 : 1;  // buffers of out2
+  static constexpr int kOut2Col = kOutCol;
+  static constexpr int kOut1Col = kOutCol + (kBoth ? D : 0);
+  static_assert(kOut1Col + kOuts * D <= 512, "TMEM budget");
+  static constexpr int kPart2Col = 64, kPart2Step = kOut2 ? 8 : 16;  // part 2 of k-step kk within a slot
+  // shared memory: R2 parts, then stages of (C1 parts, C2 parts)
+  static constexpr int kStages = D == 64 || !kOut1 ? 2 : 1;
+  static constexpr int kCPart = kTcJob * D * 2;
+  static constexpr int kCTile = 3 * kCPart;
+  static constexpr int kRPart = kTcRows * D * 2;
+  static constexpr int kC1Off = kR2Smem ? 3 * kRPart : 0;
+  static constexpr int kC2Off = kC1Off + kStages * kCTile;
+  static constexpr int kBarOff = kC2Off + kStages * kCTile;
+  static constexpr int kC1Full = 0;                    // [kStages] tile converted (4 warps)
+  static constexpr int kC2Full = kC1Full + kStages;
+  static constexpr int kC1Empty = kC2Full + kStages;   // [kStages] every product that reads the tile is complete
+  static constexpr int kC2Empty = kC1Empty + kStages;
+  static constexpr int kSFull = kC2Empty + kStages;    // [kSlots]
+  static constexpr int kDpFull = kSFull + kSlots;      // [kSlots] (both outputs: 1)
+  static constexpr int kPReady = kDpFull + kSlots;     // [kSlots] P written (16 warps)
+  static constexpr int kDsReady = kPReady + kSlots;    // [kSlots]
+  static constexpr int kOut1Full = kDsReady + kSlots;  // products of the job complete
+  static constexpr int kOut2Full = kOut1Full + 1;      // [kOuts]
+  static constexpr int kOut1Free = kOut2Full + 2;      // output added to the registers (16 warps)
+  static constexpr int kOut2Free = kOut1Free + 1;      // [kOuts]
+  static constexpr int kNumBars = kOut2Free + 2;
+  static constexpr int kMiscOff = kBarOff + 8 * kNumBars;
+  // (the FMA code reuses the space from the start)
+  using Fallback = F32Shape<D, 4, 4>;
+  static constexpr int kFallbackBytes = kMode == kTcFwd ? Fallback::kFwdBytes : kKeyRows ? Fallback::kDkdvBytes : Fallback::kDqBytes;
+  static_assert(kFallbackBytes <= kBarOff, "shared memory of the FMA code");
+  static constexpr int kDynBytes = kMiscOff + 16 + 1024;
+  static_assert(kDynBytes <= 232448, "shared memory budget");
+};
+
+// The three bf16 parts of 2 N floats, in packed pairs.
+template <int N>
+__device__ __forceinline__ void tc_split(const float (&x)[2 * N], uint32_t (&p0)[N], uint32_t (&p1)[N], uint32_t (&p2)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    float2 r = make_float2(x[2 * i], x[2 * i + 1]);
+    p0[i] = pack2<true>(r.x, r.y);
+    r = __fadd2_rn(r, make_float2(-__uint_as_float(p0[i] << 16), -__uint_as_float(p0[i] & 0xffff0000u)));
+    p1[i] = pack2<true>(r.x, r.y);
+    r = __fadd2_rn(r, make_float2(-__uint_as_float(p1[i] << 16), -__uint_as_float(p1[i] & 0xffff0000u)));
+    p2[i] = pack2<true>(r.x, r.y);
+  }
+}
+
+template <int D, int kMode>
+__global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32Params p, const int n_tiles) {
+  using L = TcShape<D, kMode>;
+  constexpr int kSite = (0x6 + kMode) << 16;
+  extern __shared__ uint8_t tc_smem[];
+  if (*reinterpret_cast<volatile int*>(&g_status_word) != 0) return;
+
+  // ---------------------------------------------------------------- the tile
+  const F32Item it = f32_item(p, n_tiles, !L::kKeyRows);
+  const int r0 = it.tile * kTcRows;
+  const int Lr = L::kKeyRows ? it.Lk : it.Lq, Lc = L::kKeyRows ? it.Lq : it.Lk;
+  const int row_lim = L::kKeyRows ? it.key_lim : it.row_lim;
+  const int c_begin = L::kKeyRows && p.causal ? r0 : 0;
+  const int c_end = !L::kKeyRows && p.causal ? min(Lc, r0 + kTcRows) : Lc;
+  const int n_jobs = r0 < Lr && c_end > c_begin ? (c_end - c_begin + kTcJob - 1) / kTcJob : 0;
+  const int n16 = (p.d_cols + 15) / 16;  // steps of 16 along the head dimension that hold anything
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int quarter = warp & 3, cg = warp >> 2;
+  const int row = r0 + quarter * 32 + lane;  // of a compute thread, within the sequence
+
+  // outputs of a compute thread: columns [cg D/4, +D/4) of its row
+  constexpr int kOutPer = D / 4;
+  auto out_row = [&](float* base, int64_t sb, int64_t st, int64_t sh, int t0) -> float* {
+    return base + (int64_t)it.bc * sb + (int64_t)it.h * sh + (int64_t)(t0 + row) * st + cg * kOutPer;
+  };
+  auto store = [&](float* dst, const float (&acc)[kOutPer], float mul) {
+#pragma unroll
+    for (int c = 0; c < kOutPer; c += 4) {
+      if (cg * kOutPer + c >= p.d_cols) continue;
+      float4 w = make_float4(acc[c] * mul, acc[c + 1] * mul, acc[c + 2] * mul, acc[c + 3] * mul);
+      if (row >= Lr) w = make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(dst + c) = w;
+    }
+  };
+  auto store_all = [&](const float (&a1)[kOutPer], const float (&a2)[kOutPer]) {
+    if (row >= row_lim) return;
+    if constexpr (kMode == kTcFwd) store(out_row(p.o, p.o_sb, p.o_st, p.o_sh, it.tq0), a2, 1.0f);
+    if constexpr (L::kKeyRows && L::kOut1) store(out_row(p.dk, p.dk_sb, p.dk_st, p.dk_sh, it.tk0), a1, p.scale);
+    if constexpr (L::kKeyRows && L::kOut2) store(out_row(p.dv, p.dv_sb, p.dv_st, p.dv_sh, it.tk0), a2, 1.0f);
+    if constexpr (kMode == kTcDq) store(out_row(p.dq, p.dq_sb, p.dq_st, p.dq_sh, it.tq0), a1, p.scale);
+  };
+  if (n_jobs == 0) {  // nothing is visible to these rows
+    if (warp < kTcComputeWarps) {
+      const float zero[kOutPer] = {};
+      store_all(zero, zero);
+    }
+    return;
+  }
+
+  // ---------------------------------------------------------------- setup
+  const uint32_t smem_base = (smem_u32(tc_smem) + 1023u) & ~1023u;
+  uint8_t* smem_gen = tc_smem + (smem_base - smem_u32(tc_smem));
+  auto bar = [&](int i) -> uint32_t { return smem_base + L::kBarOff + 8u * i; };
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + L::kMiscOff + 4);
+  volatile int* redo_flag = reinterpret_cast<volatile int*>(smem_gen + L::kMiscOff + 8);
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    *redo_flag = 0;
+    for (int i = 0; i < L::kStages; ++i) {
+      mbar_init(bar(L::kC1Full + i), kTcConvWarps);
+      mbar_init(bar(L::kC2Full + i), kTcConvWarps);
+      mbar_init(bar(L::kC1Empty + i), 1);
+      mbar_init(bar(L::kC2Empty + i), 1);
+    }
+    for (int i = 0; i < L::kSlots; ++i) {
+      mbar_init(bar(L::kSFull + i), 1);
+      mbar_init(bar(L::kDpFull + i), 1);
+      mbar_init(bar(L::kPReady + i), kTcComputeWarps);
+      mbar_init(bar(L::kDsReady + i), kTcComputeWarps);
+    }
+    mbar_init(bar(L::kOut1Full), 1);
+    mbar_init(bar(L::kOut1Free), kTcComputeWarps);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(L::kOut2Full + i), 1);
+      mbar_init(bar(L::kOut2Free + i), kTcComputeWarps);
+    }
+    fence_mbar_init();
+  }
+  if (warp == kTcIssuerWarp) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+
+  const float* q_base = p.q + (int64_t)it.bc * p.q_sb + (int64_t)it.h * p.q_sh + (int64_t)it.tq0 * p.q_st;
+  const float* k_base = p.k + (int64_t)it.bc * p.k_sb + (int64_t)it.h * p.k_sh + (int64_t)it.tk0 * p.k_st;
+  const float* v_base = p.v + (int64_t)it.bc * p.v_sb + (int64_t)it.h * p.v_sh + (int64_t)it.tk0 * p.v_st;
+  const float* do_base = !p.dout ? nullptr
+                                         : p.dout + (int64_t)it.bc * p.do_sb + (int64_t)it.h * p.do_sh + (int64_t)it.tq0 * p.do_st;
+
+  if (warp >= kTcIssuerWarp) {
+    // ============================================================ issuer
+    setmaxnreg_dec<48>();
+    if (warp == kTcIssuerWarp) {
+      asm volatile("bar.sync 9, %0;" ::"n"(32 * kTcComputeWarps + 32) : "memory");  // R has been written
+      tc_fence_after_sync();
+      const bool leader = elect_one();
+      constexpr uint32_t id_in = make_idesc(128, kTcJob, true, false, false);
+      const uint32_t id_out = make_idesc(128, 0, true, false, true) | (uint32_t)(n16 * 2) << 17;  // N = 16 n16
+      const uint64_t c1_d = smem_desc_sw128(smem_base + L::kC1Off, 16, 1024);
+      const uint32_t hi = (uint32_t)(c1_d >> 32);
+      const uint32_t c1_in = (uint32_t)c1_d;
+      const uint32_t c2_in = (uint32_t)smem_desc_sw128(smem_base + L::kC2Off, 16, 1024);
+      const uint32_t r2_in = (uint32_t)smem_desc_sw128(smem_base, 16, 1024);
+      const uint32_t c1_out = (uint32_t)smem_desc_sw128(smem_base + L::kC1Off, kTcJob * 128, 1024);
+      const uint32_t c2_out = (uint32_t)smem_desc_sw128(smem_base + L::kC2Off, kTcJob * 128, 1024);
+      constexpr uint32_t kStage16 = L::kCTile >> 4;
+      // the six products, small terms first
+      constexpr int kA[6] = {2, 1, 0, 1, 0, 0}, kB[6] = {0, 1, 2, 0, 1, 0};
+      // scores: A = R1 in TMEM / R2 in TMEM or shared memory, B = a streamed tile, K = head dimension
+      auto in_ts = [&](uint32_t dcol, uint32_t acol, uint32_t b_lo) {
+#pragma unroll
+        for (int t = 0; t < 6; ++t)
+          for (int kk = 0; kk < n16; ++kk)
+            mma_ts(leader, tmem + dcol, tmem + acol + kA[t] * L::kPartCols + 8 * kk,
+                   make_desc(b_lo + kB[t] * (L::kCPart >> 4) + (kk >> 2) * (kTcJob * 128 >> 4) + (kk & 3) * 2, hi), id_in,
+                   t > 0 || kk > 0);
+      };
+      auto in_ss = [&](uint32_t dcol, uint32_t a_lo, uint32_t b_lo) {
+#pragma unroll
+        for (int t = 0; t < 6; ++t)
+          for (int kk = 0; kk < n16; ++kk)
+            mma_ss(leader, tmem + dcol,
+                   make_desc(a_lo + kA[t] * (L::kRPart >> 4) + (kk >> 2) * (kTcRows * 128 >> 4) + (kk & 3) * 2, hi),
+                   make_desc(b_lo + kB[t] * (L::kCPart >> 4) + (kk >> 2) * (kTcJob * 128 >> 4) + (kk & 3) * 2, hi), id_in,
+                   t > 0 || kk > 0);
+      };
+      // outputs of a job: A = P or dS in a slot, B = the streamed tile, K = its 64 rows
+      auto out = [&](uint32_t dcol, uint32_t slot_col, uint32_t b_lo) {
+#pragma unroll
+        for (int t = 0; t < 6; ++t)
+#pragma unroll
+          for (int kk = 0; kk < kTcJob / 16; ++kk)
+            mma_ts(leader, tmem + dcol,
+                   tmem + slot_col + (kA[t] < 2 ? 16 * kk + 8 * kA[t] : L::kPart2Col + L::kPart2Step * kk),
+                   make_desc(b_lo + kB[t] * (L::kCPart >> 4) + kk * (2048 >> 4), hi), id_out, t > 0 || kk > 0);
+      };
+      bool ok = true;
+      auto wait = [&](int b, int n_th, int site) {  // completion number n_th (from 0) of a barrier
+        ok = ok && mbar_wait_warp(bar(b), (uint32_t)n_th & 1u, abort_flag, kSite + site);
+        tc_fence_after_sync();
+      };
+      auto stage16 = [&](int j) -> uint32_t { return (uint32_t)(j % L::kStages) * kStage16; };
+      auto scores = [&](int j) {
+        wait(L::kC1Full + j % L::kStages, j / L::kStages, 1);
+        if (!ok) return;
+        in_ts(L::kSCol + (j % L::kSlots) * L::kSlotCols, L::kR1Col, c1_in + stage16(j));
+        mma_commit(leader, bar(L::kSFull + j % L::kSlots));
+        if (!L::kOut1) mma_commit(leader, bar(L::kC1Empty + j % L::kStages));
+      };
+      auto dscores = [&](int j) {
+        wait(L::kC2Full + j % L::kStages, j / L::kStages, 2);
+        if (!ok) return;
+        const uint32_t dcol = L::kDpCol + (!L::kBoth ? (j % L::kSlots) * L::kSlotCols : 0);
+        if constexpr (L::kR2Smem) in_ss(dcol, r2_in, c2_in + stage16(j));
+        else in_ts(dcol, L::kR2Col, c2_in + stage16(j));
+        mma_commit(leader, bar(L::kDpFull + (!L::kBoth ? j % L::kSlots : 0)));
+        if (!L::kOut2) mma_commit(leader, bar(L::kC2Empty + j % L::kStages));
+      };
+      auto out2 = [&](int j) {
+        const int b = j % L::kOuts;
+        wait(L::kPReady + j % L::kSlots, j / L::kSlots, 3);
+        if (!L::kOut1) wait(L::kC2Full + j % L::kStages, j / L::kStages, 2);
+        if (j >= L::kOuts) wait(L::kOut2Free + b, j / L::kOuts - 1, 4);
+        if (!ok) return;
+        out(L::kOut2Col + b * D, L::kSCol + (j % L::kSlots) * L::kSlotCols, c2_out + stage16(j));
+        mma_commit(leader, bar(L::kOut2Full + b));
+        mma_commit(leader, bar(L::kC2Empty + j % L::kStages));
+      };
+      auto out1 = [&](int j) {
+        const int s = !L::kBoth ? j % L::kSlots : 0;
+        wait(L::kDsReady + s, !L::kBoth ? j / L::kSlots : j, 5);
+        if (j > 0) wait(L::kOut1Free, j - 1, 6);
+        if (!ok) return;
+        out(L::kOut1Col, (!L::kBoth ? L::kSCol : L::kDpCol) + s * L::kSlotCols, c1_out + stage16(j));
+        mma_commit(leader, bar(L::kOut1Full));
+        mma_commit(leader, bar(L::kC1Empty + j % L::kStages));
+      };
+      // A slot's scores may be overwritten when the output products that read the P / dS written over them are complete.
+      if constexpr (!L::kOut1) {
+        scores(0);
+        for (int j = 0; j < n_jobs && ok; ++j) {
+          if (j + 1 < n_jobs) {
+            const int f = j + 1 - L::kSlots;
+            if (f >= 0) wait(L::kOut2Full + f % L::kOuts, f / L::kOuts, 7);
+            if (ok) scores(j + 1);
+          }
+          if (ok) out2(j);
+        }
+      } else if constexpr (L::kBoth) {
+        scores(0);
+        if (ok) dscores(0);
+        for (int j = 0; j < n_jobs && ok; ++j) {
+          if (j + 1 < n_jobs) {
+            if (j > 0) wait(L::kOut2Full, j - 1, 7);
+            if (ok) scores(j + 1);
+          }
+          if (ok) out2(j);
+          if (ok) out1(j);
+          if (j + 1 < n_jobs) {
+            wait(L::kOut1Full, j, 8);
+            if (ok) dscores(j + 1);
+          }
+        }
+      } else {
+        constexpr int kAhead = L::kSlots - 1;
+        if (kAhead) {
+          scores(0);
+          if (ok) dscores(0);
+        }
+        for (int j = 0; j < n_jobs && ok; ++j) {
+          const int n = j + kAhead;
+          if (n < n_jobs) {
+            if (n >= L::kSlots) wait(L::kOut1Full, n - L::kSlots, 7);
+            if (ok) scores(n);
+            if (ok) dscores(n);
+          }
+          if (ok) out1(j);
+        }
+      }
+    }
+  } else if (warp >= kTcComputeWarps) {
+    // ============================================================ conversion of the streamed rows
+    // A chunk is 64 rows x 64 columns of one tensor; a thread takes 8 consecutive columns of four of its rows.  The loads of
+    // the next chunk are issued as the registers of this one become free.  (This group keeps the 80 registers of the launch.)
+    const int wc = warp - kTcComputeWarps;
+    const int rr = 4 * wc + (lane >> 3), c8 = lane & 7;
+    const float* src1 = (L::kKeyRows ? q_base : k_base) + 8 * c8;
+    const float* src2 = (L::kKeyRows ? do_base : v_base) + 8 * c8;
+    const int64_t st1 = L::kKeyRows ? p.q_st : p.k_st, st2 = L::kKeyRows ? p.do_st : p.v_st;
+    constexpr int kHalves = D / 64;
+    const int n_chunks = n_jobs * 2 * kHalves;
+    float4 x[4][2];
+    auto load = [&](int chunk, int u) {
+      const int j = chunk / (2 * kHalves), half = chunk % kHalves;
+      const bool second = (chunk / kHalves) & 1;
+      const int r = c_begin + j * kTcJob + 16 * u + rr, c = 64 * half + 8 * c8;
+      const float* s = (second ? src2 + r * st2 : src1 + r * st1) + 64 * half;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      const bool live = chunk < n_chunks && r < Lc;
+      x[u][0] = live && c < p.d_cols ? __ldg(reinterpret_cast<const float4*>(s)) : zero;
+      x[u][1] = live && c + 4 < p.d_cols ? __ldg(reinterpret_cast<const float4*>(s) + 1) : zero;
+    };
+#pragma unroll
+    for (int u = 0; u < 4; ++u) load(0, u);
+    bool ok = true;
+    for (int chunk = 0; chunk < n_chunks; ++chunk) {
+      const int j = chunk / (2 * kHalves), half = chunk % kHalves;
+      const bool second = (chunk / kHalves) & 1;
+      const int st = j % L::kStages;
+      if (half == 0 && j >= L::kStages) {
+        ok = mbar_wait_warp(bar((second ? L::kC2Empty : L::kC1Empty) + st), (uint32_t)(j / L::kStages - 1) & 1u, abort_flag, kSite + 9);
+        if (!ok) break;
+      }
+      uint8_t* tile = smem_gen + (second ? L::kC2Off : L::kC1Off) + st * L::kCTile + half * (kTcJob * 128) + rr * 128 +
+                      ((c8 ^ (rr & 7)) << 4);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float f[8] = {x[u][0].x, x[u][0].y, x[u][0].z, x[u][0].w, x[u][1].x, x[u][1].y, x[u][1].z, x[u][1].w};
+        uint32_t p0[4], p1[4], p2[4];
+        tc_split<4>(f, p0, p1, p2);
+        load(chunk + 1, u);
+        uint8_t* dst = tile + u * 2048;
+        *reinterpret_cast<uint4*>(dst) = make_uint4(p0[0], p0[1], p0[2], p0[3]);
+        *reinterpret_cast<uint4*>(dst + L::kCPart) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+        *reinterpret_cast<uint4*>(dst + 2 * L::kCPart) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+      }
+      if (half == kHalves - 1) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar((second ? L::kC2Full : L::kC1Full) + st));
+      }
+    }
+  } else {
+    // ============================================================ compute
+    setmaxnreg_inc<88>();
+    const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
+    // ------------------------------------------------------------ R: this thread's row, columns [cg D/4, +D/4)
+    auto split_rows = [&](const float* base, int64_t st, bool to_smem, int col) {
+      const float* src = base + (int64_t)row * st;
+#pragma unroll
+      for (int s = 0; s < D / 64; ++s) {
+        const int kk = cg * (D / 64) + s;
+        float f[16];
+#pragma unroll
+        for (int c = 0; c < 16; c += 4) {
+          const float4 w = row < Lr && 16 * kk + c < p.d_cols ? __ldg(reinterpret_cast<const float4*>(src + 16 * kk + c))
+                                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+          f[c] = w.x; f[c + 1] = w.y; f[c + 2] = w.z; f[c + 3] = w.w;
+        }
+        uint32_t part[3][8];
+        tc_split<8>(f, part[0], part[1], part[2]);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+          if (!to_smem) {
+            tmem_st8(lanes + col + t * L::kPartCols + 8 * kk, part[t]);
+          } else {
+            const int rr = quarter * 32 + lane;
+            uint8_t* dst = smem_gen + t * L::kRPart + (kk >> 2) * (kTcRows * 128) + rr * 128;
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              *reinterpret_cast<uint4*>(dst + (((2 * (kk & 3) + e) ^ (rr & 7)) << 4)) =
+                  make_uint4(part[t][4 * e], part[t][4 * e + 1], part[t][4 * e + 2], part[t][4 * e + 3]);
+          }
+        }
+      }
+    };
+    split_rows(L::kKeyRows ? k_base : q_base, L::kKeyRows ? p.k_st : p.q_st, false, L::kR1Col);
+    if constexpr (L::kOut1)
+      split_rows(L::kKeyRows ? v_base : do_base, L::kKeyRows ? p.v_st : p.do_st, L::kR2Smem, L::kR2Col);
+    tmem_st_wait();
+    fence_proxy_async_smem();
+    tc_fence_before_sync();
+    asm volatile("bar.arrive 9, %0;" ::"n"(32 * kTcComputeWarps + 32) : "memory");
+
+    float bias = item_bias(p.bias, p.bias_scalar, it.b, it.Lk);
+    const float* sm = p.score_mod ? p.score_mod + it.sm_off : nullptr;
+    const float row_mod = L::kKeyRows && sm && row < it.key_lim ? sm[row] : 0.f;
+    const int lo = L::kKeyRows && p.causal ? row : 0;  // visible columns of this row: [lo, hi)
+    const int hi = !L::kKeyRows && p.causal ? min(Lc, row + 1) : Lc;
+
+    bool ok = true;
+    auto wait = [&](int b, int n_th, int site) {
+      ok = mbar_wait_warp(bar(b), (uint32_t)n_th & 1u, abort_flag, kSite + site);
+      tc_fence_after_sync();
+    };
+    auto arrive = [&](int b) {
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(b));
+    };
+    float acc1[kOutPer], acc2[kOutPer];
+#pragma unroll
+    for (int c = 0; c < kOutPer; ++c) acc1[c] = acc2[c] = 0.f;
+    // adds a job's output to the registers
+    auto drain = [&](float (&acc)[kOutPer], int full, int free, int n_th, int col) {
+      wait(full, n_th, 13);
+      if (!ok) return;
+#pragma unroll
+      for (int s = 0; s < kOutPer / 16; ++s) {
+        if (cg * (kOutPer / 16) + s >= n16) continue;  // columns that no product wrote
+        uint32_t r[16];
+        tmem_ld(lanes + col + cg * kOutPer + 16 * s, r);
+        tmem_ld_wait_for(r);
+#pragma unroll
+        for (int c = 0; c < 16; c += 2) {
+          const float2 a = __fadd2_rn(make_float2(acc[16 * s + c], acc[16 * s + c + 1]),
+                                      make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])));
+          acc[16 * s + c] = a.x;
+          acc[16 * s + c + 1] = a.y;
+        }
+      }
+      arrive(free);
+    };
+    auto drain_all = [&](int j) {
+      if constexpr (L::kOut2) drain(acc2, L::kOut2Full + j % L::kOuts, L::kOut2Free + j % L::kOuts, j / L::kOuts, L::kOut2Col + (j % L::kOuts) * D);
+      if constexpr (L::kOut1) if (ok) drain(acc1, L::kOut1Full, L::kOut1Free, j, L::kOut1Col);
+    };
+    // parts of a 128 x 64 operand over the scores that it was computed from
+    auto put = [&](uint32_t slot, const float (&x)[16]) {
+      uint32_t p01[16], p2[8];
+      {
+        uint32_t p0[8], p1[8];
+        tc_split<8>(x, p0, p1, p2);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { p01[i] = p0[i]; p01[8 + i] = p1[i]; }
+      }
+      tmem_st(slot + 16 * cg, p01);
+      tmem_st(slot + L::kPart2Col + L::kPart2Step * cg, p2);
+      tmem_st_wait();
+    };
+
+    for (int j = 0; j < n_jobs; ++j) {
+      const int s = j % L::kSlots;
+      const uint32_t slot = lanes + L::kSCol + s * L::kSlotCols;
+      const int job0 = c_begin + j * kTcJob, col0 = job0 + 16 * cg;
+      const bool mask = job0 + kTcJob > Lc || (p.causal && (L::kKeyRows ? job0 < r0 + kTcRows - 1 : job0 + kTcJob - 1 > r0));
+      float pr[16];
+      wait(L::kSFull + s, j / L::kSlots, 10);
+      if (!ok) break;
+      {
+        uint32_t r[16];
+        tmem_ld(slot + 16 * cg, r);
+        tmem_ld_wait_for(r);
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          float x = __uint_as_float(r[c]) * p.scale + bias;
+          if (sm) x += L::kKeyRows ? row_mod : (col0 + c < it.key_lim ? __ldg(sm + col0 + c) : 0.f);
+          pr[c] = f32_sigmoid(x);
+        }
+        if (mask) {
+#pragma unroll
+          for (int c = 0; c < 16; ++c) pr[c] = col0 + c >= lo && col0 + c < hi ? pr[c] : 0.f;
+        }
+      }
+      if constexpr (L::kOut2) {
+        put(slot, pr);
+        arrive(L::kPReady + s);
+      }
+      if constexpr (L::kOut1) {
+        if (L::kBoth && j > 0) drain_all(j - 1);
+        if (!ok) break;
+        wait(L::kDpFull + (!L::kBoth ? s : 0), !L::kBoth ? j / L::kSlots : j, 11);
+        if (!ok) break;
+        const uint32_t dslot = !L::kBoth ? slot : lanes + L::kDpCol;
+        uint32_t r[16];
+        tmem_ld((!L::kBoth ? slot + 64 : dslot) + 16 * cg, r);
+        tmem_ld_wait_for(r);
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const float ds = pr[c] * (1.0f - pr[c]) * __uint_as_float(r[c]);
+          pr[c] = !mask || (col0 + c >= lo && col0 + c < hi) ? ds : 0.f;
+        }
+        put(dslot, pr);
+        arrive(L::kDsReady + (!L::kBoth ? s : 0));
+      }
+      if (!L::kBoth && j > 0) drain_all(j - 1);
+      if (!ok) break;
+    }
+    if (ok) drain_all(n_jobs - 1);
+
+    // ------------------------------------------------------------ epilogue
+    float finite = 0.f;  // NaN when a sum is not finite
+#pragma unroll
+    for (int c = 0; c < kOutPer; ++c) {
+      if constexpr (L::kOut1) finite = fmaf(acc1[c], 0.f, finite);
+      if constexpr (L::kOut2) finite = fmaf(acc2[c], 0.f, finite);
+    }
+    if (row < Lr && !(finite == 0.f)) *redo_flag = 1;
+    asm volatile("bar.sync 10, %0;" ::"n"(32 * kTcComputeWarps) : "memory");
+    if (*abort_flag == 0) {
+      if (*redo_flag == 0) {
+        store_all(acc1, acc2);
+      } else {
+        float* space = reinterpret_cast<float*>(smem_gen);
+#pragma unroll 1
+        for (int r = r0; r < min(r0 + kTcRows, row_lim); r += 64) {
+          if constexpr (kMode == kTcFwd) f32_fwd_rows<D, 4, 4, 11>(p, it, r, space);
+          if constexpr (L::kKeyRows) f32_dkdv_rows<D, 4, 4, 11>(p, it, r, space);
+          if constexpr (kMode == kTcDq) f32_dq_rows<D, 4, 4, 11>(p, it, r, space);
+        }
+      }
+    }
+  }
+
+  // ---------------------------------------------------------------- teardown
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == kTcIssuerWarp) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+}  // namespace sigattn

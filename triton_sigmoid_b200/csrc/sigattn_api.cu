@@ -13,6 +13,7 @@
 #include "bwd_kernel.cuh"
 #include "bwd_stream_kernel.cuh"
 #include "f32_kernels.cuh"
+#include "f32_tc_kernel.cuh"
 #include "fwd_kernel.cuh"
 
 namespace {
@@ -557,7 +558,7 @@ int static_scratch_ptr(int device, float** out) {
   return 0;
 }
 
-// float32 tensors: the FMA-pipe kernels (no tensor maps, no workspace).
+// float32 tensors on the FMA pipe (no tensor maps, no workspace).
 template <int D, int kR, int kC>
 int launch_f32_shape(const SigAttnParams* p, const sigattn::F32Params& fp, bool backward) {
   using namespace sigattn;
@@ -583,6 +584,30 @@ int launch_f32_shape(const SigAttnParams* p, const sigattn::F32Params& fp, bool 
     SIG_CUDA(cudaGetLastError());
   }
   return 0;
+}
+
+// float32 tensors on the tensor cores (no tensor maps, no workspace either).
+template <int D, int kMode>
+int launch_f32_tc(const SigAttnParams* p, const sigattn::F32Params& fp) {
+  using namespace sigattn;
+  using S = TcShape<D, kMode>;
+  const int n_tiles = ((S::kKeyRows ? p->Tk : p->Tq) + kTcRows - 1) / kTcRows;
+  const int64_t ctas = (int64_t)p->B * p->H * n_tiles;
+  if (ctas > INT32_MAX) return fail(-2, "too many (batch, head, tile) items: %lld", (long long)ctas);
+  auto kernel = sigattn_f32_tc_kernel<D, kMode>;
+  if (int rc = set_smem(kernel, S::kDynBytes, p->device)) return rc;
+  kernel<<<(unsigned int)ctas, kTcThreads, S::kDynBytes, static_cast<cudaStream_t>(p->stream)>>>(fp, n_tiles);
+  SIG_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// Whether float32 tensors take the tensor-core kernels: whose tiles of 128 rows need long sequences, or many of them, to pay.
+// Forward and backward, FMA kernels -> these: D=64 B=1 H=4 T=512 26 and 87 us -> 27 and 95, T=1000 57 and 183 -> 43 and 158; B=4 H=3
+// T=777 106 and 258 -> 43 and 143; B=2 H=4 T=256 16 and 67 -> 19 and 68; D=32 B=2 H=4 T=512 30 and 95 -> 24 and 82; D=128 B=1 H=4 T=512
+// 37 and 127 -> 40 and 178, T=2048 257 and 864 -> 120 and 566.
+bool f32_tc(const SigAttnParams* p) {
+  const int shorter = std::min(p->Tq, p->Tk);
+  return shorter >= 768 || (shorter >= 256 && (int64_t)p->B * p->H * ((shorter + 63) / 64) >= 64);
 }
 
 // Rows per CTA: 64 once such tiles occupy half of the SMs; below that 16, with four times the threads per row, which take
@@ -628,7 +653,21 @@ int launch_f32_d(const SigAttnParams* p, bool backward) {
   FwdDeviceInfo info;
   if (int rc = fwd_device_info(p->device, &info)) return rc;
   if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
-  const int rc = f32_tile_rows(p, info.n_sm) == 64 ? launch_f32_shape<D, 4, D / 64>(p, fp, backward) : launch_f32_shape<D, 1, 4>(p, fp, backward);
+  int rc = 0;
+  if (f32_tc(p)) {
+    if (!backward) {
+      rc = launch_f32_tc<D, kTcFwd>(p, fp);
+    } else {
+      if constexpr (D == 64) {
+        rc = launch_f32_tc<D, kTcDkdv>(p, fp);
+      } else {
+        rc = launch_f32_tc<D, kTcDv>(p, fp);
+        if (!rc) rc = launch_f32_tc<D, kTcDk>(p, fp);
+      }
+      if (!rc) rc = launch_f32_tc<D, kTcDq>(p, fp);
+    }
+  } else
+    rc = f32_tile_rows(p, info.n_sm) == 64 ? launch_f32_shape<D, 4, D / 64>(p, fp, backward) : launch_f32_shape<D, 1, 4>(p, fp, backward);
   if (rc) return rc;
   if (p->ev_main_stop) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_stop), stream));
   return 0;
@@ -690,7 +729,10 @@ int sigattn_form(const SigAttnParams* p, int backward, int n_sm) {
   if (!p) return fail(-1, "params is NULL");
   if (p->struct_bytes != sizeof(SigAttnParams)) return fail(-1, "struct_bytes %u != sizeof(SigAttnParams) %zu (ABI mismatch)", p->struct_bytes, sizeof(SigAttnParams));
   if (n_sm < 1) return fail(-2, "n_sm must be positive, got %d", n_sm);
-  if (p->dtype == SIGATTN_FP32) return f32_tile_rows(p, n_sm) == 64 ? SIGATTN_FORM_F32_64 : SIGATTN_FORM_F32_16;
+  if (p->dtype == SIGATTN_FP32) {
+    if (f32_tc(p)) return SIGATTN_FORM_F32_TC;
+    return f32_tile_rows(p, n_sm) == 64 ? SIGATTN_FORM_F32_64 : SIGATTN_FORM_F32_16;
+  }
   if (!backward) return fwd_split(p, n_sm) ? SIGATTN_FORM_FWD_SPLIT : SIGATTN_FORM_FWD;
   if (p->flags & SIGATTN_BWD_SPLIT) return SIGATTN_FORM_BWD_STREAM;
   return bwd_by_head(p, n_sm) ? SIGATTN_FORM_BWD_BY_HEAD : SIGATTN_FORM_BWD;
