@@ -1,0 +1,31 @@
+"""Which float32 calls the tensor-core kernels take, on 148 SMs."""
+
+import pytest
+import torch
+
+from tests.gpu_util import launch_form
+from triton_sigmoid_b200._cabi import FORM_F32_16, FORM_F32_64, FORM_F32_TC
+
+
+@pytest.mark.parametrize("B,H,Tq,Tk,D,forward,backward", [
+    (4, 8, 2048, 2048, 64, FORM_F32_TC, FORM_F32_TC),
+    (2, 4, 256, 256, 64, FORM_F32_16, FORM_F32_16),     # 32 tiles
+    (2, 8, 256, 256, 64, FORM_F32_TC, FORM_F32_TC),     # 64
+    (1000, 8, 255, 255, 64, FORM_F32_64, FORM_F32_64),
+    (1, 1, 383, 383, 64, FORM_F32_16, FORM_F32_16),
+    (1, 1, 384, 384, 64, FORM_F32_16, FORM_F32_TC),
+    (1, 1, 511, 511, 32, FORM_F32_16, FORM_F32_TC),
+    (1, 1, 512, 512, 32, FORM_F32_TC, FORM_F32_TC),
+    (1, 1, 16, 4096, 64, FORM_F32_TC, FORM_F32_TC),
+    (1, 1, 15, 4096, 64, FORM_F32_16, FORM_F32_16),
+    (1, 16, 4096, 63, 64, FORM_F32_16, FORM_F32_16),
+    (1, 17, 256, 256, 128, FORM_F32_16, FORM_F32_16),   # 68 tiles
+    (1, 18, 256, 256, 128, FORM_F32_TC, FORM_F32_16),   # 72
+    (1, 24, 256, 256, 128, FORM_F32_TC, FORM_F32_TC),   # 96
+    (1, 8, 512, 512, 128, FORM_F32_TC, FORM_F32_TC),
+    (1, 7, 512, 512, 128, FORM_F32_TC, FORM_F32_16),
+    (65535, 65535, 2 ** 31 - 1, 2 ** 31 - 1, 128, FORM_F32_TC, FORM_F32_TC),
+])
+def test_form(B, H, Tq, Tk, D, forward, backward):
+    for is_backward, want in ((False, forward), (True, backward)):
+        assert launch_form(B, H, Tq, Tk, D, torch.float32, is_backward, n_sm=148) == want

@@ -89,7 +89,7 @@ def test_values_that_the_parts_cannot_carry(bad, causal, D):
     assert torch.equal(got[inf], ref[inf])
     got[inf] = ref[inf] = 0.0
     assert got.isfinite().all()
-    scale = ref.abs().amax(dim=(0, 1, 3), keepdim=True) if bad != 3.4e38 else ref.abs().clamp(min=1.0)
+    scale = ref.abs().amax(dim=(0, 1, 3), keepdim=True).clamp(min=1e-30) if bad != 3.4e38 else ref.abs().clamp(min=1.0)
     assert ((got - ref).abs() / scale).max().item() <= 1e-5
 
 
@@ -98,7 +98,7 @@ def test_values_that_the_parts_cannot_carry(bad, causal, D):
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 def test_nonfinite_values_pass_through_probabilities_of_zero(bad, causal, D):
     """As in tests/test_f32_tiles_gpu.py: dS = P (1 - P) dP of a visible pair is NaN also where P has underflowed."""
-    T, j = 800, 70
+    T, j = 2112, 70
     assert launch_form(1, 2, T, T, D, torch.float32, True, causal) == FORM_F32_TC
     q, k, v, do = make_inputs(1, T, T, 2, D, torch.float32, std=0.5, seed=1)
     v[:, j] = bad

@@ -7,10 +7,11 @@
 // tiles are made in registers, rounded to nearest, so that the tensor core's own summation never runs over more than
 // 64 terms.
 //
-// B=4 T=2048 H=8 D=64, forward + backward: 1512 us (the FMA kernels 3652, and 1670 at the rate of the FMA pipe alone).
-// Relative error of O, dQ, dK, dV against 64 bits, FMA kernels in brackets: T=256 2.5 - 3.1e-7 (3.4 - 3.6), T=2048 3.1 - 3.8e-7 (8.3 -
-// 8.5), T=32768 causal 4.7 - 5.1e-7 (2.7e-6); D = 128, T=2048 2.0 - 3.0e-7 (8.3 - 8.4), T=16384 4.1 - 4.7e-7 (2.3e-6).  Accumulators
-// kept for 128 or 256 terms would make it 6 and 15e-7, small and large terms in turn 4e-7: the tensor core truncates its sums.
+// B=4 T=2048 H=8 D=64: 213 us forward, 625 backward (the FMA kernels 840 and 2820; 434 for all products at the tensor core's
+// rate).  Relative error of O, dQ, dK, dV against 64 bits, FMA kernels in brackets: T=512 2.3 - 2.9e-7 (4.5 - 4.7), T=2048 2.6 - 3.3e-7
+// (8.3 - 8.5), bias 0 1.3 - 1.8e-7 (7.8 - 8.2), T=32768 causal 4.3 - 4.7e-7 (2.7e-6); D = 128, T=2048 1.3 - 2.3e-7 (8.3 - 8.4), T=16384
+// 2.9 - 3.6e-7 (2.3e-6).  Accumulators kept for 128 or 256 terms would make it 6 and 15e-7, small and large terms in turn 4e-7: the
+// tensor core truncates its sums.
 //
 // One kernel, five modes, one CTA per (batch, head, 128-row tile); R = stationary side, C = streamed side:
 //     kTcFwd   R1 = Q            C1 = K  C2 = V     S = R1 C1^T, P = sigmoid;         out2 = O  += P C2
@@ -20,20 +21,28 @@
 //                                                   more registers and more TMEM than there are
 // A job is the row tile times 64 streamed rows.
 //
-// 24 warps, registers re-split with setmaxnreg:
-//   0-15   compute: 32 rows x 16 columns of a job each (thread = one row): scores out of TMEM, probability (the same
-//          f32_sigmoid as the FMA kernels) or dS, the three bf16 parts back into TMEM as the A operand of the next product,
-//          and the sums over jobs, 1/16 of the output tile per warp
-//   16-19  conversion: the streamed rows from global memory (loads run ahead by one tile), split, into swizzled tiles that
-//          serve as K-major operand (scores) and as MN-major one (outputs); rows beyond the valid length are zero
-//   20     issues every product
-// R1 (and R2 where it fits) is a TMEM operand: a product of 128 x 64 whose A lies in shared memory would read 6 KB in the 32
-// clocks that it takes, half again what shared memory delivers.
+// 28 warps, registers re-split with setmaxnreg:
+//   0-15   compute: 32 rows x 16 columns of a job each (thread = one row): scores out of TMEM, probability or dS, the three
+//          bf16 parts back into TMEM as the A operand of the next product, and the sums over jobs, 1/16 of the output tile per
+//          warp
+//   16-23  conversion: the streamed rows from global memory, split, into swizzled tiles that serve as K-major operand
+//          (scores) and as MN-major one (outputs); rows beyond the valid length are zero
+//   24, 25 issue the products: scores, outputs
+// R1 (and R2 where it fits) is a TMEM operand: a product of 128 x 64 takes 32 clocks then, and 48 with A in shared memory, of
+// which it reads 6 KB.
+//
+// What bounds it: a job needs 1536 (forward), 3456 (kTcDkdv) and 2304 (kTcDq) clocks of the tensor core and takes about 2700,
+// 4800 and 4200; splitting and the elementwise step are 1600 to 1900 instructions per scheduler and job, at half of the issue rate.
+// One issuing warp for scores and outputs, with loops over the k-steps, made it 95 clocks per product (286 us forward, 1211
+// backward); four conversion warps are 650 clocks per 64 x 64 chunk behind (D = 128 forward 118 us at B=2 H=8 T=2048 causal, 104
+// with eight; D = 64 the same), and more of them leave the compute warps too few registers.
 //
 // Values that the split cannot carry (infinities and NaN; finite ones within 2^-9 of the largest float) turn into NaN in
 // every result that they reach.  A CTA that finds an accumulator that is not finite computes its tile again with the FMA
 // code (f32_fwd_rows and so on), which gives what single precision gives.
 #pragma once
+
+#include <type_traits>
 
 #include "f32_kernels.cuh"
 #include "ptx.cuh"
@@ -45,9 +54,13 @@ enum TcMode { kTcFwd = 0, kTcDkdv = 1, kTcDq = 2, kTcDv = 3, kTcDk = 4 };
 constexpr int kTcRows = 128;
 constexpr int kTcJob = 64;
 constexpr int kTcComputeWarps = 16;
-constexpr int kTcConvWarps = 4;
-constexpr int kTcIssuerWarp = 20;
-constexpr int kTcThreads = 24 * 32;
+constexpr int kTcConvWarps = 8;
+constexpr int kTcIssuerIn = 24;   // scores; owns the TMEM allocation
+constexpr int kTcIssuerOut = 25;  // outputs
+constexpr int kTcThreads = 28 * 32;
+// Registers per thread: 72 at launch (65536 / 896, rounded down to a multiple of 8), then by role.
+constexpr int kTcConvRegs = 48, kTcIssuerRegs = 56, kTcComputeRegs = 88;
+static_assert(kTcComputeWarps * kTcComputeRegs + kTcConvWarps * kTcConvRegs + 4 * kTcIssuerRegs <= 28 * 72, "no more than the launch gave");
 
 template <int D, int kMode>
 struct TcShape {
@@ -81,8 +94,14 @@ struct TcShape {
   static constexpr int kRPart = kTcRows * D * 2;
   static constexpr int kC1Off = kR2Smem ? 3 * kRPart : 0;
   static constexpr int kC2Off = kC1Off + kStages * kCTile;
-  static constexpr int kBarOff = kC2Off + kStages * kCTile;
-  static constexpr int kC1Full = 0;                    // [kStages] tile converted (4 warps)
+  // rows on their way to the conversion warps: a ring of chunks of 64 rows x 64 floats
+  static constexpr int kRing = D == 64 ? 4 : 2;
+  static constexpr int kRingOff = kC2Off + kStages * kCTile;
+  static constexpr int kChunk = kTcJob * 64 * 4;
+  static constexpr int kBarOff = kRingOff + kRing * kChunk;
+  // With one stage, the tile that only dP reads is free again before the one that the output product reads too: it comes first.
+  static constexpr bool kC2First = kStages == 1;
+  static constexpr int kC1Full = 0;                    // [kStages] tile converted (8 warps)
   static constexpr int kC2Full = kC1Full + kStages;
   static constexpr int kC1Empty = kC2Full + kStages;   // [kStages] every product that reads the tile is complete
   static constexpr int kC2Empty = kC1Empty + kStages;
@@ -94,7 +113,9 @@ struct TcShape {
   static constexpr int kOut2Full = kOut1Full + 1;      // [kOuts]
   static constexpr int kOut1Free = kOut2Full + 2;      // output added to the registers (16 warps)
   static constexpr int kOut2Free = kOut1Free + 1;      // [kOuts]
-  static constexpr int kNumBars = kOut2Free + 2;
+  static constexpr int kSlotFree = kOut2Free + 2;      // [kSlots] output product that reads the slot complete
+  static constexpr int kDpFree = kSlotFree + kSlots;   // both outputs: the same for the slot of dP / dS
+  static constexpr int kNumBars = kDpFree + 1;
   static constexpr int kMiscOff = kBarOff + 8 * kNumBars;
   // (the FMA code reuses the space from the start)
   using Fallback = F32Shape<D, 4, 4>;
@@ -109,13 +130,23 @@ template <int N>
 __device__ __forceinline__ void tc_split(const float (&x)[2 * N], uint32_t (&p0)[N], uint32_t (&p1)[N], uint32_t (&p2)[N]) {
 #pragma unroll
   for (int i = 0; i < N; ++i) {
+    const float2 minus = make_float2(-1.0f, -1.0f);  // (packed operations have no negated operands)
     float2 r = make_float2(x[2 * i], x[2 * i + 1]);
     p0[i] = pack2<true>(r.x, r.y);
-    r = __fadd2_rn(r, make_float2(-__uint_as_float(p0[i] << 16), -__uint_as_float(p0[i] & 0xffff0000u)));
+    r = __ffma2_rn(make_float2(__uint_as_float(p0[i] << 16), __uint_as_float(p0[i] & 0xffff0000u)), minus, r);
     p1[i] = pack2<true>(r.x, r.y);
-    r = __fadd2_rn(r, make_float2(-__uint_as_float(p1[i] << 16), -__uint_as_float(p1[i] & 0xffff0000u)));
+    r = __ffma2_rn(make_float2(__uint_as_float(p1[i] << 16), __uint_as_float(p1[i] & 0xffff0000u)), minus, r);
     p2[i] = pack2<true>(r.x, r.y);
   }
+}
+
+// Two sigmoids 1 / (1 + u), u = e^-x = 2^-y * factor: the bias is in the factor, e^-bias, so that y, which is rounded, is as
+// small as the scaled score.  (With the bias in y, as in the FMA kernels' logits, this rounding is most of the error of O: T=2048
+// 3.6e-7, T=256 causal dQ 3.6e-7.)  Infinite u gives 0, as it should.
+__device__ __forceinline__ float2 tc_sigmoid2(float2 minus_y, float factor) {
+  const float2 e = make_float2(ex2_approx(minus_y.x), ex2_approx(minus_y.y));
+  const float2 d = __ffma2_rn(e, make_float2(factor, factor), make_float2(1.0f, 1.0f));
+  return make_float2(rcp_approx(d.x), rcp_approx(d.y));
 }
 
 template <int D, int kMode>
@@ -189,7 +220,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
       mbar_init(bar(L::kDpFull + i), 1);
       mbar_init(bar(L::kPReady + i), kTcComputeWarps);
       mbar_init(bar(L::kDsReady + i), kTcComputeWarps);
+      mbar_init(bar(L::kSlotFree + i), 1);
     }
+    mbar_init(bar(L::kDpFree), 1);
     mbar_init(bar(L::kOut1Full), 1);
     mbar_init(bar(L::kOut1Free), kTcComputeWarps);
     for (int i = 0; i < 2; ++i) {
@@ -198,7 +231,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
     }
     fence_mbar_init();
   }
-  if (warp == kTcIssuerWarp) {
+  if (warp == kTcIssuerIn) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
     tmem_relinquish();
   }
@@ -213,192 +246,183 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
   const float* do_base = !p.dout ? nullptr
                                          : p.dout + (int64_t)it.bc * p.do_sb + (int64_t)it.h * p.do_sh + (int64_t)it.tq0 * p.do_st;
 
-  if (warp >= kTcIssuerWarp) {
-    // ============================================================ issuer
-    setmaxnreg_dec<48>();
-    if (warp == kTcIssuerWarp) {
-      asm volatile("bar.sync 9, %0;" ::"n"(32 * kTcComputeWarps + 32) : "memory");  // R has been written
+  constexpr int kRReady = 9;  // named barrier: the R operands have been written
+  constexpr int kRReadyThreads = 32 * (kTcComputeWarps + 1);
+  if (warp >= kTcIssuerIn) {
+    // ============================================================ issuers
+    setmaxnreg_dec<kTcIssuerRegs>();
+    const bool leader = elect_one();
+    constexpr uint32_t kStage16 = L::kCTile >> 4;
+    auto stage16 = [](int j) -> uint32_t { return (uint32_t)(j % L::kStages) * kStage16; };
+    // the six products, small terms first
+    constexpr int kA[6] = {2, 1, 0, 1, 0, 0}, kB[6] = {0, 1, 2, 0, 1, 0};
+    bool ok = true;
+    auto wait = [&](int b, int n_th, int site) {  // completion number n_th (from 0) of a barrier
+      ok = ok && mbar_wait_warp(bar(b), (uint32_t)n_th & 1u, abort_flag, kSite + site);
+    };
+    if (warp == kTcIssuerIn) {
+      asm volatile("bar.sync %0, %1;" ::"n"(kRReady), "n"(kRReadyThreads) : "memory");
       tc_fence_after_sync();
-      const bool leader = elect_one();
       constexpr uint32_t id_in = make_idesc(128, kTcJob, true, false, false);
-      const uint32_t id_out = make_idesc(128, 0, true, false, true) | (uint32_t)(n16 * 2) << 17;  // N = 16 n16
       const uint64_t c1_d = smem_desc_sw128(smem_base + L::kC1Off, 16, 1024);
-      const uint32_t hi = (uint32_t)(c1_d >> 32);
-      const uint32_t c1_in = (uint32_t)c1_d;
-      const uint32_t c2_in = (uint32_t)smem_desc_sw128(smem_base + L::kC2Off, 16, 1024);
-      const uint32_t r2_in = (uint32_t)smem_desc_sw128(smem_base, 16, 1024);
-      const uint32_t c1_out = (uint32_t)smem_desc_sw128(smem_base + L::kC1Off, kTcJob * 128, 1024);
-      const uint32_t c2_out = (uint32_t)smem_desc_sw128(smem_base + L::kC2Off, kTcJob * 128, 1024);
-      constexpr uint32_t kStage16 = L::kCTile >> 4;
-      // the six products, small terms first
-      constexpr int kA[6] = {2, 1, 0, 1, 0, 0}, kB[6] = {0, 1, 2, 0, 1, 0};
-      // scores: A = R1 in TMEM / R2 in TMEM or shared memory, B = a streamed tile, K = head dimension
-      auto in_ts = [&](uint32_t dcol, uint32_t acol, uint32_t b_lo) {
+      const uint32_t c1 = (uint32_t)c1_d, hi = (uint32_t)(c1_d >> 32);
+      const uint32_t c2 = c1 + ((L::kC2Off - L::kC1Off) >> 4), r2 = (uint32_t)smem_desc_sw128(smem_base, 16, 1024);
+      // A = R1 in TMEM / R2 in TMEM or shared memory, B = a streamed tile, K = head dimension
+      auto products = [&](uint32_t dcol, uint32_t a0, uint32_t b0, auto smem_a, auto steps) {
+        const int n = decltype(steps)::value ? decltype(steps)::value : n16;
 #pragma unroll
         for (int t = 0; t < 6; ++t)
-          for (int kk = 0; kk < n16; ++kk)
-            mma_ts(leader, tmem + dcol, tmem + acol + kA[t] * L::kPartCols + 8 * kk,
-                   make_desc(b_lo + kB[t] * (L::kCPart >> 4) + (kk >> 2) * (kTcJob * 128 >> 4) + (kk & 3) * 2, hi), id_in,
-                   t > 0 || kk > 0);
-      };
-      auto in_ss = [&](uint32_t dcol, uint32_t a_lo, uint32_t b_lo) {
 #pragma unroll
-        for (int t = 0; t < 6; ++t)
-          for (int kk = 0; kk < n16; ++kk)
-            mma_ss(leader, tmem + dcol,
-                   make_desc(a_lo + kA[t] * (L::kRPart >> 4) + (kk >> 2) * (kTcRows * 128 >> 4) + (kk & 3) * 2, hi),
-                   make_desc(b_lo + kB[t] * (L::kCPart >> 4) + (kk >> 2) * (kTcJob * 128 >> 4) + (kk & 3) * 2, hi), id_in,
-                   t > 0 || kk > 0);
+          for (int kk = 0; kk < n; ++kk) {
+            const uint64_t b = make_desc(b0 + kB[t] * (L::kCPart >> 4) + (kk >> 2) * (kTcJob * 128 >> 4) + (kk & 3) * 2, hi);
+            if constexpr (decltype(smem_a)::value)
+              mma_ss(leader, tmem + dcol, make_desc(a0 + kA[t] * (L::kRPart >> 4) + (kk >> 2) * (kTcRows * 128 >> 4) + (kk & 3) * 2, hi),
+                     b, id_in, t > 0 || kk > 0);
+            else
+              mma_ts(leader, tmem + dcol, tmem + a0 + kA[t] * L::kPartCols + 8 * kk, b, id_in, t > 0 || kk > 0);
+          }
       };
-      // outputs of a job: A = P or dS in a slot, B = the streamed tile, K = its 64 rows
-      auto out = [&](uint32_t dcol, uint32_t slot_col, uint32_t b_lo) {
+      auto issue = [&](uint32_t dcol, uint32_t a0, uint32_t b0, auto smem_a) {
+        if (n16 == D / 16) products(dcol, a0, b0, smem_a, std::integral_constant<int, D / 16>());
+        else products(dcol, a0, b0, smem_a, std::integral_constant<int, 0>());
+      };
+      for (int j = 0; j < n_jobs && ok; ++j) {
+        const int sl = j % L::kSlots, st = j % L::kStages;
+        if (j >= L::kSlots) wait(L::kSlotFree + sl, j / L::kSlots - 1, 7);
+        auto scores = [&]() {
+          wait(L::kC1Full + st, j / L::kStages, 1);
+          if (!ok) return;
+          tc_fence_after_sync();
+          issue(L::kSCol + sl * L::kSlotCols, L::kR1Col, c1 + stage16(j), std::false_type());
+          mma_commit(leader, bar(L::kSFull + sl));
+          if (!L::kOut1) mma_commit(leader, bar(L::kC1Empty + st));
+        };
+        if constexpr (!L::kC2First) scores();
+        if constexpr (L::kOut1) {
+          wait(L::kC2Full + st, j / L::kStages, 2);
+          if (L::kBoth && j > 0) wait(L::kDpFree, j - 1, 8);
+          if (!ok) break;
+          tc_fence_after_sync();
+          issue(L::kBoth ? L::kDpCol : L::kDpCol + sl * L::kSlotCols, L::kR2Smem ? r2 : L::kR2Col, c2 + stage16(j),
+                std::bool_constant<L::kR2Smem>());
+          mma_commit(leader, bar(L::kDpFull + (L::kBoth ? 0 : sl)));
+          if (!L::kOut2) mma_commit(leader, bar(L::kC2Empty + st));
+        }
+        if constexpr (L::kC2First) scores();
+      }
+    } else if (warp == kTcIssuerOut) {
+      const uint32_t id_out = make_idesc(128, 0, true, false, true) | (uint32_t)(n16 * 2) << 17;  // N = 16 n16
+      const uint64_t c1_d = smem_desc_sw128(smem_base + L::kC1Off, kTcJob * 128, 1024);
+      const uint32_t c1 = (uint32_t)c1_d, hi = (uint32_t)(c1_d >> 32);
+      const uint32_t c2 = c1 + ((L::kC2Off - L::kC1Off) >> 4);
+      // A = P or dS in a slot, B = the streamed tile, K = its 64 rows
+      auto issue = [&](uint32_t dcol, uint32_t slot_col, uint32_t b0) {
 #pragma unroll
         for (int t = 0; t < 6; ++t)
 #pragma unroll
           for (int kk = 0; kk < kTcJob / 16; ++kk)
             mma_ts(leader, tmem + dcol,
                    tmem + slot_col + (kA[t] < 2 ? 16 * kk + 8 * kA[t] : L::kPart2Col + L::kPart2Step * kk),
-                   make_desc(b_lo + kB[t] * (L::kCPart >> 4) + kk * (2048 >> 4), hi), id_out, t > 0 || kk > 0);
+                   make_desc(b0 + kB[t] * (L::kCPart >> 4) + kk * (2048 >> 4), hi), id_out, t > 0 || kk > 0);
       };
-      bool ok = true;
-      auto wait = [&](int b, int n_th, int site) {  // completion number n_th (from 0) of a barrier
-        ok = ok && mbar_wait_warp(bar(b), (uint32_t)n_th & 1u, abort_flag, kSite + site);
-        tc_fence_after_sync();
-      };
-      auto stage16 = [&](int j) -> uint32_t { return (uint32_t)(j % L::kStages) * kStage16; };
-      auto scores = [&](int j) {
-        wait(L::kC1Full + j % L::kStages, j / L::kStages, 1);
-        if (!ok) return;
-        in_ts(L::kSCol + (j % L::kSlots) * L::kSlotCols, L::kR1Col, c1_in + stage16(j));
-        mma_commit(leader, bar(L::kSFull + j % L::kSlots));
-        if (!L::kOut1) mma_commit(leader, bar(L::kC1Empty + j % L::kStages));
-      };
-      auto dscores = [&](int j) {
-        wait(L::kC2Full + j % L::kStages, j / L::kStages, 2);
-        if (!ok) return;
-        const uint32_t dcol = L::kDpCol + (!L::kBoth ? (j % L::kSlots) * L::kSlotCols : 0);
-        if constexpr (L::kR2Smem) in_ss(dcol, r2_in, c2_in + stage16(j));
-        else in_ts(dcol, L::kR2Col, c2_in + stage16(j));
-        mma_commit(leader, bar(L::kDpFull + (!L::kBoth ? j % L::kSlots : 0)));
-        if (!L::kOut2) mma_commit(leader, bar(L::kC2Empty + j % L::kStages));
-      };
-      auto out2 = [&](int j) {
-        const int b = j % L::kOuts;
-        wait(L::kPReady + j % L::kSlots, j / L::kSlots, 3);
-        if (!L::kOut1) wait(L::kC2Full + j % L::kStages, j / L::kStages, 2);
-        if (j >= L::kOuts) wait(L::kOut2Free + b, j / L::kOuts - 1, 4);
-        if (!ok) return;
-        out(L::kOut2Col + b * D, L::kSCol + (j % L::kSlots) * L::kSlotCols, c2_out + stage16(j));
-        mma_commit(leader, bar(L::kOut2Full + b));
-        mma_commit(leader, bar(L::kC2Empty + j % L::kStages));
-      };
-      auto out1 = [&](int j) {
-        const int s = !L::kBoth ? j % L::kSlots : 0;
-        wait(L::kDsReady + s, !L::kBoth ? j / L::kSlots : j, 5);
-        if (j > 0) wait(L::kOut1Free, j - 1, 6);
-        if (!ok) return;
-        out(L::kOut1Col, (!L::kBoth ? L::kSCol : L::kDpCol) + s * L::kSlotCols, c1_out + stage16(j));
-        mma_commit(leader, bar(L::kOut1Full));
-        mma_commit(leader, bar(L::kC1Empty + j % L::kStages));
-      };
-      // A slot's scores may be overwritten when the output products that read the P / dS written over them are complete.
-      if constexpr (!L::kOut1) {
-        scores(0);
-        for (int j = 0; j < n_jobs && ok; ++j) {
-          if (j + 1 < n_jobs) {
-            const int f = j + 1 - L::kSlots;
-            if (f >= 0) wait(L::kOut2Full + f % L::kOuts, f / L::kOuts, 7);
-            if (ok) scores(j + 1);
-          }
-          if (ok) out2(j);
+      // (the scores of job j are complete, and with them what they read, when its P or dS are ready)
+      for (int j = 0; j < n_jobs && ok; ++j) {
+        const int sl = j % L::kSlots, st = j % L::kStages;
+        if constexpr (L::kOut2) {
+          const int b = j % L::kOuts;
+          wait(L::kC2Full + st, j / L::kStages, 2);
+          wait(L::kPReady + sl, j / L::kSlots, 3);
+          if (j >= L::kOuts) wait(L::kOut2Free + b, j / L::kOuts - 1, 4);
+          if (!ok) break;
+          tc_fence_after_sync();
+          issue(L::kOut2Col + b * D, L::kSCol + sl * L::kSlotCols, c2 + stage16(j));
+          mma_commit(leader, bar(L::kOut2Full + b));
+          mma_commit(leader, bar(L::kSlotFree + sl));
+          if (!L::kBoth) mma_commit(leader, bar(L::kC2Empty + st));
         }
-      } else if constexpr (L::kBoth) {
-        scores(0);
-        if (ok) dscores(0);
-        for (int j = 0; j < n_jobs && ok; ++j) {
-          if (j + 1 < n_jobs) {
-            if (j > 0) wait(L::kOut2Full, j - 1, 7);
-            if (ok) scores(j + 1);
-          }
-          if (ok) out2(j);
-          if (ok) out1(j);
-          if (j + 1 < n_jobs) {
-            wait(L::kOut1Full, j, 8);
-            if (ok) dscores(j + 1);
-          }
-        }
-      } else {
-        constexpr int kAhead = L::kSlots - 1;
-        if (kAhead) {
-          scores(0);
-          if (ok) dscores(0);
-        }
-        for (int j = 0; j < n_jobs && ok; ++j) {
-          const int n = j + kAhead;
-          if (n < n_jobs) {
-            if (n >= L::kSlots) wait(L::kOut1Full, n - L::kSlots, 7);
-            if (ok) scores(n);
-            if (ok) dscores(n);
-          }
-          if (ok) out1(j);
+        if constexpr (L::kOut1) {
+          wait(L::kDsReady + (L::kBoth ? 0 : sl), L::kBoth ? j : j / L::kSlots, 5);
+          if (j > 0) wait(L::kOut1Free, j - 1, 6);
+          if (!ok) break;
+          tc_fence_after_sync();
+          if (L::kBoth) mma_commit(leader, bar(L::kC2Empty + st));  // (dP of the job is complete too, else dS were not)
+          issue(L::kOut1Col, L::kBoth ? L::kDpCol : L::kSCol + sl * L::kSlotCols, c1 + stage16(j));
+          mma_commit(leader, bar(L::kOut1Full));
+          mma_commit(leader, bar(L::kBoth ? L::kDpFree : L::kSlotFree + sl));
+          mma_commit(leader, bar(L::kC1Empty + st));
         }
       }
     }
   } else if (warp >= kTcComputeWarps) {
     // ============================================================ conversion of the streamed rows
-    // A chunk is 64 rows x 64 columns of one tensor; a thread takes 8 consecutive columns of four of its rows.  The loads of
-    // the next chunk are issued as the registers of this one become free.  (This group keeps the 80 registers of the launch.)
+    // A chunk is 64 rows x 64 columns of one tensor; a thread takes 4 consecutive columns of four of its rows, a warp whole
+    // rows at a time.  What a thread converts it has fetched itself, kRing - 1 chunks ahead, by asynchronous copies into places
+    // of its own (neighbours adjacent): no synchronisation, no registers held for loads in flight.
+    setmaxnreg_dec<kTcConvRegs>();
     const int wc = warp - kTcComputeWarps;
-    const int rr = 4 * wc + (lane >> 3), c8 = lane & 7;
-    const float* src1 = (L::kKeyRows ? q_base : k_base) + 8 * c8;
-    const float* src2 = (L::kKeyRows ? do_base : v_base) + 8 * c8;
-    const int64_t st1 = L::kKeyRows ? p.q_st : p.k_st, st2 = L::kKeyRows ? p.do_st : p.v_st;
+    const int rr = 2 * wc + (lane >> 4), c4 = lane & 15;
     constexpr int kHalves = D / 64;
     const int n_chunks = n_jobs * 2 * kHalves;
-    float4 x[4][2];
-    auto load = [&](int chunk, int u) {
-      const int j = chunk / (2 * kHalves), half = chunk % kHalves;
-      const bool second = (chunk / kHalves) & 1;
-      const int r = c_begin + j * kTcJob + 16 * u + rr, c = 64 * half + 8 * c8;
-      const float* s = (second ? src2 + r * st2 : src1 + r * st1) + 64 * half;
-      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-      const bool live = chunk < n_chunks && r < Lc;
-      x[u][0] = live && c < p.d_cols ? __ldg(reinterpret_cast<const float4*>(s)) : zero;
-      x[u][1] = live && c + 4 < p.d_cols ? __ldg(reinterpret_cast<const float4*>(s) + 1) : zero;
+    const int64_t st1 = L::kKeyRows ? p.q_st : p.k_st, st2 = L::kKeyRows ? p.do_st : p.v_st;
+    const float* src1 = (L::kKeyRows ? q_base : k_base) + (c_begin + rr) * st1 + 4 * c4;
+    const float* src2 = (L::kKeyRows ? do_base : v_base) + (c_begin + rr) * st2 + 4 * c4;
+    uint8_t* mine = smem_gen + L::kRingOff + (threadIdx.x & 255) * 16;
+    auto second = [](int chunk) -> bool { return (((chunk / kHalves) & 1) != 0) != L::kC2First; };
+    auto fetch = [&](int chunk) {
+      if (chunk < n_chunks) {
+        const int j = chunk / (2 * kHalves), half = chunk % kHalves;
+        const bool two = second(chunk);
+        const int64_t step = two ? 16 * st2 : 16 * st1;
+        const float* src = (two ? src2 : src1) + 4 * j * step + 64 * half;
+        const int rows = Lc - (c_begin + j * kTcJob + rr);  // from this thread's first one
+        const bool in_head = 64 * half + 4 * c4 < p.d_cols;
+        float* dst = reinterpret_cast<float*>(mine + (chunk % L::kRing) * L::kChunk);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          f32_cp16(dst + u * 1024, src, in_head && 16 * u < rows);
+          src += step;
+        }
+      }
+      f32_commit();
     };
 #pragma unroll
-    for (int u = 0; u < 4; ++u) load(0, u);
+    for (int i = 0; i < L::kRing - 1; ++i) fetch(i);
     bool ok = true;
     for (int chunk = 0; chunk < n_chunks; ++chunk) {
       const int j = chunk / (2 * kHalves), half = chunk % kHalves;
-      const bool second = (chunk / kHalves) & 1;
+      const bool two = second(chunk);
       const int st = j % L::kStages;
+      fetch(chunk + L::kRing - 1);
+      f32_wait<L::kRing - 1>();
       if (half == 0 && j >= L::kStages) {
-        ok = mbar_wait_warp(bar((second ? L::kC2Empty : L::kC1Empty) + st), (uint32_t)(j / L::kStages - 1) & 1u, abort_flag, kSite + 9);
+        ok = mbar_wait_warp(bar((two ? L::kC2Empty : L::kC1Empty) + st), (uint32_t)(j / L::kStages - 1) & 1u, abort_flag, kSite + 9);
         if (!ok) break;
       }
-      uint8_t* tile = smem_gen + (second ? L::kC2Off : L::kC1Off) + st * L::kCTile + half * (kTcJob * 128) + rr * 128 +
-                      ((c8 ^ (rr & 7)) << 4);
+      const float4* got = reinterpret_cast<const float4*>(mine + (chunk % L::kRing) * L::kChunk);
+      // (row 16 u + rr: its place in the swizzle, rr & 7, is the same for every u)
+      uint8_t* tile = smem_gen + (two ? L::kC2Off : L::kC1Off) + st * L::kCTile + half * (kTcJob * 128) + rr * 128 +
+                      (((c4 >> 1) ^ (rr & 7)) << 4) + 8 * (c4 & 1);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const float f[8] = {x[u][0].x, x[u][0].y, x[u][0].z, x[u][0].w, x[u][1].x, x[u][1].y, x[u][1].z, x[u][1].w};
-        uint32_t p0[4], p1[4], p2[4];
-        tc_split<4>(f, p0, p1, p2);
-        load(chunk + 1, u);
+        const float4 x = got[u * 256];
+        const float f[4] = {x.x, x.y, x.z, x.w};
+        uint32_t p0[2], p1[2], p2[2];
+        tc_split<2>(f, p0, p1, p2);
         uint8_t* dst = tile + u * 2048;
-        *reinterpret_cast<uint4*>(dst) = make_uint4(p0[0], p0[1], p0[2], p0[3]);
-        *reinterpret_cast<uint4*>(dst + L::kCPart) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
-        *reinterpret_cast<uint4*>(dst + 2 * L::kCPart) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+        *reinterpret_cast<uint2*>(dst) = make_uint2(p0[0], p0[1]);
+        *reinterpret_cast<uint2*>(dst + L::kCPart) = make_uint2(p1[0], p1[1]);
+        *reinterpret_cast<uint2*>(dst + 2 * L::kCPart) = make_uint2(p2[0], p2[1]);
       }
       if (half == kHalves - 1) {
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar((second ? L::kC2Full : L::kC1Full) + st));
+        if (lane == 0) mbar_arrive(bar((two ? L::kC2Full : L::kC1Full) + st));
       }
     }
+    f32_wait<0>();  // (the fallback of the compute warps reuses the space)
   } else {
     // ============================================================ compute
-    setmaxnreg_inc<88>();
+    setmaxnreg_inc<kTcComputeRegs>();
     const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
     // ------------------------------------------------------------ R: this thread's row, columns [cg D/4, +D/4)
     auto split_rows = [&](const float* base, int64_t st, bool to_smem, int col) {
@@ -436,11 +460,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
     tmem_st_wait();
     fence_proxy_async_smem();
     tc_fence_before_sync();
-    asm volatile("bar.arrive 9, %0;" ::"n"(32 * kTcComputeWarps + 32) : "memory");
+    asm volatile("bar.arrive %0, %1;" ::"n"(kRReady), "n"(kRReadyThreads) : "memory");
 
-    float bias = item_bias(p.bias, p.bias_scalar, it.b, it.Lk);
+    constexpr float kLog2 = 1.4426950408889634f;
     const float* sm = p.score_mod ? p.score_mod + it.sm_off : nullptr;
     const float row_mod = L::kKeyRows && sm && row < it.key_lim ? sm[row] : 0.f;
+    // a bias between 0 and -44 is a factor (2^64 at most: nothing overflows that the sigmoid does not send to 0 or 1), what is
+    // beyond that remains in the exponent
+    const float bias = item_bias(p.bias, p.bias_scalar, it.b, it.Lk) + row_mod;
+    const float bias_in = fminf(fmaxf(bias, -44.0f), 0.0f);
+    const float factor = expf(-bias_in), y1 = -p.scale * kLog2, y0 = (bias_in - bias) * kLog2;
+    const float* col_mod = L::kKeyRows ? nullptr : sm;
     const int lo = L::kKeyRows && p.causal ? row : 0;  // visible columns of this row: [lo, hi)
     const int hi = !L::kKeyRows && p.causal ? min(Lc, row + 1) : Lc;
 
@@ -508,10 +538,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
         tmem_ld(slot + 16 * cg, r);
         tmem_ld_wait_for(r);
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          float x = __uint_as_float(r[c]) * p.scale + bias;
-          if (sm) x += L::kKeyRows ? row_mod : (col0 + c < it.key_lim ? __ldg(sm + col0 + c) : 0.f);
-          pr[c] = f32_sigmoid(x);
+        for (int c = 0; c < 16; c += 2) {
+          float2 y = __ffma2_rn(make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])), make_float2(y1, y1), make_float2(y0, y0));
+          if (col_mod) {
+            y.x = fmaf(col0 + c < it.key_lim ? __ldg(col_mod + col0 + c) : 0.f, -kLog2, y.x);
+            y.y = fmaf(col0 + c + 1 < it.key_lim ? __ldg(col_mod + col0 + c + 1) : 0.f, -kLog2, y.y);
+          }
+          const float2 w = tc_sigmoid2(y, factor);
+          pr[c] = w.x;
+          pr[c + 1] = w.y;
         }
         if (mask) {
 #pragma unroll
@@ -532,9 +567,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
         tmem_ld((!L::kBoth ? slot + 64 : dslot) + 16 * cg, r);
         tmem_ld_wait_for(r);
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          const float ds = pr[c] * (1.0f - pr[c]) * __uint_as_float(r[c]);
-          pr[c] = !mask || (col0 + c >= lo && col0 + c < hi) ? ds : 0.f;
+        for (int c = 0; c < 16; c += 2) {
+          const float2 w = make_float2(pr[c], pr[c + 1]);
+          const float2 v = __ffma2_rn(w, make_float2(-1.0f, -1.0f), make_float2(1.0f, 1.0f));
+          const float2 ds = __fmul2_rn(__fmul2_rn(w, v), make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])));
+          pr[c] = ds.x;
+          pr[c + 1] = ds.y;
+        }
+        if (mask) {
+#pragma unroll
+          for (int c = 0; c < 16; ++c) pr[c] = col0 + c >= lo && col0 + c < hi ? pr[c] : 0.f;
         }
         put(dslot, pr);
         arrive(L::kDsReady + (!L::kBoth ? s : 0));
@@ -571,7 +613,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
   // ---------------------------------------------------------------- teardown
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == kTcIssuerWarp) {
+  if (warp == kTcIssuerIn) {
     tc_fence_after_sync();
     tmem_dealloc(tmem, 512);
   }

@@ -601,13 +601,23 @@ int launch_f32_tc(const SigAttnParams* p, const sigattn::F32Params& fp) {
   return 0;
 }
 
-// Whether float32 tensors take the tensor-core kernels: whose tiles of 128 rows need long sequences, or many of them, to pay.
-// Forward and backward, FMA kernels -> these: D=64 B=1 H=4 T=512 26 and 87 us -> 27 and 95, T=1000 57 and 183 -> 43 and 158; B=4 H=3
-// T=777 106 and 258 -> 43 and 143; B=2 H=4 T=256 16 and 67 -> 19 and 68; D=32 B=2 H=4 T=512 30 and 95 -> 24 and 82; D=128 B=1 H=4 T=512
-// 37 and 127 -> 40 and 178, T=2048 257 and 864 -> 120 and 566.
-bool f32_tc(const SigAttnParams* p) {
-  const int shorter = std::min(p->Tq, p->Tk);
-  return shorter >= 768 || (shorter >= 256 && (int64_t)p->B * p->H * ((shorter + 63) / 64) >= 64);
+// Whether float32 tensors take the tensor-core kernels.  Their tiles have 128 rows, and setting one up takes as long as two of
+// its steps of 64: so they need enough 64-row tiles to occupy half of the SMs (in a forward of the queries, in a backward of
+// queries and keys on average), or sequences that are long enough for the faster steps to pay even where 16-row tiles of the
+// FMA kernels would occupy more of the chip.  Device time of these over FMA kernels, from 477 shapes (means over those that
+// differ in B H only):
+//  - D = 64 forward: T=256, 64 tiles or more 0.42 - 0.77, fewer 1.08; T=512 0.31 - 0.88, T=1024 0.25 - 0.75; backward T=384 0.30 - 0.80,
+//    T=1024 0.22 - 0.63.  Heads of 32 columns, which get the same kernels (and the same bits as heads filled up with zeros):
+//    T=512 0.37 - 1.01, backward T=384 0.40 - 1.04.
+//  - D = 128 forward: T=256 0.36 - 0.69 from 148 tiles on, 0.88 at 64 and 1.05 there with a causal mask, 1.3 below; Tk = 512 0.98;
+//    backward (three kernels): 0.35 - 0.71 from 96 tiles on, 0.76 - 0.89 at 64 with T >= 512 (causal 0.94 - 1.06), 1.1 - 1.6 below.
+//  - below 256 rows on both sides 0.5 - 2.2, and below 64 keys or 16 queries mostly padding: FMA kernels.
+bool f32_tc(const SigAttnParams* p, bool backward) {
+  const int64_t Tq = p->Tq, Tk = p->Tk, longer = std::max(Tq, Tk);
+  if (Tk < 64 || Tq < 16 || longer < 256) return false;
+  const int64_t tiles = (int64_t)p->B * p->H * (((backward ? (Tq + Tk) / 2 : Tq) + 63) / 64);
+  if (p->D == 128) return backward ? tiles >= 96 || (tiles >= 64 && longer >= 512) : tiles >= 72 || Tk >= 512;
+  return tiles >= 64 || longer >= (backward ? 384 : 512);
 }
 
 // Rows per CTA: 64 once such tiles occupy half of the SMs; below that 16, with four times the threads per row, which take
@@ -654,7 +664,7 @@ int launch_f32_d(const SigAttnParams* p, bool backward) {
   if (int rc = fwd_device_info(p->device, &info)) return rc;
   if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
   int rc = 0;
-  if (f32_tc(p)) {
+  if (f32_tc(p, backward)) {
     if (!backward) {
       rc = launch_f32_tc<D, kTcFwd>(p, fp);
     } else {
@@ -730,7 +740,7 @@ int sigattn_form(const SigAttnParams* p, int backward, int n_sm) {
   if (p->struct_bytes != sizeof(SigAttnParams)) return fail(-1, "struct_bytes %u != sizeof(SigAttnParams) %zu (ABI mismatch)", p->struct_bytes, sizeof(SigAttnParams));
   if (n_sm < 1) return fail(-2, "n_sm must be positive, got %d", n_sm);
   if (p->dtype == SIGATTN_FP32) {
-    if (f32_tc(p)) return SIGATTN_FORM_F32_TC;
+    if (f32_tc(p, backward != 0)) return SIGATTN_FORM_F32_TC;
     return f32_tile_rows(p, n_sm) == 64 ? SIGATTN_FORM_F32_64 : SIGATTN_FORM_F32_16;
   }
   if (!backward) return fwd_split(p, n_sm) ? SIGATTN_FORM_FWD_SPLIT : SIGATTN_FORM_FWD;
