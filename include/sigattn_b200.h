@@ -68,6 +68,9 @@ enum SigAttnFlags {
    * few small tensor kernels before the launch); `bias` and `bias_scalar` are ignored.  An element without
    * keys gets +inf, where every probability is masked anyway. */
   SIGATTN_BIAS_NEG_LOG_LK = 1u << 3,
+  /* Packed layout, at least one sequence: rows of the outputs that belong to no sequence (see cu_seqlens_q below) are written as
+   * zeros instead of being left untouched.  The outputs must be contiguous. */
+  SIGATTN_ZERO_GAPS = 1u << 4,
 };
 
 enum SigAttnQuery {

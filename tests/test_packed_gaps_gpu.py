@@ -1,0 +1,61 @@
+"""Rows of packed tensors that belong to no sequence are zero in every output, whatever the memory held before: in front of the
+first sequence, behind the last one, and rows of a sequence beyond the given maximum."""
+
+import pytest
+import torch
+
+import triton_sigmoid_b200 as sa
+from tests.gpu_util import launch_form
+from triton_sigmoid_b200._cabi import FORM_BWD, FORM_BWD_BY_HEAD
+
+pytestmark = pytest.mark.gpu
+
+
+def _poison(shape, dtype):
+    """Memory of this size goes back to the allocator full of NaN, for the outputs to be made from."""
+    keep = [torch.full(shape, float("nan"), dtype=dtype, device="cuda") for _ in range(4)]
+    del keep
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("n,H,D,dtype,form", [
+    (3, 2, 64, torch.bfloat16, FORM_BWD),            # fewer items than SMs: a fill before the kernels
+    (40, 8, 64, torch.float16, FORM_BWD),            # zeroed by the kernels
+    (40, 8, 128, torch.bfloat16, FORM_BWD),
+    (40, 8, 24, torch.bfloat16, FORM_BWD),
+    (260, 8, 64, torch.bfloat16, FORM_BWD_BY_HEAD),
+    (6, 2, 64, torch.float32, None),
+])
+def test_rows_outside_the_sequences(n, H, D, dtype, form, split, monkeypatch):
+    T, cut, front, behind = 300, 260, 37, 1000
+    if split:
+        monkeypatch.setenv("SIGATTN_B200_BWD_SPLIT", "1")
+    g = torch.Generator().manual_seed(n)
+    lens = torch.randint(T // 2, T + 1, (n,), generator=g)
+    lens[0], lens[n // 2], lens[-1] = T, 0, T
+    cu = torch.cat([torch.zeros(1, dtype=torch.long), lens.cumsum(0)]) + front
+    rows = int(cu[-1]) + behind
+    if form is not None:
+        assert launch_form(n, H, cut, cut, D, dtype, True, packed_rows=rows) == form
+    at = torch.arange(rows)
+    seq = (torch.searchsorted(cu, at, right=True) - 1).clamp(0, n - 1)
+    inside = ((at >= front) & (at < cu[-1]) & (at - cu[seq] < cut)).cuda()
+    cu = cu.int().cuda()
+    leaf = [(torch.randn(rows, H, D, device="cuda") * 0.5).to(dtype).requires_grad_() for _ in range(3)]
+    do = torch.randn(rows, H, D, device="cuda").to(dtype)
+    _poison((rows, H, D), dtype)
+    out = sa.sigmoid_attention_varlen(*leaf, cu, cu, cut, cut)
+    _poison((rows, H, D), dtype)
+    for t in (out,) + torch.autograd.grad(out, leaf, do):
+        assert (t[~inside] == 0).all() and t.isfinite().all()
+        assert (t[inside] != 0).any(dim=-1).all()
+
+
+def test_no_sequences_at_all():
+    leaf = [torch.randn(500, 2, 64, device="cuda", dtype=torch.float16).requires_grad_() for _ in range(3)]
+    cu = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _poison((500, 2, 64), torch.float16)
+    out = sa.sigmoid_attention_varlen(*leaf, cu, cu, 64, 64)
+    _poison((500, 2, 64), torch.float16)
+    for t in (out,) + torch.autograd.grad(out, leaf, torch.ones_like(out)):
+        assert (t == 0).all()

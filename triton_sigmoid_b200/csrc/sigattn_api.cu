@@ -138,6 +138,26 @@ int zero_fill(void* ptr, const int64_t* strides, int B, int T, int H, int D, int
   return 0;
 }
 
+// SIGATTN_ZERO_GAPS, where the kernel does not do it on the way: the whole output (before the kernel writes the sequences).
+int zero_gaps_first(const SigAttnParams* p, void* ptr, const int64_t* strides, int total, const char* name) {
+  if (!(p->flags & SIGATTN_ZERO_GAPS) || !p->cu_seqlens_q) return 0;
+  const int D = head_cols(p);
+  const Strides3 s = map_strides(strides, total, true);
+  if (!is_contiguous(s.s, total > 0 ? total : 1, p->H, D)) return fail(-2, "%s: SIGATTN_ZERO_GAPS needs contiguous outputs", name);
+  return zero_fill(ptr, s.s, 1, total, p->H, D, p->dtype, static_cast<cudaStream_t>(p->stream), name);
+}
+int zero_grad_gaps_first(const SigAttnParams* p) {
+  if (int rc = zero_gaps_first(p, p->dq, p->dq_strides, p->total_q, "dq")) return rc;
+  if (int rc = zero_gaps_first(p, p->dk, p->dk_strides, p->total_k, "dk")) return rc;
+  return zero_gaps_first(p, p->dv, p->dv_strides, p->total_k, "dv");
+}
+// The spare warps of the 16-bit kernels zero the rows outside the sequences while the others work, if there are as many as SMs
+// (fewer would take longer than a fill over a long unused tail): four fills of whole tensors less per training step.  24 causal
+// sequences up to 1500, H=8, D=128: 411 -> 361 us forward + backward.
+bool zero_gaps_inside(const SigAttnParams* p, int64_t n_items, int n_sm) {
+  return (p->flags & SIGATTN_ZERO_GAPS) && p->cu_seqlens_q && n_items >= n_sm;
+}
+
 struct DeviceGuard {
   int prev = -1;
   bool switched = false;
@@ -340,6 +360,9 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
   if (int rc = fwd_device_info(p->device, &info)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   fp.split = fwd_split(p, info.n_sm);
+  fp.zero_total = -1;
+  if (zero_gaps_inside(p, n_items, info.n_sm)) fp.zero_total = p->total_q;
+  else if (int rc = zero_gaps_first(p, p->o, p->o_strides, p->total_q, "o")) return rc;
   fp.sorted = !fp.causal && worth_sorting(p, n_items, info.n_sm, p->seq_lens_k || p->cu_seqlens_k);
   if (fp.split) {
     auto kernel = sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, true>;
@@ -453,6 +476,13 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
   bp.group = by_head ? 1 : schedule_group(bp.causal != 0, n_bh, (int64_t)p->Tq * D * (2 + 2 + 4), 32ll << 20);
   bp.sorted = (by_head || !bp.causal) && worth_sorting(p, by_head ? n_bh : n_items, info.n_sm,
                                                        p->seq_lens_q || p->cu_seqlens_q || (by_head && p->seq_lens_k));
+  bp.zero_total_q = bp.zero_total_k = -1;
+  if (zero_gaps_inside(p, by_head ? n_bh : n_items, info.n_sm)) {
+    bp.zero_total_q = p->total_q;
+    bp.zero_total_k = p->total_k;
+  } else if (int rc = zero_grad_gaps_first(p)) {
+    return rc;
+  }
   bp.ticket = next_ticket_pair(info, p->device, stream);
 
   {
@@ -537,6 +567,7 @@ int launch_bwd_stream(const SigAttnParams* p, const CUtensorMap& qm, const CUten
   FwdDeviceInfo info;
   if (int rc = fwd_device_info(p->device, &info)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
+  if (int rc = zero_grad_gaps_first(p)) return rc;
   if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
   if (int rc = launch_bwd_stream_mode<D, kBF16, true, kAccurate>(p, km, vm, qm, dom, info)) return rc;
   if (int rc = launch_bwd_stream_mode<D, kBF16, false, kAccurate>(p, qm, dom, km, vm, info)) return rc;
@@ -673,6 +704,7 @@ int launch_f32_d(const SigAttnParams* p, bool backward) {
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   FwdDeviceInfo info;
   if (int rc = fwd_device_info(p->device, &info)) return rc;
+  if (int rc = backward ? zero_grad_gaps_first(p) : zero_gaps_first(p, p->o, p->o_strides, p->total_q, "o")) return rc;
   if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
   int rc = 0;
   if (f32_tc(p, backward)) {
@@ -816,7 +848,8 @@ int sigattn_fwd(const SigAttnParams* p) {
   DeviceGuard g;
   SIG_CUDA(g.enter(p->device));
   const Extents ex = extents(p);
-  if (ex.Tq == 0 || p->Tq == 0) return 0;
+  if (ex.Tq == 0) return 0;
+  if (p->Tq == 0) return zero_gaps_first(p, p->o, p->o_strides, p->total_q, "o");
   if (ex.Tk == 0 || p->Tk == 0) {  // no keys at all: the output is all zeros
     const Strides3 os = map_strides(p->o_strides, ex.Tq, ex.packed);
     return zero_fill(p->o, os.s, ex.B, ex.Tq, p->H, head_cols(p), p->dtype, static_cast<cudaStream_t>(p->stream), "o");

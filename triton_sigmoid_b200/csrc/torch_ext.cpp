@@ -149,6 +149,8 @@ void fill_common(SigAttnParams& p, const Tensors& t, const Call& c, const Switch
   }
   p.flags = (c.causal ? SIGATTN_CAUSAL : 0u) | (sw.accurate ? SIGATTN_ACCURATE : 0u) |
             (c.bias_neg_log_lk ? SIGATTN_BIAS_NEG_LOG_LK : 0u);
+  // rows between or behind the sequences, and rows of a sequence beyond max_seqlen, are zero in every output
+  if (packed) p.flags |= SIGATTN_ZERO_GAPS;
   p.scale = c.scale;
   p.bias_scalar = c.bias;
   p.device = t.q.get_device();
@@ -184,9 +186,7 @@ void launch(int (*fn)(const SigAttnParams*), const SigAttnParams& p, const char*
 Tensor run_forward(const Tensors& t, const Call& c, const Switches& sw) {
   Tensor out = new_like(t.q);
   if (out.numel() == 0) return out;
-  // packed: only rows of the sequences are written; rows between or behind them, and rows of a sequence beyond
-  // max_seqlen_q, stay zero (as in the backward)
-  if (t.cu_q.defined()) out.zero_();
+  if (t.cu_q.defined() && t.cu_q.numel() == 1) return out.zero_();  // no sequence at all
   SigAttnParams p;
   fill_common(p, t, c, sw);
   p.o = out.mutable_data_ptr();
@@ -199,13 +199,9 @@ void run_backward(const Tensors& t, const Call& c, const Switches& sw, const Ten
   dq = new_like(t.q);
   dk = new_like(t.k);
   dv = new_like(t.v);
-  const bool packed = t.cu_q.defined();
-  if (packed) {
-    dq.zero_();
-    dk.zero_();
-    dv.zero_();
-    if (dq.numel() == 0 || dk.numel() == 0) return;
-  } else if (dq.numel() == 0 && dk.numel() == 0) {
+  if (dq.numel() == 0 && dk.numel() == 0) return;
+  if (t.cu_q.defined() && (dq.numel() == 0 || dk.numel() == 0 || t.cu_q.numel() == 1)) {
+    for (Tensor* g : {&dq, &dk, &dv}) g->zero_();
     return;
   }
   SigAttnParams p;
