@@ -165,9 +165,8 @@ struct FwdCursor {
 // 32 score columns of one TMEM lane (this thread's query row), already in registers -> logits in the
 // base-2 domain, t = (scale * s + bias) * log2(e).  Chunks that need no element
 // predicate work on logits shifted up by kDeepShift (see sigmoid2_from_shifted_log2_deep).
-template <bool kMask, bool kAccurate>
+template <bool kShift>
 __device__ __forceinline__ void fwd_chunk_logits(const uint32_t (&r)[32], float2 (&t)[16], float c1, float c0) {
-  constexpr bool kShift = !kMask && !kAccurate;
   const float c0s = kShift ? c0 + kDeepShift : c0;
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
@@ -215,7 +214,7 @@ __device__ __forceinline__ void fwd_add_score_mod(float2 (&t)[16], int col0, con
 
 // Logits of fwd_chunk_logits -> 16-bit probabilities, written over the first 16 of the chunk's 32 TMEM
 // columns at s_addr.  lim = largest visible key index of this row (used only when kMask).
-template <bool kBF16, bool kMask, bool kAccurate>
+template <bool kBF16, bool kMask, bool kAccurate, bool kDeep>
 __device__ __forceinline__ void fwd_chunk_probs(uint32_t s_addr, float2 (&t)[16], int col0, int lim) {
   constexpr int kCh = 32;
   uint32_t pk[kCh / 2];
@@ -233,12 +232,12 @@ __device__ __forceinline__ void fwd_chunk_probs(uint32_t s_addr, float2 (&t)[16]
   } else {
     // Under the default bias every logit of a chunk is far below zero: the short series applies
     // and the sign handling (one compare and one select per element) is skipped for the whole warp.
-    if (!kMask && warp_all_negative(t)) {
+    if (!kMask && kDeep && warp_all_negative(t)) {
 #pragma unroll
       for (int i = 0; i < kCh / 2; ++i) pk[i] = sigmoid2_deep_packed<kBF16>(t[i], (i & 7) == 7);
     } else {
       bool all_neg = false;
-      if constexpr (!kMask) {
+      if constexpr (!kMask && kDeep) {
 #pragma unroll
         for (int i = 0; i < kCh / 2; ++i) t[i] = __fadd2_rn(t[i], make_float2(-kDeepShift, -kDeepShift));
         all_neg = warp_all_negative(t);  // negative but not far below zero: full polynomial, still no select
@@ -267,13 +266,13 @@ __device__ __forceinline__ void fwd_chunk_probs(uint32_t s_addr, float2 (&t)[16]
 }
 
 // All steps for a chunk whose scores are in registers.  mod_args: those of fwd_add_score_mod after the logits.
-template <bool kBF16, bool kScoreMod, bool kMask, bool kAccurate, typename... ModArgs>
+template <bool kBF16, bool kScoreMod, bool kMask, bool kAccurate, bool kDeep, typename... ModArgs>
 __device__ __forceinline__ void fwd_sigmoid_chunk(uint32_t s_addr, const uint32_t (&r)[32], float c1, float c0, int col0,
                                                   int lim, ModArgs... mod_args) {
   float2 t[16];
-  fwd_chunk_logits<kMask, kAccurate>(r, t, c1, c0);
+  fwd_chunk_logits<kDeep && !kMask && !kAccurate>(r, t, c1, c0);
   if constexpr (kScoreMod) fwd_add_score_mod(t, mod_args...);
-  fwd_chunk_probs<kBF16, kMask, kAccurate>(s_addr, t, col0, lim);
+  fwd_chunk_probs<kBF16, kMask, kAccurate, kDeep>(s_addr, t, col0, lim);
 }
 
 // One work item.  The producer warp decodes it once (integer divisions, length and bias loads from global
@@ -368,7 +367,9 @@ __device__ __forceinline__ void fwd_take_part(FwdItem& it, int rank, int split) 
   it.n_max = j1 - j0;
 }
 
-template <int D, bool kBF16, bool kScoreMod, bool kAccurate, bool kSplit>
+// kDeep: chunks whose logits are all far below zero take the short series.  The form without it skips the test, which costs a
+// chunk that fails it a packed addition per pair and two votes: for biases with which none passes, see fwd_shallow().
+template <int D, bool kBF16, bool kScoreMod, bool kAccurate, bool kSplit, bool kDeep>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                    const __grid_constant__ CUtensorMap v_map, const FwdParams p) {
@@ -929,9 +930,9 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
                 tmem_ld32_sync(s_addr, r);
                 // the predicate code exists only in the instantiation used by boundary chunks
                 if (col0 + 32 > mask_from[s])
-                  fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate>(s_addr, r, c1, c0, col0, lim[s], col0, sm_row, sm_lim);
+                  fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate, kDeep>(s_addr, r, c1, c0, col0, lim[s], col0, sm_row, sm_lim);
                 else
-                  fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate>(s_addr, r, c1, c0, col0, lim[s], col0, sm_row, sm_lim);
+                  fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate, kDeep>(s_addr, r, c1, c0, col0, lim[s], col0, sm_row, sm_lim);
                 tmem_st_wait();
                 tc_fence_before_sync();
                 __syncwarp();
@@ -983,9 +984,9 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
             tmem_ld_wait_for(r);
             if (c == 0) tmem_ld(s_addr + 32, rbuf[1]);
             if (col0 + 32 * c + 32 > mask_from[s])
-              fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], mod[c], mod_patch);
+              fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate, kDeep>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], mod[c], mod_patch);
             else
-              fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], mod[c], mod_patch);
+              fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate, kDeep>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], mod[c], mod_patch);
             if constexpr (kScoreMod) mod[c] = load_mod((j + j_step) * kTileN + 64 * g + 32 * c + lane);
           }
           tmem_st_wait();

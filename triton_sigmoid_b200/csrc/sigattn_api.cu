@@ -326,6 +326,14 @@ bool worth_sorting(const SigAttnParams* p, int64_t n_items, int n_sm, bool lengt
   return lengths && p->B > 1 && p->B <= sigattn::kMaxOrdered && n_items > n_sm;
 }
 
+// Whether the forward leaves out the test for logits far below zero (below -3.5, all 1024 of a warp's chunk): with a bias of
+// the caller's, the same for the whole batch and above -3, scores would have to be below zero throughout to pass it.
+// B=4 T=4096 H=32 D=64, bias 0: 944 -> 787 us.  (Choosing by the chunk before, at run time: 879, and 1.4 % more with the default
+// bias, whose chunks pass.)
+bool fwd_shallow(const SigAttnParams* p) {
+  return !p->bias && !p->score_mod && !(p->flags & (SIGATTN_ACCURATE | SIGATTN_BIAS_NEG_LOG_LK)) && p->bias_scalar > -3.0f;
+}
+
 template <int D, bool kBF16, bool kScoreMod, bool kAccurate>
 int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap& km, const CUtensorMap& vm) {
   using namespace sigattn;
@@ -365,7 +373,7 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
   else if (int rc = zero_gaps_first(p, p->o, p->o_strides, p->total_q, "o")) return rc;
   fp.sorted = !fp.causal && worth_sorting(p, n_items, info.n_sm, p->seq_lens_k || p->cu_seqlens_k);
   if (fp.split) {
-    auto kernel = sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, true>;
+    auto kernel = sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, true, true>;
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
     fp.ticket = nullptr;
     cudaLaunchAttribute attr = {};
@@ -382,7 +390,9 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
     if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
     SIG_CUDA(cudaLaunchKernelEx(&cfg, kernel, qm, km, vm, fp));
   } else {
-    auto kernel = sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, false>;
+    constexpr bool kCanBeShallow = !kScoreMod && !kAccurate;
+    auto kernel = kCanBeShallow && fwd_shallow(p) ? sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, false, !kCanBeShallow>
+                                                  : sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, false, true>;
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
     fp.ticket = next_ticket_pair(info, p->device, stream);
     // persistent: one CTA per SM (the kernel's shared memory allows no more), fewer when there are fewer items
