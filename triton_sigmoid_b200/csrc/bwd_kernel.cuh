@@ -150,11 +150,11 @@ struct BwdSmem {
 // of the 32 columns read (the operand of dV).  Both phases move 16 columns at a time, so that besides the 32
 // probabilities only few registers are live.
 // q0 = query index of the first column; valid queries for this key row are [q_lo, q_hi).
-template <bool kBF16, bool kMask, bool kAccurate>
+template <bool kBF16, bool kMask, bool kAccurate, bool kDeep>
 __device__ __forceinline__ void bwd_phase_a(uint32_t s_addr, float c1, float c0, int q0, int q_lo, int q_hi,
                                             float2 (&pv)[16]) {
   // unmasked tiles work on logits shifted up by kDeepShift (see sigmoid2_from_shifted_log2_deep)
-  const float c0s = (kMask || kAccurate) ? c0 : c0 + kDeepShift;
+  const float c0s = (kMask || kAccurate || !kDeep) ? c0 : c0 + kDeepShift;
   {
     uint32_t r[32];
     tmem_ld32_sync(s_addr, r);
@@ -185,12 +185,12 @@ __device__ __forceinline__ void bwd_phase_a(uint32_t s_addr, float c1, float c0,
   if constexpr (kAccurate) {
     // exponential and reciprocal both on the special-function unit (see sigmoid2_accurate_from_log2)
     emit([](float2 x) { return sigmoid2_accurate_from_log2(x); });
-  } else if (!kMask && warp_all_negative(pv)) {
+  } else if (!kMask && kDeep && warp_all_negative(pv)) {
     // all logits far below zero (the usual case under the default bias): short series, no compare / select per element
     emit([](float2 x) { return sigmoid2_from_shifted_log2_deep<kBF16>(x); });
   } else {
     bool all_neg = false;
-    if constexpr (!kMask) {
+    if constexpr (!kMask && kDeep) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) pv[i] = __fadd2_rn(pv[i], make_float2(-kDeepShift, -kDeepShift));
       all_neg = warp_all_negative(pv);  // negative but not far below zero: full polynomial, still no select
@@ -236,13 +236,13 @@ __device__ __forceinline__ void bwd_phase_b(uint32_t dp_addr, uint32_t ds_line, 
 // (32 registers per thread that the drain warps' share of the register file cannot spare) but read back
 // from TMEM in the 16-bit form they were stored in for the dV product, and dS = P (1 - P) dP is formed on
 // packed 16-bit pairs.
-template <bool kBF16, bool kMask, bool kAccurate>
+template <bool kBF16, bool kMask, bool kAccurate, bool kDeep>
 __device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c0, int q0, int q_lo, int q_hi) {
   uint32_t r[32];
   tmem_ld32_sync(s_addr, r);
   uint32_t pk[16];
   float2 t[16];
-  const float c0s = (kMask || kAccurate) ? c0 : c0 + kDeepShift;
+  const float c0s = (kMask || kAccurate || !kDeep) ? c0 : c0 + kDeepShift;
 #pragma unroll
   for (int i = 0; i < 16; ++i)
     t[i] = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), make_float2(c1, c1),
@@ -258,13 +258,13 @@ __device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c
       }
       pk[i] = pack2<kBF16>(pe.x, pe.y);
     }
-  } else if (!kMask && warp_all_negative(t)) {
+  } else if (!kMask && kDeep && warp_all_negative(t)) {
     // all logits far below zero (the usual case under the default bias): short series on packed pairs
 #pragma unroll
     for (int i = 0; i < 16; ++i) pk[i] = sigmoid2_deep_packed<kBF16>(t[i], false);
   } else {
     bool all_neg = false;
-    if constexpr (!kMask) {
+    if constexpr (!kMask && kDeep) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) t[i] = __fadd2_rn(t[i], make_float2(-kDeepShift, -kDeepShift));
       all_neg = warp_all_negative(t);
@@ -408,7 +408,8 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item,
 // tickets count (batch, head) pairs.  (This form spills more: 132 / 188 bytes of stores / loads by -Xptxas -v at D = 64
 // against 68 / 76 in the general one, 208 / 300 against 120 / 188 at D = 128.  All registers of the CTA are handed out, see
 // below; the figures of the rule that chooses the form, bwd_by_head(), include these spills.)
-template <int D, bool kBF16, bool kAccurate, bool kByHead>
+// kDeep: as in the forward kernel.
+template <int D, bool kBF16, bool kAccurate, bool kByHead, bool kDeep>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                    const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap do_map,
@@ -1072,11 +1073,11 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         if (!ok) break;
         tc_fence_after_sync();
         if constexpr (D == 64) {
-          if (need_mask) bwd_phase_a16<kBF16, true, kAccurate>(s_addr, c1, c0, q0, q_lo, q_hi);
-          else           bwd_phase_a16<kBF16, false, kAccurate>(s_addr, c1, c0, q0, q_lo, q_hi);
+          if (need_mask) bwd_phase_a16<kBF16, true, kAccurate, kDeep>(s_addr, c1, c0, q0, q_lo, q_hi);
+          else           bwd_phase_a16<kBF16, false, kAccurate, kDeep>(s_addr, c1, c0, q0, q_lo, q_hi);
         } else {
-          if (need_mask) bwd_phase_a<kBF16, true, kAccurate>(s_addr, c1, c0, q0, q_lo, q_hi, pv);
-          else           bwd_phase_a<kBF16, false, kAccurate>(s_addr, c1, c0, q0, q_lo, q_hi, pv);
+          if (need_mask) bwd_phase_a<kBF16, true, kAccurate, kDeep>(s_addr, c1, c0, q0, q_lo, q_hi, pv);
+          else           bwd_phase_a<kBF16, false, kAccurate, kDeep>(s_addr, c1, c0, q0, q_lo, q_hi, pv);
         }
         tmem_st_wait();
         tc_fence_before_sync();

@@ -368,7 +368,7 @@ __device__ __forceinline__ void fwd_take_part(FwdItem& it, int rank, int split) 
 }
 
 // kDeep: chunks whose logits are all far below zero take the short series.  The form without it skips the test, which costs a
-// chunk that fails it a packed addition per pair and two votes: for biases with which none passes, see fwd_shallow().
+// chunk that fails it a packed addition per pair and two votes: for biases with which none passes, see few_deep_logits().
 template <int D, bool kBF16, bool kScoreMod, bool kAccurate, bool kSplit, bool kDeep>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,

@@ -326,11 +326,11 @@ bool worth_sorting(const SigAttnParams* p, int64_t n_items, int n_sm, bool lengt
   return lengths && p->B > 1 && p->B <= sigattn::kMaxOrdered && n_items > n_sm;
 }
 
-// Whether the forward leaves out the test for logits far below zero (below -3.5, all 1024 of a warp's chunk): with a bias of
+// Whether the 16-bit kernels leave out the test for logits far below zero (below -3.5, all 1024 of a warp's chunk): with a bias of
 // the caller's, the same for the whole batch and above -3, scores would have to be below zero throughout to pass it.
-// B=4 T=4096 H=32 D=64, bias 0: 944 -> 787 us.  (Choosing by the chunk before, at run time: 879, and 1.4 % more with the default
-// bias, whose chunks pass.)
-bool fwd_shallow(const SigAttnParams* p) {
+// Bias 0, B=4 T=4096 H=32 D=64, forward: 944 -> 787 us; H=16, forward and backward: 467 and 850 -> 366 and 815, D=128 580 and 1540 ->
+// 462 and 1350.  (Choosing by the chunk before, at run time: 879, and 1.4 % more with the default bias, whose chunks pass.)
+bool few_deep_logits(const SigAttnParams* p) {
   return !p->bias && !p->score_mod && !(p->flags & (SIGATTN_ACCURATE | SIGATTN_BIAS_NEG_LOG_LK)) && p->bias_scalar > -3.0f;
 }
 
@@ -391,7 +391,7 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
     SIG_CUDA(cudaLaunchKernelEx(&cfg, kernel, qm, km, vm, fp));
   } else {
     constexpr bool kCanBeShallow = !kScoreMod && !kAccurate;
-    auto kernel = kCanBeShallow && fwd_shallow(p) ? sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, false, !kCanBeShallow>
+    auto kernel = kCanBeShallow && few_deep_logits(p) ? sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, false, !kCanBeShallow>
                                                   : sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, false, true>;
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
     fp.ticket = next_ticket_pair(info, p->device, stream);
@@ -496,7 +496,9 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
   bp.ticket = next_ticket_pair(info, p->device, stream);
 
   {
-    auto kernel = by_head ? sigattn_bwd_kernel<D, kBF16, kAccurate, !kAccurate> : sigattn_bwd_kernel<D, kBF16, kAccurate, false>;
+    const bool shallow = !kAccurate && few_deep_logits(p);
+    auto kernel = by_head ? (shallow ? sigattn_bwd_kernel<D, kBF16, kAccurate, !kAccurate, kAccurate> : sigattn_bwd_kernel<D, kBF16, kAccurate, !kAccurate, true>)
+                          : (shallow ? sigattn_bwd_kernel<D, kBF16, kAccurate, false, kAccurate> : sigattn_bwd_kernel<D, kBF16, kAccurate, false, true>);
     constexpr int smem = BwdSmem<D>::kDynBytes;
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
     // persistent: one CTA per SM (the kernel's shared memory allows no more), fewer when there are fewer items
