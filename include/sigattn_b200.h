@@ -69,7 +69,7 @@ enum SigAttnFlags {
    * keys gets +inf, where every probability is masked anyway. */
   SIGATTN_BIAS_NEG_LOG_LK = 1u << 3,
   /* Packed layout, at least one sequence: rows of the outputs that belong to no sequence (see cu_seqlens_q below) are written as
-   * zeros instead of being left untouched.  The outputs must be contiguous. */
+   * zeros instead of being left untouched. */
   SIGATTN_ZERO_GAPS = 1u << 4,
 };
 

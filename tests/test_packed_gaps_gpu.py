@@ -19,8 +19,8 @@ def _poison(shape, dtype):
 
 @pytest.mark.parametrize("split", [False, True])
 @pytest.mark.parametrize("n,H,D,dtype,form", [
-    (3, 2, 64, torch.bfloat16, FORM_BWD),            # fewer items than SMs: a fill before the kernels
-    (40, 8, 64, torch.float16, FORM_BWD),            # zeroed by the kernels
+    (3, 2, 64, torch.bfloat16, FORM_BWD),
+    (40, 8, 64, torch.float16, FORM_BWD),
     (40, 8, 128, torch.bfloat16, FORM_BWD),
     (40, 8, 24, torch.bfloat16, FORM_BWD),
     (260, 8, 64, torch.bfloat16, FORM_BWD_BY_HEAD),

@@ -61,7 +61,6 @@ struct BwdParams {
   // one region per head and sequence.  nullptr = (B, T, H, D).
   const int* cu_q;
   const int* cu_k;
-  int zero_total_q, zero_total_k;  // packed: rows of dq and of dk, dv, those outside the sequences are zeroed; -1: left alone
   const float* bias;
   const float* score_mod;
   float scale;
@@ -73,7 +72,7 @@ struct BwdParams {
   int n_items;  // B * H * n_kvblk
   int group;    // (batch, head) pairs per scheduling group, >= 1 (see bwd_decode_item)
   int sorted;   // batch elements are taken by falling weight of what a ticket stands for (see worth_sorting())
-  void* dq;     // (rows of sequences: kByHead only, else sigattn_dq_convert_kernel writes them)
+  void* dq;     // kByHead only (else sigattn_dq_convert_kernel writes dQ)
   int64_t dq_sb, dq_st, dq_sh;
   // two counters, zero between launches: [0] items handed out beyond the first per CTA,
   // [1] CTAs that have finished (the last one clears both)
@@ -1005,14 +1004,6 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       mma_commit(leader, bar(L::kKvEmpty + kb));  // the dQ products were this warp's readers of K_j
       g += it.n_q;
       ++act;
-    }
-  }
-  else if (warp == kBwdIssuerB + 1) {  // the spare warp
-    if (p.zero_total_q >= 0) {
-      const int w = (int)blockIdx.x, n = (int)gridDim.x;
-      zero_gap_rows(p.dq, p.dq_st, p.dq_sh, p.H, p.d_cols, p.cu_q, p.B, p.Tq, p.zero_total_q, w, n);
-      zero_gap_rows(p.dk, p.dk_st, p.dk_sh, p.H, p.d_cols, p.cu_k, p.B, p.Tk, p.zero_total_k, w, n);
-      zero_gap_rows(p.dv, p.dv_st, p.dv_sh, p.H, p.d_cols, p.cu_k, p.B, p.Tk, p.zero_total_k, w, n);
     }
   }
   else if (warp < kBwdComputeWarps) {

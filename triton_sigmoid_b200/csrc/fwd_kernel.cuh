@@ -57,7 +57,6 @@ struct FwdParams {
   // tensor (likewise cu_k for keys / values); Tq, Tk are then upper bounds of the lengths.  nullptr = (B, T, H, D).
   const int* cu_q;
   const int* cu_k;
-  int zero_total;          // packed: rows of o, those outside the sequences are zeroed; -1: they are left alone
   const float* bias;       // [B] or nullptr
   const float* score_mod;  // [B, Tk] (packed: [total keys]) or nullptr
   float scale;
@@ -856,9 +855,6 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       mma_commit(leader, bar(L::kOFull));
       ++act;
     }
-  }
-  else if (!kSplit && warp == kFwdProducerWarp + 3 && p.zero_total >= 0) {  // the spare warp
-    zero_gap_rows(p.o, p.o_st, p.o_sh, p.H, p.d_cols, p.cu_q, p.B, p.Tq, p.zero_total, (int)blockIdx.x, (int)gridDim.x);
   }
   if constexpr (kSplit) { cluster_sync(); cluster_sync(); }
   }  // role warps

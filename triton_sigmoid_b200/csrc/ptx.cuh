@@ -371,32 +371,6 @@ __device__ __forceinline__ int seq_rows(const int* lens, const int* cu, int b, i
   return min(max(n, 0), T);
 }
 
-// One warp's share of zeroing the rows of a packed 16-bit tensor that belong to no sequence: rows before the first one, rows
-// of a sequence beyond T, rows behind the last one.  Usually there are none, and this is a look at the offsets.
-// strides in elements; d_cols a multiple of 8.
-__device__ __forceinline__ void zero_gap_rows(void* base, int64_t st, int64_t sh, int H, int d_cols, const int* cu, int B, int T,
-                                              int total, int worker, int n_workers) {
-  const int lane = threadIdx.x & 31;
-  const int chunks = d_cols / 8, per_row = H * chunks;
-  for (int g0 = 0; g0 <= B; g0 += 32) {
-    const int g = g0 + lane;  // the gap in front of sequence g
-    int lo = 0, hi = 0;
-    if (g <= B) {
-      if (g > 0) lo = cu[g - 1] + min(max(cu[g] - cu[g - 1], 0), T);
-      hi = g < B ? cu[g] : total;
-    }
-    for (unsigned int m = __ballot_sync(0xffffffffu, lo < hi); m; m &= m - 1) {
-      const int src = __ffs(m) - 1;
-      const int first = __shfl_sync(0xffffffffu, lo, src), end = __shfl_sync(0xffffffffu, hi, src);
-      for (int64_t r = (int64_t)first + worker; r < end; r += n_workers)
-        for (int i = lane; i < per_row; i += 32) {
-          const int h = i / chunks, c = i - h * chunks;
-          reinterpret_cast<uint4*>(static_cast<uint8_t*>(base) + 2 * (r * st + h * sh))[c] = make_uint4(0, 0, 0, 0);
-        }
-    }
-  }
-}
-
 // ---------------------------------------------------------------- math
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;

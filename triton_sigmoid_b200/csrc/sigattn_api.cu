@@ -138,24 +138,62 @@ int zero_fill(void* ptr, const int64_t* strides, int B, int T, int H, int D, int
   return 0;
 }
 
-// SIGATTN_ZERO_GAPS, where the kernel does not do it on the way: the whole output (before the kernel writes the sequences).
-int zero_gaps_first(const SigAttnParams* p, void* ptr, const int64_t* strides, int total, const char* name) {
+// SIGATTN_ZERO_GAPS: rows of packed outputs that belong to no sequence - before the first one, beyond T within one, behind the
+// last one - are zeroed by a kernel that usually finds none, a look at the offsets.  24 causal sequences up to 1500, H=8, D=128,
+// forward + backward: 411 -> 368 us without the fills.  (Done by the spare warps of the attention kernels it costs no launch, 361 us, but the
+// backward's code moves: a dense causal step of B=8 T=1000 H=16 D=64 took 179 us instead of 174.)
+struct GapTensor {
+  uint8_t* base;
+  int64_t st, sh;  // bytes
+  const int* cu;
+  int T, total;
+};
+struct GapParams {
+  GapTensor t[3];
+  int n, B, H, chunks;  // 16-byte pieces of a row of one head
+};
+__global__ void __launch_bounds__(256) sigattn_zero_gaps_kernel(const GapParams p) {
+  const int lane = threadIdx.x & 31, worker = (blockIdx.x * 256 + threadIdx.x) >> 5, n_workers = gridDim.x * 8;
+  for (int k = 0; k < p.n; ++k) {
+    const GapTensor t = p.t[k];
+    for (int g0 = 0; g0 <= p.B; g0 += 32) {
+      const int g = g0 + lane;  // the gap in front of sequence g
+      int lo = 0, hi = 0;
+      if (g <= p.B) {
+        if (g > 0) lo = t.cu[g - 1] + min(max(t.cu[g] - t.cu[g - 1], 0), t.T);
+        hi = min(g < p.B ? t.cu[g] : t.total, t.total);
+      }
+      for (unsigned int m = __ballot_sync(0xffffffffu, lo < hi); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const int first = __shfl_sync(0xffffffffu, lo, src), end = __shfl_sync(0xffffffffu, hi, src);
+        for (int64_t r = (int64_t)first + worker; r < end; r += n_workers)
+          for (int i = lane; i < p.H * p.chunks; i += 32) {
+            const int h = i / p.chunks, c = i - h * p.chunks;
+            reinterpret_cast<uint4*>(t.base + r * t.st + h * t.sh)[c] = make_uint4(0, 0, 0, 0);
+          }
+      }
+    }
+  }
+}
+int zero_gaps(const SigAttnParams* p, bool backward, int n_sm) {
   if (!(p->flags & SIGATTN_ZERO_GAPS) || !p->cu_seqlens_q) return 0;
-  const int D = head_cols(p);
-  const Strides3 s = map_strides(strides, total, true);
-  if (!is_contiguous(s.s, total > 0 ? total : 1, p->H, D)) return fail(-2, "%s: SIGATTN_ZERO_GAPS needs contiguous outputs", name);
-  return zero_fill(ptr, s.s, 1, total, p->H, D, p->dtype, static_cast<cudaStream_t>(p->stream), name);
-}
-int zero_grad_gaps_first(const SigAttnParams* p) {
-  if (int rc = zero_gaps_first(p, p->dq, p->dq_strides, p->total_q, "dq")) return rc;
-  if (int rc = zero_gaps_first(p, p->dk, p->dk_strides, p->total_k, "dk")) return rc;
-  return zero_gaps_first(p, p->dv, p->dv_strides, p->total_k, "dv");
-}
-// The spare warps of the 16-bit kernels zero the rows outside the sequences while the others work, if there are as many as SMs
-// (fewer would take longer than a fill over a long unused tail): four fills of whole tensors less per training step.  24 causal
-// sequences up to 1500, H=8, D=128: 411 -> 361 us forward + backward.
-bool zero_gaps_inside(const SigAttnParams* p, int64_t n_items, int n_sm) {
-  return (p->flags & SIGATTN_ZERO_GAPS) && p->cu_seqlens_q && n_items >= n_sm;
+  const int es = p->dtype == SIGATTN_FP32 ? 4 : 2;
+  void* ptr[3] = {backward ? p->dq : p->o, p->dk, p->dv};
+  const int64_t* strides[3] = {backward ? p->dq_strides : p->o_strides, p->dk_strides, p->dv_strides};
+  GapParams gp = {};
+  gp.n = backward ? 3 : 1;
+  gp.B = p->B;
+  gp.H = p->H;
+  gp.chunks = head_cols(p) * es / 16;
+  for (int k = 0; k < gp.n; ++k) {
+    if ((reinterpret_cast<uintptr_t>(ptr[k]) & 15u) != 0 || strides[k][1] * es % 16 != 0 || strides[k][2] * es % 16 != 0)
+      return fail(-3, "SIGATTN_ZERO_GAPS: outputs and their strides must be 16-byte aligned");
+    gp.t[k] = GapTensor{static_cast<uint8_t*>(ptr[k]), strides[k][1] * es, strides[k][2] * es, k ? p->cu_seqlens_k : p->cu_seqlens_q,
+                        k ? p->Tk : p->Tq, k ? p->total_k : p->total_q};
+  }
+  sigattn_zero_gaps_kernel<<<n_sm, 256, 0, static_cast<cudaStream_t>(p->stream)>>>(gp);
+  SIG_CUDA(cudaGetLastError());
+  return 0;
 }
 
 struct DeviceGuard {
@@ -368,9 +406,7 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
   if (int rc = fwd_device_info(p->device, &info)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   fp.split = fwd_split(p, info.n_sm);
-  fp.zero_total = -1;
-  if (zero_gaps_inside(p, n_items, info.n_sm)) fp.zero_total = p->total_q;
-  else if (int rc = zero_gaps_first(p, p->o, p->o_strides, p->total_q, "o")) return rc;
+  if (int rc = zero_gaps(p, false, info.n_sm)) return rc;
   fp.sorted = !fp.causal && worth_sorting(p, n_items, info.n_sm, p->seq_lens_k || p->cu_seqlens_k);
   if (fp.split) {
     auto kernel = sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, true, true>;
@@ -486,13 +522,7 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
   bp.group = by_head ? 1 : schedule_group(bp.causal != 0, n_bh, (int64_t)p->Tq * D * (2 + 2 + 4), 32ll << 20);
   bp.sorted = (by_head || !bp.causal) && worth_sorting(p, by_head ? n_bh : n_items, info.n_sm,
                                                        p->seq_lens_q || p->cu_seqlens_q || (by_head && p->seq_lens_k));
-  bp.zero_total_q = bp.zero_total_k = -1;
-  if (zero_gaps_inside(p, by_head ? n_bh : n_items, info.n_sm)) {
-    bp.zero_total_q = p->total_q;
-    bp.zero_total_k = p->total_k;
-  } else if (int rc = zero_grad_gaps_first(p)) {
-    return rc;
-  }
+  if (int rc = zero_gaps(p, true, info.n_sm)) return rc;
   bp.ticket = next_ticket_pair(info, p->device, stream);
 
   {
@@ -579,7 +609,7 @@ int launch_bwd_stream(const SigAttnParams* p, const CUtensorMap& qm, const CUten
   FwdDeviceInfo info;
   if (int rc = fwd_device_info(p->device, &info)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-  if (int rc = zero_grad_gaps_first(p)) return rc;
+  if (int rc = zero_gaps(p, true, info.n_sm)) return rc;
   if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
   if (int rc = launch_bwd_stream_mode<D, kBF16, true, kAccurate>(p, km, vm, qm, dom, info)) return rc;
   if (int rc = launch_bwd_stream_mode<D, kBF16, false, kAccurate>(p, qm, dom, km, vm, info)) return rc;
@@ -716,7 +746,7 @@ int launch_f32_d(const SigAttnParams* p, bool backward) {
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   FwdDeviceInfo info;
   if (int rc = fwd_device_info(p->device, &info)) return rc;
-  if (int rc = backward ? zero_grad_gaps_first(p) : zero_gaps_first(p, p->o, p->o_strides, p->total_q, "o")) return rc;
+  if (int rc = zero_gaps(p, backward, info.n_sm)) return rc;
   if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
   int rc = 0;
   if (f32_tc(p, backward)) {
@@ -861,7 +891,11 @@ int sigattn_fwd(const SigAttnParams* p) {
   SIG_CUDA(g.enter(p->device));
   const Extents ex = extents(p);
   if (ex.Tq == 0) return 0;
-  if (p->Tq == 0) return zero_gaps_first(p, p->o, p->o_strides, p->total_q, "o");
+  if (p->Tq == 0) {  // every row is outside a sequence
+    FwdDeviceInfo info;
+    if ((rc = fwd_device_info(p->device, &info))) return rc;
+    return zero_gaps(p, false, info.n_sm);
+  }
   if (ex.Tk == 0 || p->Tk == 0) {  // no keys at all: the output is all zeros
     const Strides3 os = map_strides(p->o_strides, ex.Tq, ex.packed);
     return zero_fill(p->o, os.s, ex.B, ex.Tq, p->H, head_cols(p), p->dtype, static_cast<cudaStream_t>(p->stream), "o");
