@@ -71,7 +71,6 @@ struct BwdParams {
   int n_kvblk;  // ceil(Tk / 128)
   int n_items;  // B * H * n_kvblk
   int group;    // (batch, head) pairs per scheduling group, >= 1 (see bwd_decode_item)
-  int sorted;   // batch elements are taken by falling weight of what a ticket stands for (see worth_sorting())
   void* dq;     // kByHead only (else sigattn_dq_convert_kernel writes dQ)
   int64_t dq_sb, dq_st, dq_sh;
   // two counters, zero between launches: [0] items handed out beyond the first per CTA,
@@ -138,8 +137,7 @@ struct BwdSmem {
   static constexpr int kItemEmpty = kItemFull + 2;    // [2] item index read by every consumer warp
   static constexpr int kNumBars = kItemEmpty + 2;
   static constexpr int kMiscOff = kBarOff + 8 * kNumBars;  // tmem base (u32), abort flag (int), 2 x item record (16 int each)
-  static constexpr int kOrderOff = kMiscOff + 16 + 2 * 64;  // 16-bit batch indices, see order_by_weight
-  static constexpr int kTotal = kOrderOff + 2 * kMaxOrdered;
+  static constexpr int kTotal = kMiscOff + 16 + 2 * 64;
   static constexpr int kDynBytes = kTotal + 1024;
 };
 
@@ -362,7 +360,7 @@ __device__ __forceinline__ BwdItem bwd_load_item(const volatile int* rec) {
   return it;
 }
 template <int D>
-__device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item, const uint16_t* order) {
+__device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item) {
   BwdItem it;
   // Groups of `group` (batch, head) pairs: within a group every pair's key tile 0 comes first, then
   // every pair's tile 1, ... (under a causal mask the early tiles are the heavy ones, so this is a
@@ -375,7 +373,6 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item,
   const int bh = grp * p.group + (r - j * g_eff);
   it.b = bh / p.H;
   it.h = bh - it.b * p.H;
-  if (order) it.b = order[it.b];
   it.kv0 = j * kBwdTileKV;
   it.Lq = p.Tq;
   it.Lk = p.Tk;
@@ -503,17 +500,6 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   if (warp == kBwdIssuerA) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
     tmem_relinquish();
-  }
-  const uint16_t* order = nullptr;
-  if (p.sorted) {
-    // what a ticket stands for: a key tile, as heavy as there are query tiles, or a pair
-    uint16_t* by_weight = reinterpret_cast<uint16_t*>(smem_gen + L::kOrderOff);
-    order_by_weight(by_weight, reinterpret_cast<int*>(smem_gen + L::kKOff), p.B, [&](int b) {
-      const int q_tiles = (seq_rows(p.lens_q, p.cu_q, b, p.Tq) + kBwdTileQ - 1) / kBwdTileQ;
-      return kByHead ? q_tiles * ((seq_rows(p.lens_k, p.cu_k, b, p.Tk) + kBwdTileKV - 1) / kBwdTileKV) : q_tiles;
-    });
-    fence_proxy_async_smem();  // (the scratch is where the first K tile will be loaded)
-    order = by_weight;
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -761,7 +747,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         }
       }
       BwdItem it = {};
-      if (item >= 0) it = bwd_decode_item<D>(p, item, order);
+      if (item >= 0) it = bwd_decode_item<D>(p, item);
       if (lane == 0) {
         if (item >= 0) bwd_publish_item(item_ring + 16 * slot, item, it);
         else item_ring[16 * slot] = -1;

@@ -67,7 +67,6 @@ struct FwdParams {
   int n_qblk;   // ceil(Tq / 256)
   int n_items;  // B * H * n_qblk
   int group;    // (batch, head) pairs per scheduling group, >= 1 (see fwd_decode_item)
-  int sorted;   // batch elements are taken by falling number of keys (see worth_sorting() on the host side)
   int split;    // kSplit: CTAs per cluster = parts of the key range of an item (no tickets then)
   // two counters, zero between launches: [0] items handed out beyond the first per CTA,
   // [1] CTAs that have finished (the last one clears both)
@@ -127,8 +126,7 @@ struct FwdSmem {
   static constexpr int kModFloats = (D == 64) ? 32 : 0;
   static constexpr int kModOff = (kMiscOff + 16 + 2 * 64 + 15) & ~15;  // read 16 bytes at a time
   static_assert(kModOff % 16 == 0 && kKOff % 16 == 0, "16-byte accesses");
-  static constexpr int kOrderOff = kModOff + kFwdSigmoidWarps * kModFloats * 4;  // 16-bit batch indices, see order_by_weight
-  static constexpr int kTotal = kOrderOff + 2 * kMaxOrdered;
+  static constexpr int kTotal = kModOff + kFwdSigmoidWarps * kModFloats * 4;
   static constexpr int kDynBytes = kTotal + 1024;  // slack to align the base to 1024 bytes
 };
 
@@ -302,7 +300,7 @@ __device__ __forceinline__ FwdItem fwd_load_item(const volatile int* rec) {
   it.n_max = rec[13]; it.bias = __int_as_float(rec[14]); it.k_first = rec[15];
   return it;
 }
-__device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item, const uint16_t* order) {
+__device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item) {
   FwdItem it;
   // Items are ordered in groups of `group` (batch, head) pairs: within a group all pairs' heaviest
   // query blocks come first, then their second heaviest, ... (a longest-first order under a causal
@@ -316,7 +314,6 @@ __device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item,
   const int bh = grp * p.group + (r - qi * g_eff);
   it.b = bh / p.H;
   it.h = bh - it.b * p.H;
-  if (order) it.b = order[it.b];
   const int qblk = p.causal ? (p.n_qblk - 1 - qi) : qi;  // heavy blocks of a head first
   it.q0 = qblk * kFwdBlockM;
   it.Lq = p.Tq;
@@ -443,14 +440,6 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   if (warp == kFwdIssuerWarp) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
     tmem_relinquish();
-  }
-  const uint16_t* order = nullptr;
-  if (!kSplit && p.sorted) {
-    uint16_t* by_keys = reinterpret_cast<uint16_t*>(smem_gen + L::kOrderOff);
-    order_by_weight(by_keys, reinterpret_cast<int*>(smem_gen + L::kKOff), p.B,
-                    [&](int b) { return seq_rows(p.lens_k, p.cu_k, b, p.Tk); });
-    fence_proxy_async_smem();  // (the scratch is where the first K tile will be loaded)
-    order = by_keys;
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -681,7 +670,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         item = __shfl_sync(0xffffffffu, item, 0);
       }
       FwdItem it = {};
-      if (item >= 0) it = fwd_decode_item(p, item, order);
+      if (item >= 0) it = fwd_decode_item(p, item);
       if constexpr (kSplit)
         if (item >= 0) fwd_take_part(it, (int)blockIdx.x % p.split, p.split);
       if (lane == 0) {
@@ -1001,7 +990,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     if constexpr (kSplit) {
       // ---- the cluster's partial O, added up in the order of the ranks: every rank finishes its share of the rows
       const int rank = (int)blockIdx.x % p.split;
-      const FwdItem it = fwd_decode_item(p, (int)blockIdx.x / p.split, nullptr);  // the whole item
+      const FwdItem it = fwd_decode_item(p, (int)blockIdx.x / p.split);  // the whole item
       cluster_sync();
       constexpr int kPieces = D / 8;  // 8 columns = 16 bytes of O
       const int share = (p.Tq <= 128 ? 128 : 256) / p.split;

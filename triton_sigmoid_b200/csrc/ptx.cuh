@@ -347,30 +347,6 @@ __device__ __forceinline__ float item_bias(const float* bias, float bias_scalar,
   return (bias_scalar != bias_scalar) ? -logf((float)n_keys) : bias_scalar;
 }
 
-// Batch elements by falling weight (ties: by index), for schedules that hand out the heaviest work first: order[i] is the
-// i-th.  Every thread of the block calls it; `weights` is scratch for B ints, and `order` may be read after the caller's
-// next __syncthreads.  O(B) steps per thread, a microsecond at kMaxOrdered.
-constexpr int kMaxOrdered = 512;
-template <typename F>
-__device__ __forceinline__ void order_by_weight(uint16_t* order, int* weights, int B, F weight) {
-  for (int b = threadIdx.x; b < B; b += blockDim.x) weights[b] = weight(b);
-  __syncthreads();
-  for (int b = threadIdx.x; b < B; b += blockDim.x) {
-    const int w = weights[b];
-    int rank = 0;
-    for (int i = 0; i < B; ++i) {
-      const int x = weights[i];
-      rank += x > w || (x == w && i < b);
-    }
-    order[rank] = (uint16_t)b;
-  }
-}
-// Rows of sequence b, from its length or the packed layout's offsets, at most T.
-__device__ __forceinline__ int seq_rows(const int* lens, const int* cu, int b, int T) {
-  const int n = cu ? cu[b + 1] - cu[b] : lens ? lens[b] : T;
-  return min(max(n, 0), T);
-}
-
 // ---------------------------------------------------------------- math
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;

@@ -356,14 +356,6 @@ int fwd_split(const SigAttnParams* p, int n_sm) {
   return split > 1 ? split : 0;
 }
 
-// Whether the persistent kernels take the batch elements by falling length: the launch ends on the last item, which in the
-// order of the batch may be one of the longest.  Not for dense batches, nor for as many items as SMs; under a causal mask the
-// general forms order by tile already.  16 sequences of 256 .. 2048, H=8, forward + backward: 375 -> 368 us (a model of the
-// schedule says 3.5 % for the backward and 10 % for the forward); packed causal ones unchanged, 410.
-bool worth_sorting(const SigAttnParams* p, int64_t n_items, int n_sm, bool lengths) {
-  return lengths && p->B > 1 && p->B <= sigattn::kMaxOrdered && n_items > n_sm;
-}
-
 // Whether the 16-bit kernels leave out the test for logits far below zero (below -3.5, all 1024 of a warp's chunk): with a bias of
 // the caller's, the same for the whole batch and above -3, scores would have to be below zero throughout to pass it.
 // Bias 0, B=4 T=4096 H=32 D=64, forward: 944 -> 787 us; H=16, forward and backward: 467 and 850 -> 366 and 815, D=128 580 and 1540 ->
@@ -407,7 +399,6 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   fp.split = fwd_split(p, info.n_sm);
   if (int rc = zero_gaps(p, false, info.n_sm)) return rc;
-  fp.sorted = !fp.causal && worth_sorting(p, n_items, info.n_sm, p->seq_lens_k || p->cu_seqlens_k);
   if (fp.split) {
     auto kernel = sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, true, true>;
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
@@ -520,8 +511,6 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
   // Q, dO and the fp32 dQ accumulator of one head; a quarter of the L2 (measured: larger groups cost the
   // reductions their locality, a few heads already balance the CTAs)
   bp.group = by_head ? 1 : schedule_group(bp.causal != 0, n_bh, (int64_t)p->Tq * D * (2 + 2 + 4), 32ll << 20);
-  bp.sorted = (by_head || !bp.causal) && worth_sorting(p, by_head ? n_bh : n_items, info.n_sm,
-                                                       p->seq_lens_q || p->cu_seqlens_q || (by_head && p->seq_lens_k));
   if (int rc = zero_gaps(p, true, info.n_sm)) return rc;
   bp.ticket = next_ticket_pair(info, p->device, stream);
 
