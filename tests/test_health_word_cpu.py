@@ -1,0 +1,19 @@
+"""A kernel that finds the health word set leaves before it has set anything up.  Its warps read the word at different times, and
+it may be written meanwhile: unless they agree on one answer, some leave and the others wait for them - at a named barrier, which
+has no limit, or with a tensor-memory address that the warp that left was to write."""
+
+import os
+import re
+
+import pytest
+
+from triton_sigmoid_b200._paths import CSRC
+
+KERNELS = ["f32_tc_kernel.cuh"]
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_early_return_is_one_answer_for_the_block(name):
+    with open(os.path.join(CSRC, name)) as f:
+        reads = [line for line in f if re.search(r"&g_status_word\)", line)]
+    assert reads and all("__syncthreads_or(" in line for line in reads), reads

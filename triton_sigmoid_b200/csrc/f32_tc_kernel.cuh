@@ -154,7 +154,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
   using L = TcShape<D, kMode>;
   constexpr int kSite = (0x6 + kMode) << 16;
   extern __shared__ uint8_t tc_smem[];
-  if (*reinterpret_cast<volatile int*>(&g_status_word) != 0) return;
+  // a kernel of this library already gave up on a wait: leave, all warps or none (the named barriers below count on every warp,
+  // and the word may change while they read it)
+  if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) return;
 
   // ---------------------------------------------------------------- the tile
   const F32Item it = f32_item(p, n_tiles, !L::kKeyRows);
@@ -205,10 +207,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
   auto bar = [&](int i) -> uint32_t { return smem_base + L::kBarOff + 8u * i; };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + L::kMiscOff + 4);
-  volatile int* redo_flag = reinterpret_cast<volatile int*>(smem_gen + L::kMiscOff + 8);
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    *redo_flag = 0;
     for (int i = 0; i < L::kStages; ++i) {
       mbar_init(bar(L::kC1Full + i), kTcConvWarps);
       mbar_init(bar(L::kC2Full + i), kTcConvWarps);
@@ -593,10 +593,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
       if constexpr (L::kOut1) finite = fmaf(acc1[c], 0.f, finite);
       if constexpr (L::kOut2) finite = fmaf(acc2[c], 0.f, finite);
     }
-    if (row < Lr && !(finite == 0.f)) *redo_flag = 1;
-    asm volatile("bar.sync 10, %0;" ::"n"(32 * kTcComputeWarps) : "memory");
-    if (*abort_flag == 0) {
-      if (*redo_flag == 0) {
+    // one answer for all compute warps: they meet at barriers again below, and another role may still give up
+    auto any = [](bool x) -> bool {
+      int r;
+      asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.or.pred q, 10, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+                   : "=r"(r)
+                   : "r"((int)x), "n"(32 * kTcComputeWarps)
+                   : "memory");
+      return r != 0;
+    };
+    const bool redo = any(row < Lr && !(finite == 0.f));
+    if (!any(!ok || *abort_flag != 0)) {
+      if (!redo) {
         store_all(acc1, acc2);
       } else {
         float* space = reinterpret_cast<float*>(smem_gen);
