@@ -9,7 +9,7 @@ import pytest
 
 from triton_sigmoid_b200._paths import CSRC
 
-KERNELS = ["f32_tc_kernel.cuh"]
+KERNELS = ["f32_tc_kernel.cuh", "fwd_kernel.cuh", "bwd_kernel.cuh", "bwd_stream_kernel.cuh"]
 
 
 @pytest.mark.parametrize("name", KERNELS)

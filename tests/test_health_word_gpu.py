@@ -11,14 +11,23 @@ from triton_sigmoid_b200 import _cabi
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("split_backward", [False, True])
 @pytest.mark.parametrize("B,T,H,D,dtype,form", [
     (1, 512, 2, 64, torch.float32, _cabi.FORM_F32_TC),
     (1, 512, 16, 128, torch.float32, _cabi.FORM_F32_TC),
+    (1, 512, 2, 64, torch.float16, _cabi.FORM_BWD),           # forward: keys split over a cluster
+    (16, 256, 16, 128, torch.bfloat16, _cabi.FORM_BWD),       # persistent forward
+    (80, 256, 16, 64, torch.bfloat16, _cabi.FORM_BWD_BY_HEAD),
 ])
-def test_replay_while_the_word_is_set(B, T, H, D, dtype, form):
+def test_replay_while_the_word_is_set(B, T, H, D, dtype, form, split_backward, monkeypatch):
     lib = _cabi.load()
     assert launch_form(B, H, T, T, D, dtype, True) == form
     assert m.device_status() == 0
+    if split_backward:
+        if dtype == torch.float32:
+            pytest.skip("an option of the 16-bit kernels")
+        monkeypatch.setenv("SIGATTN_B200_BWD_SPLIT", "1")
+        form = None
     q, k, v, do = make_inputs(B, T, T, H, D, dtype, std=0.5, seed=1, requires_grad=True)
 
     def step():

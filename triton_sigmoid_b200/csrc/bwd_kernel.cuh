@@ -451,7 +451,8 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   const int lane = threadIdx.x & 31;
 
   // a kernel of this library already gave up on a wait: do not pile more work on a sick device
-  if (*reinterpret_cast<volatile int*>(&g_status_word) != 0) return;
+  // (one answer for the CTA: the word may change while its warps read it)
+  if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) return;
 
   // ---------------------------------------------------------------- setup
   if (threadIdx.x == 0) {

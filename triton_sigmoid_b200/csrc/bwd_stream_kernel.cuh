@@ -249,7 +249,8 @@ sigattn_bwd_stream_kernel(const __grid_constant__ CUtensorMap r1_map, const __gr
   const int lane = threadIdx.x & 31;
 
   // a kernel of this library already gave up on a wait: do not pile more work on a sick device
-  if (*reinterpret_cast<volatile int*>(&g_status_word) != 0) return;
+  // (one answer for the CTA: the word may change while its warps read it)
+  if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) return;
 
   // ---------------------------------------------------------------- setup
   if (threadIdx.x == 0) {

@@ -395,14 +395,12 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   const int lane = threadIdx.x & 31;
 
   // a kernel of this library already gave up on a wait: do not pile more work on a sick device
-  if constexpr (kSplit) {
-    // (one answer for the CTA; the others of the cluster may get another, and read this one's shared memory)
-    if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) {
+  // (one answer for the CTA: the word may change while its warps read it)
+  if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) {
+    if constexpr (kSplit) {  // (the others of the cluster may have got another one, and read this CTA's shared memory)
       cluster_sync();
       cluster_sync();
-      return;
     }
-  } else if (*reinterpret_cast<volatile int*>(&g_status_word) != 0) {
     return;
   }
 
