@@ -1,6 +1,8 @@
 """The float32 kernels on the tensor cores at the edges of their tiles (128 stationary rows, 64 streamed ones), against the
 float64 oracle with the gates of tests/test_f32_gpu.py."""
 
+import math
+
 import pytest
 import torch
 
@@ -111,3 +113,70 @@ def test_nonfinite_values_pass_through_probabilities_of_zero(bad, causal, D):
     assert dq[:, sees].isnan().all() and (dq[:, ~sees] == 0).all()
     at = torch.arange(T, device="cuda") == j
     assert dk[:, at].isnan().all() and (dk[:, ~at] == 0).all() and (dv == 0).all()
+
+
+def _against_float64(q, k, v, do, bias, causal=False, scale=None, more=0.0):
+    """Relative errors (2-norm) of O, dQ, dK, dV at most 1e-6 - the six products leave some 4e-7 over 2048 terms, the FMA kernels up
+    to 9e-7 - plus what the rounding of the logit costs (2^-24 of it, as a factor of the probability), plus half a unit of the
+    smallest float where the results are that small, plus `more`."""
+    B, T, H, D = q.shape
+    for backward in (False, True):
+        assert launch_form(B, H, T, T, D, torch.float32, backward) == FORM_F32_TC
+    scale = D ** -0.5 if scale is None else scale
+    leaf = [t.requires_grad_() for t in (q, k, v)]
+    out = sa.sigmoid_attention(*leaf, is_causal=causal, scale=scale, sigmoid_bias=bias)
+    got = (out,) + torch.autograd.grad(out, leaf, do)
+    qd, kd, vd, dd = (t.detach().double().transpose(1, 2) for t in (q, k, v, do))
+    x = qd @ kd.transpose(-1, -2) * scale + bias
+    p = torch.sigmoid(x)
+    if causal:
+        p = p.tril()
+    ds = p * torch.sigmoid(-x) * (dd @ vd.transpose(-1, -2))
+    ref = [t.transpose(1, 2) for t in (p @ vd, ds @ kd * scale, ds.transpose(-1, -2) @ qd * scale, p.transpose(-1, -2) @ dd)]
+    rounding = 2.0 ** -24 * x.clamp(max=0.0).abs().max().item()
+    for name, a, r in zip(("o", "dq", "dk", "dv"), got, ref):
+        smallest = 2.0 ** -150 / r.square().mean().sqrt().item()
+        assert rel_l2(a, r) <= 1e-6 + rounding + smallest + more, (name, rel_l2(a, r), rounding, smallest)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("which", ["q", "k", "v", "do"])
+@pytest.mark.parametrize("size", [1e-30, 1e-33, 1e-35, 1e-37, 1e-38])
+def test_small_values_keep_their_bits(size, which, D):
+    """bf16 parts of a float below 1e-33 reach into bf16's subnormal numbers."""
+    q, k, v, do = make_inputs(1, 520, 520, 8, D, torch.float32, std=0.5, seed=D)
+    t = dict(q=q, k=k, v=v, do=do)[which]
+    t *= size
+    if which in "qk":  # (the other one's gradient is as large as the scale, and must stay a float)
+        do *= 1e-3
+    _against_float64(q, k, v, do, -math.log(520.0), scale=1.0 / size if which in "qk" else None)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("bias", [-50.0, -75.0, -84.0, -87.0, -90.0, -95.0, -100.0])
+def test_probabilities_down_to_the_smallest_float(bias, D):
+    q, k, v, do = make_inputs(1, 520, 520, 8, D, torch.float32, std=0.5, seed=D)
+    _against_float64(q, k, v * 1e6, do * 1e6, bias)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("score", [-20.0, -60.0, -84.0, -87.0, -90.0, -95.0, -100.0])
+def test_large_scores(score, D):
+    """Every score is about that: one product of 64 or 128.  The tensor core cuts off its sum after each of the D / 16 steps,
+    up to 2^-23 of it."""
+    q, k, v, do = make_inputs(1, 520, 520, 8, D, torch.float32, std=0.5, seed=D)
+    q[..., 0] = 8.0
+    k[..., 0] = score * D ** 0.5 / 8
+    _against_float64(q, k, v * 1e6, do * 1e6, 0.0, more=D / 16 * 2.0 ** -23 * abs(score))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_scores_beyond_the_scaled_range(D):
+    """Sums that are floats, but not 2^32 times: 2e28, 2e29 and 4e29, which a small scale and a large bias make ordinary logits
+    of (-231000, -83000 and 83000)."""
+    q, k, v, do = make_inputs(1, 520, 520, 8, D, torch.float32, std=0.5, seed=D)
+    q[..., 0] = 2.0e14
+    k[..., 0] = torch.tensor([1.0e14, 1.0e15, 2.0e15], device="cuda").repeat(174)[:520][None, :, None]
+    scale = 2.0 ** -80
+    out = sa.sigmoid_attention(q, k, v, scale=scale, sigmoid_bias=-3.0e29 * scale)
+    assert rel_l2(out, v[:, 2::3].double().sum(1, keepdim=True).expand_as(out)) <= 1e-6

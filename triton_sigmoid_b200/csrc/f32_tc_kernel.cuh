@@ -1,8 +1,12 @@
 // fp32 on the tensor cores: forward, dK/dV and dQ of float32 tensors with every product done as six bf16 products.
 //
 // A float is the sum of three bf16 numbers, x = x0 + x1 + x2 (each the rounded remainder of the ones before it; 24 bits
-// and three signs lose nothing but subnormal tails), so x y = x0 y0 + (x0 y1 + x1 y0) + (x0 y2 + x1 y1 + x2 y0) up to terms
-// of 2^-27 |x y|: six products of the bf16 pipe, whose products of 8-bit significands are exact and whose sums are fp32.
+// and three signs lose nothing), so x y = x0 y0 + (x0 y1 + x1 y0) + (x0 y2 + x1 y1 + x2 y0) up to terms of 2^-24 |x y| (2^-27
+// RMS): six products of the bf16 pipe, whose products of 8-bit significands are exact and whose sums are fp32.
+// What is split is 2^16 times the value.  A bf16 number is a multiple of 2^-133 and a float one of 2^-149, so that the parts
+// are exact down to the smallest float; unscaled, the third one would begin to lose bits at 3e-33 and the first at 1e-38
+// (V of 1e-35: relative error of O 2.7e-6, of dQ 6e-4).  The factors are powers of two that the constants behind the products
+// take up.
 // The small terms go into the accumulator first, and an accumulator takes one tile of 64 streamed rows only: the sums over
 // tiles are made in registers, rounded to nearest, so that the tensor core's own summation never runs over more than
 // 64 terms.
@@ -37,7 +41,7 @@
 // backward); four conversion warps are 650 clocks per 64 x 64 chunk behind (D = 128 forward 118 us at B=2 H=8 T=2048 causal, 104
 // with eight; D = 64 the same), and more of them leave the compute warps too few registers.
 //
-// Values that the split cannot carry (infinities and NaN; finite ones within 2^-9 of the largest float) turn into NaN in
+// Values that the split cannot carry (infinities and NaN; finite ones from 2^112 on) and sums that overflow turn into NaN in
 // every result that they reach.  A CTA that finds an accumulator that is not finite computes its tile again with the FMA
 // code (f32_fwd_rows and so on), which gives what single precision gives.
 #pragma once
@@ -125,6 +129,10 @@ struct TcShape {
   static_assert(kDynBytes <= 232448, "shared memory budget");
 };
 
+// Powers of two that the operands carry: inputs and probabilities 2^16; so a score and dP 2^32, O and dV 2^32, dS 2^48, dQ and
+// dK 2^64.
+constexpr float kTcUp = 65536.0f, kTcDown = 1.0f / 65536.0f;
+
 // The three bf16 parts of 2 N floats, in packed pairs.
 template <int N>
 __device__ __forceinline__ void tc_split(const float (&x)[2 * N], uint32_t (&p0)[N], uint32_t (&p1)[N], uint32_t (&p2)[N]) {
@@ -140,14 +148,17 @@ __device__ __forceinline__ void tc_split(const float (&x)[2 * N], uint32_t (&p0)
   }
 }
 
-// Two sigmoids 1 / (1 + u), u = e^-x = 2^-y * factor: the bias is in the factor, e^-bias, so that y, which is rounded, is as
-// small as the scaled score.  (With the bias in y, as in the FMA kernels' logits, this rounding is most of the error of O: T=2048
-// 3.6e-7, T=256 causal dQ 3.6e-7.)  Infinite u gives 0, as it should.
-__device__ __forceinline__ float2 tc_sigmoid2(float2 minus_y, float factor) {
-  const float2 e = make_float2(ex2_approx(minus_y.x), ex2_approx(minus_y.y));
-  const float2 d = __ffma2_rn(e, make_float2(factor, factor), make_float2(1.0f, 1.0f));
+// Two sigmoids 1 / (1 + u), times kTcUp; u = e^-x = 2^y * factor: the bias is in the factor, e^-bias, so that y, which is
+// rounded, is as small as the scaled score.  (With the bias in y, as in the FMA kernels' logits, this rounding is most of the
+// error of O: T=2048 3.6e-7, T=256 causal dQ 3.6e-7.)  factor_down: factor * kTcDown.
+__device__ __forceinline__ float2 tc_sigmoid2(float2 y, float factor_down) {
+  const float2 e = make_float2(ex2_approx(y.x), ex2_approx(y.y));
+  const float2 d = __ffma2_rn(e, make_float2(factor_down, factor_down), make_float2(kTcDown, kTcDown));
   return make_float2(rcp_approx(d.x), rcp_approx(d.y));
 }
+// The same where u, from 2^120 on, would end up beyond the floats: 2^-y / factor.  below = 2^-24 / factor.  (Probabilities go
+// on to the smallest float this way, as in the FMA kernels.)
+__device__ __forceinline__ float tc_sigmoid_tiny(float y, float below) { return ex2_approx(40.0f - y) * below; }
 
 template <int D, int kMode>
 __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32Params p, const int n_tiles) {
@@ -177,21 +188,23 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
   auto out_row = [&](float* base, int64_t sb, int64_t st, int64_t sh, int t0) -> float* {
     return base + (int64_t)it.bc * sb + (int64_t)it.h * sh + (int64_t)(t0 + row) * st + cg * kOutPer;
   };
-  auto store = [&](float* dst, const float (&acc)[kOutPer], float mul) {
+  auto store = [&](float* dst, const float (&acc)[kOutPer], float down, float mul) {
 #pragma unroll
     for (int c = 0; c < kOutPer; c += 4) {
       if (cg * kOutPer + c >= p.d_cols) continue;
-      float4 w = make_float4(acc[c] * mul, acc[c + 1] * mul, acc[c + 2] * mul, acc[c + 3] * mul);
+      // (two factors: their product may be too small for a float)
+      float4 w = make_float4(acc[c] * down * mul, acc[c + 1] * down * mul, acc[c + 2] * down * mul, acc[c + 3] * down * mul);
       if (row >= Lr) w = make_float4(0.f, 0.f, 0.f, 0.f);
       *reinterpret_cast<float4*>(dst + c) = w;
     }
   };
   auto store_all = [&](const float (&a1)[kOutPer], const float (&a2)[kOutPer]) {
     if (row >= row_lim) return;
-    if constexpr (kMode == kTcFwd) store(out_row(p.o, p.o_sb, p.o_st, p.o_sh, it.tq0), a2, 1.0f);
-    if constexpr (L::kKeyRows && L::kOut1) store(out_row(p.dk, p.dk_sb, p.dk_st, p.dk_sh, it.tk0), a1, p.scale);
-    if constexpr (L::kKeyRows && L::kOut2) store(out_row(p.dv, p.dv_sb, p.dv_st, p.dv_sh, it.tk0), a2, 1.0f);
-    if constexpr (kMode == kTcDq) store(out_row(p.dq, p.dq_sb, p.dq_st, p.dq_sh, it.tq0), a1, p.scale);
+    constexpr float kDown2 = kTcDown * kTcDown, kDown4 = kDown2 * kDown2;
+    if constexpr (kMode == kTcFwd) store(out_row(p.o, p.o_sb, p.o_st, p.o_sh, it.tq0), a2, kDown2, 1.0f);
+    if constexpr (L::kKeyRows && L::kOut1) store(out_row(p.dk, p.dk_sb, p.dk_st, p.dk_sh, it.tk0), a1, kDown4, p.scale);
+    if constexpr (L::kKeyRows && L::kOut2) store(out_row(p.dv, p.dv_sb, p.dv_st, p.dv_sh, it.tk0), a2, kDown2, 1.0f);
+    if constexpr (kMode == kTcDq) store(out_row(p.dq, p.dq_sb, p.dq_st, p.dq_sh, it.tq0), a1, kDown4, p.scale);
   };
   if (n_jobs == 0) {  // nothing is visible to these rows
     if (warp < kTcComputeWarps) {
@@ -405,7 +418,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const float4 x = got[u * 256];
-        const float f[4] = {x.x, x.y, x.z, x.w};
+        const float2 lo = __fmul2_rn(make_float2(x.x, x.y), make_float2(kTcUp, kTcUp));
+        const float2 hi = __fmul2_rn(make_float2(x.z, x.w), make_float2(kTcUp, kTcUp));
+        const float f[4] = {lo.x, lo.y, hi.x, hi.y};
         uint32_t p0[2], p1[2], p2[2];
         tc_split<2>(f, p0, p1, p2);
         uint8_t* dst = tile + u * 2048;
@@ -435,7 +450,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
         for (int c = 0; c < 16; c += 4) {
           const float4 w = row < Lr && 16 * kk + c < p.d_cols ? __ldg(reinterpret_cast<const float4*>(src + 16 * kk + c))
                                                                : make_float4(0.f, 0.f, 0.f, 0.f);
-          f[c] = w.x; f[c + 1] = w.y; f[c + 2] = w.z; f[c + 3] = w.w;
+          f[c] = w.x * kTcUp; f[c + 1] = w.y * kTcUp; f[c + 2] = w.z * kTcUp; f[c + 3] = w.w * kTcUp;
         }
         uint32_t part[3][8];
         tc_split<8>(f, part[0], part[1], part[2]);
@@ -469,7 +484,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
     // beyond that remains in the exponent
     const float bias = item_bias(p.bias, p.bias_scalar, it.b, it.Lk) + row_mod;
     const float bias_in = fminf(fmaxf(bias, -44.0f), 0.0f);
-    const float factor = expf(-bias_in), y1 = -p.scale * kLog2, y0 = (bias_in - bias) * kLog2;
+    const float factor = expf(-bias_in), factor_down = factor * kTcDown;
+    const float y1 = -p.scale * (kLog2 * kTcDown * kTcDown), y0 = (bias_in - bias) * kLog2;
+    const float y_most = 120.0f + bias_in * kLog2;  // (u = 2^120)
     const float* col_mod = L::kKeyRows ? nullptr : sm;
     const int lo = L::kKeyRows && p.causal ? row : 0;  // visible columns of this row: [lo, hi)
     const int hi = !L::kKeyRows && p.causal ? min(Lc, row + 1) : Lc;
@@ -537,6 +554,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
         uint32_t r[16];
         tmem_ld(slot + 16 * cg, r);
         tmem_ld_wait_for(r);
+        float most = 0.f;
 #pragma unroll
         for (int c = 0; c < 16; c += 2) {
           float2 y = __ffma2_rn(make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])), make_float2(y1, y1), make_float2(y0, y0));
@@ -544,9 +562,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
             y.x = fmaf(col0 + c < it.key_lim ? __ldg(col_mod + col0 + c) : 0.f, -kLog2, y.x);
             y.y = fmaf(col0 + c + 1 < it.key_lim ? __ldg(col_mod + col0 + c + 1) : 0.f, -kLog2, y.y);
           }
-          const float2 w = tc_sigmoid2(y, factor);
-          pr[c] = w.x;
-          pr[c + 1] = w.y;
+          most = fmaxf(most, fmaxf(fabsf(y.x), fabsf(y.y)));
+          pr[c] = y.x;
+          pr[c + 1] = y.y;
+        }
+        if (!__any_sync(0xffffffffu, most > y_most)) {
+#pragma unroll
+          for (int c = 0; c < 16; c += 2) {
+            const float2 w = tc_sigmoid2(make_float2(pr[c], pr[c + 1]), factor_down);
+            pr[c] = w.x;
+            pr[c + 1] = w.y;
+          }
+        } else {  // scores so large that a probability is next to 0 or 1, or that their sum has overflowed
+          const float below = 5.9604644775390625e-8f / factor;
+          tmem_ld(slot + 16 * cg, r);
+          tmem_ld_wait_for(r);
+#pragma unroll
+          for (int c = 0; c < 16; ++c) {
+            const float w = pr[c] > y_most ? tc_sigmoid_tiny(pr[c], below) : rcp_approx(fmaf(ex2_approx(pr[c]), factor_down, kTcDown));
+            pr[c] = fmaf(__uint_as_float(r[c]), 0.f, w);  // (NaN for an infinite sum)
+          }
         }
         if (mask) {
 #pragma unroll
@@ -569,7 +604,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
 #pragma unroll
         for (int c = 0; c < 16; c += 2) {
           const float2 w = make_float2(pr[c], pr[c + 1]);
-          const float2 v = __ffma2_rn(w, make_float2(-1.0f, -1.0f), make_float2(1.0f, 1.0f));
+          const float2 v = __ffma2_rn(w, make_float2(-kTcDown, -kTcDown), make_float2(1.0f, 1.0f));
           const float2 ds = __fmul2_rn(__fmul2_rn(w, v), make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])));
           pr[c] = ds.x;
           pr[c + 1] = ds.y;

@@ -5,6 +5,7 @@
 #include <stdarg.h>
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 #include <stdio.h>
 #include <string.h>
@@ -688,6 +689,8 @@ int launch_f32_tc(const SigAttnParams* p, const sigattn::F32Params& fp) {
 bool f32_tc(const SigAttnParams* p, bool backward) {
   const int64_t Tq = p->Tq, Tk = p->Tk, longer = std::max(Tq, Tk);
   if (Tk < 64 || Tq < 16 || longer < 256) return false;
+  // (the kernels' factor of the score is 2^-31.5 scale, which must not be a subnormal number)
+  if (p->scale != 0.0f && !(std::abs(p->scale) >= 1e-25f)) return false;
   const int64_t tiles = (int64_t)p->B * p->H * (((backward ? (Tq + Tk) / 2 : Tq) + 63) / 64);
   if (p->D == 128) return backward ? tiles >= 96 || (tiles >= 64 && longer >= 512) : tiles >= 72 || Tk >= 512;
   return tiles >= 64 || longer >= (backward ? 384 : 512);
