@@ -189,11 +189,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
     return base + (int64_t)it.bc * sb + (int64_t)it.h * sh + (int64_t)(t0 + row) * st + cg * kOutPer;
   };
   auto store = [&](float* dst, const float (&acc)[kOutPer], float down, float mul) {
+    // acc * down * mul; in one factor, if that is not too small for a float, since acc * down may be
+    const bool one = fabsf(down * mul) >= 1.1754944e-38f;
+    const float m1 = one ? down * mul : down, m2 = one ? 1.0f : mul;
 #pragma unroll
     for (int c = 0; c < kOutPer; c += 4) {
       if (cg * kOutPer + c >= p.d_cols) continue;
-      // (two factors: their product may be too small for a float)
-      float4 w = make_float4(acc[c] * down * mul, acc[c + 1] * down * mul, acc[c + 2] * down * mul, acc[c + 3] * down * mul);
+      float4 w = make_float4(acc[c] * m1 * m2, acc[c + 1] * m1 * m2, acc[c + 2] * m1 * m2, acc[c + 3] * m1 * m2);
       if (row >= Lr) w = make_float4(0.f, 0.f, 0.f, 0.f);
       *reinterpret_cast<float4*>(dst + c) = w;
     }
