@@ -49,3 +49,33 @@ def test_padded_and_by_head(B, H, T, form, D):
     for a, r in zip((out,) + grads, (ref,) + ref_g):
         assert a.isfinite().all() and (a.masked_select(~valid) == 0).all()
         assert ((a.float() - r).norm() / r.norm()).item() <= 1e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("every", [0, 700, 96, 40])
+def test_scores_far_below_zero_without_a_bias(every, D, dtype):
+    """Logits about -10 take the short series, whose leading term is exact, also where the scores make them: no common factor on the
+    probabilities beyond what the 16-bit type leaves (the polynomial for all logits has 3.0e-4 in fp16 and 1.7e-3 in bf16 there;
+    the series in 16 bits at most e^-10 = 4.5e-5, plus the mean of some 10^6 roundings).  `every`: that many keys apart one at a score
+    of 0, so that tests for the series fail now and then."""
+    B, T, H = 4, 1300, 8
+    q, k, v, do = make_inputs(B, T, T, H, D, dtype, std=0.4, seed=D + every)
+    q[..., 0] = 8.0
+    k[..., 0] = -10.0 * D ** 0.5 / 8
+    if every:
+        k[:, 5::every, :, 0] = 0.0
+    v += 1.0
+    leaf = [t.requires_grad_() for t in (q, k, v)]
+    out = m.sigmoid_attention(*leaf, sigmoid_bias=0.0)
+    got = (out,) + torch.autograd.grad(out, leaf, do)
+    qd, kd, vd, dd = (t.detach().double().transpose(1, 2) for t in (q, k, v, do))
+    p = torch.sigmoid(qd @ kd.transpose(-1, -2) / D ** 0.5)
+    ds = p * (1 - p) * (dd @ vd.transpose(-1, -2)) / D ** 0.5
+    ref = [t.transpose(1, 2) for t in (p @ vd, ds @ kd, ds.transpose(-1, -2) @ qd, p.transpose(-1, -2) @ dd)]
+    rel, factor = {torch.float16: (1e-3, 1.5e-4), torch.bfloat16: (6e-3, 6e-4)}[dtype]
+    for name, a, r in zip(("o", "dq", "dk", "dv"), got, ref):
+        a = a.double()
+        assert ((a - r).norm() / r.norm()).item() <= rel, name
+        if not every:
+            assert abs((a * r).sum() / (r * r).sum() - 1).item() <= factor, name

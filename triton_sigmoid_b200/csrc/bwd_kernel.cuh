@@ -147,11 +147,11 @@ struct BwdSmem {
 // of the 32 columns read (the operand of dV).  Both phases move 16 columns at a time, so that besides the 32
 // probabilities only few registers are live.
 // q0 = query index of the first column; valid queries for this key row are [q_lo, q_hi).
-template <bool kBF16, bool kMask, bool kAccurate, bool kDeep>
+template <bool kBF16, bool kMask, bool kAccurate, DeepTest kTest>
 __device__ __forceinline__ void bwd_phase_a(uint32_t s_addr, float c1, float c0, int q0, int q_lo, int q_hi,
-                                            float2 (&pv)[16]) {
-  // unmasked tiles work on logits shifted up by kDeepShift (see sigmoid2_from_shifted_log2_deep)
-  const float c0s = (kMask || kAccurate || !kDeep) ? c0 : c0 + kDeepShift;
+                                            float2 (&pv)[16], DeepWatch& watch) {
+  // tested tiles work on logits shifted up by kDeepShift (see sigmoid2_from_shifted_log2_deep)
+  const float c0s = kTest == kNoTest ? c0 : c0 + kDeepShift;
   {
     uint32_t r[32];
     tmem_ld32_sync(s_addr, r);
@@ -182,15 +182,17 @@ __device__ __forceinline__ void bwd_phase_a(uint32_t s_addr, float c1, float c0,
   if constexpr (kAccurate) {
     // exponential and reciprocal both on the special-function unit (see sigmoid2_accurate_from_log2)
     emit([](float2 x) { return sigmoid2_accurate_from_log2(x); });
-  } else if (!kMask && kDeep && warp_all_negative(pv)) {
+  } else if (kTest != kNoTest && warp_all_negative(pv)) {
+    watch.passed();
     // all logits far below zero (the usual case under the default bias): short series, no compare / select per element
     emit([](float2 x) { return sigmoid2_from_shifted_log2_deep<kBF16>(x); });
   } else {
     bool all_neg = false;
-    if constexpr (!kMask && kDeep) {
+    if constexpr (kTest != kNoTest) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) pv[i] = __fadd2_rn(pv[i], make_float2(-kDeepShift, -kDeepShift));
-      all_neg = warp_all_negative(pv);  // negative but not far below zero: full polynomial, still no select
+      if constexpr (kTest == kTestAll) all_neg = warp_all_negative(pv);  // negative but not far below zero: full polynomial, still no select
+      else watch.failed();
     }
     if (all_neg) emit([](float2 x) { return sigmoid2_from_log2_neg<kBF16>(x); });
     else         emit([](float2 x) { return sigmoid2_from_log2<kBF16>(x); });
@@ -233,13 +235,13 @@ __device__ __forceinline__ void bwd_phase_b(uint32_t dp_addr, uint32_t ds_line, 
 // (32 registers per thread that the drain warps' share of the register file cannot spare) but read back
 // from TMEM in the 16-bit form they were stored in for the dV product, and dS = P (1 - P) dP is formed on
 // packed 16-bit pairs.
-template <bool kBF16, bool kMask, bool kAccurate, bool kDeep>
-__device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c0, int q0, int q_lo, int q_hi) {
+template <bool kBF16, bool kMask, bool kAccurate, DeepTest kTest>
+__device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c0, int q0, int q_lo, int q_hi, DeepWatch& watch) {
   uint32_t r[32];
   tmem_ld32_sync(s_addr, r);
   uint32_t pk[16];
   float2 t[16];
-  const float c0s = (kMask || kAccurate || !kDeep) ? c0 : c0 + kDeepShift;
+  const float c0s = kTest == kNoTest ? c0 : c0 + kDeepShift;
 #pragma unroll
   for (int i = 0; i < 16; ++i)
     t[i] = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), make_float2(c1, c1),
@@ -255,16 +257,18 @@ __device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c
       }
       pk[i] = pack2<kBF16>(pe.x, pe.y);
     }
-  } else if (!kMask && kDeep && warp_all_negative(t)) {
+  } else if (kTest != kNoTest && warp_all_negative(t)) {
+    watch.passed();
     // all logits far below zero (the usual case under the default bias): short series on packed pairs
 #pragma unroll
     for (int i = 0; i < 16; ++i) pk[i] = sigmoid2_deep_packed<kBF16>(t[i], false);
   } else {
     bool all_neg = false;
-    if constexpr (!kMask && kDeep) {
+    if constexpr (kTest != kNoTest) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) t[i] = __fadd2_rn(t[i], make_float2(-kDeepShift, -kDeepShift));
-      all_neg = warp_all_negative(t);
+      if constexpr (kTest == kTestAll) all_neg = warp_all_negative(t);
+      else watch.failed();
     }
     if (all_neg) {
 #pragma unroll
@@ -1009,6 +1013,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     int g = 0;    // query tiles processed so far (all items)
     int act = 0;  // items with work so far
     bool ok = true;
+    DeepWatch watch;
 
     for (int k = 0; ok; ++k) {
       BwdItem it;
@@ -1050,13 +1055,18 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         const uint32_t s_addr = s_addr0 + 128u * (uint32_t)sbuf(gt);
         if (!ok) break;
         tc_fence_after_sync();
+        constexpr DeepTest kTest = kDeep && !kAccurate ? kTestAll : kNoTest;
+        const bool test_now = !kDeep && !kAccurate && watch.due();
         if constexpr (D == 64) {
-          if (need_mask) bwd_phase_a16<kBF16, true, kAccurate, kDeep>(s_addr, c1, c0, q0, q_lo, q_hi);
-          else           bwd_phase_a16<kBF16, false, kAccurate, kDeep>(s_addr, c1, c0, q0, q_lo, q_hi);
+          if (need_mask)     bwd_phase_a16<kBF16, true, kAccurate, kNoTest>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
+          else if (test_now) bwd_phase_a16<kBF16, false, kAccurate, kTestNow>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
+          else               bwd_phase_a16<kBF16, false, kAccurate, kTest>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
         } else {
-          if (need_mask) bwd_phase_a<kBF16, true, kAccurate, kDeep>(s_addr, c1, c0, q0, q_lo, q_hi, pv);
-          else           bwd_phase_a<kBF16, false, kAccurate, kDeep>(s_addr, c1, c0, q0, q_lo, q_hi, pv);
+          if (need_mask)     bwd_phase_a<kBF16, true, kAccurate, kNoTest>(s_addr, c1, c0, q0, q_lo, q_hi, pv, watch);
+          else if (test_now) bwd_phase_a<kBF16, false, kAccurate, kTestNow>(s_addr, c1, c0, q0, q_lo, q_hi, pv, watch);
+          else               bwd_phase_a<kBF16, false, kAccurate, kTest>(s_addr, c1, c0, q0, q_lo, q_hi, pv, watch);
         }
+        if (!kDeep && !need_mask && !test_now) watch.skipped();
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();

@@ -357,10 +357,14 @@ int fwd_split(const SigAttnParams* p, int n_sm) {
   return split > 1 ? split : 0;
 }
 
-// Whether the 16-bit kernels leave out the test for logits far below zero (below -3.5, all 1024 of a warp's chunk): with a bias of
-// the caller's, the same for the whole batch and above -3, scores would have to be below zero throughout to pass it.
-// Bias 0, B=4 T=4096 H=32 D=64, forward: 944 -> 787 us; H=16, forward and backward: 467 and 850 -> 366 and 815, D=128 580 and 1540 ->
-// 462 and 1350.  (Choosing by the chunk before, at run time: 879, and 1.4 % more with the default bias, whose chunks pass.)
+// Whether the 16-bit kernels test for logits far below zero (below -3.5, all 1024 of a warp's chunk) only while chunks pass, instead
+// of always: with a bias of the caller's, the same for the whole batch and above -3, scores would have to be below zero
+// throughout to pass.  D = 64 or D = 128, B=4 T=4096, bf16, bias 0, always -> while it pays, us, forward (H=32, H=16) and with the backward:
+//  - scores of both signs, D = 64 924 -> 740 and 2560 -> 2340; D = 128 582 -> 545 and 1904 -> 1880.  Never tested 725 and 2290, 500 and 1830;
+//  - scores about -8, which trained weights may well have, D = 64 755 -> 778, 2260 -> 2310; D = 128 507 -> 520, 1870 -> 1880.  Never tested 810
+//    and 2430, 530 and 1910, and probabilities that are all too small by what the polynomial lacks at 0 (see rcp1p_poly);
+//  - about -8 with every 512th key at 0 (a quarter of the chunks fails): 745 -> 790.
+// The default bias takes the form that always tests: its chunks pass, and are 3 % slower in the other form (second line).
 bool few_deep_logits(const SigAttnParams* p) {
   return !p->bias && !p->score_mod && !(p->flags & (SIGATTN_ACCURATE | SIGATTN_BIAS_NEG_LOG_LK)) && p->bias_scalar > -3.0f;
 }

@@ -83,6 +83,19 @@ __device__ __forceinline__ bool warp_all_negative(const float2 (&t)[N]) {
   return __all_sync(0xffffffffu, (int)sgn < 0) != 0;
 }
 
+// Whether a warp's next chunk is tested for logits far below zero, in the forms without kDeep.  After a test that failed, 1, 3,
+// 7, 15 and then always 31 chunks go untested, after one that passed none.
+struct DeepWatch {
+  int state = 0;  // chunks to go untested, + 256 times as many as that were after the last failure
+  __device__ __forceinline__ bool due() const { return (state & 255) == 0; }
+  __device__ __forceinline__ void passed() { state = 0; }
+  __device__ __forceinline__ void failed() { state = 257 * min(2 * (state >> 8) + 1, 31); }
+  __device__ __forceinline__ void skipped() { --state; }
+};
+// What the code of one chunk does about it: no test; a test, and the shorter form for logits that are all negative where it
+// fails; a test alone, where most fail.
+enum DeepTest { kNoTest, kTestAll, kTestNow };
+
 // ---------------------------------------------------------------- cheaper forms for the deep regime
 // 2^u for u <= 0 without the MUFU unit: floor(u) by the magic-number addition (rounded down, so the low
 // mantissa bits of the sum hold the integer part), a minimax polynomial of the fraction (degree 3:
