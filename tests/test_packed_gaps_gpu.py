@@ -59,3 +59,27 @@ def test_no_sequences_at_all():
     _poison((500, 2, 64), torch.float16)
     for t in (out,) + torch.autograd.grad(out, leaf, torch.ones_like(out)):
         assert (t == 0).all()
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 1025, 5000])
+@pytest.mark.parametrize("H,D", [(1, 64), (3, 40), (9, 128)])
+def test_many_short_sequences(n, H, D):
+    """Every warp of the kernel that zeroes the gaps searches for its part of the offsets, and many parts hold several gaps."""
+    cut, front, behind = 24, 5, 4000 if n == 33 else 3
+    g = torch.Generator().manual_seed(n)
+    lens = torch.randint(0, 41, (n,), generator=g)
+    lens[0] = 41
+    cu = torch.cat([torch.zeros(1, dtype=torch.long), lens.cumsum(0)]) + front
+    rows = int(cu[-1]) + behind
+    at = torch.arange(rows)
+    seq = (torch.searchsorted(cu, at, right=True) - 1).clamp(0, n - 1)
+    inside = ((at >= front) & (at < cu[-1]) & (at - cu[seq] < cut)).cuda()
+    cu = cu.int().cuda()
+    leaf = [(torch.randn(rows, H, D, device="cuda") * 0.5).bfloat16().requires_grad_() for _ in range(3)]
+    do = torch.randn(rows, H, D, device="cuda").bfloat16()
+    _poison((rows, H, D), torch.bfloat16)
+    out = sa.sigmoid_attention_varlen(*leaf, cu, cu, cut, cut)
+    _poison((rows, H, D), torch.bfloat16)
+    for t in (out,) + torch.autograd.grad(out, leaf, do):
+        assert (t[~inside] == 0).all() and t.isfinite().all()
+        assert (t[inside] != 0).any(dim=-1).all()
