@@ -165,12 +165,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
   using L = TcShape<D, kMode>;
   constexpr int kSite = (0x6 + kMode) << 16;
   extern __shared__ uint8_t tc_smem[];
-  // a kernel of this library already gave up on a wait: leave, all warps or none (the named barriers below count on every warp,
-  // and the word may change while they read it)
-  if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) return;
 
   // ---------------------------------------------------------------- the tile
   const F32Item it = f32_item(p, n_tiles, !L::kKeyRows);
+  // a kernel of this library already gave up on a wait: leave, all warps or none (the named barriers below count on every warp,
+  // and the word may change while they read it)
+  if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) return;
   const int r0 = it.tile * kTcRows;
   const int Lr = L::kKeyRows ? it.Lk : it.Lq, Lc = L::kKeyRows ? it.Lq : it.Lk;
   const int row_lim = L::kKeyRows ? it.key_lim : it.row_lim;
@@ -208,11 +208,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
     if constexpr (L::kKeyRows && L::kOut2) store(out_row(p.dv, p.dv_sb, p.dv_st, p.dv_sh, it.tk0), a2, kDown2, 1.0f);
     if constexpr (kMode == kTcDq) store(out_row(p.dq, p.dq_sb, p.dq_st, p.dq_sh, it.tq0), a1, kDown4, p.scale);
   };
-  if (n_jobs == 0) {  // nothing is visible to these rows
-    if (warp < kTcComputeWarps) {
-      const float zero[kOutPer] = {};
-      store_all(zero, zero);
-    }
+  if (n_jobs == 0) {  // nothing is visible to these rows: zeros, by whole rows
+    const int pieces = p.d_cols / 4, rows = min(kTcRows, row_lim - r0);
+    auto zero = [&](float* base, int64_t sb, int64_t st, int64_t sh, int t0) {
+      base += (int64_t)it.bc * sb + (int64_t)it.h * sh + (int64_t)(t0 + r0) * st;
+      for (int i = threadIdx.x; i < rows * pieces; i += kTcThreads)
+        *reinterpret_cast<float4*>(base + (i / pieces) * st + 4 * (i % pieces)) = make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    if constexpr (kMode == kTcFwd) zero(p.o, p.o_sb, p.o_st, p.o_sh, it.tq0);
+    if constexpr (L::kKeyRows && L::kOut1) zero(p.dk, p.dk_sb, p.dk_st, p.dk_sh, it.tk0);
+    if constexpr (L::kKeyRows && L::kOut2) zero(p.dv, p.dv_sb, p.dv_st, p.dv_sh, it.tk0);
+    if constexpr (kMode == kTcDq) zero(p.dq, p.dq_sb, p.dq_st, p.dq_sh, it.tq0);
     return;
   }
 
