@@ -29,3 +29,20 @@ from triton_sigmoid_b200._cabi import FORM_F32_16, FORM_F32_64, FORM_F32_TC
 def test_form(B, H, Tq, Tk, D, forward, backward):
     for is_backward, want in ((False, forward), (True, backward)):
         assert launch_form(B, H, Tq, Tk, D, torch.float32, is_backward, n_sm=148) == want
+
+
+@pytest.mark.parametrize("D,causal,mean,forward,backward", [
+    (64, False, 79, FORM_F32_64, FORM_F32_64),
+    (64, False, 80, FORM_F32_64, FORM_F32_TC),
+    (64, False, 95, FORM_F32_64, FORM_F32_TC),
+    (64, False, 96, FORM_F32_TC, FORM_F32_TC),
+    (64, True, 191, FORM_F32_64, FORM_F32_TC),
+    (64, True, 192, FORM_F32_TC, FORM_F32_TC),
+    (128, False, 32, FORM_F32_TC, FORM_F32_64),
+    (128, True, 80, FORM_F32_TC, FORM_F32_TC),
+])
+def test_mean_length_of_packed_sequences(D, causal, mean, forward, backward):
+    """Many sequences, the longest of 1024: the mean length decides.  Few: the longest."""
+    for is_backward, want in ((False, forward), (True, backward)):
+        assert launch_form(1000, 8, 1024, 1024, D, torch.float32, is_backward, causal, packed_rows=1000 * mean, n_sm=148) == want
+        assert launch_form(20, 8, 1024, 1024, D, torch.float32, is_backward, causal, packed_rows=20 * mean, n_sm=148) == FORM_F32_TC

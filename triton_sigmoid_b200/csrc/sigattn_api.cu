@@ -723,11 +723,23 @@ int launch_f32_tc(const SigAttnParams* p, const sigattn::F32Params& fp) {
 //  - D = 128 forward: T=256 0.36 - 0.69 from 148 tiles on, 0.88 at 64 and 1.05 there with a causal mask, 1.3 below; Tk = 512 0.98;
 //    backward (three kernels): 0.35 - 0.71 from 96 tiles on, 0.76 - 0.89 at 64 with T >= 512 (causal 0.94 - 1.06), 1.1 - 1.6 below.
 //  - below 256 rows on both sides 0.5 - 2.2, and below 64 keys or 16 queries mostly padding: FMA kernels.
-bool f32_tc(const SigAttnParams* p, bool backward) {
+//  - packed sequences that are shorter on average than a tile is worth, whatever the longest one, once the rows are so many that the FMA
+//    kernels are not waiting for that one alone (as many per SM as it has).  Forward D = 64, mean length 32 and 64 1.9 - 2.0, 96
+//    0.95 - 1.03 and 128 0.98 - 1.09, causal 96 1.17, 128 1.2, 192 1.00 - 1.04, 256 0.76; D = 128 0.87 - 0.97 from 32 on; backward 64
+//    1.25 - 1.39 and 1.23, 96 0.66 - 0.69 and 0.73 (causal 0.82).  With one of 1024 among few of 64, 0.66 and 0.61 (step).
+//    (Padded ones, whose lengths the host does not know, go by the padded extents.  Where a tenth or less of those is filled they are slower than
+//    the FMA kernels: T=1024 B=128 H=8 filled to 48, D = 64 forward 1.28, with the backward 1.09, D = 128 0.88 and 0.97; T=512 B=256 to 40 1.65
+//    and 1.37, 1.09 and 1.23; to 200 of 1024 0.56 and 0.47, 0.43 and 0.49; full 0.26, 0.26, 0.21 and 0.28.)
+bool f32_tc(const SigAttnParams* p, bool backward, int n_sm) {
   const int64_t Tq = p->Tq, Tk = p->Tk, longer = std::max(Tq, Tk);
   if (Tk < 64 || Tq < 16 || longer < 256) return false;
   // (the kernels' factor of the score is 2^-31.5 scale, which must not be a subnormal number)
   if (p->scale != 0.0f && !(std::abs(p->scale) >= 1e-25f)) return false;
+  if (p->cu_seqlens_q && (backward || p->D == 64)) {
+    const int64_t rows = std::max(p->total_q, p->total_k);  // B sequences of `line` would have more
+    const int64_t line = backward ? 80 : (p->flags & SIGATTN_CAUSAL) ? 192 : 96;
+    if (rows < line * p->B && rows * p->H >= n_sm * longer) return false;
+  }
   const int64_t tiles = (int64_t)p->B * p->H * (((backward ? (Tq + Tk) / 2 : Tq) + 63) / 64);
   if (p->D == 128) return backward ? tiles >= 96 || (tiles >= 64 && longer >= 512) : tiles >= 72 || Tk >= 512;
   return tiles >= 64 || longer >= (backward ? 384 : 512);
@@ -778,7 +790,7 @@ int launch_f32_d(const SigAttnParams* p, bool backward) {
   if (int rc = zero_gaps(p, backward, info.n_sm)) return rc;
   if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
   int rc = 0;
-  if (f32_tc(p, backward)) {
+  if (f32_tc(p, backward, info.n_sm)) {
     if (!backward) {
       rc = launch_f32_tc<D, kTcFwd>(p, fp);
     } else {
@@ -854,7 +866,7 @@ int sigattn_form(const SigAttnParams* p, int backward, int n_sm) {
   if (p->struct_bytes != sizeof(SigAttnParams)) return fail(-1, "struct_bytes %u != sizeof(SigAttnParams) %zu (ABI mismatch)", p->struct_bytes, sizeof(SigAttnParams));
   if (n_sm < 1) return fail(-2, "n_sm must be positive, got %d", n_sm);
   if (p->dtype == SIGATTN_FP32) {
-    if (f32_tc(p, backward != 0)) return SIGATTN_FORM_F32_TC;
+    if (f32_tc(p, backward != 0, n_sm)) return SIGATTN_FORM_F32_TC;
     return f32_tile_rows(p, n_sm) == 64 ? SIGATTN_FORM_F32_64 : SIGATTN_FORM_F32_16;
   }
   if (!backward) return fwd_split(p, n_sm) ? SIGATTN_FORM_FWD_SPLIT : SIGATTN_FORM_FWD;
