@@ -130,8 +130,8 @@ typedef struct SigAttnParams {
    * there), the batch strides are ignored, seq_lens_* must be NULL, score_mod is [total_k], the backward
    * workspace is sigattn_bwd_workspace_bytes(1, total_q, H, D) bytes (none for fp32), and only rows of
    * the sequences are written: rows of q-side / k-side tensors that belong to no sequence (gaps, rows behind
- * the last sequence, rows of a sequence beyond Tq / Tk) are left untouched in o, dq, dk, dv - pre-zero
- * them if they are read afterwards. */
+   * the last sequence, rows of a sequence beyond Tq / Tk) are left untouched in o, dq, dk, dv - unless SIGATTN_ZERO_GAPS is
+   * set, pre-zero them if they are read afterwards. */
   const int32_t *cu_seqlens_q; /* [B+1] device, non-decreasing, cu_seqlens_q[B] <= total_q */
   const int32_t *cu_seqlens_k; /* [B+1] device */
   int32_t total_q, total_k;

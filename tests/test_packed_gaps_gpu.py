@@ -83,3 +83,16 @@ def test_many_short_sequences(n, H, D):
     for t in (out,) + torch.autograd.grad(out, leaf, do):
         assert (t[~inside] == 0).all() and t.isfinite().all()
         assert (t[inside] != 0).any(dim=-1).all()
+
+
+def test_debug_mode_poisons_packed_outputs_too(monkeypatch):
+    """Outputs of packed calls are made from memory that nobody has cleared: a row that no kernel writes has to show."""
+    monkeypatch.setenv("SIGATTN_B200_DEBUG", "1")
+    leaf = [torch.randn(300, 2, 64, device="cuda", dtype=torch.float16).requires_grad_() for _ in range(3)]
+    cu = torch.tensor([0, 100, 300], dtype=torch.int32, device="cuda")
+    do = torch.randn(300, 2, 64, device="cuda", dtype=torch.float16)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as seen:
+        out = sa.sigmoid_attention_varlen(*leaf, cu, cu, 200, 200)
+        grads = torch.autograd.grad(out, leaf, do)
+    assert sum(e.name == "aten::fill_" for e in seen.events()) == 4
+    assert all(t.isfinite().all() and (t != 0).any(dim=-1).all() for t in (out,) + grads)

@@ -170,7 +170,7 @@ void fill_common(SigAttnParams& p, const Tensors& t, const Call& c, const Switch
 // is synchronised and checked after the launch.
 void launch(int (*fn)(const SigAttnParams*), const SigAttnParams& p, const char* what, bool debug,
             std::initializer_list<Tensor*> outs) {
-  if (debug && !p.cu_seqlens_q)
+  if (debug && (!p.cu_seqlens_q || (p.flags & SIGATTN_ZERO_GAPS)))  // (calls that write every row)
     for (Tensor* t : outs) t->fill_(std::nan(""));
   const int rc = fn(&p);
   TORCH_CHECK(rc == 0, what, " failed (code ", rc, "): ", g_abi.last_error());
