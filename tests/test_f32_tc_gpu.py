@@ -115,9 +115,9 @@ def test_nonfinite_values_pass_through_probabilities_of_zero(bad, causal, D):
     assert dk[:, at].isnan().all() and (dk[:, ~at] == 0).all() and (dv == 0).all()
 
 
-def _against_float64(q, k, v, do, bias, causal=False, scale=None, more=0.0):
+def _against_float64(q, k, v, do, bias, causal=False, scale=None, more=0.0, logits=True):
     """Relative errors (2-norm) of O, dQ, dK, dV at most 1e-6 - the six products leave some 4e-7 over 2048 terms, the FMA kernels up
-    to 9e-7 - plus what the rounding of the logit costs (2^-24 of it, as a factor of the probability), plus half a unit of the
+    to 9e-7 - plus what the rounding of the logit costs (2^-24 of it, as a factor of the probability; `logits`), plus half a unit of the
     smallest float where the results are that small, plus `more`."""
     B, T, H, D = q.shape
     for backward in (False, True):
@@ -133,7 +133,7 @@ def _against_float64(q, k, v, do, bias, causal=False, scale=None, more=0.0):
         p = p.tril()
     ds = p * torch.sigmoid(-x) * (dd @ vd.transpose(-1, -2))
     ref = [t.transpose(1, 2) for t in (p @ vd, ds @ kd * scale, ds.transpose(-1, -2) @ qd * scale, p.transpose(-1, -2) @ dd)]
-    rounding = 2.0 ** -24 * x.clamp(max=0.0).abs().max().item()
+    rounding = 2.0 ** -24 * x.clamp(max=0.0).abs().max().item() if logits else 0.0
     for name, a, r in zip(("o", "dq", "dk", "dv"), got, ref):
         smallest = 2.0 ** -150 / r.square().mean().sqrt().item()
         assert rel_l2(a, r) <= 1e-6 + rounding + smallest + more, (name, rel_l2(a, r), rounding, smallest)
@@ -180,3 +180,61 @@ def test_scores_beyond_the_scaled_range(D):
     scale = 2.0 ** -80
     out = sa.sigmoid_attention(q, k, v, scale=scale, sigmoid_bias=-3.0e29 * scale)
     assert rel_l2(out, v[:, 2::3].double().sum(1, keepdim=True).expand_as(out)) <= 1e-6
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("std", [0.5, 1.0, 4.0])
+@pytest.mark.parametrize("T", [520, 2048])
+def test_all_six_products_count(T, std, D):
+    """1e-6 (see _against_float64): without one of the three smallest products the errors are 2.5e-6 to 2e-5 at these inputs (a
+    computation of the split products in 64 bits).  std 4: scores up to 80."""
+    q, k, v, do = make_inputs(1, T, T, 8, D, torch.float32, std=std, seed=T + D)
+    _against_float64(q, k, v, do, -math.log(T), logits=False)
+
+
+@pytest.mark.parametrize("lo,hi", [(-80, -20), (-20, -10), (-10, -4), (-4, 0), (0, 8)])
+@pytest.mark.parametrize("bias", [0.0, -7.3, -60.0])
+def test_sigmoid_of_a_score(bias, lo, hi):
+    """One of 64 keys with a value, one-hot: O is the sigmoid of the query's first column.  The exponent y = scale score log2(e) is rounded
+    (2^-24 of it) and has a rounded factor (three roundings at most 2^-24 each), beyond a bias of -44 also the rest of the bias; ex2.approx
+    has 2 units, rcp.approx 1, their arguments and e^-bias one each: 2^-23 a unit, and half of one for the smallest results."""
+    T, H, scale = 4096, 16, 0.1
+    f32 = lambda y: torch.tensor(y, dtype=torch.float32).item()  # noqa: E731
+    s = torch.linspace((lo - bias) / scale, (hi - bias) / scale, T * H + 2, device="cuda", dtype=torch.float64)[1:-1].float().reshape(T, H)
+    q = torch.zeros(1, T, H, 64, device="cuda")
+    q[0, :, :, 0] = s
+    one = torch.zeros(1, 64, H, 64, device="cuda")
+    one[:, 9, :, 0] = 1.0
+    assert launch_form(1, H, T, 64, 64, torch.float32, False) == FORM_F32_TC
+    out = sa.sigmoid_attention_padded(q, one, one, scale=scale, sigmoid_bias=bias)[0, :, :, 0].double()
+    x = s.double() * f32(scale)
+    ref = torch.sigmoid(x + f32(bias))
+    bound = 2.0 ** -24 * 4 * (x.abs() + max(0.0, -44.0 - bias)) + 5 * 2.0 ** -23 + 2.0 ** -150 / ref
+    assert (((out - ref).abs() / ref) <= bound).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("where", ["k", "v", "do"])
+def test_backward_of_values_that_the_parts_cannot_carry(where, causal, D):
+    """One value of 1e34, which turns into NaN in the parts, in a column that the other operand has as 1e-34: the gradients are
+    ordinary numbers, which only the repeat in single precision gives (every query tile sees key 64, every key tile query 790).
+    Columns are compared one by one, with the gate of tests/test_f32_gpu.py."""
+    B, T, H = 3, 800, 2
+    assert launch_form(B, H, T, T, D, torch.float32, True, causal) == FORM_F32_TC
+    q, k, v, do = make_inputs(B, T, T, H, D, torch.float32, std=0.5, seed=D)
+    other = dict(k=q, v=do, do=v)[where]
+    dict(k=k, v=v, do=do)[where][:, 790 if where == "do" else 64, :, 1] = 1.0e34
+    other[..., 1] *= 1.0e-34
+    leaf = [t.requires_grad_() for t in (q, k, v)]
+    out = sa.sigmoid_attention(*leaf, is_causal=causal, sigmoid_bias=0.0)
+    got = (out,) + torch.autograd.grad(out, leaf, do)
+    qd, kd, vd, dd = (t.detach().double().transpose(1, 2) for t in (q, k, v, do))
+    p = torch.sigmoid(qd @ kd.transpose(-1, -2) / D ** 0.5)
+    if causal:
+        p = p.tril()
+    ds = p * (1 - p) * (dd @ vd.transpose(-1, -2)) / D ** 0.5
+    for name, a, r in zip(("o", "dq", "dk", "dv"), got, (p @ vd, ds @ kd, ds.transpose(-1, -2) @ qd, p.transpose(-1, -2) @ dd)):
+        assert a.isfinite().all(), name
+        err = (a.transpose(1, 2).double() - r).norm(dim=2) / r.norm(dim=2)
+        assert err.max().item() <= 1e-5, (name, err.max().item())

@@ -96,3 +96,28 @@ def test_debug_mode_poisons_packed_outputs_too(monkeypatch):
         grads = torch.autograd.grad(out, leaf, do)
     assert sum(e.name == "aten::fill_" for e in seen.events()) == 4
     assert all(t.isfinite().all() and (t != 0).any(dim=-1).all() for t in (out,) + grads)
+
+
+@pytest.mark.parametrize("dtype,H,n", [(torch.bfloat16, 4, 6), (torch.bfloat16, 8, 200), (torch.float32, 4, 6), (torch.float32, 1, 2)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("split", [False, True])
+def test_queries_without_keys_and_keys_without_queries(split, D, dtype, H, n, monkeypatch):
+    """Their rows belong to a sequence, so they are the attention kernels' to write: zeros."""
+    if split:
+        monkeypatch.setenv("SIGATTN_B200_BWD_SPLIT", "1")
+    T = 300
+    lq, lk = torch.full((n,), T), torch.full((n,), T)
+    lq[::2] = torch.tensor([T, 0, 17]).repeat(n)[:len(lq[::2])]
+    lk[1::2] = torch.tensor([0, 129, T]).repeat(n)[:len(lk[1::2])]
+    cq, ck = (torch.cat([torch.zeros(1, dtype=torch.long), x.cumsum(0)]).int().cuda() for x in (lq, lk))
+    alive = (lq > 0) & (lk > 0)
+    rows_q, rows_k = (torch.repeat_interleave(alive, x).cuda() for x in (lq, lk))
+    q, do = ((torch.randn(int(lq.sum()), H, D, device="cuda") * 0.5).to(dtype) for _ in range(2))
+    k, v = ((torch.randn(int(lk.sum()), H, D, device="cuda") * 0.5).to(dtype) for _ in range(2))
+    leaf = [t.requires_grad_() for t in (q, k, v)]
+    _poison(q.shape, dtype)
+    out = sa.sigmoid_attention_varlen(*leaf, cq, ck, T, T)
+    _poison(q.shape, dtype), _poison(k.shape, dtype)
+    for t, live in zip((out,) + torch.autograd.grad(out, leaf, do), (rows_q, rows_q, rows_k, rows_k)):
+        assert (t[~live] == 0).all() and t.isfinite().all()
+        assert (t[live] != 0).any(dim=-1).all()
