@@ -1041,6 +1041,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       if (p.score_mod && kv < it.key_lim) c0 += p.score_mod[(p.cu_k ? (int64_t)it.tk0 : (int64_t)b * p.Tk) + kv];
       c0 *= kLog2e;
       const bool row_ok = kv < Lk;
+      watch.start();
 
       for (int t = 0; t < n_q; ++t) {
         const int gt = g + t;

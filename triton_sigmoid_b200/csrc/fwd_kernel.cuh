@@ -909,6 +909,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         }
       }
       const int n_max = max(n0, n1);
+      watch.start();
 
       if constexpr (kJobWarps == 16) {
         // every warp works on every job, in the fixed order (0,0) (1,0) (0,1) (1,1) ... restricted to j < n_s

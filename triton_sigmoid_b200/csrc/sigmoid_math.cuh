@@ -83,10 +83,12 @@ __device__ __forceinline__ bool warp_all_negative(const float2 (&t)[N]) {
   return __all_sync(0xffffffffu, (int)sgn < 0) != 0;
 }
 
-// Whether a warp's next chunk is tested for logits far below zero, in the forms without kDeep.  After a test that failed, 1, 3,
-// 7, 15 and then always 31 chunks go untested, after one that passed none.
+// Whether a warp's next chunk is tested for logits far below zero, in the forms without kDeep.  The first chunk of an item is; after
+// a failure 7, 15 and then always 31 chunks go untested, after one behind a test that passed 1, 3, 7, ...  Every item starts
+// anew: which CTA takes it, and after which others, must not show in its results.
 struct DeepWatch {
-  int state = 0;  // chunks to go untested, + 256 times as many as that were after the last failure
+  int state;  // chunks to go untested, + 256 times as many as that were after the last failure
+  __device__ __forceinline__ void start() { state = 256 * 3; }
   __device__ __forceinline__ bool due() const { return (state & 255) == 0; }
   __device__ __forceinline__ void passed() { state = 0; }
   __device__ __forceinline__ void failed() { state = 257 * min(2 * (state >> 8) + 1, 31); }
