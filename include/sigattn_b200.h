@@ -44,9 +44,9 @@ extern "C" {
 
 #define SIGATTN_ABI_VERSION 2
 
-/* fp16 / bf16: tensor-core kernels.  fp32: single-precision kernels on the FMA pipe (the
- * reference accepts float32, src/triton_sigmoid/__init__.py:48, and tests it to 1e-5); they need no
- * workspace, and base pointers / strides must be multiples of 16 bytes as for the other types. */
+/* fp16 / bf16: tensor-core kernels.  fp32: single precision, by products of bf16 parts on the tensor cores or,
+ * for few or short sequences, on the FMA pipe (the reference accepts float32, src/triton_sigmoid/__init__.py:48, and
+ * tests it to 1e-5; see sigattn_form); these kernels need no workspace, and base pointers / strides must be multiples of 16 bytes as for the other types. */
 enum SigAttnDtype { SIGATTN_FP16 = 0, SIGATTN_BF16 = 1, SIGATTN_FP32 = 2 };
 
 enum SigAttnFlags {

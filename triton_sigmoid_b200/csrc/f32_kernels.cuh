@@ -1,10 +1,10 @@
-// fp32 path: the same forward and backward for float32 tensors, products and sums in single precision on
-// the FMA pipe.
+// fp32 on the FMA pipe: the same forward and backward for float32 tensors, products and sums in single precision.  Calls with few or
+// short sequences take these kernels, and tiles of the others that hold infinities, NaN or numbers that the tensor cores' parts
+// cannot carry (f32_tc_kernel.cuh).
 //
 // The reference accepts float32 (src/triton_sigmoid/__init__.py:48) and its tests hold that
 // dtype to 1e-5 (tests/conftest.py:27-34), which a tf32 tensor-core product (10-bit mantissa)
-// cannot meet; the 16-bit tcgen05 kernels are the fast path, this one is the accurate path (relative
-// error of O and of the gradients 3e-7 to 9e-7 against float64, that of the sigmoid at f32_sigmoid()).  The
+// cannot meet (relative error of O and of the gradients here 3e-7 to 9e-7 against float64, that of the sigmoid at f32_sigmoid()).  The
 // work is split as in the reference: one forward kernel, a dK/dV kernel that walks the query
 // tiles of one key tile and a dQ kernel that walks the key tiles of one query tile
 // (src/triton_sigmoid/sigmoid_triton_dense.py:23-154, 162-467), so nothing is accumulated
@@ -18,8 +18,8 @@
 //   accumulation acc[row][d] += W[row][col] X[col][d]       W = P or dS from shared memory, 16-byte reads along col
 // so that a step of 4 in the contraction costs a thread 12 shared-memory reads for 128 FMAs (kC = 1), half of what the
 // shared memory delivers in that time.  What is left is latency (2 - 3 warps per scheduler) and the elementwise step:
-// B=4 T=2048 H=8 D=64 takes 0.85 ms forward and 2.82 ms backward, 41 and 43 TFLOP/s of products done against 25 and 28
-// for 4 x 4 blocks of scalar FMAs with two __syncthreads more per tile (1.37 and 4.31 ms).  W rows are produced and
+// B=4 T=2048 H=8 D=64 (which the tensor cores take by now, in 0.22 and 0.63) took 0.85 ms forward and 2.82 ms backward, 41 and
+// 43 TFLOP/s of products done against 25 and 28 for 4 x 4 blocks of scalar FMAs with two __syncthreads more per tile (1.37 and 4.31 ms).  W rows are produced and
 // read by the warps of one row group only: a __syncwarp (kC = 1) or a barrier of those kC warps orders them.  Tiles
 // arrive by cp.async, each while the product that does not need it runs.
 //
@@ -552,7 +552,7 @@ __device__ __forceinline__ void f32_dq_rows(const F32Params& p, const F32Item& i
 }
 
 // ---------------------------------------------------------------- kernels: one row tile per CTA
-// (Three CTAs per SM at D = 64, kR = 4, at 168 registers and 72 / 88 bytes of spills: 844 us at B=4 T=2048 H=8, 870 with the 222
+// (Three CTAs per SM at D = 64, kR = 4, at 168 registers and 72 / 88 bytes of spills: 844 us at B=4 T=2048 H=8 (the tensor cores' by now), 870 with the 222
 // registers and two CTAs that it takes unbounded.)
 template <int D, int kR, int kC>
 __global__ void __launch_bounds__(32 * kR * kC, D == 64 && kR == 4 ? 3 : 1) sigattn_fwd_f32_kernel(const F32Params p, const int n_tiles) {

@@ -1,4 +1,5 @@
-// fp32 on the tensor cores: forward, dK/dV and dQ of float32 tensors with every product done as six bf16 products.
+// fp32 on the tensor cores: forward, dK/dV and dQ of float32 tensors with every product done as six bf16 products (the method of
+// Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations", 2019).
 //
 // A float is the sum of three bf16 numbers, x = x0 + x1 + x2 (each the rounded remainder of the ones before it; 24 bits
 // and three signs lose nothing), so x y = x0 y0 + (x0 y1 + x1 y0) + (x0 y2 + x1 y1 + x2 y0) up to terms of 2^-24 |x y| (2^-27
@@ -7,15 +8,17 @@
 // are exact down to the smallest float; unscaled, the third one would begin to lose bits at 3e-33 and the first at 1e-38
 // (V of 1e-35: relative error of O 2.7e-6, of dQ 6e-4).  The factors are powers of two that the constants behind the products
 // take up.
-// The small terms go into the accumulator first, and an accumulator takes one tile of 64 streamed rows only: the sums over
-// tiles are made in registers, rounded to nearest, so that the tensor core's own summation never runs over more than
-// 64 terms.
+// The small terms go into the accumulator first, and an accumulator of outputs takes one tile of 64 streamed rows only: the sums
+// over tiles are made in registers, rounded to nearest, so that the tensor core's own summation runs over 64 terms, or, for scores
+// and dP, over the head dimension.
 //
-// B=4 T=2048 H=8 D=64: 213 us forward, 625 backward (the FMA kernels 840 and 2820; 434 for all products at the tensor core's
-// rate).  Relative error of O, dQ, dK, dV against 64 bits, FMA kernels in brackets: T=512 2.3 - 2.9e-7 (4.5 - 4.7), T=2048 2.6 - 3.3e-7
+// B=4 T=2048 H=8 D=64: 221 us forward, 631 backward (the FMA kernels 840 and 2820; 434 for all products at the tensor core's
+// rate; 213 and 615 without the scaling and the test for large scores).  Relative error of O, dQ, dK, dV against 64 bits, FMA kernels in brackets: T=512 2.3 - 2.9e-7 (4.5 - 4.7), T=2048 2.6 - 3.3e-7
 // (8.3 - 8.5), bias 0 1.3 - 1.8e-7 (7.8 - 8.2), T=32768 causal 4.3 - 4.7e-7 (2.7e-6); D = 128, T=2048 1.3 - 2.3e-7 (8.3 - 8.4), T=16384
 // 2.9 - 3.6e-7 (2.3e-6).  Accumulators kept for 128 or 256 terms would make it 6 and 15e-7, small and large terms in turn 4e-7: the
-// tensor core truncates its sums.
+// tensor core truncates its sums.  It shows where one product makes up a score: every score -20 by the head's first column, 3.4e-6
+// at D = 64 and 4.2e-6 at 128 (3.1 and 3.2e-6), by the last one 1.2 and 0.7e-6 (0.9 and 0.9e-6), by all alike 1.3 and 1.5e-6 (1.2
+// and 1.8e-6); random scores of deviation 16 1.5 to 6e-7 (3.7 to 11e-7).
 //
 // One kernel, five modes, one CTA per (batch, head, 128-row tile); R = stationary side, C = streamed side:
 //     kTcFwd   R1 = Q            C1 = K  C2 = V     S = R1 C1^T, P = sigmoid;         out2 = O  += P C2
@@ -35,15 +38,18 @@
 // R1 (and R2 where it fits) is a TMEM operand: a product of 128 x 64 takes 32 clocks then, and 48 with A in shared memory, of
 // which it reads 6 KB.
 //
-// What bounds it: a job needs 1536 (forward), 3456 (kTcDkdv) and 2304 (kTcDq) clocks of the tensor core and takes about 2700,
-// 4800 and 4200; splitting and the elementwise step are 1600 to 1900 instructions per scheduler and job, at half of the issue rate.
+// What bounds it: a job needs 1536 (forward), 3456 (kTcDkdv) and 2304 (kTcDq) clocks of the tensor core and takes about 3000,
+// 4900 and 4000; splitting and the elementwise step are 1940, 2770 and 2250 instructions per scheduler and job, at 66, 57 and 56 % of the
+// issue rate, with the tensor pipe active for 52, 63 and 58 % of the time (D = 128, T=2048: 63 forward, 63 dV, 47 dK, 46 dQ).
 // One issuing warp for scores and outputs, with loops over the k-steps, made it 95 clocks per product (286 us forward, 1211
 // backward); four conversion warps are 650 clocks per 64 x 64 chunk behind (D = 128 forward 118 us at B=2 H=8 T=2048 causal, 104
 // with eight; D = 64 the same), and more of them leave the compute warps too few registers.
 //
 // Values that the split cannot carry (infinities and NaN; finite ones from 2^112 on) and sums that overflow turn into NaN in
 // every result that they reach.  A CTA that finds an accumulator that is not finite computes its tile again with the FMA
-// code (f32_fwd_rows and so on), which gives what single precision gives.
+// code (f32_fwd_rows and so on), which gives what single precision gives.  That costs both: with a NaN that every row sees, B=4
+// T=2048 H=8, forward 1.89 ms (the FMA kernels 0.85) and 5.7 with the backward (3.7); D = 128, where dV's and dK's kernels each
+// repeat dK and dV, 2.95 (1.77) and 11.3 (7.7).
 #pragma once
 
 #include <type_traits>
@@ -62,7 +68,9 @@ constexpr int kTcConvWarps = 8;
 constexpr int kTcIssuerIn = 24;   // scores; owns the TMEM allocation
 constexpr int kTcIssuerOut = 25;  // outputs
 constexpr int kTcThreads = 28 * 32;
-// Registers per thread: 72 at launch (65536 / 896, rounded down to a multiple of 8), then by role.
+// Registers per thread: 72 at launch (65536 / 896, rounded down to a multiple of 8), then by role.  Spills (bytes of stores / loads,
+// -Xptxas -v): D = 64 forward 0 / 0, dK/dV 56 / 64, dQ 12 / 44; D = 128 forward 12 / 28, dQ 56 / 76, dV 44 / 76, dK 80 / 152, most of them in
+// the FMA code.
 constexpr int kTcConvRegs = 48, kTcIssuerRegs = 56, kTcComputeRegs = 88;
 static_assert(kTcComputeWarps * kTcComputeRegs + kTcConvWarps * kTcConvRegs + 4 * kTcIssuerRegs <= 28 * 72, "no more than the launch gave");
 

@@ -497,8 +497,8 @@ def _pad_head_dim(x: torch.Tensor, D_kernel: int) -> torch.Tensor:
 
 
 def _check_dtype(query, key, value):
-    """float16 / bfloat16 run on the tensor cores; float32 runs the single-precision
-    kernels (slower by design: the reference holds float32 to 1e-5, which tf32 cannot meet)."""
+    """float16 / bfloat16 run on the tensor cores; float32 runs the single-precision kernels (six products of bf16 parts for
+    each one, or the FMA pipe: the reference holds float32 to 1e-5, which tf32 cannot meet)."""
     if query.dtype not in _SUPPORTED_DTYPES:
         raise NotImplementedError(f"unsupported dtype {query.dtype}: use float16, bfloat16 or float32")
     if key.dtype != query.dtype or value.dtype != query.dtype:
