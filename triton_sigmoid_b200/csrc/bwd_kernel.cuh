@@ -455,8 +455,8 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   const int lane = threadIdx.x & 31;
 
   // a kernel of this library already gave up on a wait: do not pile more work on a sick device
-  // (one answer for the CTA: the word may change while its warps read it)
-  if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) return;
+  // (looked at behind the set-up, where the warps meet anyway)
+  const bool sick = *reinterpret_cast<volatile int*>(&g_status_word) != 0;
 
   // ---------------------------------------------------------------- setup
   if (threadIdx.x == 0) {
@@ -507,9 +507,14 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     tmem_relinquish();
   }
   tc_fence_before_sync();
-  __syncthreads();
+  // one answer for the CTA: the word may change while its warps read it
+  const bool leave = __syncthreads_or(sick);
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  if (leave) {
+    if (warp == kBwdIssuerA) tmem_dealloc(tmem, kTmemCols);
+    return;
+  }
 
   // Consumer side of the item ring: returns the k-th item of this CTA, or -1 when there is none
   // (also on a failed wait).  Called by all 32 lanes of a reader warp.

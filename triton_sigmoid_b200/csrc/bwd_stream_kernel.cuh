@@ -249,8 +249,8 @@ sigattn_bwd_stream_kernel(const __grid_constant__ CUtensorMap r1_map, const __gr
   const int lane = threadIdx.x & 31;
 
   // a kernel of this library already gave up on a wait: do not pile more work on a sick device
-  // (one answer for the CTA: the word may change while its warps read it)
-  if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) return;
+  // (looked at behind the set-up, where the warps meet anyway)
+  const bool sick = *reinterpret_cast<volatile int*>(&g_status_word) != 0;
 
   // ---------------------------------------------------------------- setup
   if (threadIdx.x == 0) {
@@ -286,9 +286,14 @@ sigattn_bwd_stream_kernel(const __grid_constant__ CUtensorMap r1_map, const __gr
     tmem_relinquish();
   }
   tc_fence_before_sync();
-  __syncthreads();
+  // one answer for the CTA: the word may change while its warps read it
+  const bool leave = __syncthreads_or(sick);
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  if (leave) {
+    if (warp == kBsIssuerIn) tmem_dealloc(tmem, kTmemCols);
+    return;
+  }
 
   auto read_item = [&](int k) -> int {
     const int slot = k & 1;

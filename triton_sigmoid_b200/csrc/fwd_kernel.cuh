@@ -408,14 +408,8 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   const int lane = threadIdx.x & 31;
 
   // a kernel of this library already gave up on a wait: do not pile more work on a sick device
-  // (one answer for the CTA: the word may change while its warps read it)
-  if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) {
-    if constexpr (kSplit) {  // (the others of the cluster may have got another one, and read this CTA's shared memory)
-      cluster_sync();
-      cluster_sync();
-    }
-    return;
-  }
+  // (looked at behind the set-up, where the warps meet anyway)
+  const bool sick = *reinterpret_cast<volatile int*>(&g_status_word) != 0;
 
   // ---------------------------------------------------------------- setup
   if (threadIdx.x == 0) {
@@ -453,9 +447,18 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     tmem_relinquish();
   }
   tc_fence_before_sync();
-  __syncthreads();
+  // one answer for the CTA: the word may change while its warps read it
+  const bool leave = __syncthreads_or(sick);
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  if (leave) {
+    if (warp == kFwdIssuerWarp) tmem_dealloc(tmem, kTmemCols);
+    if constexpr (kSplit) {  // (the others of the cluster may have got another answer, and read this CTA's shared memory)
+      cluster_sync();
+      cluster_sync();
+    }
+    return;
+  }
 
   // The sigmoid warps hold 64 scores each in flight and want more registers than an even split
   // gives; the role warps and the output warps need few.  Registers only move within what the CTA was
