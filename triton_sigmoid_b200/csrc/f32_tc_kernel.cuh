@@ -12,8 +12,8 @@
 // over tiles are made in registers, rounded to nearest, so that the tensor core's own summation runs over 64 terms, or, for scores
 // and dP, over the head dimension.
 //
-// B=4 T=2048 H=8 D=64: 221 us forward, 631 backward (the FMA kernels 840 and 2820; 434 for all products at the tensor core's
-// rate; 213 and 615 without the scaling and the test for large scores).  Relative error of O, dQ, dK, dV against 64 bits, FMA kernels in brackets: T=512 2.3 - 2.9e-7 (4.5 - 4.7), T=2048 2.6 - 3.3e-7
+// B=4 T=2048 H=8 D=64: 210 us forward, 589 backward (the FMA kernels 840 and 2820; 434 for all products at the tensor core's
+// rate).  Relative error of O, dQ, dK, dV against 64 bits, FMA kernels in brackets: T=512 2.3 - 2.9e-7 (4.5 - 4.7), T=2048 2.6 - 3.3e-7
 // (8.3 - 8.5), bias 0 1.3 - 1.8e-7 (7.8 - 8.2), T=32768 causal 4.3 - 4.7e-7 (2.7e-6); D = 128, T=2048 1.3 - 2.3e-7 (8.3 - 8.4), T=16384
 // 2.9 - 3.6e-7 (2.3e-6).  Accumulators kept for 128 or 256 terms would make it 6 and 15e-7, small and large terms in turn 4e-7: the
 // tensor core truncates its sums.  It shows where one product makes up a score: every score -20 by the head's first column, 3.4e-6
@@ -168,14 +168,15 @@ __device__ __forceinline__ float2 tc_sigmoid2(float2 y, float factor_down) {
 // on to the smallest float this way, as in the FMA kernels.)
 __device__ __forceinline__ float tc_sigmoid_tiny(float y, float below) { return ex2_approx(40.0f - y) * below; }
 
+// One tile; `block` counts those of the mode.
 template <int D, int kMode>
-__global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32Params p, const int n_tiles) {
+__device__ __forceinline__ void f32_tc_tile(const F32Params& p, const unsigned int block, const int n_tiles) {
   using L = TcShape<D, kMode>;
   constexpr int kSite = (0x6 + kMode) << 16;
   extern __shared__ uint8_t tc_smem[];
 
   // ---------------------------------------------------------------- the tile
-  const F32Item it = f32_item(p, n_tiles, !L::kKeyRows);
+  const F32Item it = f32_item(p, block, n_tiles, !L::kKeyRows);
   // a kernel of this library already gave up on a wait: leave, all warps or none (the named barriers below count on every warp,
   // and the word may change while they read it)
   if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) return;
@@ -675,6 +676,35 @@ __global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_kernel(const F32
   if (warp == kTcIssuerIn) {
     tc_fence_after_sync();
     tmem_dealloc(tmem, 512);
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_fwd_kernel(const F32Params p, const int n_tiles) {
+  f32_tc_tile<D, kTcFwd>(p, blockIdx.x, n_tiles);
+}
+template <int D>
+constexpr int tc_bwd_bytes() {
+  if constexpr (D == 64) return TcShape<D, kTcDkdv>::kDynBytes > TcShape<D, kTcDq>::kDynBytes ? TcShape<D, kTcDkdv>::kDynBytes : TcShape<D, kTcDq>::kDynBytes;
+  else {
+    constexpr int dk = TcShape<D, kTcDk>::kDynBytes, dv = TcShape<D, kTcDv>::kDynBytes, dq = TcShape<D, kTcDq>::kDynBytes;
+    return dk > dv ? (dk > dq ? dk : dq) : (dv > dq ? dv : dq);
+  }
+}
+// All tiles of the backward in one launch, the heavier kinds first: they need nothing of each other, and one CTA per SM in turn
+// leaves SMs idle at the end of each launch.  One launch per kind -> one, us: B=4 T=2048 H=8 D=64 (512 tiles of each kind, 3.46 waves) 683 -> 589,
+// D=128 1873 -> 1686; B=64 T=384 H=8 538 -> 525; B=1 T=8192 H=4 1302 -> 1272.
+template <int D>
+__global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_bwd_kernel(const F32Params p, const int n_k_tiles, const int n_q_tiles) {
+  const unsigned int n_bh = (unsigned int)(p.B * p.H), n_k = n_bh * (unsigned int)n_k_tiles, n_q = n_bh * (unsigned int)n_q_tiles;
+  const unsigned int block = blockIdx.x;
+  if constexpr (D == 64) {
+    if (block < n_k) f32_tc_tile<D, kTcDkdv>(p, block, n_k_tiles);
+    else f32_tc_tile<D, kTcDq>(p, block - n_k, n_q_tiles);
+  } else {
+    if (block < n_q) f32_tc_tile<D, kTcDq>(p, block, n_q_tiles);
+    else if (block < n_q + n_k) f32_tc_tile<D, kTcDk>(p, block - n_q, n_k_tiles);
+    else f32_tc_tile<D, kTcDv>(p, block - n_q - n_k, n_k_tiles);
   }
 }
 

@@ -685,29 +685,37 @@ int launch_f32_shape(const SigAttnParams* p, const sigattn::F32Params& fp, bool 
     kernel<<<(unsigned int)(n_bh * n_q), S::kThreads, S::kFwdBytes, stream>>>(fp, n_q);
     SIG_CUDA(cudaGetLastError());
   } else {
-    auto kdkdv = sigattn_bwd_dkdv_f32_kernel<D, kR, kC>;
-    auto kdq = sigattn_bwd_dq_f32_kernel<D, kR, kC>;
-    if (int rc = set_smem(kdkdv, S::kDkdvBytes, p->device)) return rc;
-    if (int rc = set_smem(kdq, S::kDqBytes, p->device)) return rc;
-    kdkdv<<<(unsigned int)(n_bh * n_k), S::kThreads, S::kDkdvBytes, stream>>>(fp, n_k);
+    auto kernel = sigattn_bwd_f32_kernel<D, kR, kC>;
+    constexpr int smem = std::max(S::kDkdvBytes, S::kDqBytes);
+    if (int rc = set_smem(kernel, smem, p->device)) return rc;
+    const bool both = n_bh * ((int64_t)n_k + n_q) <= INT32_MAX;
+    kernel<<<(unsigned int)(n_bh * (n_k + (both ? n_q : 0))), S::kThreads, smem, stream>>>(fp, n_k, n_q);
     SIG_CUDA(cudaGetLastError());
-    kdq<<<(unsigned int)(n_bh * n_q), S::kThreads, S::kDqBytes, stream>>>(fp, n_q);
-    SIG_CUDA(cudaGetLastError());
+    if (!both) {
+      kernel<<<(unsigned int)(n_bh * n_q), S::kThreads, smem, stream>>>(fp, 0, n_q);
+      SIG_CUDA(cudaGetLastError());
+    }
   }
   return 0;
 }
 
 // float32 tensors on the tensor cores (no tensor maps, no workspace either).
-template <int D, int kMode>
-int launch_f32_tc(const SigAttnParams* p, const sigattn::F32Params& fp) {
+template <int D>
+int launch_f32_tc(const SigAttnParams* p, const sigattn::F32Params& fp, bool backward) {
   using namespace sigattn;
-  using S = TcShape<D, kMode>;
-  const int n_tiles = ((S::kKeyRows ? p->Tk : p->Tq) + kTcRows - 1) / kTcRows;
-  const int64_t ctas = (int64_t)p->B * p->H * n_tiles;
+  cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
+  const int n_q = (p->Tq + kTcRows - 1) / kTcRows, n_k = (p->Tk + kTcRows - 1) / kTcRows;
+  const int64_t ctas = (int64_t)p->B * p->H * (backward ? n_q + (int64_t)n_k * (D == 64 ? 1 : 2) : n_q);
   if (ctas > INT32_MAX) return fail(-2, "too many (batch, head, tile) items: %lld", (long long)ctas);
-  auto kernel = sigattn_f32_tc_kernel<D, kMode>;
-  if (int rc = set_smem(kernel, S::kDynBytes, p->device)) return rc;
-  kernel<<<(unsigned int)ctas, kTcThreads, S::kDynBytes, static_cast<cudaStream_t>(p->stream)>>>(fp, n_tiles);
+  if (!backward) {
+    constexpr int smem = TcShape<D, kTcFwd>::kDynBytes;
+    if (int rc = set_smem(sigattn_f32_tc_fwd_kernel<D>, smem, p->device)) return rc;
+    sigattn_f32_tc_fwd_kernel<D><<<(unsigned int)ctas, kTcThreads, smem, stream>>>(fp, n_q);
+  } else {
+    constexpr int smem = tc_bwd_bytes<D>();
+    if (int rc = set_smem(sigattn_f32_tc_bwd_kernel<D>, smem, p->device)) return rc;
+    sigattn_f32_tc_bwd_kernel<D><<<(unsigned int)ctas, kTcThreads, smem, stream>>>(fp, n_k, n_q);
+  }
   SIG_CUDA(cudaGetLastError());
   return 0;
 }
@@ -791,17 +799,7 @@ int launch_f32_d(const SigAttnParams* p, bool backward) {
   if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
   int rc = 0;
   if (f32_tc(p, backward, info.n_sm)) {
-    if (!backward) {
-      rc = launch_f32_tc<D, kTcFwd>(p, fp);
-    } else {
-      if constexpr (D == 64) {
-        rc = launch_f32_tc<D, kTcDkdv>(p, fp);
-      } else {
-        rc = launch_f32_tc<D, kTcDv>(p, fp);
-        if (!rc) rc = launch_f32_tc<D, kTcDk>(p, fp);
-      }
-      if (!rc) rc = launch_f32_tc<D, kTcDq>(p, fp);
-    }
+    rc = launch_f32_tc<D>(p, fp, backward);
   } else
     rc = f32_tile_rows(p, info.n_sm) == 64 ? launch_f32_shape<D, 4, D / 64>(p, fp, backward) : launch_f32_shape<D, 1, 4>(p, fp, backward);
   if (rc) return rc;
