@@ -1,0 +1,57 @@
+"""The short polynomials for logits below zero: logits on both sides of each polynomial's limit, in the three forms that the
+bias and the number of keys select, against 64 bits."""
+
+import pytest
+import torch
+
+import triton_sigmoid_b200 as m
+from tests.gpu_util import make_inputs
+
+pytestmark = pytest.mark.gpu
+
+# limit of the logits, largest relative error of the polynomial; above the limit the one for all logits
+NEAR = {torch.float16: (-2.08, 6.4e-5), torch.bfloat16: (-1.386, 4.4e-4)}
+FAR = {torch.float16: (-3.466, 3.1e-5), torch.bfloat16: (-3.466, 9.8e-4)}
+GENERAL = {torch.float16: 3.0e-4, torch.bfloat16: 1.74e-3}
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("bias,T", [(0.0, 520), (-3.1, 520), (-3.1, 1024), (-3.1, 1025)])
+@pytest.mark.parametrize("centre", [-0.7, -1.85, -2.55, -3.95, -9.0])
+def test_common_factor(centre, bias, T, D, dtype):
+    """Logits within 0.46 of `centre` (deviation 0.1), V and dO of mean 1: an error that all probabilities share shows as a factor on O
+    and dV.  Bound: the polynomial's error, plus what rounding to 16 bits (2^-9, 2^-12 at most) leaves of itself: an eighth where only the
+    product is rounded, averaged over 10^6 of them; a whole one on packed pairs, whose last factor, between 0.97 and 1, changes so little
+    over these logits that its rounding does not average out."""
+    B, H = 6, 4  # (too many items for the split form)
+    q, k, v, do = make_inputs(B, T, T, H, D, dtype, std=1.0, seed=D)
+    with torch.no_grad():
+        scores = 0.1 * torch.randn(B, T, 1, device="cuda").clamp(-4.5, 4.5) + centre - bias
+        q.zero_()
+        k.zero_()
+        q[..., 0] = 8.0
+        k[..., 0] = scores * D ** 0.5 / 8
+        k[..., 1] = scores * D ** 0.5 / 8 - k[..., 0].float()  # what the 16-bit type leaves of the score
+        q[..., 1] = 8.0
+        v += 1.0
+        do += 1.0
+    leaf = [t.requires_grad_() for t in (q, k, v)]
+    out = m.sigmoid_attention(*leaf, sigmoid_bias=bias)
+    got = (out,) + torch.autograd.grad(out, leaf, do)
+    qd, kd, vd, dd = (t.detach().double().transpose(1, 2) for t in (q, k, v, do))
+    x = qd @ kd.transpose(-1, -2) / D ** 0.5 + bias
+    p = torch.sigmoid(x)
+    ref = [t.transpose(1, 2) for t in (p @ vd, p.transpose(-1, -2) @ dd)]
+    unit = {torch.float16: 2.0 ** -12, torch.bfloat16: 2.0 ** -9}[dtype]
+    if dtype == torch.float16 and p.min() < 6.2e-5:
+        unit *= 6.2e-5 / p.min().item()  # subnormal probabilities
+
+    def bound(far):
+        limit, poly = (FAR if far else NEAR)[dtype]
+        most = poly + (unit if far else unit / 8) if x.max() < limit else GENERAL[dtype] + unit / 8
+        return max(most, GENERAL[dtype] + unit / 8) if bias > -3.0 else most  # (above -3 not every chunk is tested)
+
+    far = T > 1024
+    for name, a, r, most in (("o", got[0], ref[0], bound(far or (D == 128 and bias <= -3.0))), ("dv", got[3], ref[1], bound(far and D == 64))):
+        assert abs((a.double() * r).sum() / (r * r).sum() - 1).item() <= most, name

@@ -150,8 +150,8 @@ struct BwdSmem {
 template <bool kBF16, bool kMask, bool kAccurate, DeepTest kTest>
 __device__ __forceinline__ void bwd_phase_a(uint32_t s_addr, float c1, float c0, int q0, int q_lo, int q_hi,
                                             float2 (&pv)[16], DeepWatch& watch) {
-  // tested tiles work on logits shifted up by kDeepShift (see sigmoid2_from_shifted_log2_deep)
-  const float c0s = kTest == kNoTest ? c0 : c0 + kDeepShift;
+  // tested tiles work on logits shifted up (see sigmoid2_near)
+  const float c0s = kTest == kNoTest ? c0 : c0 + kNearShift<kBF16>;
   {
     uint32_t r[32];
     tmem_ld32_sync(s_addr, r);
@@ -184,13 +184,13 @@ __device__ __forceinline__ void bwd_phase_a(uint32_t s_addr, float c1, float c0,
     emit([](float2 x) { return sigmoid2_accurate_from_log2(x); });
   } else if (kTest != kNoTest && warp_all_negative(pv)) {
     watch.passed();
-    // all logits far below zero (the usual case under the default bias): short series, no compare / select per element
-    emit([](float2 x) { return sigmoid2_from_shifted_log2_deep<kBF16>(x); });
+    // all logits far below zero (the usual case under the default bias): short polynomial, no compare / select per element
+    emit([](float2 x) { return sigmoid2_near<kBF16>(x); });
   } else {
     bool all_neg = false;
     if constexpr (kTest != kNoTest) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) pv[i] = __fadd2_rn(pv[i], make_float2(-kDeepShift, -kDeepShift));
+      for (int i = 0; i < 16; ++i) pv[i] = __fadd2_rn(pv[i], make_float2(-kNearShift<kBF16>, -kNearShift<kBF16>));
       if constexpr (kTest == kTestAll) all_neg = warp_all_negative(pv);  // negative but not far below zero: full polynomial, still no select
       else watch.failed();
     }
@@ -235,13 +235,13 @@ __device__ __forceinline__ void bwd_phase_b(uint32_t dp_addr, uint32_t ds_line, 
 // (32 registers per thread that the drain warps' share of the register file cannot spare) but read back
 // from TMEM in the 16-bit form they were stored in for the dV product, and dS = P (1 - P) dP is formed on
 // packed 16-bit pairs.
-template <bool kBF16, bool kMask, bool kAccurate, DeepTest kTest>
+template <bool kBF16, bool kMask, bool kAccurate, DeepTest kTest, DeepRange kRange>
 __device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c0, int q0, int q_lo, int q_hi, DeepWatch& watch) {
   uint32_t r[32];
   tmem_ld32_sync(s_addr, r);
   uint32_t pk[16];
   float2 t[16];
-  const float c0s = kTest == kNoTest ? c0 : c0 + kDeepShift;
+  const float c0s = kTest == kNoTest ? c0 : c0 + kDeepShift<kRange, kBF16>;
 #pragma unroll
   for (int i = 0; i < 16; ++i)
     t[i] = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), make_float2(c1, c1),
@@ -259,14 +259,21 @@ __device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c
     }
   } else if (kTest != kNoTest && warp_all_negative(t)) {
     watch.passed();
-    // all logits far below zero (the usual case under the default bias): short series on packed pairs
+    // the usual case under the default bias: short polynomial, no compare / select per element
 #pragma unroll
-    for (int i = 0; i < 16; ++i) pk[i] = sigmoid2_deep_packed<kBF16>(t[i], false);
+    for (int i = 0; i < 16; ++i) {
+      if constexpr (kRange == kFar) {
+        pk[i] = sigmoid2_far_packed<kBF16>(t[i], false);
+      } else {
+        const float2 pe = sigmoid2_near<kBF16>(t[i]);
+        pk[i] = pack2<kBF16>(pe.x, pe.y);
+      }
+    }
   } else {
     bool all_neg = false;
     if constexpr (kTest != kNoTest) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) t[i] = __fadd2_rn(t[i], make_float2(-kDeepShift, -kDeepShift));
+      for (int i = 0; i < 16; ++i) t[i] = __fadd2_rn(t[i], make_float2(-kDeepShift<kRange, kBF16>, -kDeepShift<kRange, kBF16>));
       if constexpr (kTest == kTestAll) all_neg = warp_all_negative(t);
       else watch.failed();
     }
@@ -408,8 +415,8 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item)
 // tickets count (batch, head) pairs.  (This form spills more: 140 / 204 bytes of stores / loads by -Xptxas -v at D = 64
 // against 68 / 80 in the general one, 208 / 300 against 120 / 188 at D = 128.  All registers of the CTA are handed out, see
 // below; the figures of the rule that chooses the form, bwd_by_head(), include these spills.)
-// kDeep: as in the forward kernel.
-template <int D, bool kBF16, bool kAccurate, bool kByHead, bool kDeep>
+// kForm: as in the forward kernel (kDeepFar at D = 64 only, where P is on packed pairs from the start).
+template <int D, bool kBF16, bool kAccurate, bool kByHead, DeepForm kForm>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                    const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap do_map,
@@ -1061,18 +1068,19 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         const uint32_t s_addr = s_addr0 + 128u * (uint32_t)sbuf(gt);
         if (!ok) break;
         tc_fence_after_sync();
-        constexpr DeepTest kTest = kDeep && !kAccurate ? kTestAll : kNoTest;
-        const bool test_now = !kDeep && !kAccurate && watch.due();
+        constexpr DeepTest kTest = kForm != kDeepWatched && !kAccurate ? kTestAll : kNoTest;
+        constexpr DeepRange kRange = kForm == kDeepFar ? kFar : kNear;
+        const bool test_now = kForm == kDeepWatched && !kAccurate && watch.due();
         if constexpr (D == 64) {
-          if (need_mask)     bwd_phase_a16<kBF16, true, kAccurate, kNoTest>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
-          else if (test_now) bwd_phase_a16<kBF16, false, kAccurate, kTestNow>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
-          else               bwd_phase_a16<kBF16, false, kAccurate, kTest>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
+          if (need_mask)     bwd_phase_a16<kBF16, true, kAccurate, kNoTest, kRange>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
+          else if (test_now) bwd_phase_a16<kBF16, false, kAccurate, kTestNow, kRange>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
+          else               bwd_phase_a16<kBF16, false, kAccurate, kTest, kRange>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
         } else {
           if (need_mask)     bwd_phase_a<kBF16, true, kAccurate, kNoTest>(s_addr, c1, c0, q0, q_lo, q_hi, pv, watch);
           else if (test_now) bwd_phase_a<kBF16, false, kAccurate, kTestNow>(s_addr, c1, c0, q0, q_lo, q_hi, pv, watch);
           else               bwd_phase_a<kBF16, false, kAccurate, kTest>(s_addr, c1, c0, q0, q_lo, q_hi, pv, watch);
         }
-        if (!kDeep && !need_mask && !test_now) watch.skipped();
+        if (kForm == kDeepWatched && !need_mask && !test_now) watch.skipped();
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();

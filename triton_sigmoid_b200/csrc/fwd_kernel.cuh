@@ -161,10 +161,10 @@ struct FwdCursor {
 
 // 32 score columns of one TMEM lane (this thread's query row), already in registers -> logits in the
 // base-2 domain, t = (scale * s + bias) * log2(e).  Chunks that are tested for logits far below zero work on logits
-// shifted up by kDeepShift (see sigmoid2_from_shifted_log2_deep).
-template <bool kShift>
+// shifted up (see sigmoid2_near).
+template <bool kShift, bool kBF16, DeepRange kRange>
 __device__ __forceinline__ void fwd_chunk_logits(const uint32_t (&r)[32], float2 (&t)[16], float c1, float c0) {
-  const float c0s = kShift ? c0 + kDeepShift : c0;
+  const float c0s = kShift ? c0 + kDeepShift<kRange, kBF16> : c0;
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     t[i] = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), make_float2(c1, c1),
@@ -210,8 +210,9 @@ __device__ __forceinline__ void fwd_add_score_mod(float2 (&t)[16], int col0, con
 }
 
 // Logits of fwd_chunk_logits -> 16-bit probabilities, written over the first 16 of the chunk's 32 TMEM
-// columns at s_addr.  lim = largest visible key index of this row (used only when kMask).
-template <bool kBF16, bool kMask, bool kAccurate, DeepTest kTest>
+// columns at s_addr.  lim = largest visible key index of this row; negative when the row is padding, whose logits then have no say in
+// the form that the others' take.
+template <bool kBF16, bool kMask, bool kAccurate, DeepTest kTest, DeepRange kRange>
 __device__ __forceinline__ void fwd_chunk_probs(uint32_t s_addr, float2 (&t)[16], int col0, int lim, DeepWatch& watch) {
   constexpr int kCh = 32;
   uint32_t pk[kCh / 2];
@@ -227,18 +228,25 @@ __device__ __forceinline__ void fwd_chunk_probs(uint32_t s_addr, float2 (&t)[16]
       pk[i] = pack2<kBF16>(pr.x, pr.y);
     }
   } else {
-    // Under the default bias every logit of a chunk is far below zero: the short series applies
+    // Under the default bias every logit of a chunk is below zero far enough for the short polynomial,
     // and the sign handling (one compare and one select per element) is skipped for the whole warp.
-    if (kTest != kNoTest && warp_all_negative(t)) {
+    if (kTest != kNoTest && warp_all_negative(t, lim)) {
       watch.passed();
 #pragma unroll
-      for (int i = 0; i < kCh / 2; ++i) pk[i] = sigmoid2_deep_packed<kBF16>(t[i], (i & 7) == 7);
+      for (int i = 0; i < kCh / 2; ++i) {
+        if constexpr (kRange == kFar) {
+          pk[i] = sigmoid2_far_packed<kBF16>(t[i], (i & 7) == 7);
+        } else {
+          const float2 pr = sigmoid2_near<kBF16>(t[i]);
+          pk[i] = pack2<kBF16>(pr.x, pr.y);
+        }
+      }
     } else {
       bool all_neg = false;
       if constexpr (kTest != kNoTest) {
 #pragma unroll
-        for (int i = 0; i < kCh / 2; ++i) t[i] = __fadd2_rn(t[i], make_float2(-kDeepShift, -kDeepShift));
-        if constexpr (kTest == kTestAll) all_neg = warp_all_negative(t);  // negative but not far below zero: full polynomial, still no select
+        for (int i = 0; i < kCh / 2; ++i) t[i] = __fadd2_rn(t[i], make_float2(-kDeepShift<kRange, kBF16>, -kDeepShift<kRange, kBF16>));
+        if constexpr (kTest == kTestAll) all_neg = warp_all_negative(t, lim);  // negative but not far below zero: full polynomial, still no select
         else watch.failed();
       }
       if (all_neg) {
@@ -266,23 +274,24 @@ __device__ __forceinline__ void fwd_chunk_probs(uint32_t s_addr, float2 (&t)[16]
 
 // All steps for a chunk whose scores are in registers.  mod_args: those of fwd_add_score_mod after the logits.  (The untested
 // chunk has code of its own: with a join behind the test, bias 0, B=4 T=4096 H=32 D=64, 782 us instead of 740.)
-template <bool kBF16, bool kScoreMod, bool kMask, bool kAccurate, bool kDeep, typename... ModArgs>
+template <bool kBF16, bool kScoreMod, bool kMask, bool kAccurate, DeepForm kForm, typename... ModArgs>
 __device__ __forceinline__ void fwd_sigmoid_chunk(uint32_t s_addr, const uint32_t (&r)[32], float c1, float c0, int col0,
                                                   int lim, DeepWatch& watch, ModArgs... mod_args) {
   float2 t[16];
-  if constexpr (!kMask && !kAccurate && !kDeep) {
+  constexpr DeepRange kRange = kForm == kDeepFar ? kFar : kNear;
+  if constexpr (!kMask && !kAccurate && kForm == kDeepWatched) {
     if (watch.due()) {
-      fwd_chunk_logits<true>(r, t, c1, c0);
+      fwd_chunk_logits<true, kBF16, kNear>(r, t, c1, c0);
       if constexpr (kScoreMod) fwd_add_score_mod(t, mod_args...);
-      fwd_chunk_probs<kBF16, false, false, kTestNow>(s_addr, t, col0, lim, watch);
+      fwd_chunk_probs<kBF16, false, false, kTestNow, kNear>(s_addr, t, col0, lim, watch);
       return;
     }
     watch.skipped();
   }
-  constexpr DeepTest kTest = kDeep && !kMask && !kAccurate ? kTestAll : kNoTest;
-  fwd_chunk_logits<kTest == kTestAll>(r, t, c1, c0);
+  constexpr DeepTest kTest = kForm != kDeepWatched && !kMask && !kAccurate ? kTestAll : kNoTest;
+  fwd_chunk_logits<kTest == kTestAll, kBF16, kRange>(r, t, c1, c0);
   if constexpr (kScoreMod) fwd_add_score_mod(t, mod_args...);
-  fwd_chunk_probs<kBF16, kMask, kAccurate, kTest>(s_addr, t, col0, lim, watch);
+  fwd_chunk_probs<kBF16, kMask, kAccurate, kTest, kRange>(s_addr, t, col0, lim, watch);
 }
 
 // One work item.  The producer warp decodes it once (integer divisions, length and bias loads from global
@@ -376,9 +385,9 @@ __device__ __forceinline__ void fwd_take_part(FwdItem& it, int rank, int split) 
   it.n_max = j1 - j0;
 }
 
-// kDeep: every chunk is tested for logits that are all far below zero, which take the short series.  A chunk that fails it
-// has paid a packed addition per pair and two votes: the form without kDeep tests while it pays (DeepWatch), see few_deep_logits().
-template <int D, bool kBF16, bool kScoreMod, bool kAccurate, bool kSplit, bool kDeep>
+// kForm: kDeepNear and kDeepFar test every chunk for logits that are all far enough below zero for a short polynomial (see sigmoid2_near).  A
+// chunk that fails the test has paid a packed addition per pair and two votes: kDeepWatched tests while it pays (DeepWatch).  See deep_form().
+template <int D, bool kBF16, bool kScoreMod, bool kAccurate, bool kSplit, DeepForm kForm>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                    const __grid_constant__ CUtensorMap v_map, const FwdParams p) {
@@ -881,7 +890,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       if (!ok) break;
       const int item = item_ring[16 * islot];
       if (item < 0) break;
-      int n0, n1, q0, Lk;  // (q0: kSplit: relative to the first key of this CTA's part, as Lk)
+      int n0, n1, q0, Lk, rows;  // (rows: valid ones from the item's first on; q0: kSplit: relative to the first key of this CTA's part, as Lk)
       float c0;
       const float* sm_row = nullptr;
       int sm_lim = 0;
@@ -891,6 +900,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         n1 = it.n1;
         q0 = it.q0 - (kSplit ? it.k_first : 0);
         Lk = it.Lk;
+        rows = it.Lq - it.q0;
         c0 = it.bias * kLog2e;
         if constexpr (kScoreMod) {
           sm_row = p.score_mod + (p.cu_k ? (int64_t)it.tk0 : (int64_t)it.b * p.Tk + (kSplit ? it.k_first : 0));
@@ -910,6 +920,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           lim[s] = min(lim[s], q0 + 128 * s + lane_row);
           mask_from[s] = min(mask_from[s], q0 + 128 * s + 1);
         }
+        if (128 * s + lane_row >= rows) lim[s] = -1;
       }
       const int n_max = max(n0, n1);
       watch.start();
@@ -931,9 +942,9 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
                 tmem_ld32_sync(s_addr, r);
                 // the predicate code exists only in the instantiation used by boundary chunks
                 if (col0 + 32 > mask_from[s])
-                  fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate, kDeep>(s_addr, r, c1, c0, col0, lim[s], watch, col0, sm_row, sm_lim);
+                  fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate, kForm>(s_addr, r, c1, c0, col0, lim[s], watch, col0, sm_row, sm_lim);
                 else
-                  fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate, kDeep>(s_addr, r, c1, c0, col0, lim[s], watch, col0, sm_row, sm_lim);
+                  fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate, kForm>(s_addr, r, c1, c0, col0, lim[s], watch, col0, sm_row, sm_lim);
                 tmem_st_wait();
                 tc_fence_before_sync();
                 __syncwarp();
@@ -985,9 +996,9 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
             tmem_ld_wait_for(r);
             if (c == 0) tmem_ld(s_addr + 32, rbuf[1]);
             if (col0 + 32 * c + 32 > mask_from[s])
-              fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate, kDeep>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], watch, mod[c], mod_patch);
+              fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate, kForm>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], watch, mod[c], mod_patch);
             else
-              fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate, kDeep>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], watch, mod[c], mod_patch);
+              fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate, kForm>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], watch, mod[c], mod_patch);
             if constexpr (kScoreMod) mod[c] = load_mod((j + j_step) * kTileN + 64 * g + 32 * c + lane);
           }
           tmem_st_wait();

@@ -390,16 +390,23 @@ int fwd_split(const SigAttnParams* p, int n_sm) {
   return split > 1 ? split : 0;
 }
 
-// Whether the 16-bit kernels test for logits far below zero (below -3.5, all 1024 of a warp's chunk) only while chunks pass, instead
-// of always: with a bias of the caller's, the same for the whole batch and above -3, scores would have to be below zero
-// throughout to pass.  D = 64 or D = 128, B=4 T=4096, bf16, bias 0, always -> while it pays, us, forward (H=32, H=16) and with the backward:
-//  - scores of both signs, D = 64 924 -> 740 and 2560 -> 2340; D = 128 582 -> 545 and 1904 -> 1880.  Never tested 725 and 2290, 500 and 1830;
-//  - scores about -8, which trained weights may well have, D = 64 755 -> 778, 2260 -> 2310; D = 128 507 -> 520, 1870 -> 1880.  Never tested 810
-//    and 2430, 530 and 1910, and probabilities that are all too small by what the polynomial lacks at 0 (see rcp1p_poly);
-//  - about -8 with every 512th key at 0 (a quarter of the chunks fails): 745 -> 790.
-// The default bias takes the form that always tests: its chunks pass, and are 3 % slower in the other form (second line).
-bool few_deep_logits(const SigAttnParams* p) {
-  return !p->bias && !p->score_mod && !(p->flags & (SIGATTN_ACCURATE | SIGATTN_BIAS_NEG_LOG_LK)) && p->bias_scalar > -3.0f;
+// Which logits below zero the 16-bit kernels test for (all 1024 of a warp's chunk; see sigmoid2_near), and when.
+//  - with a bias of the caller's, the same for the whole batch and above -3, scores would have to be below zero throughout to pass:
+//    kDeepWatched tests only while chunks pass.  bf16, bias 0, B=4 T=4096, a test for every chunk -> while it pays, us, forward (H=32 D=64,
+//    H=16 D=128) and with the backward: scores of both signs 924 -> 740 and 2560 -> 2340, 582 -> 545 and 1904 -> 1880; about -8, which
+//    trained weights may well have, 755 -> 778 and 2260 -> 2310, 507 -> 520 and 1870 -> 1880; about -8 with every 512th key at 0 745 -> 790.
+//    (Never tested 725 and 2290, 810 and 2430, and probabilities that are all too small by what the polynomial lacks at 0, see rcp1p_poly.)
+//  - D = 64, up to 1024 keys: kDeepNear, which scores of deviation 1 pass under the default bias, where kDeepFar, which is two operations
+//    shorter per pair, sends them on to the polynomial for all logits.  Far -> near, us, H=16: forward bf16 512 x 512 960 -> 844, 256 x 256
+//    158 -> 145, 32 x 1024 214 -> 214, 16 x 2048 380 -> 405; fp16 128 x 512 266 -> 230, 32 x 1000 234 -> 219, 4 x 4096 382 -> 393; backward
+//    512 x 512 2345 -> 2286, 32 x 1000 650 -> 600, 32 x 1024 520 -> 518, 16 x 2048 926 -> 933.  The errors are smaller than before: T=512 bf16, dV
+//    2.63e-3 -> 2.36e-3, dQ 3.88e-3 -> 3.72e-3; fp16 3.4e-4 -> 3.0e-4, 4.9e-4 -> 4.6e-4.
+//    (By the keys and not by the bias, which some callers pass as an array: the result is the same either way.)  At D = 128 the forward does
+//    not gain (scores of deviation 0.25, T=512 175 -> 183).
+sigattn::DeepForm deep_form(const SigAttnParams* p) {
+  if (!p->bias && !p->score_mod && !(p->flags & (SIGATTN_ACCURATE | SIGATTN_BIAS_NEG_LOG_LK)) && p->bias_scalar > -3.0f)
+    return sigattn::kDeepWatched;
+  return p->D == 64 && p->Tk <= 1024 && !(p->flags & SIGATTN_ACCURATE) ? sigattn::kDeepNear : sigattn::kDeepFar;
 }
 
 template <int D, bool kBF16, bool kScoreMod, bool kAccurate>
@@ -438,7 +445,7 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
   fp.split = fwd_split(p, info.n_sm);
   if (int rc = zero_gaps(p, false, info.n_sm)) return rc;
   if (fp.split) {
-    auto kernel = sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, true, true>;
+    auto kernel = sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, true, kDeepFar>;
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
     fp.ticket = nullptr;
     cudaLaunchAttribute attr = {};
@@ -455,9 +462,14 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
     if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
     SIG_CUDA(cudaLaunchKernelEx(&cfg, kernel, qm, km, vm, fp));
   } else {
-    constexpr bool kCanBeShallow = !kScoreMod && !kAccurate;
-    auto kernel = kCanBeShallow && few_deep_logits(p) ? sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, false, !kCanBeShallow>
-                                                  : sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, false, true>;
+    auto pick = [&]() {
+      if constexpr (!kScoreMod && !kAccurate)
+        if (deep_form(p) == kDeepWatched) return sigattn_fwd_kernel<D, kBF16, false, false, false, kDeepWatched>;
+      if constexpr (D == 64 && !kAccurate)
+        if (deep_form(p) == kDeepNear) return sigattn_fwd_kernel<D, kBF16, kScoreMod, false, false, kDeepNear>;
+      return sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, false, kDeepFar>;
+    };
+    auto kernel = pick();
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
     fp.ticket = next_ticket_pair(info, p->device, stream);
     // persistent: one CTA per SM (the kernel's shared memory allows no more), fewer when there are fewer items
@@ -553,9 +565,17 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
   bp.ticket = next_ticket_pair(info, p->device, stream);
 
   {
-    const bool shallow = !kAccurate && few_deep_logits(p);
-    auto kernel = by_head ? (shallow ? sigattn_bwd_kernel<D, kBF16, kAccurate, !kAccurate, kAccurate> : sigattn_bwd_kernel<D, kBF16, kAccurate, !kAccurate, true>)
-                          : (shallow ? sigattn_bwd_kernel<D, kBF16, kAccurate, false, kAccurate> : sigattn_bwd_kernel<D, kBF16, kAccurate, false, true>);
+    // (the accurate sigmoid has one form, and D = 128, where P is fp32 throughout, one for both ranges)
+    auto pick = [&]() {
+      if constexpr (!kAccurate) {
+        if (deep_form(p) == kDeepWatched) return by_head ? sigattn_bwd_kernel<D, kBF16, false, true, kDeepWatched> : sigattn_bwd_kernel<D, kBF16, false, false, kDeepWatched>;
+        if constexpr (D == 64)
+          if (deep_form(p) == kDeepFar) return by_head ? sigattn_bwd_kernel<D, kBF16, false, true, kDeepFar> : sigattn_bwd_kernel<D, kBF16, false, false, kDeepFar>;
+        if (by_head) return sigattn_bwd_kernel<D, kBF16, false, true, kDeepNear>;
+      }
+      return sigattn_bwd_kernel<D, kBF16, kAccurate, false, kDeepNear>;
+    };
+    auto kernel = pick();
     constexpr int smem = BwdSmem<D>::kDynBytes;
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
     // persistent: one CTA per SM (the kernel's shared memory allows no more), fewer when there are fewer items

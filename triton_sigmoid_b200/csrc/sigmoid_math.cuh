@@ -7,6 +7,11 @@ namespace sigattn {
 
 constexpr float kLog2e = 1.4426950408889634f;
 
+// The forms of the kernels: chunks of logits below zero are looked for in the near range (see sigmoid2_near) while chunks pass, there
+// always, and in the far one.
+enum DeepForm { kDeepWatched, kDeepNear, kDeepFar };
+enum DeepRange { kNear, kFar };
+
 // sigmoid(x) with x given in the base-2 domain (t = x * log2(e)).
 // e = 2^-|t| in (0,1] (one MUFU op); sigmoid = (t < 0 ? e : 1) / (1 + e).  This keeps RELATIVE
 // accuracy for strongly negative logits (the default bias is -log(T), so a typical probability
@@ -51,39 +56,38 @@ __device__ __forceinline__ float2 sigmoid2_from_log2_neg(float2 t) {
   return __fmul2_rn(e, rcp1p_poly<kBF16>(e));
 }
 
-// Far below zero the series sigmoid(x) = e - e^2 + e^3 - ... (e = exp(x)) needs very few terms.  The
-// kernels evaluate their logits shifted up by kDeepShift (in the base-2 domain, folded into the bias
-// they add anyway), u = t + kDeepShift, so that "every logit of the warp is below -kDeepShift" is the
-// same sign-bit test as warp_all_negative(); that is the usual case under the default bias -log(T)
-// (a typical probability is 1/T).  With e' = 2^u = 2^kDeepShift e:
-//   fp16: p = e' (a + e' (b + e' c)),  a = 2^-5, b = -2^-10, c = 2^-15   (relative error < e^3 <= 3.1e-5)
-//   bf16: p = e' (a + e' b)                                             (relative error < e^2 <= 9.8e-4)
-// i.e. two or three packed operations after the exponential instead of four or five.
-constexpr float kDeepShift = 5.0f;
+// Below zero, sigmoid(x) = e / (1 + e) with e = exp(x) <= E needs a short polynomial only.  The kernels evaluate their logits shifted
+// up by -log2 E (in the base-2 domain, folded into the bias they add anyway), u = t - log2 E, so that "every logit of the warp is below
+// log E" is the same sign-bit test as warp_all_negative(), and e' = 2^u = e / E.  Two ranges:
+//   near  E = 1/4 (bf16), 1/8 (fp16), x < -1.39, -2.08: p = e' (a + e' (b + e' c)) in fp32, fitted for the least relative error with a = E exact:
+//         4.4e-4 and 6.4e-5 at most, 1.4e-4 and 3.1e-5 at e = 1/128
+//   far   E = 1/32, x < -3.47: the series e - e^2 (bf16; relative error e^2 <= 9.8e-4), e - e^2 + e^3 (fp16; e^3 <= 3.1e-5) on packed 16-bit
+//         pairs, see sigmoid2_far_packed
+// What matters is E.  Under the default bias -log(T) and scores of deviation 1, a chunk of 1024 logits passes the far test from T = 2000 on
+// and the near one from T = 256 on (bf16; fp16 512).  See deep_form() for
+// which is taken and what it measured.
+constexpr float kFarShift = 5.0f;
+template <bool kBF16> constexpr float kNearShift = kBF16 ? 2.0f : 3.0f;
+template <DeepRange kRange, bool kBF16> constexpr float kDeepShift = kRange == kFar ? kFarShift : kNearShift<kBF16>;
 template <bool kBF16>
-__device__ __forceinline__ float2 sigmoid2_from_shifted_log2_deep(float2 u) {
+__device__ __forceinline__ float2 sigmoid2_near(float2 u) {
+  constexpr float a = kBF16 ? 0.25f : 0.125f, b = kBF16 ? -0.98041906f * a * a : -0.99429952f * a * a, c = kBF16 ? 0.72727273f * a * a * a : 0.84690567f * a * a * a;
   const float2 e = make_float2(ex2_approx(u.x), ex2_approx(u.y));
-  constexpr float a = 0.03125f, b = -0.0009765625f, c = 0.000030517578125f;
-  float2 r;
-  if constexpr (kBF16) {
-    r = __ffma2_rn(e, make_float2(b, b), make_float2(a, a));
-  } else {
-    r = __ffma2_rn(e, make_float2(c, c), make_float2(b, b));
-    r = __ffma2_rn(r, e, make_float2(a, a));
-  }
+  float2 r = __ffma2_rn(e, make_float2(c, c), make_float2(b, b));
+  r = __ffma2_rn(r, e, make_float2(a, a));
   return __fmul2_rn(e, r);
 }
 
-// True when every one of a warp's logits t[0..N) (all 32 lanes) is negative: AND of the sign bits.
+// True when every one of a warp's logits t[0..N) (all 32 lanes) is negative: AND of the sign bits.  Lanes with a negative `dead` do not count.
 template <int N>
-__device__ __forceinline__ bool warp_all_negative(const float2 (&t)[N]) {
+__device__ __forceinline__ bool warp_all_negative(const float2 (&t)[N], int dead = 0) {
   uint32_t sgn = 0x80000000u;
 #pragma unroll
   for (int i = 0; i < N; ++i) sgn &= __float_as_uint(t[i].x) & __float_as_uint(t[i].y);
-  return __all_sync(0xffffffffu, (int)sgn < 0) != 0;
+  return __all_sync(0xffffffffu, ((int)sgn | dead) < 0) != 0;
 }
 
-// Whether a warp's next chunk is tested for logits far below zero, in the forms without kDeep.  The first chunk of an item is; after
+// Whether a warp's next chunk is tested for logits far below zero, in the kDeepWatched forms.  The first chunk of an item is; after
 // a failure 7, 15 and then always 31 chunks go untested, after one behind a test that passed 1, 3, 7, ...  Every item starts
 // anew: which CTA takes it, and after which others, must not show in its results.
 struct DeepWatch {
@@ -116,8 +120,8 @@ __device__ __forceinline__ float2 ex2_emulated2(float2 u) {
   asm("add.rm.ftz.f32x2 %0, %1, %2;"
       : "=l"(*reinterpret_cast<unsigned long long*>(&y))
       : "l"(*reinterpret_cast<const unsigned long long*>(&u)), "l"(*reinterpret_cast<const unsigned long long*>(&magic2)));
-  const float2 yb = __fadd2_rn(y, make_float2(-kMagic, -kMagic));
-  const float2 r = __fadd2_rn(u, make_float2(-yb.x, -yb.y));  // fraction in [0, 1)
+  const float2 nb = __ffma2_rn(y, make_float2(-1.0f, -1.0f), magic2);  // -floor(u)
+  const float2 r = __fadd2_rn(u, nb);  // fraction in [0, 1)
   float2 p;
   if constexpr (kBF16) {
     p = __ffma2_rn(make_float2(0.3371894061565399f, 0.3371894061565399f), r, make_float2(0.657636284828186f, 0.657636284828186f));
@@ -149,14 +153,14 @@ __device__ __forceinline__ uint32_t hmul2(uint32_t a, uint32_t b) {
   return d;
 }
 
-// The deep-regime series of sigmoid2_from_shifted_log2_deep() evaluated in the 16-bit type the result is
-// stored in anyway: e' = 2^u is rounded to 16 bits first and the series runs on packed pairs,
+// The series of the far range evaluated in the 16-bit type the result is stored in anyway: e' = 2^u is rounded to 16 bits first and the
+// series runs on packed pairs,
 //   fp16: p = e' (a + e' (b + e' c)),   bf16: p = e' (a + e' b),   a = 2^-5, b = -2^-10, c = 2^-15,
 // which halves the instructions after the exponential (one conversion, two or three packed operations
 // per PAIR of elements).  Relative error: two roundings of the 16-bit type instead of one.
 // `emulate` selects the FMA-pipe exponential for this pair.
 template <bool kBF16>
-__device__ __forceinline__ uint32_t sigmoid2_deep_packed(float2 u, bool emulate) {
+__device__ __forceinline__ uint32_t sigmoid2_far_packed(float2 u, bool emulate) {
   const float2 e = emulate ? ex2_emulated2<kBF16>(u) : make_float2(ex2_approx(u.x), ex2_approx(u.y));
   const uint32_t eh = pack2<kBF16>(e.x, e.y);
   if constexpr (kBF16) {
