@@ -465,6 +465,10 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   // (looked at behind the set-up, where the warps meet anyway)
   const bool sick = *reinterpret_cast<volatile int*>(&g_status_word) != 0;
 
+  // (without a second item, or pair, for any CTA nobody asks for one, and the counters stay as they are)
+  const int n_tickets = kByHead ? p.B * p.H : p.n_items;
+  const bool tickets = n_tickets > (int)gridDim.x;
+
   // ---------------------------------------------------------------- setup
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -751,12 +755,14 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       if (kByHead && tile > 0 && tile < p.n_kvblk) {
         item = head * p.n_kvblk + tile++;
       } else {
-        const int n_tickets = kByHead ? p.B * p.H : p.n_items;
-        if (lane == 0 && k > 0) {
-          const unsigned int tk = atomicAdd(p.ticket, 1u) + gridDim.x;
-          item = tk < (unsigned int)n_tickets ? (int)tk : -1;
+        if (k > 0) {
+          item = -1;
+          if (lane == 0 && tickets) {
+            const unsigned int tk = atomicAdd(p.ticket, 1u) + gridDim.x;
+            item = tk < (unsigned int)n_tickets ? (int)tk : -1;
+          }
+          item = __shfl_sync(0xffffffffu, item, 0);
         }
-        item = __shfl_sync(0xffffffffu, item, 0);
         if (kByHead && item >= 0) {
           head = item;
           tile = 1;
@@ -1193,7 +1199,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     tc_fence_after_sync();
     tmem_dealloc(tmem, kTmemCols);
   }
-  if (threadIdx.x == 0) {
+  if (tickets && threadIdx.x == 0) {
     // the last CTA to finish leaves both counters at zero for the next launch that uses them
     __threadfence();
     const unsigned int done = atomicAdd(p.ticket + 1, 1u);

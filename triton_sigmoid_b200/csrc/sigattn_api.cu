@@ -471,7 +471,7 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
     };
     auto kernel = pick();
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
-    fp.ticket = next_ticket_pair(info, p->device, stream);
+    fp.ticket = n_items > info.n_sm ? next_ticket_pair(info, p->device, stream) : nullptr;  // (more items than CTAs)
     // persistent: one CTA per SM (the kernel's shared memory allows no more), fewer when there are fewer items
     dim3 grid((unsigned int)std::min<int64_t>(n_items, info.n_sm));
     if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
