@@ -20,7 +20,8 @@ def test_against_64_bits(B, H, Tq, Tk, form, causal, D):
     assert launch_form(B, H, Tq, Tk, D, torch.float32, True, causal) == form
     q, k, v, do = make_inputs(B, Tq, Tk, H, D, torch.float32, std=0.5, seed=Tq + Tk)
     leaf = [t.requires_grad_() for t in (q, k, v)]
-    got = torch.autograd.grad(m.sigmoid_attention(*leaf, is_causal=causal, sigmoid_bias=-1.0), leaf, do)
+    full = [torch.full((B,), n, dtype=torch.int32, device="cuda") for n in (Tk, Tq)]
+    got = torch.autograd.grad(m.sigmoid_attention_padded(*leaf, *full, is_causal=causal, sigmoid_bias=-1.0), leaf, do)
     qd, kd, vd, dd = (t.detach().double().transpose(1, 2) for t in (q, k, v, do))
     p = torch.sigmoid(qd @ kd.transpose(-1, -2) / D ** 0.5 - 1.0)
     if causal:

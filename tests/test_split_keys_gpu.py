@@ -75,3 +75,40 @@ def test_split_keys_accurate(Tq, Tk, causal, D):
         with sa.accurate_sigmoid():
             check_against_oracle(sa.sigmoid_attention_padded, q, k, v, do, torch.float16, backward=False, is_causal=causal,
                                  score_mod=score_mod)
+
+
+@pytest.mark.parametrize("D", [8, 64])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,H,Tq,Tk,causal,accurate", [
+    (2, 4, 256, 256, False, False),   # two items of 128 rows per head, one key tile per group of warps
+    (1, 2, 300, 300, True, False),    # the last item has 44 rows
+    (3, 5, 1, 64, False, False),      # one query, one key tile: the second group has no work
+    (2, 2, 64, 129, False, True),     # the queries twice, second key tile of one column
+    (2, 2, 63, 300, True, False),
+    (2, 3, 65, 65, True, True),       # one row too many for that
+    (4, 8, 64, 1500, False, False),   # and with several parts
+    (3, 2, 33, 2100, True, False),
+    (1, 148, 64, 200, False, False),  # as many items as SMs
+    (2, 37, 129, 1030, False, False),
+])
+def test_items_of_128_rows(B, H, Tq, Tk, causal, accurate, dtype, D):
+    q, k, v, do = make_inputs(B, Tq, Tk, H, D, dtype, std=0.7, seed=Tk + D)
+    g = torch.Generator().manual_seed(Tk)
+    lens_k = torch.randint(1, Tk + 1, (B,), generator=g, dtype=torch.int32)
+    lens_q = torch.randint(1, Tq + 1, (B,), generator=g, dtype=torch.int32)
+    lens_k[0], lens_q[0] = Tk, Tq
+    if B > 2:
+        lens_k[1] = 0
+    for b in range(B):
+        q[b, int(lens_q[b]):] = float("nan")
+        k[b, int(lens_k[b]):] = float("nan")
+        v[b, int(lens_k[b]):] = float("nan")
+    mod = 0.5 * torch.randn(B, Tk, generator=g).cuda()
+    lq, lk = lens_q.cuda(), lens_k.cuda()
+    with sa.accurate_sigmoid(accurate):
+        for score_mod in (None, mod):
+            kw = dict(is_causal=causal, sigmoid_bias=-2.0, score_mod=score_mod)
+            check_against_oracle(lambda a, b, c, **x: sa.sigmoid_attention_padded(q, k, v, **x), torch.nan_to_num(q), torch.nan_to_num(k),
+                                 torch.nan_to_num(v), do, dtype, lens_q=lq, lens_k=lk, backward=False, **kw)
+            one, two = (sa.sigmoid_attention_padded(q, k, v, seq_lens_k=lk, seq_lens_q=lq, **kw) for _ in range(2))
+            assert torch.equal(one, two)

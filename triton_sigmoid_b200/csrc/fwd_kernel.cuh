@@ -37,7 +37,9 @@
 //
 // Split form (kSplit), for problems with too few items to occupy the SMs: a cluster of p.split CTAs shares one item, each
 // takes a contiguous part of its key tiles, and the partial O, in fp32, are added through distributed shared memory (no
-// workspace, no atomics, a fixed order).  See fwd_split() on the host side for when.
+// workspace, no atomics, a fixed order).  At D = 64 items may have 128 rows there, whose key tiles the two groups of sigmoid warps
+// take alternately; and with at most 64 queries the tile holds them twice, each copy for half of every key tile's columns, so that no
+// lane of TMEM is without work (p.twice).  See fwd_plan() on the host side for when.
 //
 // Masking: key tiles beyond the causal diagonal or the valid key length are skipped
 // entirely; tiles that straddle either boundary apply an element predicate.
@@ -68,6 +70,8 @@ struct FwdParams {
   int n_items;  // B * H * n_qblk
   int group;    // (batch, head) pairs per scheduling group, >= 1 (see fwd_decode_item)
   int split;    // kSplit: CTAs per cluster = parts of the key range of an item (no tickets then)
+  int block_m;  // kSplit: query rows per item, 256 or, D = 64, 128
+  int twice;    // kSplit, block_m = 128: at most 64 queries, which are both halves of the tile (the Q map's box has 64 rows)
   // two counters, zero between launches: [0] items handed out beyond the first per CTA,
   // [1] CTAs that have finished (the last one clears both)
   unsigned int* ticket;
@@ -322,7 +326,7 @@ __device__ __forceinline__ FwdItem fwd_load_item(const volatile int* rec) {
   it.n_max = rec[13]; it.bias = __int_as_float(rec[14]); it.k_first = rec[15];
   return it;
 }
-__device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item) {
+__device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item, int block_m = kFwdBlockM) {
   FwdItem it;
   // Items are ordered in groups of `group` (batch, head) pairs: within a group all pairs' heaviest
   // query blocks come first, then their second heaviest, ... (a longest-first order under a causal
@@ -337,7 +341,7 @@ __device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item)
   it.b = bh / p.H;
   it.h = bh - it.b * p.H;
   const int qblk = p.causal ? (p.n_qblk - 1 - qi) : qi;  // heavy blocks of a head first
-  it.q0 = qblk * kFwdBlockM;
+  it.q0 = qblk * block_m;
   it.Lq = p.Tq;
   it.Lk = p.Tk;
   if (p.lens_q) it.Lq = min(max(p.lens_q[it.b], 0), p.Tq);
@@ -361,7 +365,7 @@ __device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item)
     const int r0 = it.q0 + 128 * s;
     int kv_end = it.Lk;
     if (p.causal) kv_end = min(kv_end, r0 + 128);
-    n_kv[s] = (r0 < it.Lq) ? (kv_end + kTileN - 1) / kTileN : 0;
+    n_kv[s] = (r0 < it.Lq && 128 * s < block_m) ? (kv_end + kTileN - 1) / kTileN : 0;
   }
   it.n0 = n_kv[0];
   it.n1 = n_kv[1];
@@ -420,12 +424,42 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   // (looked at behind the set-up, where the warps meet anyway)
   const bool sick = *reinterpret_cast<volatile int*>(&g_status_word) != 0;
 
+  // kSplit, single: no item has a second query tile, so the two groups of sigmoid warps and the two accumulators of
+  // D = 64 take the key tiles alternately instead (job j: group j & 1, O_(j & 1)); the output warps add the two.
+  const bool single = kSplit && D == 64 && p.block_m == 128;
+  const bool twice = kSplit && D == 64 && p.twice != 0;
+  // Loads of the producer warp (one lane).
+  auto load_q = [&](const FwdItem& it) {
+#pragma unroll 1
+    for (int s = 0; s < 2; ++s) {
+      if ((s == 0 ? it.n0 : it.n1) > 0) {
+        mbar_expect_tx(bar(L::kQFull + s), kTileBytes);
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c)
+          tma_load_4d(smem_base + L::kQOff + s * kTileBytes + c * 16384, &q_map, bar(L::kQFull + s), c * 64, it.h,
+                      it.tq0 + it.q0 + 128 * s, it.bc);
+        if (kSplit && D == 64 && p.twice) tma_load_4d(smem_base + L::kQOff + 8192, &q_map, bar(L::kQFull), 0, it.h, it.tq0 + it.q0, it.bc);
+      }
+    }
+  };
+  auto load_k = [&](const FwdItem& it, int j, int st) {
+    mbar_expect_tx(bar(L::kKFull + st), kTileBytes);
+#pragma unroll
+    for (int c = 0; c < D / 64; ++c)
+      tma_load_4d(smem_base + L::kKOff + st * kTileBytes + c * 16384, &k_map, bar(L::kKFull + st), c * 64, it.h, it.tk0 + j * kTileN, it.bc);
+  };
+  auto load_v = [&](const FwdItem& it, int j, int st) {
+    mbar_expect_tx(bar(L::kVFull + st), kTileBytes);
+#pragma unroll
+    for (int c = 0; c < D / 64; ++c)
+      tma_load_4d(smem_base + L::kVOff + st * kTileBytes + c * 16384, &v_map, bar(L::kVFull + st), c * 64, it.h, it.tk0 + j * kTileN, it.bc);
+  };
   // Without a second item for any CTA nobody asks for one, and the counters stay as they are (their clean-up by the last CTA took 1900
   // clocks of a small launch: B=2 T=256 H=4 D=64 12.6 -> 10.7 us).
   const bool tickets = !kSplit && p.n_items > (int)gridDim.x;
 
   // ---------------------------------------------------------------- setup
-  if (threadIdx.x == 0) {
+  auto init = [&]() {
     *abort_flag = 0;
     mbar_init(bar(L::kQFull + 0), 1);
     mbar_init(bar(L::kQFull + 1), 1);
@@ -449,11 +483,45 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       mbar_init(bar(L::kItemEmpty + i), kItemReaders);
     }
     fence_mbar_init();
-  }
-  if (warp == kFwdProducerWarp && lane == 0) {
+  };
+  FwdItem first = {};    // kSplit: this CTA's part of its item
+  bool loading = false;  // kSplit: loads under way
+  if (warp == kFwdIssuerWarp2 && lane == 0) {
     tma_prefetch_desc(&q_map);
     tma_prefetch_desc(&k_map);
     tma_prefetch_desc(&v_map);
+  }
+  if (threadIdx.x == 0) init();
+  if constexpr (kSplit) {
+    // One item per CTA, and few CTAs: the launch is as long as one item's chain, which starts before the warps meet, with the decoding, the
+    // records and the first loads.
+    constexpr int kBarsReady = 1;  // named barrier: the mbarriers are initialised (warp 0, producer warp)
+    if (warp == 0) {
+      __syncwarp();
+      asm volatile("bar.arrive %0, 64;" ::"n"(kBarsReady) : "memory");
+    } else if (warp == kFwdProducerWarp) {
+      first = fwd_decode_item(p, (int)blockIdx.x / p.split, p.block_m);
+      const int n0 = first.n0, n1 = first.n1, n_max = first.n_max;
+      fwd_take_part(first, (int)blockIdx.x % p.split, p.split);
+      if (lane == 0) {
+        fwd_publish_item(item_ring, 0, first);
+        item_ring[16] = -1;  // no second one; in its record the key tiles of the whole item
+        item_ring[17] = n0;
+        item_ring[18] = n1;
+        item_ring[19] = n_max;
+      }
+      asm volatile("bar.sync %0, 64;" ::"n"(kBarsReady) : "memory");
+      if (lane == 0) {
+        mbar_arrive(bar(L::kItemFull + 0));
+        mbar_arrive(bar(L::kItemFull + 1));
+        if (first.n_max > 0 && !sick) {
+          load_q(first);
+          load_k(first, 0, 0);
+          load_v(first, 0, 0);
+          loading = true;
+        }
+      }
+    }
   }
   if (warp == kFwdIssuerWarp) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
@@ -465,6 +533,12 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   if (leave) {
+    if (kSplit && loading) {  // (they write to this CTA's shared memory)
+      for (int q = 0; q < 2; ++q)
+        if ((q == 0 ? first.n0 : first.n1) > 0) mbar_wait(bar(L::kQFull + q), 0u, abort_flag, kSiteBase + 3);
+      mbar_wait(bar(L::kKFull), 0u, abort_flag, kSiteBase + 5);
+      mbar_wait(bar(L::kVFull), 0u, abort_flag, kSiteBase + 6);
+    }
     if (warp == kFwdIssuerWarp) tmem_dealloc(tmem, kTmemCols);
     if constexpr (kSplit) {  // (the others of the cluster may have got another answer, and read this CTA's shared memory)
       cluster_sync();
@@ -488,10 +562,6 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     if (lane == 0) mbar_arrive(bar(L::kItemEmpty + slot));
     return item;
   };
-
-  // kSplit, single: no item has a second query tile, so the two groups of sigmoid warps and the two accumulators of
-  // D = 64 take the key tiles alternately instead (job j: group j & 1, O_(j & 1)); the output warps add the two.
-  const bool single = kSplit && D == 64 && p.Tq <= 128;
 
   if (warp >= kFwdOutputWarp0) {
     // ============================================================ output warps: O from TMEM to global memory
@@ -517,6 +587,18 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         tc_fence_after_sync();
       }
       if constexpr (kSplit) {
+        auto load_o = [&](int s, int c, uint32_t (&ra)[16]) {  // 16 columns of a lane's row
+          uint32_t rb[16];
+          tmem_ld16(tmem_lane + kColO + D * s + 16 * c, ra);
+          const bool two = single && it.n0 > 1;
+          if (two) tmem_ld16(tmem_lane + kColO + D + 16 * c, rb);
+          tmem_ld_wait_for(ra);
+          if (two) {
+            tmem_ld_wait_for(rb);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) ra[i] = __float_as_uint(__uint_as_float(ra[i]) + __uint_as_float(rb[i]));
+          }
+        };
         // The partial O of this CTA, fp32, over the K / V stages: every tile has been loaded and every product that reads
         // one is complete.  [tile][row][D], 16-byte pieces swizzled by the row.
         uint8_t* part = smem_gen + L::kKOff;
@@ -526,15 +608,8 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
             uint8_t* row = part + (s * 128 + lane_row) * (4 * D);
 #pragma unroll 1
             for (int c = 0; c < D / 16; ++c) {
-              uint32_t ra[16], rb[16];
-              tmem_ld16(tmem_lane + kColO + D * s + 16 * c, ra);
-              tmem_ld_wait_for(ra);
-              if (single && it.n0 > 1) {
-                tmem_ld16(tmem_lane + kColO + D + 16 * c, rb);
-                tmem_ld_wait_for(rb);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) ra[i] = __float_as_uint(__uint_as_float(ra[i]) + __uint_as_float(rb[i]));
-              }
+              uint32_t ra[16];
+              load_o(s, c, ra);
 #pragma unroll
               for (int i = 0; i < 4; ++i)
                 *reinterpret_cast<uint4*>(row + (((4 * c + i) ^ (lane & 7)) << 4)) =
@@ -683,13 +758,15 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     int act = 0;         // items with work so far
     bool ok = true;
     for (int k = 0; ok; ++k) {
-      const int slot = k & 1;
-      ok = mbar_wait_warp(bar(L::kItemEmpty + slot), ((uint32_t)(k >> 1) & 1u) ^ 1u, abort_flag, kSiteBase + 31);
-      if (!ok) break;
-      int item = blockIdx.x;  // the first item needs no ticket
+      FwdItem it = {};
       if constexpr (kSplit) {
-        item = k == 0 ? (int)blockIdx.x / p.split : -1;
+        if (k > 0) break;
+        it = first;
       } else {
+        const int slot = k & 1;
+        ok = mbar_wait_warp(bar(L::kItemEmpty + slot), ((uint32_t)(k >> 1) & 1u) ^ 1u, abort_flag, kSiteBase + 31);
+        if (!ok) break;
+        int item = blockIdx.x;  // the first item needs no ticket
         if (k > 0) {
           item = -1;
           if (lane == 0 && tickets) {
@@ -698,54 +775,32 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           }
           item = __shfl_sync(0xffffffffu, item, 0);
         }
+        if (item >= 0) it = fwd_decode_item(p, item);
+        if (lane == 0) {
+          if (item >= 0) fwd_publish_item(item_ring + 16 * slot, item, it);
+          else item_ring[16 * slot] = -1;
+          mbar_arrive(bar(L::kItemFull + slot));  // (release: the record is visible to whoever sees the phase)
+        }
+        if (item < 0) break;
       }
-      FwdItem it = {};
-      if (item >= 0) it = fwd_decode_item(p, item);
-      if constexpr (kSplit)
-        if (item >= 0) fwd_take_part(it, (int)blockIdx.x % p.split, p.split);
-      if (lane == 0) {
-        if (item >= 0) fwd_publish_item(item_ring + 16 * slot, item, it);
-        else item_ring[16 * slot] = -1;
-        mbar_arrive(bar(L::kItemFull + slot));  // (release: the record is visible to whoever sees the phase)
-      }
-      if (item < 0) break;
       if (it.n_max == 0) continue;
 
-      // Q tiles of this item: the previous item's score products must have read theirs
-      if (act > 0) ok = mbar_wait_warp(bar(L::kQEmpty), (uint32_t)(act - 1) & 1u, abort_flag, kSiteBase + 32);
-      if (!ok) break;
-      if (lane == 0) {
-#pragma unroll 1
-        for (int s = 0; s < 2; ++s) {
-          if ((s == 0 ? it.n0 : it.n1) > 0) {
-            mbar_expect_tx(bar(L::kQFull + s), kTileBytes);
-#pragma unroll
-            for (int c = 0; c < D / 64; ++c)
-              tma_load_4d(smem_base + L::kQOff + s * kTileBytes + c * 16384, &q_map, bar(L::kQFull + s), c * 64, it.h,
-                          it.tq0 + it.q0 + 128 * s, it.bc);
-          }
-        }
+      if constexpr (!kSplit) {
+        // Q tiles of this item: the previous item's score products must have read theirs
+        if (act > 0) ok = mbar_wait_warp(bar(L::kQEmpty), (uint32_t)(act - 1) & 1u, abort_flag, kSiteBase + 32);
+        if (!ok) break;
+        if (lane == 0) load_q(it);
       }
       int st = tile % kStages;
       uint32_t ph = (uint32_t)(tile / kStages) & 1u;
       for (int j = 0; j < it.n_max && ok; ++j) {
-        ok = mbar_wait_warp(bar(L::kKEmpty + st), ph ^ 1u, abort_flag, kSiteBase + 1);
-        if (!ok) break;
-        if (lane == 0) {
-          mbar_expect_tx(bar(L::kKFull + st), kTileBytes);
-#pragma unroll
-          for (int c = 0; c < D / 64; ++c)
-            tma_load_4d(smem_base + L::kKOff + st * kTileBytes + c * 16384, &k_map, bar(L::kKFull + st), c * 64, it.h,
-                        it.tk0 + j * kTileN, it.bc);
-        }
-        ok = mbar_wait_warp(bar(L::kVEmpty + st), ph ^ 1u, abort_flag, kSiteBase + 2);
-        if (!ok) break;
-        if (lane == 0) {
-          mbar_expect_tx(bar(L::kVFull + st), kTileBytes);
-#pragma unroll
-          for (int c = 0; c < D / 64; ++c)
-            tma_load_4d(smem_base + L::kVOff + st * kTileBytes + c * 16384, &v_map, bar(L::kVFull + st), c * 64, it.h,
-                        it.tk0 + j * kTileN, it.bc);
+        if (!kSplit || j > 0) {  // (else under way since the set-up)
+          ok = mbar_wait_warp(bar(L::kKEmpty + st), ph ^ 1u, abort_flag, kSiteBase + 1);
+          if (!ok) break;
+          if (lane == 0) load_k(it, j, st);
+          ok = mbar_wait_warp(bar(L::kVEmpty + st), ph ^ 1u, abort_flag, kSiteBase + 2);
+          if (!ok) break;
+          if (lane == 0) load_v(it, j, st);
         }
         if (j * kTileN + kTileN > it.Lk) {
           // The tile straddles the valid key length.  P is zero for the padded keys, but 0 * NaN
@@ -916,6 +971,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(L::kItemEmpty + islot));  // the record is in registers
+      const int q_row = twice ? lane_row & 63 : lane_row;
       // per query tile: largest visible key index of this thread's row, and the first key index at which a
       // chunk needs the element predicate (it reaches beyond the keys every row of the tile sees)
       int lim[2], mask_from[2];
@@ -924,10 +980,10 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         lim[s] = Lk - 1;
         mask_from[s] = Lk;
         if (p.causal) {
-          lim[s] = min(lim[s], q0 + 128 * s + lane_row);
+          lim[s] = min(lim[s], q0 + 128 * s + q_row);
           mask_from[s] = min(mask_from[s], q0 + 128 * s + 1);
         }
-        if (128 * s + lane_row >= rows) lim[s] = -1;
+        if (128 * s + q_row >= rows) lim[s] = -1;
       }
       const int n_max = max(n0, n1);
       watch.start();
@@ -982,9 +1038,12 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         }
         auto load_mod = [&](int key) -> float { return key < sm_lim ? __ldg(sm_row + key) * kLog2e : 0.0f; };
         float mod[2] = {0.0f, 0.0f};  // this lane's terms of the two chunks, loaded one key tile ahead
+        // first column of a warp's two chunks, or, with the queries twice, of its only one: the first copy's rows are for columns 0 to 63, the
+        // second one's for the rest, and the other half of the P of each is zero
+        const int my_col = twice ? 64 * ((warp & 3) >> 1) + 32 * g : 64 * g;
         if constexpr (kScoreMod) {
-          mod[0] = load_mod(j_first * kTileN + 64 * g + lane);
-          mod[1] = load_mod(j_first * kTileN + 64 * g + 32 + lane);
+          mod[0] = load_mod(j_first * kTileN + my_col + lane);
+          mod[1] = load_mod(j_first * kTileN + my_col + 32 + lane);
         }
         for (int j = j_first; j < n_mine && ok; j += j_step) {
           const int n = jobs_base + (s == 0 ? j + min(j, n1) : j + min(j + 1, n0));
@@ -992,8 +1051,28 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           ok = mbar_wait_warp(bar(L::kSFull + jb), (uint32_t)(n / kSBufs) & 1u, abort_flag, kSiteBase + 10 + s);
           if (!ok) break;
           tc_fence_after_sync();
-          const uint32_t s_addr = tmem_lane + kColS + 128u * (uint32_t)jb + 64u * (uint32_t)g;
-          const int col0 = j * kTileN + 64 * g;
+          const uint32_t s_addr = tmem_lane + kColS + 128u * (uint32_t)jb + (uint32_t)my_col;
+          const int col0 = j * kTileN + my_col;
+          if constexpr (kSplit) {
+            if (twice) {
+              uint32_t r[32], none[16];
+              tmem_ld(s_addr, r);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) none[i] = 0u;
+              tmem_st(tmem_lane + kColS + 128u * (uint32_t)jb + (uint32_t)(my_col ^ 64), none);
+              tmem_ld_wait_for(r);
+              if (col0 + 32 > mask_from[s])
+                fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate, kForm>(s_addr, r, c1, c0, col0, lim[s], watch, mod[0], mod_patch);
+              else
+                fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate, kForm>(s_addr, r, c1, c0, col0, lim[s], watch, mod[0], mod_patch);
+              if constexpr (kScoreMod) mod[0] = load_mod((j + j_step) * kTileN + my_col + lane);
+              tmem_st_wait();
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar(L::kPFull + jb));
+              continue;
+            }
+          }
           // two register buffers: the load of the second chunk is in flight while the first is computed
           uint32_t rbuf[2][32];
           tmem_ld(s_addr, rbuf[0]);
@@ -1006,7 +1085,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
               fwd_sigmoid_chunk<kBF16, kScoreMod, true, kAccurate, kForm>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], watch, mod[c], mod_patch);
             else
               fwd_sigmoid_chunk<kBF16, kScoreMod, false, kAccurate, kForm>(s_addr + 32 * c, r, c1, c0, col0 + 32 * c, lim[s], watch, mod[c], mod_patch);
-            if constexpr (kScoreMod) mod[c] = load_mod((j + j_step) * kTileN + 64 * g + 32 * c + lane);
+            if constexpr (kScoreMod) mod[c] = load_mod((j + j_step) * kTileN + my_col + 32 * c + lane);
           }
           tmem_st_wait();
           tc_fence_before_sync();
@@ -1022,39 +1101,61 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     }
 
     if constexpr (kSplit) {
-      // ---- the cluster's partial O, added up in the order of the ranks: every rank finishes its share of the rows
+      // ---- the cluster's partial O, added up in the order of the ranks (and of the copies): every rank finishes its share of the rows,
+      // a thread twice four columns, with eight loads under way at a time.
       const int rank = (int)blockIdx.x % p.split;
-      const FwdItem it = fwd_decode_item(p, (int)blockIdx.x / p.split);  // the whole item
+      const FwdItem it = fwd_load_item(item_ring);  // (the fields that do not depend on the part)
+      const int n0 = item_ring[17], n1 = item_ring[18], n_max = item_ring[19];
+      uint32_t have0 = 0u, have1 = 0u;  // ranks with keys, per query tile
+      for (int r = 0; r < p.split; ++r) {
+        const int j0 = fwd_part_begin(n_max, r, p.split), j1 = fwd_part_begin(n_max, r + 1, p.split);
+        if (j0 < min(n0, j1)) have0 |= 1u << r;
+        if (j0 < min(n1, j1)) have1 |= 1u << r;
+      }
+      if (twice) have0 |= have0 << p.split;  // (the second copies' rows are 64 on, with the same swizzle)
+      const int sources = twice ? 2 * p.split : p.split;
+      const int share = (twice ? 64 : p.Tq <= 128 || single ? 128 : 256) / p.split;
+      constexpr int kPieces = D / 4;
       cluster_sync();
-      constexpr int kPieces = D / 8;  // 8 columns = 16 bytes of O
-      const int share = (p.Tq <= 128 ? 128 : 256) / p.split;
-      for (int i = threadIdx.x; i < share * kPieces; i += kFwdSigmoidWarps * 32) {
-        const int row = rank * share + i / kPieces, piece = i % kPieces;  // row of the item's 256
-        const int n_s = row < 128 ? it.n0 : it.n1;
-        const int qrow = it.q0 + row;
-        if (qrow >= it.row_lim || 8 * piece >= p.d_cols) continue;
-        float acc[8];
+#pragma unroll 1
+      for (int i0 = threadIdx.x; i0 < share * kPieces; i0 += 2 * kFwdSigmoidWarps * 32) {
+        float4 acc[2];
+        uint32_t at[2], have[2];
+        uint8_t* dst[2];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] = 0.0f;
-        if (qrow < it.Lq) {  // rows beyond the valid length are written as zeros
-          const uint32_t at = smem_base + L::kKOff + (uint32_t)row * (4 * D);
-          for (int r = 0; r < p.split; ++r) {
-            if (fwd_part_begin(it.n_max, r, p.split) >= min(n_s, fwd_part_begin(it.n_max, r + 1, p.split))) continue;  // no keys there
+        for (int u = 0; u < 2; ++u) {
+          const int i = i0 + u * kFwdSigmoidWarps * 32;
+          const int row = rank * share + i / kPieces, piece = i % kPieces;  // row of the item
+          const int qrow = it.q0 + row;
+          const bool written = i < share * kPieces && qrow < it.row_lim && 4 * piece < p.d_cols;
+          dst[u] = written ? reinterpret_cast<uint8_t*>(p.o) + 2 * ((int64_t)it.bc * p.o_sb + (int64_t)it.h * p.o_sh + (int64_t)(it.tq0 + qrow) * p.o_st) + 8 * piece
+                           : nullptr;
+          acc[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          at[u] = smem_base + L::kKOff + (uint32_t)row * (4 * D) + (uint32_t)((piece ^ (row & 7)) << 4);
+          have[u] = !written || qrow >= it.Lq ? 0u : row < 128 ? have0 : have1;  // rows beyond the valid length are written as zeros
+        }
+#pragma unroll 1
+        for (int r0 = 0; r0 < sources; r0 += 4) {
+          float4 x[2][4];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const float4 x = ld_cluster_f4(at + (((2 * piece + h) ^ (row & 7)) << 4), (uint32_t)r);
-              acc[4 * h + 0] += x.x; acc[4 * h + 1] += x.y; acc[4 * h + 2] += x.z; acc[4 * h + 3] += x.w;
+          for (int e = 0; e < 4; ++e) {
+            const int n = r0 + e, copy = n >= p.split ? 1 : 0;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              x[u][e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+              if ((have[u] >> n) & 1u) x[u][e] = ld_cluster_f4(at[u] + copy * (64 * 4 * D), (uint32_t)(n - copy * p.split));
             }
           }
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              acc[u].x += x[u][e].x; acc[u].y += x[u][e].y; acc[u].z += x[u][e].z; acc[u].w += x[u][e].w;
+            }
         }
-        uint4 w;
-        w.x = pack2<kBF16>(acc[0], acc[1]);
-        w.y = pack2<kBF16>(acc[2], acc[3]);
-        w.z = pack2<kBF16>(acc[4], acc[5]);
-        w.w = pack2<kBF16>(acc[6], acc[7]);
-        *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.o) +
-                                  2 * ((int64_t)it.bc * p.o_sb + (int64_t)it.h * p.o_sh + (int64_t)(it.tq0 + qrow) * p.o_st) +
-                                  16 * piece) = w;
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (dst[u]) *reinterpret_cast<uint2*>(dst[u]) = make_uint2(pack2<kBF16>(acc[u].x, acc[u].y), pack2<kBF16>(acc[u].z, acc[u].w));
       }
       cluster_sync();  // no CTA's shared memory goes away while another reads it
     }

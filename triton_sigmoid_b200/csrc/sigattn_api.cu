@@ -373,21 +373,39 @@ unsigned int* next_ticket_pair(const FwdDeviceInfo& info, int device, cudaStream
   return info.tickets + 2 * (kEagerTicketSlots + next_captured[device].fetch_add(1u) % (kTicketSlots - kEagerTicketSlots));
 }
 
-// CTAs per item of the forward: 0 = the persistent form, else the split form with clusters of that many.
-// With fewer items than half of the SMs the key range of each is split, as long as every part keeps two key tiles (a part
+// How the forward divides its work: the persistent form, or, with fewer items than half of the SMs, the split one with clusters of `split`
+// CTAs per item.
+// The key range of each is split, as long as every part keeps two key tiles (a part
 // of one costs as much in the cluster's hand-over as it saves) and the clusters still find room at once (they must lie
 // within a GPC, whose SM counts are not all multiples of 8: 7/8 of the SMs are counted on).
 // B=8 H=8, 64 queries on 1024 .. 4096 keys: 47 -> 29 us; B=1 T=4096 H=2, D = 64 61 -> 33, D = 128 74 -> 37; B=1 T=1024 H=4
 // 24.6 -> 20.5; with two parts of two tiles, B=1 T=512 H=4, 20 -> 18.4; unchanged beyond 64 items, B=1 T=8192 H=4.
-int64_t fwd_items(const SigAttnParams* p) {
-  return (int64_t)((p->Tq + sigattn::kFwdBlockM - 1) / sigattn::kFwdBlockM) * p->H * p->B;
-}
-int fwd_split(const SigAttnParams* p, int n_sm) {
-  const int64_t n_items = fwd_items(p);
+// At D = 64 with items of 128 rows, whose key tiles the two groups of sigmoid warps take alternately, there are twice as many to split, and up
+// to 64 queries fill both halves of a tile (FwdParams::twice): 64 queries as above with a per-key term 26.9 -> 20.7 us, without 23.4 -> 18.7, B=1
+// 14.5 -> 12.5; one query on 4096 keys 22.7 -> 18.7.
+int64_t fwd_items(const SigAttnParams* p, int rows) { return (int64_t)((p->Tq + rows - 1) / rows) * p->H * p->B; }
+struct FwdPlan {
+  int block_m = sigattn::kFwdBlockM;  // query rows per item
+  int split = 0;                      // 0: persistent
+  bool twice = false;
+};
+FwdPlan fwd_plan(const SigAttnParams* p, int n_sm) {
   const int tiles = (p->Tk + sigattn::kTileN - 1) / sigattn::kTileN;
-  int split = 1;
-  while (split < 8 && n_items * split * 2 <= n_sm * 7 / 8 && tiles >= 4 * split) split *= 2;
-  return split > 1 ? split : 0;
+  auto parts = [&](int64_t n_items) {
+    int split = 1;
+    while (split < 8 && n_items * split * 2 <= n_sm * 7 / 8 && tiles >= 4 * split) split *= 2;
+    return split;
+  };
+  FwdPlan plan;
+  const int64_t narrow = fwd_items(p, 128);
+  const int split = parts(fwd_items(p, sigattn::kFwdBlockM));
+  if (split > 1) plan.split = split;
+  if (p->D == 64 && narrow <= n_sm && (parts(narrow) > 1 || (split == 1 && p->Tq <= 64))) {
+    plan.block_m = 128;
+    plan.split = parts(narrow);
+    plan.twice = p->Tq <= 64;
+  }
+  return plan;
 }
 
 // Which logits below zero the 16-bit kernels test for (all 1024 of a warp's chunk; see sigmoid2_near), and when.
@@ -403,10 +421,11 @@ int fwd_split(const SigAttnParams* p, int n_sm) {
 //    2.63e-3 -> 2.36e-3, dQ 3.88e-3 -> 3.72e-3; fp16 3.4e-4 -> 3.0e-4, 4.9e-4 -> 4.6e-4.
 //    (By the keys and not by the bias, which some callers pass as an array: the result is the same either way.)  At D = 128 the forward does
 //    not gain (scores of deviation 0.25, T=512 175 -> 183).
+constexpr int kNearKeys = 1024;
 sigattn::DeepForm deep_form(const SigAttnParams* p) {
   if (!p->bias && !p->score_mod && !(p->flags & (SIGATTN_ACCURATE | SIGATTN_BIAS_NEG_LOG_LK)) && p->bias_scalar > -3.0f)
     return sigattn::kDeepWatched;
-  return p->D == 64 && p->Tk <= 1024 && !(p->flags & SIGATTN_ACCURATE) ? sigattn::kDeepNear : sigattn::kDeepFar;
+  return p->D == 64 && p->Tk <= kNearKeys && !(p->flags & SIGATTN_ACCURATE) ? sigattn::kDeepNear : sigattn::kDeepFar;
 }
 
 template <int D, bool kBF16, bool kScoreMod, bool kAccurate>
@@ -433,19 +452,27 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
   fp.Tk = p->Tk;
   fp.d_cols = head_cols(p);
   fp.causal = (p->flags & SIGATTN_CAUSAL) ? 1 : 0;
-  fp.n_qblk = (p->Tq + kFwdBlockM - 1) / kFwdBlockM;
-  const int64_t n_items = fwd_items(p);
+  FwdDeviceInfo info;
+  if (int rc = fwd_device_info(p->device, &info)) return rc;
+  const FwdPlan plan = fwd_plan(p, info.n_sm);
+  fp.split = plan.split;
+  fp.block_m = plan.block_m;
+  fp.twice = plan.twice ? 1 : 0;
+  fp.n_qblk = (p->Tq + plan.block_m - 1) / plan.block_m;
+  const int64_t n_items = fwd_items(p, plan.block_m);
   if (n_items > INT32_MAX) return fail(-2, "too many (batch, head, query block) items: %lld", (long long)n_items);
   fp.n_items = (int)n_items;
   // K and V of one head, half of the L2 for them
   fp.group = schedule_group(fp.causal != 0, (int64_t)p->B * p->H, (int64_t)p->Tk * D * 2 * 2, 64ll << 20);
-  FwdDeviceInfo info;
-  if (int rc = fwd_device_info(p->device, &info)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-  fp.split = fwd_split(p, info.n_sm);
   if (int rc = zero_gaps(p, false, info.n_sm)) return rc;
   if (fp.split) {
-    auto kernel = sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, true, kDeepFar>;
+    auto pick = [&]() {
+      if constexpr (D == 64 && !kAccurate)
+        if (p->Tk <= kNearKeys) return sigattn_fwd_kernel<D, kBF16, kScoreMod, false, true, kDeepNear>;
+      return sigattn_fwd_kernel<D, kBF16, kScoreMod, kAccurate, true, kDeepFar>;
+    };
+    auto kernel = pick();
     if (int rc = set_smem(kernel, smem, p->device)) return rc;
     fp.ticket = nullptr;
     cudaLaunchAttribute attr = {};
@@ -562,7 +589,7 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
   // reductions their locality, a few heads already balance the CTAs)
   bp.group = by_head ? 1 : schedule_group(bp.causal != 0, n_bh, (int64_t)p->Tq * D * (2 + 2 + 4), 32ll << 20);
   if (int rc = zero_gaps(p, true, info.n_sm)) return rc;
-  bp.ticket = next_ticket_pair(info, p->device, stream);
+  bp.ticket = (by_head ? n_bh : n_items) > info.n_sm ? next_ticket_pair(info, p->device, stream) : nullptr;  // (more items than CTAs)
 
   {
     // (the accurate sigmoid has one form, and D = 128, where P is fp32 throughout, one for both ranges)
@@ -887,7 +914,7 @@ int sigattn_form(const SigAttnParams* p, int backward, int n_sm) {
     if (f32_tc(p, backward != 0, n_sm)) return SIGATTN_FORM_F32_TC;
     return f32_tile_rows(p, n_sm) == 64 ? SIGATTN_FORM_F32_64 : SIGATTN_FORM_F32_16;
   }
-  if (!backward) return fwd_split(p, n_sm) ? SIGATTN_FORM_FWD_SPLIT : SIGATTN_FORM_FWD;
+  if (!backward) return fwd_plan(p, n_sm).split > 1 ? SIGATTN_FORM_FWD_SPLIT : SIGATTN_FORM_FWD;
   if (p->flags & SIGATTN_BWD_SPLIT) return SIGATTN_FORM_BWD_STREAM;
   return bwd_by_head(p, n_sm) ? SIGATTN_FORM_BWD_BY_HEAD : SIGATTN_FORM_BWD;
 }
@@ -961,7 +988,10 @@ int sigattn_fwd(const SigAttnParams* p) {
   }
   if (p->dtype == SIGATTN_FP32) return launch_f32(p, false);
   CUtensorMap qm, km, vm;
-  if ((rc = make_map(&qm, p->q, p->dtype, ex.B, ex.Tq, p->H, head_cols(p), map_strides(p->q_strides, ex.Tq, ex.packed).s, 128, "q"))) return rc;
+  FwdDeviceInfo info;
+  if ((rc = fwd_device_info(p->device, &info))) return rc;
+  const int q_rows = fwd_plan(p, info.n_sm).twice ? 64 : 128;  // of a load
+  if ((rc = make_map(&qm, p->q, p->dtype, ex.B, ex.Tq, p->H, head_cols(p), map_strides(p->q_strides, ex.Tq, ex.packed).s, q_rows, "q"))) return rc;
   if ((rc = make_map(&km, p->k, p->dtype, ex.B, ex.Tk, p->H, head_cols(p), map_strides(p->k_strides, ex.Tk, ex.packed).s, 128, "k"))) return rc;
   if ((rc = make_map(&vm, p->v, p->dtype, ex.B, ex.Tk, p->H, head_cols(p), map_strides(p->v_strides, ex.Tk, ex.packed).s, 128, "v"))) return rc;
   if ((reinterpret_cast<uintptr_t>(p->o) & 15u) != 0) return fail(-3, "o: base pointer must be 16-byte aligned");
