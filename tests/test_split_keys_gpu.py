@@ -90,6 +90,7 @@ def test_split_keys_accurate(Tq, Tk, causal, D):
     (3, 2, 33, 2100, True, False),
     (1, 148, 64, 200, False, False),  # as many items as SMs
     (2, 37, 129, 1030, False, False),
+    (5, 40, 40, 2000, False, False),  # more items than SMs, 16 key tiles
 ])
 def test_items_of_128_rows(B, H, Tq, Tk, causal, accurate, dtype, D):
     q, k, v, do = make_inputs(B, Tq, Tk, H, D, dtype, std=0.7, seed=Tk + D)

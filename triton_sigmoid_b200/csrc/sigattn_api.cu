@@ -383,6 +383,9 @@ unsigned int* next_ticket_pair(const FwdDeviceInfo& info, int device, cudaStream
 // At D = 64 with items of 128 rows, whose key tiles the two groups of sigmoid warps take alternately, there are twice as many to split, and up
 // to 64 queries fill both halves of a tile (FwdParams::twice): 64 queries as above with a per-key term 26.9 -> 20.7 us, without 23.4 -> 18.7, B=1
 // 14.5 -> 12.5; one query on 4096 keys 22.7 -> 18.7.
+// In one part, that pays for any number of items of up to 64 queries once their key tiles outweigh that its CTAs are not persistent: 512 items,
+// 64 queries, keys up to 4096 106 -> 85 us, 160 items 51 -> 41, 512 items up to 2048 69 -> 66, up to 1024 47 -> 49; 2048 items of one query up
+// to 1500 158 -> 172.
 int64_t fwd_items(const SigAttnParams* p, int rows) { return (int64_t)((p->Tq + rows - 1) / rows) * p->H * p->B; }
 struct FwdPlan {
   int block_m = sigattn::kFwdBlockM;  // query rows per item
@@ -400,7 +403,7 @@ FwdPlan fwd_plan(const SigAttnParams* p, int n_sm) {
   const int64_t narrow = fwd_items(p, 128);
   const int split = parts(fwd_items(p, sigattn::kFwdBlockM));
   if (split > 1) plan.split = split;
-  if (p->D == 64 && narrow <= n_sm && (parts(narrow) > 1 || (split == 1 && p->Tq <= 64))) {
+  if (p->D == 64 && ((narrow <= n_sm && parts(narrow) > 1) || (split == 1 && p->Tq <= 64 && (narrow <= n_sm || tiles >= 16)))) {
     plan.block_m = 128;
     plan.split = parts(narrow);
     plan.twice = p->Tq <= 64;
