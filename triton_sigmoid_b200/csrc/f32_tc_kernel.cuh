@@ -169,8 +169,10 @@ __device__ __forceinline__ float2 tc_sigmoid2(float2 y, float factor_down) {
 __device__ __forceinline__ float tc_sigmoid_tiny(float y, float below) { return ex2_approx(40.0f - y) * below; }
 
 // One tile; `block` counts those of the mode.
-template <int D, int kMode>
-__device__ __forceinline__ void f32_tc_tile(const F32Params& p, const unsigned int block, const int n_tiles) {
+// kSplit: a cluster of `split` CTAs shares it, each takes a contiguous part of the jobs; the sums of the others go to the first one's
+// registers through distributed shared memory, in the order of the ranks.  See tc_split() on the host side for when.
+template <int D, int kMode, bool kSplit>
+__device__ __forceinline__ void f32_tc_tile(const F32Params& p, const unsigned int block, const int n_tiles, const int split) {
   using L = TcShape<D, kMode>;
   constexpr int kSite = (0x6 + kMode) << 16;
   extern __shared__ uint8_t tc_smem[];
@@ -179,13 +181,19 @@ __device__ __forceinline__ void f32_tc_tile(const F32Params& p, const unsigned i
   const F32Item it = f32_item(p, block, n_tiles, !L::kKeyRows);
   // a kernel of this library already gave up on a wait: leave, all warps or none (the named barriers below count on every warp,
   // and the word may change while they read it)
-  if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) return;
+  if (__syncthreads_or(*reinterpret_cast<volatile int*>(&g_status_word) != 0)) {
+    if constexpr (kSplit) {  // (the others of the cluster may have got another answer, and read this CTA's shared memory)
+      cluster_sync();
+      cluster_sync();
+    }
+    return;
+  }
   const int r0 = it.tile * kTcRows;
   const int Lr = L::kKeyRows ? it.Lk : it.Lq, Lc = L::kKeyRows ? it.Lq : it.Lk;
   const int row_lim = L::kKeyRows ? it.key_lim : it.row_lim;
-  const int c_begin = L::kKeyRows && p.causal ? r0 : 0;
+  int c_begin = L::kKeyRows && p.causal ? r0 : 0;
   const int c_end = !L::kKeyRows && p.causal ? min(Lc, r0 + kTcRows) : Lc;
-  const int n_jobs = r0 < Lr && c_end > c_begin ? (c_end - c_begin + kTcJob - 1) / kTcJob : 0;
+  int n_jobs = r0 < Lr && c_end > c_begin ? (c_end - c_begin + kTcJob - 1) / kTcJob : 0;
   const int n16 = (p.d_cols + 15) / 16;  // steps of 16 along the head dimension that hold anything
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -229,6 +237,13 @@ __device__ __forceinline__ void f32_tc_tile(const F32Params& p, const unsigned i
     if constexpr (L::kKeyRows && L::kOut2) zero(p.dv, p.dv_sb, p.dv_st, p.dv_sh, it.tk0);
     if constexpr (kMode == kTcDq) zero(p.dq, p.dq_sb, p.dq_st, p.dq_sh, it.tq0);
     return;
+  }
+
+  const int rank = kSplit ? (int)blockIdx.x % split : 0;
+  if constexpr (kSplit) {
+    const int j0 = n_jobs * rank / split, j1 = n_jobs * (rank + 1) / split;
+    c_begin += j0 * kTcJob;
+    n_jobs = j1 - j0;
   }
 
   // ---------------------------------------------------------------- setup
@@ -383,6 +398,7 @@ __device__ __forceinline__ void f32_tc_tile(const F32Params& p, const unsigned i
         }
       }
     }
+    if constexpr (kSplit) { cluster_sync(); cluster_sync(); }
   } else if (warp >= kTcComputeWarps) {
     // ============================================================ conversion of the streamed rows
     // A chunk is 64 rows x 64 columns of one tensor; a thread takes 4 consecutive columns of four of its rows, a warp whole
@@ -451,7 +467,8 @@ __device__ __forceinline__ void f32_tc_tile(const F32Params& p, const unsigned i
         if (lane == 0) mbar_arrive(bar((two ? L::kC2Full : L::kC1Full) + st));
       }
     }
-    f32_wait<0>();  // (the fallback of the compute warps reuses the space)
+    f32_wait<0>();  // (the compute warps reuse the space)
+    if constexpr (kSplit) { cluster_sync(); cluster_sync(); }
   } else {
     // ============================================================ compute
     setmaxnreg_inc<kTcComputeRegs>();
@@ -636,8 +653,36 @@ __device__ __forceinline__ void f32_tc_tile(const F32Params& p, const unsigned i
       if (!L::kBoth && j > 0) drain_all(j - 1);
       if (!ok) break;
     }
-    if (ok) drain_all(n_jobs - 1);
+    if (ok && (!kSplit || n_jobs > 0)) drain_all(n_jobs - 1);
 
+    if constexpr (kSplit) {
+      // (every product has been performed and drained: the space of the streamed tiles is free)
+      constexpr int kPieces = kOutPer / 4;
+      auto at = [&](int out, int c) -> uint32_t { return (uint32_t)(((out * kPieces + c) * (32 * kTcComputeWarps) + (int)threadIdx.x) * 16); };
+      if (rank > 0) {
+#pragma unroll
+        for (int c = 0; c < kPieces; ++c) {
+          if constexpr (L::kOut1) *reinterpret_cast<float4*>(smem_gen + at(0, c)) = make_float4(acc1[4 * c], acc1[4 * c + 1], acc1[4 * c + 2], acc1[4 * c + 3]);
+          if constexpr (L::kOut2) *reinterpret_cast<float4*>(smem_gen + at(1, c)) = make_float4(acc2[4 * c], acc2[4 * c + 1], acc2[4 * c + 2], acc2[4 * c + 3]);
+        }
+      }
+      cluster_sync();
+      if (rank == 0) {
+        auto add = [&](float (&acc)[kOutPer], int out, int r) {
+#pragma unroll
+          for (int c = 0; c < kPieces; ++c) {
+            const float4 x = ld_cluster_f4(smem_base + at(out, c), (uint32_t)r);
+            acc[4 * c] += x.x; acc[4 * c + 1] += x.y; acc[4 * c + 2] += x.z; acc[4 * c + 3] += x.w;
+          }
+        };
+#pragma unroll 1
+        for (int r = 1; r < split; ++r) {
+          if constexpr (L::kOut1) add(acc1, 0, r);
+          if constexpr (L::kOut2) add(acc2, 1, r);
+        }
+      }
+      cluster_sync();  // no CTA's shared memory goes away while another reads it
+    }
     // ------------------------------------------------------------ epilogue
     float finite = 0.f;  // NaN when a sum is not finite
 #pragma unroll
@@ -655,7 +700,7 @@ __device__ __forceinline__ void f32_tc_tile(const F32Params& p, const unsigned i
       return r != 0;
     };
     const bool redo = any(row < Lr && !(finite == 0.f));
-    if (!any(!ok || *abort_flag != 0)) {
+    if (!any(!ok || *abort_flag != 0) && rank == 0) {
       if (!redo) {
         store_all(acc1, acc2);
       } else {
@@ -679,9 +724,11 @@ __device__ __forceinline__ void f32_tc_tile(const F32Params& p, const unsigned i
   }
 }
 
-template <int D>
-__global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_fwd_kernel(const F32Params p, const int n_tiles) {
-  f32_tc_tile<D, kTcFwd>(p, blockIdx.x, n_tiles);
+// Tiles from `first` on.
+template <int D, bool kSplit>
+__global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_fwd_kernel(const F32Params p, const int n_tiles, const int split, const int first) {
+  if constexpr (kSplit) f32_tc_tile<D, kTcFwd, true>(p, first + blockIdx.x / split, n_tiles, split);
+  else f32_tc_tile<D, kTcFwd, false>(p, blockIdx.x, n_tiles, 1);
 }
 template <int D>
 constexpr int tc_bwd_bytes() {
@@ -694,17 +741,17 @@ constexpr int tc_bwd_bytes() {
 // All tiles of the backward in one launch, the heavier kinds first: they need nothing of each other, and one CTA per SM in turn
 // leaves SMs idle at the end of each launch.  One launch per kind -> one, us: B=4 T=2048 H=8 D=64 (512 tiles of each kind, 3.46 waves) 683 -> 589,
 // D=128 1873 -> 1686; B=64 T=384 H=8 538 -> 525; B=1 T=8192 H=4 1302 -> 1272.
-template <int D>
-__global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_bwd_kernel(const F32Params p, const int n_k_tiles, const int n_q_tiles) {
+template <int D, bool kSplit>
+__global__ void __launch_bounds__(kTcThreads, 1) sigattn_f32_tc_bwd_kernel(const F32Params p, const int n_k_tiles, const int n_q_tiles, const int split) {
   const unsigned int n_bh = (unsigned int)(p.B * p.H), n_k = n_bh * (unsigned int)n_k_tiles, n_q = n_bh * (unsigned int)n_q_tiles;
-  const unsigned int block = blockIdx.x;
+  const unsigned int block = kSplit ? blockIdx.x / split : blockIdx.x;
   if constexpr (D == 64) {
-    if (block < n_k) f32_tc_tile<D, kTcDkdv>(p, block, n_k_tiles);
-    else f32_tc_tile<D, kTcDq>(p, block - n_k, n_q_tiles);
+    if (block < n_k) f32_tc_tile<D, kTcDkdv, kSplit>(p, block, n_k_tiles, split);
+    else f32_tc_tile<D, kTcDq, kSplit>(p, block - n_k, n_q_tiles, split);
   } else {
-    if (block < n_q) f32_tc_tile<D, kTcDq>(p, block, n_q_tiles);
-    else if (block < n_q + n_k) f32_tc_tile<D, kTcDk>(p, block - n_q, n_k_tiles);
-    else f32_tc_tile<D, kTcDv>(p, block - n_q - n_k, n_k_tiles);
+    if (block < n_q) f32_tc_tile<D, kTcDq, kSplit>(p, block, n_q_tiles, split);
+    else if (block < n_q + n_k) f32_tc_tile<D, kTcDk, kSplit>(p, block - n_q, n_k_tiles, split);
+    else f32_tc_tile<D, kTcDv, kSplit>(p, block - n_q - n_k, n_k_tiles, split);
   }
 }
 

@@ -750,22 +750,65 @@ int launch_f32_shape(const SigAttnParams* p, const sigattn::F32Params& fp, bool 
 }
 
 // float32 tensors on the tensor cores (no tensor maps, no workspace either).
+// CTAs per tile of the float32 tensor-core kernels: with fewer tiles than half of the SMs, the jobs of each are split over a cluster, as long as
+// a part keeps four jobs of 64 rows (clusters of two find room on every SM, larger ones on 7/8 of them, see fwd_plan()).
+// D = 64, us, forward and backward: B=1 H=1 T=4096 103 -> 41 and 159 -> 95; B=1 H=4 T=1024 31 -> 21 and 51 -> 37, T=2048 54 -> 36 and 89 -> 87 (136 tiles
+// of the backward: not split); D = 128 H=1 T=8192 300 -> 170 and 947 -> 939.
+// The last wave of more tiles, forward: B=4 T=2048 H=8 (3.46 waves) 208 -> 195, D = 128 367 -> 349; B=5 T=1024 H=8 90 -> 82.
+int tc_split(int64_t ctas, int jobs, int n_sm) {
+  int split = 1;
+  while (split < 8 && ctas * split * 2 <= (split == 1 ? n_sm : n_sm * 7 / 8) && jobs >= 8 * split) split *= 2;
+  return split;
+}
+template <typename K, typename... Args>
+int launch_clusters(K kernel, int64_t ctas, int split, int threads, int smem, cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned int)split;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned int)(ctas * split));
+  cfg.blockDim = dim3((unsigned int)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  SIG_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  return 0;
+}
+
 template <int D>
-int launch_f32_tc(const SigAttnParams* p, const sigattn::F32Params& fp, bool backward) {
+int launch_f32_tc(const SigAttnParams* p, const sigattn::F32Params& fp, bool backward, int n_sm) {
   using namespace sigattn;
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   const int n_q = (p->Tq + kTcRows - 1) / kTcRows, n_k = (p->Tk + kTcRows - 1) / kTcRows;
   const int64_t ctas = (int64_t)p->B * p->H * (backward ? n_q + (int64_t)n_k * (D == 64 ? 1 : 2) : n_q);
   if (ctas > INT32_MAX) return fail(-2, "too many (batch, head, tile) items: %lld", (long long)ctas);
+  const int split = tc_split(ctas, ((backward ? std::min(p->Tq, p->Tk) : p->Tk) + kTcJob - 1) / kTcJob, n_sm);
   if (!backward) {
     constexpr int smem = TcShape<D, kTcFwd>::kDynBytes;
-    if (int rc = set_smem(sigattn_f32_tc_fwd_kernel<D>, smem, p->device)) return rc;
-    sigattn_f32_tc_fwd_kernel<D><<<(unsigned int)ctas, kTcThreads, smem, stream>>>(fp, n_q);
-  } else {
-    constexpr int smem = tc_bwd_bytes<D>();
-    if (int rc = set_smem(sigattn_f32_tc_bwd_kernel<D>, smem, p->device)) return rc;
-    sigattn_f32_tc_bwd_kernel<D><<<(unsigned int)ctas, kTcThreads, smem, stream>>>(fp, n_k, n_q);
+    auto whole = sigattn_f32_tc_fwd_kernel<D, false>;
+    auto parts = sigattn_f32_tc_fwd_kernel<D, true>;
+    if (int rc = set_smem(whole, smem, p->device)) return rc;
+    if (int rc = set_smem(parts, smem, p->device)) return rc;
+    if (split > 1) return launch_clusters(parts, ctas, split, kTcThreads, smem, stream, fp, n_q, split, 0);
+    // A last wave that half of the SMs would sit out is split in two as well, where all tiles take the same time.
+    const int64_t rest = ctas % n_sm;
+    const bool even = !(p->flags & SIGATTN_CAUSAL) && !p->seq_lens_q && !p->seq_lens_k && !p->cu_seqlens_q && p->Tq % kTcRows == 0;
+    const int last = even && ctas > n_sm && rest > 0 && p->Tk >= 16 * kTcJob ? tc_split(rest, 16, n_sm) : 1;
+    whole<<<(unsigned int)(last > 1 ? ctas - rest : ctas), kTcThreads, smem, stream>>>(fp, n_q, 1, 0);
+    SIG_CUDA(cudaGetLastError());
+    return last > 1 ? launch_clusters(parts, rest, last, kTcThreads, smem, stream, fp, n_q, last, (int)(ctas - rest)) : 0;
   }
+  constexpr int smem = tc_bwd_bytes<D>();
+  if (split > 1) {
+    auto parts = sigattn_f32_tc_bwd_kernel<D, true>;
+    if (int rc = set_smem(parts, smem, p->device)) return rc;
+    return launch_clusters(parts, ctas, split, kTcThreads, smem, stream, fp, n_k, n_q, split);
+  }
+  auto whole = sigattn_f32_tc_bwd_kernel<D, false>;
+  if (int rc = set_smem(whole, smem, p->device)) return rc;
+  whole<<<(unsigned int)ctas, kTcThreads, smem, stream>>>(fp, n_k, n_q, 1);
   SIG_CUDA(cudaGetLastError());
   return 0;
 }
@@ -849,7 +892,7 @@ int launch_f32_d(const SigAttnParams* p, bool backward) {
   if (p->ev_main_start) SIG_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream));
   int rc = 0;
   if (f32_tc(p, backward, info.n_sm)) {
-    rc = launch_f32_tc<D>(p, fp, backward);
+    rc = launch_f32_tc<D>(p, fp, backward, info.n_sm);
   } else
     rc = f32_tile_rows(p, info.n_sm) == 64 ? launch_f32_shape<D, 4, D / 64>(p, fp, backward) : launch_f32_shape<D, 1, 4>(p, fp, backward);
   if (rc) return rc;
