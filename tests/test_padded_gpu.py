@@ -237,3 +237,18 @@ def test_backward_repeatable_with_short_and_long_items_mixed(D, T):
             assert gr[~mask].abs().max().item() == 0
             if mask.any() and r[mask].abs().max() > 0:
                 assert rel_l2(gr[mask], r[mask]) <= 1e-2
+
+
+@pytest.mark.parametrize("D", [64, 96])
+@pytest.mark.parametrize("causal", [False, True])
+def test_dq_accumulator_is_filled_where_it_is_read(causal, D):
+    """Only the query tiles with valid rows are zero-filled and converted: whatever the workspace held, edges of tiles included."""
+    lens = [0, 1, 127, 128, 129, 300, 256]
+    B, T, H = len(lens), 300, 2
+    q, k, v, do = make_inputs(B, T, T, H, D, torch.bfloat16, std=0.5, seed=D, requires_grad=True)
+    lt = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    torch.cuda.empty_cache()
+    size = B * T * H * 128 + 4096
+    spoilt = [torch.full((size,), float("nan"), device="cuda") for _ in range(4)]  # (what the allocator hands out next)
+    del spoilt
+    check_against_oracle(m.sigmoid_attention_padded, q, k, v, do, torch.bfloat16, lens_q=lt, lens_k=lt, is_causal=causal)

@@ -1211,6 +1211,19 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   }
 }
 
+// Padded batches: zero-fills the accumulator's query tiles with valid rows, which a fill of everything does not know: 16 sequences of 256 to
+// 2048, H=8, D = 64 266 -> 258 us for the backward (with a conversion that reads valid rows only), D = 128 (8 of them) 198 -> 189; 64 sequences of 10 to
+// 4096, H=4, 1340 -> 1273.
+template <int D>
+__global__ void __launch_bounds__(256) sigattn_dq_fill_kernel(float* acc, const int* lens_q, int n_tiles, int T, int H) {
+  const int i = (int)(blockIdx.x % (unsigned)n_tiles), bh = (int)(blockIdx.x / (unsigned)n_tiles);
+  if (128 * i >= min(lens_q[bh / H], T)) return;
+  float4* dst = reinterpret_cast<float4*>(acc + ((int64_t)bh * T + 128 * i) * D);
+  const int n = min(128, T - 128 * i) * (D / 4);
+#pragma unroll 4
+  for (int k = threadIdx.x; k < n; k += 256) dst[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+}
+
 // dQ = scale * accumulator, cast to the 16-bit type.  One block per (batch element, head, query tile): the accumulator's
 // pieces in as they lie, turned through shared memory, whole rows out.
 struct DqConvertParams {
@@ -1247,14 +1260,15 @@ __global__ void __launch_bounds__(256) sigattn_dq_convert_kernel(const DqConvert
     const int qrows = min(rows - 32 * quarter, 32);
     const float4* src = reinterpret_cast<const float4*>(p.acc + (int64_t)bc * p.acc_sb + (int64_t)h * p.acc_sh +
                                                         (int64_t)(tq0 + 128 * i + 32 * quarter) * D);
+    if (r < live) {
 #pragma unroll 8
-    for (int c = threadIdx.x >> 7; c < D / 4; c += 2) {
-      const float4 a = __ldg(src + acc_piece(qrows, c, r & 31) / 4);
-      uint2 w;
-      w.x = pack2<kBF16>(a.x * p.scale, a.y * p.scale);
-      w.y = pack2<kBF16>(a.z * p.scale, a.w * p.scale);
-      if (r >= live) w = make_uint2(0u, 0u);
-      *reinterpret_cast<uint2*>(tile + r * kRowBytes + 8 * c) = w;
+      for (int c = threadIdx.x >> 7; c < D / 4; c += 2) {
+        const float4 a = __ldg(src + acc_piece(qrows, c, r & 31) / 4);
+        *reinterpret_cast<uint2*>(tile + r * kRowBytes + 8 * c) = make_uint2(pack2<kBF16>(a.x * p.scale, a.y * p.scale), pack2<kBF16>(a.z * p.scale, a.w * p.scale));
+      }
+    } else {  // (the accumulator may not have been filled there, see sigattn_dq_fill_kernel)
+#pragma unroll 8
+      for (int c = threadIdx.x >> 7; c < D / 4; c += 2) *reinterpret_cast<uint2*>(tile + r * kRowBytes + 8 * c) = make_uint2(0u, 0u);
     }
   }
   __syncthreads();

@@ -560,7 +560,14 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
   if (int rc = fwd_device_info(p->device, &info)) return rc;
   const int64_t n_bh = (int64_t)p->B * p->H;
   const bool by_head = bwd_by_head(p, info.n_sm);
-  if (!by_head) SIG_CUDA(cudaMemsetAsync(dq_acc, 0, need, stream));
+  const int64_t q_tiles = n_bh * ((p->Tq + 127) / 128);
+  if (!by_head && q_tiles > INT32_MAX) return fail(-2, "too many (batch, head, query tile) items: %lld", (long long)q_tiles);
+  if (!by_head && p->seq_lens_q) {
+    sigattn_dq_fill_kernel<D><<<(unsigned int)q_tiles, 256, 0, stream>>>(dq_acc, p->seq_lens_q, (p->Tq + 127) / 128, p->Tq, p->H);
+    SIG_CUDA(cudaGetLastError());
+  } else if (!by_head) {
+    SIG_CUDA(cudaMemsetAsync(dq_acc, 0, need, stream));
+  }
 
   BwdParams bp;
   bp.dq_acc = dq_acc;
@@ -627,9 +634,7 @@ int launch_bwd_fused(const SigAttnParams* p, const CUtensorMap& qm, const CUtens
     cp.n_tiles = (p->Tq + 127) / 128; cp.T = p->Tq; cp.H = p->H;
     cp.d_cols = head_cols(p);
     cp.scale = p->scale;
-    const int64_t blocks = (int64_t)p->B * p->H * cp.n_tiles;
-    if (blocks > INT32_MAX) return fail(-2, "too many (batch, head, query tile) items: %lld", (long long)blocks);
-    sigattn_dq_convert_kernel<D, kBF16><<<(unsigned int)blocks, 256, 0, stream>>>(cp);
+    sigattn_dq_convert_kernel<D, kBF16><<<(unsigned int)q_tiles, 256, 0, stream>>>(cp);
     SIG_CUDA(cudaGetLastError());
   }
   return 0;
