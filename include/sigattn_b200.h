@@ -180,7 +180,7 @@ int sigattn_bwd_static_scratch(const SigAttnParams *p);
  * same results up to the order of fp32 sums).  Looks at extents, dtype and flags only, no pointer is followed and no GPU is
  * needed: for tests and for explaining a measurement. */
 enum SigAttnForm {
-  SIGATTN_FORM_FWD = 0,         /* persistent */
+  SIGATTN_FORM_FWD = 0,         /* persistent (or, with up to 64 queries, the next one in one part) */
   SIGATTN_FORM_FWD_SPLIT = 1,   /* few items: the keys of each are split over a cluster */
   SIGATTN_FORM_BWD = 2,         /* fused, dQ accumulated over the whole workspace and converted */
   SIGATTN_FORM_BWD_BY_HEAD = 3, /* fused, a CTA takes whole (batch element, head) pairs */

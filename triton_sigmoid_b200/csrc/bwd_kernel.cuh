@@ -412,7 +412,7 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item)
 
 // kByHead: a CTA takes all key tiles of a (batch element, head), in order, and finishes its dQ itself (see the drain
 // warps), so that the accumulator needs neither the fill nor the conversion pass and stays in the L2.  group is 1 and the
-// tickets count (batch, head) pairs.  (This form spills more: 140 / 204 bytes of stores / loads by -Xptxas -v at D = 64
+// tickets count (batch, head) pairs.  (This form spills more: 132 / 192 bytes of stores / loads by -Xptxas -v at D = 64
 // against 68 / 80 in the general one, 208 / 300 against 120 / 188 at D = 128.  All registers of the CTA are handed out, see
 // below; the figures of the rule that chooses the form, bwd_by_head(), include these spills.)
 // kForm: as in the forward kernel (kDeepFar at D = 64 only, where P is on packed pairs from the start).

@@ -20,7 +20,7 @@
 // at D = 64 and 4.2e-6 at 128 (3.1 and 3.2e-6), by the last one 1.2 and 0.7e-6 (0.9 and 0.9e-6), by all alike 1.3 and 1.5e-6 (1.2
 // and 1.8e-6); random scores of deviation 16 1.5 to 6e-7 (3.7 to 11e-7).
 //
-// One kernel, five modes, one CTA per (batch, head, 128-row tile); R = stationary side, C = streamed side:
+// Five modes, one CTA (or cluster, see f32_tc_tile) per (batch, head, 128-row tile); R = stationary side, C = streamed side:
 //     kTcFwd   R1 = Q            C1 = K  C2 = V     S = R1 C1^T, P = sigmoid;         out2 = O  += P C2
 //     kTcDkdv  R1 = K  R2 = V    C1 = Q  C2 = dO    S, P, dP = R2 C2^T, dS;           out2 = dV += P C2, out1 = dK += dS C1
 //     kTcDq    R1 = Q  R2 = dO   C1 = K  C2 = V     S, P, dP, dS;                     out1 = dQ += dS C1
@@ -69,8 +69,8 @@ constexpr int kTcIssuerIn = 24;   // scores; owns the TMEM allocation
 constexpr int kTcIssuerOut = 25;  // outputs
 constexpr int kTcThreads = 28 * 32;
 // Registers per thread: 72 at launch (65536 / 896, rounded down to a multiple of 8), then by role.  Spills (bytes of stores / loads,
-// -Xptxas -v): D = 64 forward 0 / 0, dK/dV 56 / 64, dQ 12 / 44; D = 128 forward 12 / 28, dQ 56 / 76, dV 44 / 76, dK 80 / 152, most of them in
-// the FMA code.
+// -Xptxas -v): D = 64 forward 0 / 0, backward (dK/dV and dQ together) 100 / 124; D = 128 forward 12 / 28, backward (three kinds of tiles) 264 / 392,
+// most of them in the FMA code.  Split: 0 / 0, 94 / 120, 16 / 36, 348 / 484.
 constexpr int kTcConvRegs = 48, kTcIssuerRegs = 56, kTcComputeRegs = 88;
 static_assert(kTcComputeWarps * kTcComputeRegs + kTcConvWarps * kTcConvRegs + 4 * kTcIssuerRegs <= 28 * 72, "no more than the launch gave");
 
