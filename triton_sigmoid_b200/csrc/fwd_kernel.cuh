@@ -415,6 +415,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   auto bar = [&](int slot) -> uint32_t { return bars + 8u * slot; };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + L::kMiscOff + 4);
+  volatile int* scored = reinterpret_cast<volatile int*>(smem_gen + L::kMiscOff + 8);  // D = 64: jobs whose scores have been issued
   volatile int* item_ring = reinterpret_cast<volatile int*>(smem_gen + L::kMiscOff + 16);  // 2 records of 16 ints
 
   const int warp = threadIdx.x >> 5;
@@ -461,6 +462,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   // ---------------------------------------------------------------- setup
   auto init = [&]() {
     *abort_flag = 0;
+    *scored = 0;
     mbar_init(bar(L::kQFull + 0), 1);
     mbar_init(bar(L::kQFull + 1), 1);
     for (int i = 0; i < kStages; ++i) {
@@ -843,6 +845,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     FwdCursor c{0, 0, 0, 0u, 0, 0u, true};
     uint32_t q_par0 = 0u, q_par1 = 0u;  // parity of each Q tile's "full" barrier
     int total = 0;                 // jobs issued so far, saturating at kSBufs
+    int issued = 0;                // jobs issued so far
     bool ok = true;
     for (int k = 0; ok; ++k) {
       FwdItem it;
@@ -869,6 +872,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           mma_ss(leader, dst, make_desc(qa + off, hi), make_desc(ka + off, hi), idesc_qk, kk > 0);
         }
         mma_commit(leader, bar(L::kSFull + c.buf));
+        if (kJobWarps == 8 && leader) *scored = ++issued;
         // last job that reads K_j: hand the stage back to the producer
         if (c.s == 1 || c.j >= n1) mma_commit(leader, bar(L::kKEmpty + c.st));
         c.advance(n0, n1, kStages, kSBufs);
@@ -944,6 +948,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     int jobs_base = 0;    // 8 warps per job: jobs of all earlier items, position of this item's first job in the S ring
     float* mod_patch = reinterpret_cast<float*>(smem_gen + L::kModOff) + L::kModFloats * warp;
     bool ok = true;
+    bool missed = false;  // 8 warps per job: jobs of other tiles have gone by since this warp's last one
     DeepWatch watch;
 
     for (int k = 0; ok; ++k) {
@@ -1025,16 +1030,21 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         // phase's parity, so a group must never ask for a job more than kSBufs positions after the last one
         // whose barrier it has seen.  Within and between items in which its tile has jobs that holds by
         // itself (n1 - n0 is 0 or 1, or n1 = 0: at most two foreign jobs in a row).  A group whose tile has
-        // NO job in an item (a query tile beyond the valid length) therefore does not just skip the item: it
-        // watches the barrier of every one of its jobs go by.
+        // NO job in an item (a query tile beyond the valid length) therefore waits, before its next job, until that job's scores have
+        // been issued by the count: the buffer was free then, so the phase before is complete, and the next one cannot be
+        // before this group has done its part.  (Watching the barriers of the foreign jobs go by instead, one after another, fails a warp that
+        // looks away for three jobs, 2 us: it takes the phase after the one it waits for for the one before, and waits for good.)
         const int group = warp >> 3;
         const int s = single ? 0 : group;
         const int g = (warp >> 2) & 1;
         const int n_mine = s == 0 ? n0 : n1;
         const int j_first = single ? group : 0, j_step = single ? 2 : 1;
         if (n_mine == 0) {
-          for (int n = jobs_base; n < jobs_base + n0 + n1 && ok; ++n)
-            ok = mbar_wait_warp(bar(L::kSFull + n % kSBufs), (uint32_t)(n / kSBufs) & 1u, abort_flag, kSiteBase + 10 + s);
+          missed = true;
+        } else if (missed) {
+          const int n = jobs_base + (s == 0 ? 0 : min(1, n0));
+          ok = __all_sync(0xffffffffu, counter_wait(scored, n, abort_flag, kSiteBase + 15)) != 0;
+          missed = false;
         }
         auto load_mod = [&](int key) -> float { return key < sm_lim ? __ldg(sm_row + key) * kLog2e : 0.0f; };
         float mod[2] = {0.0f, 0.0f};  // this lane's terms of the two chunks, loaded one key tile ahead

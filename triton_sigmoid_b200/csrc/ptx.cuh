@@ -85,6 +85,23 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// The same for a counter in shared memory that another warp raises: until it is above `value`.
+__device__ __forceinline__ bool counter_wait(const volatile int* counter, int value, volatile int* abort_flag, int site) {
+  const uint64_t t0 = global_timer_ns();
+  for (uint32_t it = 1; *counter <= value; ++it) {
+    __nanosleep(50);
+    if ((it & 63u) == 0u) {
+      if (*abort_flag) return false;
+      if (global_timer_ns() - t0 > kWaitLimitNs) {
+        *abort_flag = 1;
+        record_abandoned_wait(site);
+        return false;
+      }
+    }
+  }
+  return true;
+}
+
 // The same for a converged warp: every lane waits, and the verdict is made warp-uniform.  The lanes of a
 // converged warp test the barrier in one access and get one answer, so the usual case - the phase is
 // already complete - returns without a vote; only a wait that has to spin pays for one.
