@@ -77,7 +77,7 @@ def test_split_keys_accurate(Tq, Tk, causal, D):
                                  score_mod=score_mod)
 
 
-@pytest.mark.parametrize("D", [8, 64])
+@pytest.mark.parametrize("D", [8, 64, 128])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("B,H,Tq,Tk,causal,accurate", [
     (2, 4, 256, 256, False, False),   # two items of 128 rows per head, one key tile per group of warps

@@ -70,7 +70,7 @@ struct FwdParams {
   int n_items;  // B * H * n_qblk
   int group;    // (batch, head) pairs per scheduling group, >= 1 (see fwd_decode_item)
   int split;    // kSplit: CTAs per cluster = parts of the key range of an item (no tickets then)
-  int block_m;  // kSplit: query rows per item, 256 or, D = 64, 128
+  int block_m;  // query rows per item, 256 or 128
   int twice;    // kSplit, block_m = 128: at most 64 queries, which are both halves of the tile (the Q map's box has 64 rows)
   // two counters, zero between launches: [0] items handed out beyond the first per CTA,
   // [1] CTAs that have finished (the last one clears both)
@@ -326,7 +326,8 @@ __device__ __forceinline__ FwdItem fwd_load_item(const volatile int* rec) {
   it.n_max = rec[13]; it.bias = __int_as_float(rec[14]); it.k_first = rec[15];
   return it;
 }
-__device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item, int block_m = kFwdBlockM) {
+__device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item) {
+  const int block_m = p.block_m;
   FwdItem it;
   // Items are ordered in groups of `group` (batch, head) pairs: within a group all pairs' heaviest
   // query blocks come first, then their second heaviest, ... (a longest-first order under a causal
@@ -367,6 +368,7 @@ __device__ __forceinline__ FwdItem fwd_decode_item(const FwdParams& p, int item,
     if (p.causal) kv_end = min(kv_end, r0 + 128);
     n_kv[s] = (r0 < it.Lq && 128 * s < block_m) ? (kv_end + kTileN - 1) / kTileN : 0;
   }
+  it.row_lim = min(it.row_lim, it.q0 + block_m);
   it.n0 = n_kv[0];
   it.n1 = n_kv[1];
   it.n_max = max(it.n0, it.n1);
@@ -502,7 +504,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       __syncwarp();
       asm volatile("bar.arrive %0, 64;" ::"n"(kBarsReady) : "memory");
     } else if (warp == kFwdProducerWarp) {
-      first = fwd_decode_item(p, (int)blockIdx.x / p.split, p.block_m);
+      first = fwd_decode_item(p, (int)blockIdx.x / p.split);
       const int n0 = first.n0, n1 = first.n1, n_max = first.n_max;
       fwd_take_part(first, (int)blockIdx.x % p.split, p.split);
       if (lane == 0) {

@@ -386,6 +386,8 @@ unsigned int* next_ticket_pair(const FwdDeviceInfo& info, int device, cudaStream
 // In one part, that pays for any number of items of up to 64 queries once their key tiles outweigh that its CTAs are not persistent: 512 items,
 // 64 queries, keys up to 4096 106 -> 85 us, 160 items 51 -> 41, 512 items up to 2048 69 -> 66, up to 1024 47 -> 49; 2048 items of one query up
 // to 1500 158 -> 172.
+// Few items with too few key tiles to split have 128 rows in the persistent form too: B=2 T=256 H=4 D = 64 10.6 -> 10.1 us, T=384 12.5 -> 10.4,
+// D = 128 12.6 -> 10.5, B=16 T=200 12.5 -> 10.4; B=9 T=130 H=8 D = 128 16.6 -> 14.5.
 int64_t fwd_items(const SigAttnParams* p, int rows) { return (int64_t)((p->Tq + rows - 1) / rows) * p->H * p->B; }
 struct FwdPlan {
   int block_m = sigattn::kFwdBlockM;  // query rows per item
@@ -407,6 +409,8 @@ FwdPlan fwd_plan(const SigAttnParams* p, int n_sm) {
     plan.block_m = 128;
     plan.split = parts(narrow);
     plan.twice = p->Tq <= 64;
+  } else if (split == 1 && narrow <= n_sm) {
+    plan.block_m = 128;
   }
   return plan;
 }
