@@ -412,9 +412,8 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item)
 
 // kByHead: a CTA takes all key tiles of a (batch element, head), in order, and finishes its dQ itself (see the drain
 // warps), so that the accumulator needs neither the fill nor the conversion pass and stays in the L2.  group is 1 and the
-// tickets count (batch, head) pairs.  (This form spills more: 132 / 192 bytes of stores / loads by -Xptxas -v at D = 64
-// against 68 / 80 in the general one, 208 / 300 against 120 / 188 at D = 128.  All registers of the CTA are handed out, see
-// below; the figures of the rule that chooses the form, bwd_by_head(), include these spills.)
+// tickets count (batch, head) pairs.  (This form spills more, see the
+// registers below; the figures of the rule that chooses the form, bwd_by_head(), include that.)
 // kForm: as in the forward kernel (at D = 128, where P is in single precision, the far range only).
 template <int D, bool kBF16, bool kAccurate, bool kByHead, DeepForm kForm>
 __global__ void __launch_bounds__(kBwdThreads, 1)
@@ -539,21 +538,17 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     return item;
   };
 
-  // 896 threads get 72 registers each at launch.  Each aligned group of four warps executes one
-  // instruction; the counts add up to exactly what the CTA holds:
-  //   D = 64:  compute 80, role 72 (the issuing warps must not spill: their instruction stream is the critical
-  //            chain), drain 56 (512 x 80 + 128 x 72 + 256 x 56);
+  // 896 threads get 72 registers each at launch.  Each aligned group of four warps executes one instruction; the counts add up to
+  // exactly what the CTA holds:
+  //   D = 64:  compute 80, role 56, drain 64 (512 x 80 + 128 x 56 + 256 x 64);
   //   D = 128: compute 72, role 56, drain 80 (a dQ tile goes from the drain warps' registers, 64 per thread, to the
   //            accumulator in two steps, so that its TMEM columns are free for the next dP at once; 512 x 72 + 128 x 56 + 256 x 80).
-  if constexpr (D == 64) {
-    if (warp < kBwdComputeWarps)         setmaxnreg_inc<80>();
-    else if (warp >= kBwdFirstDrainWarp) setmaxnreg_dec<56>();
-  } else {
-    if (warp >= kBwdFirstDrainWarp)      setmaxnreg_inc<80>();
-    else if (warp >= kBwdComputeWarps)   setmaxnreg_dec<56>();
-  }
-
+  // The instructions stand inside the roles' branches: the compiler allocates registers up to a count only in code that it alone leads to.
+  // Before a join it kept to 72 everywhere, and all roles spilled (bytes of stores / loads, by -Xptxas -v, general and by head: D = 64 68 / 80
+  // and 132 / 192, now 20 / 16 and 72 / 92; D = 128 120 / 188 and 208 / 300, now 60 / 76 and 148 / 188).  Backward, B=512 T=512 H=16 bf16 2190 ->
+  // 2060 us, 24 packed sequences <= 1500, H=8, D=128 287 -> 278, B=8 T=8192 H=32 D=128 causal 11.91 -> 11.45 ms at the power cap.
   if (warp >= kBwdFirstDrainWarp) {
+    if constexpr (D == 64) setmaxnreg_dec<64>(); else setmaxnreg_inc<80>();
     // ============================================================ dQ drain
     // Warp d = warp - 20: lane quarter d & 3 (32 query rows, one per lane), half of the head columns d >> 2.  Per tile:
     // wait for the dQ product, take the block into registers, release the TMEM columns, then add it into the
@@ -729,7 +724,9 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       }
       if (lane == 0) bulk_wait_all();  // every reduction has been performed when the kernel ends
     }
-  } else if (warp == kBwdProducerWarp) {
+  } else if (warp >= kBwdComputeWarps) {
+  setmaxnreg_dec<56>();
+  if (warp == kBwdProducerWarp) {
     // ============================================================ item scheduler + TMA producer
     // Rows beyond the valid lengths may hold anything (NaN included).  Masked probabilities are
     // exactly zero, but 0 * NaN is NaN inside an MMA, so the padded rows of every tile that is
@@ -1015,7 +1012,8 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       ++act;
     }
   }
-  else if (warp < kBwdComputeWarps) {
+  } else {
+    if constexpr (D == 64) setmaxnreg_inc<80>();
     // ============================================================ compute warps
     const int quarter = warp & 3;                         // TMEM lane quarter this warp may access
     const int cg = warp >> 2;                             // query-column group: columns 32 cg .. 32 cg + 31
