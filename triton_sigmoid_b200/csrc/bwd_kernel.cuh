@@ -429,6 +429,10 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   // D = 128: no room for that: one S^T buffer, dQ over the dP^T columns:  S 0 | dP 128 | dV 256 | dK 384.
   // Column group c keeps its 16-bit P^T in S columns 32c + [0,16), dS^T likewise in the dP columns.
   constexpr bool kTwoS = (D == 64);
+  // Products per pass of the loops that issue them.  The roles' code together is more than the SM's instruction caches hold: at D = 128 loops of
+  // two passes are 1 to 3 % faster for it (B=8 T=8192 H=32 causal 11.21 -> 10.92 ms, B=128 T=512 H=8 573 -> 563 us; four passes or eight 1 to 20 %
+  // slower), at D = 64, whose products are half as long, none is.
+  constexpr int kMmaUnroll = (D == 64) ? 8 : 4;
   constexpr uint32_t kColS = 0;
   constexpr uint32_t kColDp = kTwoS ? 256 : 128;
   constexpr uint32_t kColDv = kTwoS ? 384 : 256;
@@ -851,7 +855,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     const uint32_t k_lo = (uint32_t)k_km, v_lo = (uint32_t)v_km, q_lo0 = (uint32_t)q_km0, do_lo0 = (uint32_t)do_km0;
     const uint32_t hi = (uint32_t)(k_km >> 32);  // identical for all four (same layout parameters)
     auto issue = [&](uint32_t dcol, uint32_t a_lo, uint32_t b_lo) {
-#pragma unroll
+#pragma unroll kMmaUnroll
       for (int kk = 0; kk < D / 16; ++kk) {
         const uint32_t off = (uint32_t)(((kk >> 2) * 16384 + (kk & 3) * 32) >> 4);
         mma_ss(leader, tmem + dcol, make_desc(a_lo + off, hi), make_desc(b_lo + off, hi), idesc_st, kk > 0);
@@ -928,7 +932,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     const uint32_t hi = (uint32_t)(k_mn >> 32);
     // acc[key, d] (+)= A^T[key, query] (16-bit, TMEM) . B[query, d]
     auto issue_acc = [&](uint32_t dcol, uint32_t acol, uint32_t b_lo, uint32_t acc0) {
-#pragma unroll
+#pragma unroll kMmaUnroll
       for (int kk = 0; kk < kBwdTileQ / 16; ++kk) {
         // queries 32c .. 32c+31 sit, 16-bit packed, in columns 32c + [0,16) of the source
         mma_ts(leader, tmem + dcol, tmem + acol + 32 * (kk >> 1) + 8 * (kk & 1), make_desc(b_lo + kk * (2048 >> 4), hi),
@@ -981,7 +985,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           // dQ first: the compute warps wait for it before they rewrite the shared-memory copy of dS, its
           // drain starts earlier, and at the last tile of an item it is complete before dK is, so that the
           // epilogue may use the dS buffer as scratch as soon as dK_j, dV_j are complete
-#pragma unroll
+#pragma unroll kMmaUnroll
           for (int kk = 0; kk < kBwdTileKV / 16; ++kk) {
             const uint64_t kd = make_desc(k_lo + kv_off + kk * (2048 >> 4), hi), dsd = make_desc(ds_lo + kk * (2048 >> 4), hi);
             mma_ss(leader, tmem + dq_col(gt), dsd, kd, idesc_dq, kk > 0);
@@ -998,7 +1002,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           ok = mbar_wait_warp(bar(L::kDqEmpty), par ^ 1u, abort_flag, kSiteBase + 10);
           if (!ok) break;
           tc_fence_after_sync();
-#pragma unroll
+#pragma unroll kMmaUnroll
           for (int kk = 0; kk < kBwdTileKV / 16; ++kk) {
             const uint64_t kd = make_desc(k_lo + kv_off + kk * (2048 >> 4), hi), dsd = make_desc(ds_lo + kk * (2048 >> 4), hi);
             mma_ss(leader, tmem + dq_col(gt), dsd, kd, idesc_dq, kk > 0);
@@ -1152,36 +1156,33 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         uint8_t* out_base = is_dk ? reinterpret_cast<uint8_t*>(p.dk) + 2 * ((int64_t)it.bc * p.dk_sb + (int64_t)h * p.dk_sh + (int64_t)it.tk0 * p.dk_st)
                                   : reinterpret_cast<uint8_t*>(p.dv) + 2 * ((int64_t)it.bc * p.dv_sb + (int64_t)h * p.dv_sh + (int64_t)it.tk0 * p.dv_st);
         out_base += 2 * col0;
-        if constexpr (D == 64) {
-          // A lane holds 64 bytes of its key row; written as they are, one store instruction would touch 32
-          // lines (the load/store unit takes them one at a time: about 2000 clocks per item for the CTA).
-          // Each warp therefore turns its 32 x 64-byte block through its own part of the shared-memory copy
-          // of dS - the rows and 16-byte slots it writes in phase B, which no product reads any more once
-          // the item's last dK is complete - so that four lanes cover a row and an instruction 8 rows.
-          uint8_t* ds_gen = smem_gen + L::kDsOff + (cg >> 1) * 16384 + quarter * 32 * 128;  // row 0 of this warp's quarter
+        // A lane holds 64 bytes of its key row (D = 128: twice); written as they are, one store instruction would touch 32
+        // lines, and the load/store unit takes them one at a time: about 2000 clocks per item for the CTA at D = 64; at D = 128 8000 went by
+        // before the slowest warp could go on to the next item.
+        // Each warp therefore turns its 32 x 64-byte block through its own part of the shared-memory copy
+        // of dS - the rows and 16-byte slots it writes in phase B - so that four lanes cover a row and an instruction 8 rows.  No product reads
+        // that any more at D = 64, where dQ is issued before the item's last dK; at D = 128 the last dQ has to be complete first.
+        if constexpr (D == 128) {
+          ok = mbar_wait_warp(bar(L::kDqFull), (uint32_t)(g + n_q - 1) & 1u, abort_flag, kSiteBase + 16);
+          if (!ok) break;
+        }
+        uint8_t* ds_gen = smem_gen + L::kDsOff + (cg >> 1) * 16384 + quarter * 32 * 128;  // row 0 of this warp's quarter
+        const int sub = lane >> 2, piece = lane & 3;
+        const int left = it.key_lim - (kv0 + quarter * 32 + sub);  // rows from this lane's first on
+        uint8_t* out = out_base + 2 * (int64_t)(kv0 + quarter * 32 + sub) * out_st + 16 * piece;
+        const int64_t out_step = 16 * out_st;
+#pragma unroll
+        for (int cc = 0; cc < D / 64; ++cc) {
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4)
-            *reinterpret_cast<uint4*>(ds_gen + lane * 128 + (((chunk0 + q4) ^ sw) << 4)) = w[0][q4];
+            *reinterpret_cast<uint4*>(ds_gen + lane * 128 + (((chunk0 + q4) ^ sw) << 4)) = w[cc][q4];
           __syncwarp();
-          const int c = lane & 3;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int r = 8 * i + (lane >> 2);  // row within the quarter (quarter * 32 is a multiple of 8: same swizzle phase)
-            const uint4 x = *reinterpret_cast<const uint4*>(ds_gen + r * 128 + (((chunk0 + c) ^ (uint32_t)(r & 7)) << 4));
-            const int krow = kv0 + quarter * 32 + r;
-            if (krow < it.key_lim && col0 + 8 * c < p.d_cols) *reinterpret_cast<uint4*>(out_base + 2 * (int64_t)krow * out_st + 16 * c) = x;
+          for (int i = 0; i < 4; ++i) {  // (row sub + 8 i of the quarter, which begins at a multiple of 8 rows: one swizzle phase)
+            const uint4 x = *reinterpret_cast<const uint4*>(ds_gen + (sub + 8 * i) * 128 + (((chunk0 + piece) ^ (uint32_t)sub) << 4));
+            if (8 * i < left && col0 + 32 * cc + 8 * piece < p.d_cols) *reinterpret_cast<uint4*>(out + i * out_step + 64 * cc) = x;
           }
-          __syncwarp();  // phase B of the next item rewrites these slots
-        } else {
-          if (kv < it.key_lim) {
-            uint8_t* out_row = out_base + 2 * (int64_t)kv * out_st;
-#pragma unroll
-            for (int c = 0; c < D / 64; ++c) {
-#pragma unroll
-              for (int q4 = 0; q4 < 4; ++q4)
-                if (col0 + 32 * c + 8 * q4 < p.d_cols) *reinterpret_cast<uint4*>(out_row + 64 * c + 16 * q4) = w[c][q4];
-            }
-          }
+          __syncwarp();  // the slots are rewritten by the next pass, or phase B of the next item
         }
       }
       }
