@@ -350,7 +350,8 @@ struct BwdItem {
   int Lq, Lk;
   int i_begin, n_q;     // first query tile that sees this key tile, number of query tiles
   bool ragged_kv;       // the key tile straddles Lk
-  bool ragged_last_q;   // the last query tile straddles Lq
+  // rows beyond the valid length have to be cleared: of K_j, of the last Q_i and dO_i (not where the tensors end there: those come as zeros)
+  bool clear_k, clear_q;
   float bias;           // additive bias of the item's batch element
 };
 // record layout in shared memory: 16 ints, the first the item index (-1: no more work).  Read and written 16 bytes at a time: 27 warps read each, and
@@ -359,7 +360,7 @@ __device__ __forceinline__ void bwd_publish_item(int4* rec, int item, const BwdI
   rec[0] = make_int4(item, it.b, it.h, it.kv0);
   rec[1] = make_int4(it.bc, it.tq0, it.tk0, it.key_lim);
   rec[2] = make_int4((int)(uint32_t)((uint64_t)it.acc_base & 0xffffffffull), (int)(uint32_t)((uint64_t)it.acc_base >> 32), it.Lq, it.Lk);
-  rec[3] = make_int4(it.i_begin, it.n_q, (it.ragged_kv ? 1 : 0) | (it.ragged_last_q ? 2 : 0), __float_as_int(it.bias));
+  rec[3] = make_int4(it.i_begin, it.n_q, (it.ragged_kv ? 1 : 0) | (it.clear_k ? 2 : 0) | (it.clear_q ? 4 : 0), __float_as_int(it.bias));
 }
 // (behind the barrier that says that the record is there: the wait is a compiler barrier)
 __device__ __forceinline__ int bwd_load_item(const int4* rec, BwdItem& it) {
@@ -369,7 +370,7 @@ __device__ __forceinline__ int bwd_load_item(const int4* rec, BwdItem& it) {
   it.acc_base = (int64_t)(((uint64_t)(uint32_t)c.y << 32) | (uint64_t)(uint32_t)c.x);
   it.Lq = c.z; it.Lk = c.w;
   it.i_begin = d.x; it.n_q = d.y;
-  it.ragged_kv = (d.z & 1) != 0; it.ragged_last_q = (d.z & 2) != 0; it.bias = __int_as_float(d.w);
+  it.ragged_kv = (d.z & 1) != 0; it.clear_k = (d.z & 2) != 0; it.clear_q = (d.z & 4) != 0; it.bias = __int_as_float(d.w);
   return a.x;
 }
 template <int D>
@@ -407,7 +408,8 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item)
   it.i_begin = p.causal ? j : 0;  // query tiles that can see this key tile (top-left aligned)
   it.n_q = (it.kv0 < it.Lk) ? max(i_end - it.i_begin, 0) : 0;
   it.ragged_kv = it.kv0 + kBwdTileKV > it.Lk;
-  it.ragged_last_q = (it.i_begin + it.n_q) * kBwdTileQ > it.Lq;  // only the last query tile can straddle Lq
+  it.clear_k = it.ragged_kv && (p.cu_q || it.Lk < p.Tk);
+  it.clear_q = (it.i_begin + it.n_q) * kBwdTileQ > it.Lq && (p.cu_q || it.Lq < p.Tq);  // only the last query tile can straddle Lq
   it.bias = item_bias(p.bias, p.bias_scalar, it.b, it.Lk);
   return it;
 }
@@ -739,14 +741,15 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     // ============================================================ item scheduler + TMA producer
     // Rows beyond the valid lengths may hold anything (NaN included).  Masked probabilities are
     // exactly zero, but 0 * NaN is NaN inside an MMA, so the padded rows of every tile that is
-    // contracted over its rows (K_j for dQ, Q_i for dK, dO_i for dV) are cleared in shared memory.
+    // contracted over its rows (K_j for dQ, Q_i for dK, dO_i for dV) are cleared in shared memory - unless the tensor ends with the
+    // valid rows, as beyond it TMA has written zeros.  The products that mind wait for this: with a division per 16 bytes, and all products behind
+    // it, up to 16,000 clocks an item (backward of 24 packed sequences <= 1500, H=8, D=128 260 -> 232 us; B=8 T=300 H=8 D=32 31.0 -> 26.8).  (The loop
+    // stays rolled: unrolled it moves the other roles' code so that B=4 T=4096 H=16 takes 924 us instead of 890.)
     auto zero_rows = [&](uint8_t* tile, int first_bad) {
-      const int n_bad = 128 - first_bad;
-      for (int i = lane; i < n_bad * 8 * (D / 64); i += 32) {
-        const int c = i / (n_bad * 8);
-        const int rem = i % (n_bad * 8);
-        *reinterpret_cast<uint4*>(tile + c * 16384 + (first_bad + rem / 8) * 128 + (rem % 8) * 16) =
-            make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+      for (int at = 128 * first_bad + 16 * lane; at < 128 * 128; at += 512) {
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c) *reinterpret_cast<uint4*>(tile + c * 16384 + at) = make_uint4(0, 0, 0, 0);
       }
     };
     int g = 0;    // query tiles loaded so far (all items)
@@ -822,7 +825,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
               tma_load_4d(smem_base + L::kVOff + kb * kTileBytes + c * 16384, &v_map, bar(L::kKvFull + kb), c * 64, it.h, it.tk0 + it.kv0, it.bc);
             }
           }
-          if (it.ragged_kv) {
+          if (it.clear_k) {
             ok = mbar_wait_warp(bar(L::kKvFull + kb), kph, abort_flag, kSiteBase + 17);
             if (!ok) break;
             zero_rows(smem_gen + L::kKOff + kb * kTileBytes, it.Lk - it.kv0);
@@ -831,7 +834,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
             if (lane == 0) mbar_arrive(bar(L::kKvFix + kb));
           }
         }
-        if (qrow + kBwdTileQ > it.Lq) {
+        if (t == it.n_q - 1 && it.clear_q) {
           ok = mbar_wait_warp(bar(L::kQFull + st), ph, abort_flag, kSiteBase + 18);
           ok = ok && mbar_wait_warp(bar(L::kDoFull + dst), dph, abort_flag, kSiteBase + 19);
           if (!ok) break;
@@ -867,8 +870,6 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     };
     int g = 0;                // query tiles issued so far (all items)
     int act = 0;              // items with work so far
-    uint32_t kvfix_par = 0u;  // bit kb: parity of buffer kb's "padded K rows cleared" (one phase per ragged key tile in it)
-    uint32_t qfix_par = 0u;   // bit st: parity of stage st's "padded Q / dO rows cleared"
     bool ok = true;
     for (int k = 0; ok; ++k) {
       BwdItem it;
@@ -878,20 +879,12 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       const int kb = act % L::kKvBufs;
       const uint32_t kv_off = (uint32_t)kb * kStageStep;  // this item's K_j / V_j buffer, in descriptor address units
       ok = mbar_wait_warp(bar(L::kKvFull + kb), (uint32_t)(act / L::kKvBufs) & 1u, abort_flag, kSiteBase + 3);
-      if (it.ragged_kv) {
-        ok = ok && mbar_wait_warp(bar(L::kKvFix + kb), (kvfix_par >> kb) & 1u, abort_flag, kSiteBase + 20);
-        kvfix_par ^= 1u << kb;
-      }
       for (int t = 0; t < it.n_q && ok; ++t) {
         const int gt = g + t;
         const int st = gt & 1;
         const uint32_t ph = (uint32_t)(gt >> 1) & 1u;  // parity of the stage's "full" barriers
         const uint32_t prev = (uint32_t)(gt - 1) & 1u;
         ok = mbar_wait_warp(bar(L::kQFull + st), ph, abort_flag, kSiteBase + 4);
-        if (t == it.n_q - 1 && it.ragged_last_q) {
-          ok = ok && mbar_wait_warp(bar(L::kQdoFix + st), (qfix_par >> st) & 1u, abort_flag, kSiteBase + 21);
-          qfix_par ^= 1u << st;
-        }
         if constexpr (kTwoS) {
           // this S buffer last held tile g-2: its P^T (read by dV) and then its dQ, until that was drained
           if (gt >= 2) ok = ok && mbar_wait_warp(bar(L::kDqEmpty + sbuf(gt)), spar(gt - 2), abort_flag, kSiteBase + 5);
@@ -945,6 +938,8 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     };
     int g = 0;    // query tiles issued so far (all items)
     int act = 0;  // items with work so far
+    uint32_t kvfix_par = 0u;  // bit kb: parity of buffer kb's "padded K rows cleared" (one phase per ragged key tile in it)
+    uint32_t qfix_par = 0u;   // bit st: parity of stage st's "padded Q / dO rows cleared"
     // who reads the accumulators of an item (0: compute warps, 1: drain warps), for the previous item, and the
     // parity of each of the two hand-back barriers' next phase
     int prev_kind = 0;
@@ -974,6 +969,16 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         // of the stage could still hold the tile of two steps earlier (seen once in some hundred runs on one
         // shape, as dV rows carrying dO of query q - 256 instead of q).
         ok = mbar_wait_warp(bar(L::kDoFull + do_stage(gt)), do_par(gt), abort_flag, kSiteBase + 22);
+        // Rows that are cleared (see the producer): the first products to mind are this warp's.  Scores and dP of padded queries or keys are
+        // masked, whatever their rows hold or change to.
+        if (t == it.n_q - 1 && it.clear_q) {
+          ok = ok && mbar_wait_warp(bar(L::kQdoFix + st), (qfix_par >> st) & 1u, abort_flag, kSiteBase + 21);
+          qfix_par ^= 1u << st;
+        }
+        if (t == 0 && it.clear_k) {
+          ok = ok && mbar_wait_warp(bar(L::kKvFix + kb), (kvfix_par >> kb) & 1u, abort_flag, kSiteBase + 20);
+          kvfix_par ^= 1u << kb;
+        }
         ok = ok && mbar_wait_warp(bar(L::kPReady + sbuf(gt)), spar(gt), abort_flag, kSiteBase + 8);
         if (!ok) break;
         tc_fence_after_sync();

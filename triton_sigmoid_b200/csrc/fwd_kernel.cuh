@@ -561,6 +561,9 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   // gives; the role warps and the output warps need few.  Registers only move within what the CTA was
   // given at launch, so the counts must add up to no more than that (else the increase never returns).
 
+  // Whether rows of V_j beyond the valid keys have to be cleared: not where the tensor ends with those, as TMA has written zeros there.
+  auto clear_v = [&](const FwdItem& it, int j) -> bool { return j * kTileN + kTileN > it.Lk && (p.cu_k || it.Lk < it.key_lim); };
+
   // Consumer side of the item ring: returns the k-th item of this CTA, or -1 when there is none
   // (also on a failed wait).  Called by all 32 lanes of a reader warp.
   auto read_item = [&](int k, FwdItem& it) -> int {
@@ -812,19 +815,17 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           if (!ok) break;
           if (lane == 0) load_v(it, j, st);
         }
-        if (j * kTileN + kTileN > it.Lk) {
+        if (clear_v(it, j)) {
           // The tile straddles the valid key length.  P is zero for the padded keys, but 0 * NaN
           // is NaN inside the MMA, so whatever sits in the padded V rows must be cleared first.
           ok = mbar_wait_warp(bar(L::kVFull + st), ph, abort_flag, kSiteBase + 13);
           if (!ok) break;
-          const int first_bad = it.Lk - j * kTileN;  // in [1, 127]
           uint8_t* vt = smem_gen + L::kVOff + st * kTileBytes;
           // each row is one 128-byte line per 64-column block; the swizzle only permutes within a line
-          for (int i = lane; i < (kTileN - first_bad) * 8 * (D / 64); i += 32) {
-            const int c = i / ((kTileN - first_bad) * 8);
-            const int rem = i % ((kTileN - first_bad) * 8);
-            const int r = first_bad + rem / 8;
-            *reinterpret_cast<uint4*>(vt + c * 16384 + r * 128 + (rem % 8) * 16) = make_uint4(0, 0, 0, 0);
+#pragma unroll 4
+          for (int at = 128 * (it.Lk - j * kTileN) + 16 * lane; at < 128 * kTileN; at += 512) {
+#pragma unroll
+            for (int c = 0; c < D / 64; ++c) *reinterpret_cast<uint4*>(vt + c * 16384 + at) = make_uint4(0, 0, 0, 0);
           }
           fence_proxy_async_smem();
           __syncwarp();
@@ -915,7 +916,7 @@ sigattn_fwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       for (int n = 0; n < n_jobs && ok; ++n) {
         if (c.fresh) {
           ok = mbar_wait_warp(bar(L::kVFull + c.st), c.ph, abort_flag, kSiteBase + 6);
-          if (c.j * kTileN + kTileN > it.Lk) {  // padded V rows are being cleared by the producer warp
+          if (clear_v(it, c.j)) {  // padded V rows are being cleared by the producer warp
             ok = ok && mbar_wait_warp(bar(L::kVFix + c.st), (fix_par >> c.st) & 1u, abort_flag, kSiteBase + 14);
             fix_par ^= 1u << c.st;
           }
