@@ -310,12 +310,10 @@ sigattn_bwd_stream_kernel(const __grid_constant__ CUtensorMap r1_map, const __gr
     // probabilities are exactly zero, but 0 * NaN is NaN inside an MMA, and the streamed rows are what
     // out1 / out2 are contracted over: they are cleared in shared memory.
     auto zero_rows = [&](uint8_t* tile, int first_bad) {
-      const int n_bad = 128 - first_bad;
-      for (int i = lane; i < n_bad * 8 * (D / 64); i += 32) {
-        const int c = i / (n_bad * 8);
-        const int rem = i % (n_bad * 8);
-        *reinterpret_cast<uint4*>(tile + c * 16384 + (first_bad + rem / 8) * 128 + (rem % 8) * 16) =
-            make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+      for (int at = 128 * first_bad + 16 * lane; at < 128 * 128; at += 512) {
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c) *reinterpret_cast<uint4*>(tile + c * 16384 + at) = make_uint4(0, 0, 0, 0);
       }
     };
     int tile = 0;  // streamed tile pairs loaded so far (all items)
