@@ -32,7 +32,8 @@
 // What bounds it (timeline of one SM, B=4 T=4096 H=16): D = 128 shared memory - the operands of S, dP and dQ, which
 // saturate its 128 bytes per clock while they run, the tiles coming in, dS, and dQ going out: 3800 of a tile's 4200
 // clocks (1.70 -> 1.42 ms for the backward when the drain moved from the compute warps to these); D = 64 the two phases
-// of the compute warps with the barriers between them, 2900 clocks (0.85 -> 0.77 ms).
+// of the compute warps with the barriers between them, 2900 clocks (0.85 -> 0.77 ms).  Repeated calls of that size run at the board's power limit,
+// so that what counts there is energy: 850 mJ at D = 64, of them 107 for the phases' arithmetic and 90 for dQ's way out.
 // Two issuing warps, because one warp's instruction stream (waits, 32 MMAs, commits per tile
 // pair) is a serial chain that otherwise bounds the kernel.  Everything the two exchange goes
 // through mbarriers: "S columns free" after dV, "dP columns free" after dK.
@@ -141,14 +142,32 @@ struct BwdSmem {
   static constexpr int kDynBytes = kTotal + 1024;
 };
 
+// Masked tiles (a key or query beyond the valid ones, the causal diagonal): a logit of minus infinity makes a probability of exactly zero on every
+// way, and has no say in the form that a chunk takes, whatever lies in the padded rows (padded batch of 16 <= 2048, H=8, 243 -> 237 us against a general
+// polynomial for all masked tiles, 24 packed sequences, D=128, 231 -> 226, B=40 T=500 H=16 D=128 410 -> 369).  One instantiation for
+// masked and other tiles, with the mask behind a branch, took 205 us for B=40 T=500 H=16 D=64 instead of 242, but 5 to 9 % more where few tiles are masked.
+// Bit i: column q0 + i is a valid query, q_lo <= q < q_hi.
+__device__ __forceinline__ uint32_t bwd_valid_columns(int q0, int q_lo, int q_hi) {
+  const int a = min(max(q_lo - q0, 0), 32), b = min(max(q_hi - q0, 0), 32);
+  const uint32_t below_b = b < 32 ? (1u << b) - 1u : 0xffffffffu, below_a = a < 32 ? (1u << a) - 1u : 0xffffffffu;
+  return below_b & ~below_a;
+}
+__device__ __forceinline__ void bwd_mask_logits(float2 (&t)[16], uint32_t valid) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    t[i].x = (valid & (1u << (2 * i))) ? t[i].x : -INFINITY;
+    t[i].y = (valid & (2u << (2 * i))) ? t[i].y : -INFINITY;
+  }
+}
+
 // The two phases of one tile for one thread (its key row, 32 query columns) in the D = 128 kernel.
 //
 // Phase A: scores -> probabilities, kept in registers for phase B; their 16-bit packing is written over the first 16
 // of the 32 columns read (the operand of dV).  Both phases move 16 columns at a time, so that besides the 32
 // probabilities only few registers are live.
-// q0 = query index of the first column; valid queries for this key row are [q_lo, q_hi).
+// masked: only columns with their bit in `valid` count.
 template <bool kBF16, bool kMask, bool kAccurate, DeepTest kTest>
-__device__ __forceinline__ void bwd_phase_a(uint32_t s_addr, float c1, float c0, int q0, int q_lo, int q_hi,
+__device__ __forceinline__ void bwd_phase_a(uint32_t s_addr, float c1, float c0, uint32_t valid,
                                             float2 (&pv)[16], DeepWatch& watch) {
   // tested tiles work on logits shifted up (see sigmoid2_far)
   const float c0s = kTest == kNoTest ? c0 : c0 + kFarShift;
@@ -160,6 +179,7 @@ __device__ __forceinline__ void bwd_phase_a(uint32_t s_addr, float c1, float c0,
       pv[i] = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), make_float2(c1, c1),
                          make_float2(c0s, c0s));
   }
+  if constexpr (kMask) bwd_mask_logits(pv, valid);
   // f(logits) -> probabilities, in place; eight pairs at a time leave for TMEM
   auto emit = [&](auto f) {
 #pragma unroll
@@ -167,12 +187,7 @@ __device__ __forceinline__ void bwd_phase_a(uint32_t s_addr, float c1, float c0,
       uint32_t pk[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        float2 pe = f(pv[8 * h + i]);
-        if constexpr (kMask) {
-          const int q = q0 + 16 * h + 2 * i;
-          pe.x = (q >= q_lo && q < q_hi) ? pe.x : 0.0f;
-          pe.y = (q + 1 >= q_lo && q + 1 < q_hi) ? pe.y : 0.0f;
-        }
+        const float2 pe = f(pv[8 * h + i]);
         pv[8 * h + i] = pe;
         pk[i] = pack2<kBF16>(pe.x, pe.y);
       }
@@ -236,7 +251,7 @@ __device__ __forceinline__ void bwd_phase_b(uint32_t dp_addr, uint32_t ds_line, 
 // from TMEM in the 16-bit form they were stored in for the dV product, and dS = P (1 - P) dP is formed on
 // packed 16-bit pairs.
 template <bool kBF16, bool kMask, bool kAccurate, DeepTest kTest, DeepRange kRange>
-__device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c0, int q0, int q_lo, int q_hi, DeepWatch& watch) {
+__device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c0, uint32_t valid, DeepWatch& watch) {
   uint32_t r[32];
   tmem_ld32_sync(s_addr, r);
   uint32_t pk[16];
@@ -246,15 +261,11 @@ __device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c
   for (int i = 0; i < 16; ++i)
     t[i] = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), make_float2(c1, c1),
                       make_float2(c0s, c0s));
+  if constexpr (kMask) bwd_mask_logits(t, valid);
   if constexpr (kAccurate) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      float2 pe = sigmoid2_accurate_from_log2(t[i]);
-      if constexpr (kMask) {
-        const int q = q0 + 2 * i;
-        pe.x = (q >= q_lo && q < q_hi) ? pe.x : 0.0f;
-        pe.y = (q + 1 >= q_lo && q + 1 < q_hi) ? pe.y : 0.0f;
-      }
+      const float2 pe = sigmoid2_accurate_from_log2(t[i]);
       pk[i] = pack2<kBF16>(pe.x, pe.y);
     }
   } else if (kTest != kNoTest && warp_all_negative(t)) {
@@ -262,8 +273,11 @@ __device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c
     // the usual case under the default bias: short polynomial, no compare / select per element
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      if constexpr (kRange == kFar) {
+      if constexpr (kRange == kFar && !kMask) {
         pk[i] = sigmoid2_far_packed<kBF16>(t[i], false);
+      } else if constexpr (kRange == kFar) {  // (in single precision: no further from the sigmoid than the general polynomial)
+        const float2 pe = sigmoid2_far<kBF16>(t[i]);
+        pk[i] = pack2<kBF16>(pe.x, pe.y);
       } else {
         const float2 pe = sigmoid2_near<kBF16>(t[i]);
         pk[i] = pack2<kBF16>(pe.x, pe.y);
@@ -286,12 +300,7 @@ __device__ __forceinline__ void bwd_phase_a16(uint32_t s_addr, float c1, float c
     } else {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        float2 pe = sigmoid2_from_log2<kBF16>(t[i]);
-        if constexpr (kMask) {
-          const int q = q0 + 2 * i;
-          pe.x = (q >= q_lo && q < q_hi) ? pe.x : 0.0f;
-          pe.y = (q + 1 >= q_lo && q + 1 < q_hi) ? pe.y : 0.0f;
-        }
+        const float2 pe = sigmoid2_from_log2<kBF16>(t[i]);
         pk[i] = pack2<kBF16>(pe.x, pe.y);
       }
     }
@@ -556,7 +565,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   //            accumulator in two steps, so that its TMEM columns are free for the next dP at once; 512 x 72 + 128 x 56 + 256 x 80).
   // The instructions stand inside the roles' branches: the compiler allocates registers up to a count only in code that it alone leads to.
   // Before a join it kept to 72 everywhere, and all roles spilled (bytes of stores / loads, by -Xptxas -v, general and by head: D = 64 68 / 80
-  // and 132 / 192, now 20 / 16 and 72 / 92; D = 128 120 / 188 and 208 / 300, now 60 / 76 and 148 / 188).  Backward, B=512 T=512 H=16 bf16 2190 ->
+  // and 132 / 192, now 20 / 16 and 72 / 92; D = 128 120 / 188 and 208 / 300, then 60 / 76 and 148 / 188).  Backward, B=512 T=512 H=16 bf16 2190 ->
   // 2060 us, 24 packed sequences <= 1500, H=8, D=128 287 -> 278, B=8 T=8192 H=32 D=128 causal 11.91 -> 11.45 ms at the power cap.
   if (warp >= kBwdFirstDrainWarp) {
     if constexpr (D == 64) setmaxnreg_dec<64>(); else setmaxnreg_inc<80>();
@@ -1089,13 +1098,13 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         constexpr DeepRange kRange = kForm == kDeepNear ? kNear : kFar;
         const bool test_now = kForm == kDeepWatched && !kAccurate && watch.due();
         if constexpr (D == 64) {
-          if (need_mask)     bwd_phase_a16<kBF16, true, kAccurate, kNoTest, kRange>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
-          else if (test_now) bwd_phase_a16<kBF16, false, kAccurate, kTestNow, kRange>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
-          else               bwd_phase_a16<kBF16, false, kAccurate, kTest, kRange>(s_addr, c1, c0, q0, q_lo, q_hi, watch);
+          if (need_mask)     bwd_phase_a16<kBF16, true, kAccurate, kTest, kRange>(s_addr, c1, c0, bwd_valid_columns(q0, q_lo, q_hi), watch);
+          else if (test_now) bwd_phase_a16<kBF16, false, kAccurate, kTestNow, kRange>(s_addr, c1, c0, 0u, watch);
+          else               bwd_phase_a16<kBF16, false, kAccurate, kTest, kRange>(s_addr, c1, c0, 0u, watch);
         } else {
-          if (need_mask)     bwd_phase_a<kBF16, true, kAccurate, kNoTest>(s_addr, c1, c0, q0, q_lo, q_hi, pv, watch);
-          else if (test_now) bwd_phase_a<kBF16, false, kAccurate, kTestNow>(s_addr, c1, c0, q0, q_lo, q_hi, pv, watch);
-          else               bwd_phase_a<kBF16, false, kAccurate, kTest>(s_addr, c1, c0, q0, q_lo, q_hi, pv, watch);
+          if (need_mask)     bwd_phase_a<kBF16, true, kAccurate, kTest>(s_addr, c1, c0, bwd_valid_columns(q0, q_lo, q_hi), pv, watch);
+          else if (test_now) bwd_phase_a<kBF16, false, kAccurate, kTestNow>(s_addr, c1, c0, 0u, pv, watch);
+          else               bwd_phase_a<kBF16, false, kAccurate, kTest>(s_addr, c1, c0, 0u, pv, watch);
         }
         if (kForm == kDeepWatched && !need_mask && !test_now) watch.skipped();
         tmem_st_wait();
