@@ -565,7 +565,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   //            accumulator in two steps, so that its TMEM columns are free for the next dP at once; 512 x 72 + 128 x 56 + 256 x 80).
   // The instructions stand inside the roles' branches: the compiler allocates registers up to a count only in code that it alone leads to.
   // Before a join it kept to 72 everywhere, and all roles spilled (bytes of stores / loads, by -Xptxas -v, general and by head: D = 64 68 / 80
-  // and 132 / 192, now 20 / 16 and 72 / 92; D = 128 120 / 188 and 208 / 300, then 60 / 76 and 148 / 188).  Backward, B=512 T=512 H=16 bf16 2190 ->
+  // and 132 / 192, now 20 / 16 and 68 / 80; D = 128 120 / 188 and 208 / 300, then 60 / 76 and 148 / 188).  Backward, B=512 T=512 H=16 bf16 2190 ->
   // 2060 us, 24 packed sequences <= 1500, H=8, D=128 287 -> 278, B=8 T=8192 H=32 D=128 causal 11.91 -> 11.45 ms at the power cap.
   if (warp >= kBwdFirstDrainWarp) {
     if constexpr (D == 64) setmaxnreg_dec<64>(); else setmaxnreg_inc<80>();
