@@ -84,9 +84,9 @@ __device__ __forceinline__ float2 sigmoid2_far(float2 u) {
   }
   return __fmul2_rn(e, r);
 }
-template <bool kBF16>
+template <bool kBF16, bool kShifted = true>  // (not shifted: of the logits as they are)
 __device__ __forceinline__ float2 sigmoid2_near(float2 u) {
-  constexpr float a = kBF16 ? 0.25f : 0.125f, b = kBF16 ? -0.98041906f * a * a : -0.99429952f * a * a, c = kBF16 ? 0.72727273f * a * a * a : 0.84690567f * a * a * a;
+  constexpr float a = !kShifted ? 1.0f : kBF16 ? 0.25f : 0.125f, b = kBF16 ? -0.98041906f * a * a : -0.99429952f * a * a, c = kBF16 ? 0.72727273f * a * a * a : 0.84690567f * a * a * a;
   const float2 e = make_float2(ex2_approx(u.x), ex2_approx(u.y));
   float2 r = __ffma2_rn(e, make_float2(c, c), make_float2(b, b));
   r = __ffma2_rn(r, e, make_float2(a, a));
@@ -100,6 +100,18 @@ __device__ __forceinline__ bool warp_all_negative(const float2 (&t)[N], int dead
 #pragma unroll
   for (int i = 0; i < N; ++i) sgn &= __float_as_uint(t[i].x) & __float_as_uint(t[i].y);
   return __all_sync(0xffffffffu, ((int)sgn | dead) < 0) != 0;
+}
+
+// The largest of a lane's logits (a NaN does not count).
+template <int N>
+__device__ __forceinline__ float largest(const float2 (&t)[N]) {
+  float a = fmaxf(t[0].x, t[0].y), b = fmaxf(t[1].x, t[1].y);
+#pragma unroll
+  for (int i = 2; i < N; i += 2) {
+    a = fmaxf(a, fmaxf(t[i].x, t[i].y));
+    b = fmaxf(b, fmaxf(t[i + 1].x, t[i + 1].y));
+  }
+  return fmaxf(a, b);
 }
 
 // Whether a warp's next chunk is tested for logits far below zero, in the kDeepWatched forms.  The first chunk of an item is; after
