@@ -771,9 +771,12 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     // contracted over its rows (K_j for dQ, Q_i for dK, dO_i for dV) are cleared in shared memory - unless the tensor ends with the
     // valid rows, as beyond it TMA has written zeros.  The products that mind wait for this: with a division per 16 bytes, and all products behind
     // it, up to 16,000 clocks an item (backward of 24 packed sequences <= 1500, H=8, D=128 260 -> 232 us; B=8 T=300 H=8 D=32 31.0 -> 26.8).  (The loop
-    // stays rolled: unrolled it moves the other roles' code so that B=4 T=4096 H=16 takes 924 us instead of 890.)
+    // stays rolled: unrolled it moves the other roles' code so that B=4 T=4096 H=16 fp16 takes 924 us instead of 890.  The form for bias above -3 at D = 128 is
+    // the other way round, without a row to clear: bf16, bias 0, B=1 T=16384 H=8 2752 us rolled, 2609 unrolled, T=20224 4292, 4099, B=4 T=4096 H=16 1467, 1412; fp16
+    // the same.)
+    constexpr int kClearUnroll = D == 128 && kForm == kDeepWatched ? 4 : 1;
     auto zero_rows = [&](uint8_t* tile, int first_bad) {
-#pragma unroll 1
+#pragma unroll kClearUnroll
       for (int at = 128 * first_bad + 16 * lane; at < 128 * 128; at += 512) {
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) *reinterpret_cast<uint4*>(tile + c * 16384 + at) = make_uint4(0, 0, 0, 0);
