@@ -461,9 +461,9 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   constexpr bool kTwoS = (D == 64);
   // Products per pass of the loops that issue them.  The roles' code together is more than the SM's instruction caches hold: at D = 128 loops of
   // two passes are 1 to 3 % faster for it (B=8 T=8192 H=32 causal 11.21 -> 10.92 ms, B=128 T=512 H=8 573 -> 563 us; four passes or eight 1 to 20 %
-  // slower), at D = 64, whose products are half as long, none is, nor in the form for bias above -3, which is bound by its elementwise phases: B=4 T=4096
-  // H=16 D=128 bias 0 1502 us in loops of two passes, 1461 unrolled (fp16 1526, 1449).
-  constexpr int kMmaUnroll = (D == 64 || kForm == kDeepWatched) ? 8 : 4;
+  // slower), at D = 64, whose products are half as long, none is, nor in the forms whose elementwise phases are longer: bias above -3, B=4 T=4096
+  // H=16 D=128 bias 0 1502 us in loops of two passes, 1461 unrolled (fp16 1526, 1449); accurate sigmoid, B=1 T=20224 H=8 4440, 4188.
+  constexpr int kMmaUnroll = (D == 64 || kForm == kDeepWatched || kAccurate) ? 8 : 4;
   constexpr uint32_t kColS = 0;
   constexpr uint32_t kColDp = kTwoS ? 256 : 128;
   constexpr uint32_t kColDv = kTwoS ? 384 : 256;
