@@ -32,8 +32,10 @@
 // What bounds it (timeline of one SM, B=4 T=4096 H=16): D = 128 shared memory - the operands of S, dP and dQ, which
 // saturate its 128 bytes per clock while they run, the tiles coming in, dS, and dQ going out: 3800 of a tile's 4200
 // clocks (1.70 -> 1.42 ms for the backward when the drain moved from the compute warps to these); D = 64 the two phases
-// of the compute warps with the barriers between them, 2900 clocks (0.85 -> 0.77 ms).  Repeated calls of that size run at the board's power limit,
-// so that what counts there is energy: 850 mJ at D = 64, of them 107 for the phases' arithmetic and 90 for dQ's way out.
+// of the compute warps with the barriers between them, 2900 clocks (0.85 -> 0.77 ms).  Times in these two are of single calls, at 1.8 to 1.9 GHz, bf16.
+// Repeated calls of that size run at the board's power limit, at 1.5 to 1.65 GHz, where a step saves what it saves in energy: B=4 T=4096 H=16 D = 64 takes 850 us
+// at 993 W (time x nvidia-smi's power.draw over a second); left out of it for the purpose, the phases' arithmetic was 107 mJ and dQ's way out 86.
+// Figures of several steps in this file are from different boards and are not to be added up; each pair was timed in turn.
 // Two issuing warps, because one warp's instruction stream (waits, 32 MMAs, commits per tile
 // pair) is a serial chain that otherwise bounds the kernel.  Everything the two exchange goes
 // through mbarriers: "S columns free" after dV, "dP columns free" after dK.
@@ -145,7 +147,7 @@ struct BwdSmem {
 // Masked tiles (a key or query beyond the valid ones, the causal diagonal): a logit of minus infinity makes a probability of exactly zero on every
 // way, and has no say in the form that a chunk takes, whatever lies in the padded rows (padded batch of 16 <= 2048, H=8, 243 -> 237 us against a general
 // polynomial for all masked tiles, 24 packed sequences, D=128, 231 -> 226, B=40 T=500 H=16 D=128 410 -> 369).  One instantiation for
-// masked and other tiles, with the mask behind a branch, took 205 us for B=40 T=500 H=16 D=64 instead of 242, but 5 to 9 % more where few tiles are masked.
+// masked and other tiles, with the mask behind a branch, took 205 us for B=40 T=500 H=16 D=64 where this took 218, but 5 to 9 % more where few tiles are masked.
 // Bit i: column q0 + i is a valid query, q_lo <= q < q_hi.
 __device__ __forceinline__ uint32_t bwd_valid_columns(int q0, int q_lo, int q_hi) {
   const int a = min(max(q_lo - q0, 0), 32), b = min(max(q_hi - q0, 0), 32);
@@ -442,8 +444,7 @@ __device__ __forceinline__ BwdItem bwd_decode_item(const BwdParams& p, int item)
 
 // kByHead: a CTA takes all key tiles of a (batch element, head), in order, and finishes its dQ itself (see the drain
 // warps), so that the accumulator needs neither the fill nor the conversion pass and stays in the L2.  group is 1 and the
-// tickets count (batch, head) pairs.  (This form spills more, see the
-// registers below; the figures of the rule that chooses the form, bwd_by_head(), include that.)
+// tickets count (batch, head) pairs.  (This form spills more, see the registers below.)
 // kForm: as in the forward kernel (at D = 128, where P is in single precision, the far range only).
 template <int D, bool kBF16, bool kAccurate, bool kByHead, DeepForm kForm>
 __global__ void __launch_bounds__(kBwdThreads, 1)
@@ -566,8 +567,9 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   auto read_item = [&](int k, BwdItem& it) -> int {
     const int slot = k & 1;
     if (!mbar_wait_warp(bar(L::kItemFull + slot), (uint32_t)(k >> 1) & 1u, abort_flag, kSiteBase + 30)) return -1;
-    // (of the last record only the -1 holds.  Reading on without a look at it first costs registers less by head and at D = 128, but time
-    // in the general form of D = 64: B=512 T=512 2335 against 2280 us, 24 packed sequences, D=128, 264 against 260, but B=8 T=1000 causal 107.5 against 110.8.)
+    // (Of the last record only the -1 holds.  The general form of D = 64 looks at it before it reads on: B=4 T=4096 H=16 fp16 893 us so, 912 without, T=1024 bf16 534
+    // and 551, 16 padded sequences 246 and 251.  The others read on at once, which spares them registers: by head B=128 T=512 H=16 fp16 598 us so, 618 with
+    // the look, D = 128 B=8 T=8192 H=32 causal 11.4 and 11.8 ms, 24 packed sequences 235 and 238 us.)
     int item = 0;
     if constexpr (D == 64 && !kByHead) item = *reinterpret_cast<const volatile int*>(item_ring + 4 * slot);
     if (item >= 0) item = bwd_load_item(item_ring + 4 * slot, it);
@@ -582,9 +584,10 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   //   D = 128: compute 72, role 56, drain 80 (a dQ tile goes from the drain warps' registers, 64 per thread, to the
   //            accumulator in two steps, so that its TMEM columns are free for the next dP at once; 512 x 72 + 128 x 56 + 256 x 80).
   // The instructions stand inside the roles' branches: the compiler allocates registers up to a count only in code that it alone leads to.
-  // Before a join it kept to 72 everywhere, and all roles spilled (bytes of stores / loads, by -Xptxas -v, general and by head: D = 64 68 / 80
-  // and 132 / 192, now 20 / 16 and 68 / 80; D = 128 120 / 188 and 208 / 300, then 60 / 76 and 148 / 188).  Backward, B=512 T=512 H=16 bf16 2190 ->
-  // 2060 us, 24 packed sequences <= 1500, H=8, D=128 287 -> 278, B=8 T=8192 H=32 D=128 causal 11.91 -> 11.45 ms at the power cap.
+  // Before a join it kept to 72 everywhere, and all roles spilled.  Bytes of stores / loads by -Xptxas -v, general and by head, bf16: D = 64 68 / 80
+  // and 132 / 192 then, 20 / 16 and 68 / 80 now (bias above -3: 32 / 52 and 84 / 96); D = 128 120 / 188 and 208 / 300 then, 56 / 72 and 156 / 188 now (fp16
+  // 40 / 40 and 140 / 156; bias above -3: 80 / 108 and 188 / 236).  Backward, B=512 T=512 H=16 bf16 2190 -> 2060 us, 24 packed sequences <= 1500, H=8, D=128
+  // 287 -> 278, B=8 T=8192 H=32 D=128 causal 11.91 -> 11.45 ms at the power cap.
   if (warp >= kBwdFirstDrainWarp) {
     if constexpr (D == 64) setmaxnreg_dec<64>(); else setmaxnreg_inc<80>();
     // ============================================================ dQ drain
@@ -762,7 +765,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       }
       if (lane == 0) bulk_wait_all();  // every reduction has been performed when the kernel ends
     }
-  } else if (warp >= kBwdComputeWarps) {
+  } else if (warp >= kBwdComputeWarps) {  // (producer, issuers and the idle warp, down to the compute warps' branch)
   setmaxnreg_dec<56>();
   if (warp == kBwdProducerWarp) {
     // ============================================================ item scheduler + TMA producer
@@ -1034,7 +1037,8 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         issue_acc(kColDk, kColDp, q_lo0 + (uint32_t)st * kStageStep, acc0);
         if (kTwoS) mma_commit(leader, bar(L::kDpFree));
         mma_commit(leader, bar(L::kQEmpty + st));
-        // dK_j, dV_j are complete with the last tile's dK: the epilogue need not wait for its dQ
+        // dK_j, dV_j are complete with the last tile's dK: to take them out of TMEM the epilogue need not wait for the last dQ.  (At D = 128 it
+        // waits for that before it writes over the shared-memory copy of dS, which the product still reads.)
         if (t == it.n_q - 1) mma_commit(leader, bar(L::kDkvFull));
         if constexpr (!kTwoS) {
           // the dQ GEMM needs the previous dQ tile read out of its columns
@@ -1054,7 +1058,7 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       g += it.n_q;
       ++act;
     }
-  }
+  }  // (issuer B)
   } else {
     if constexpr (D == 64) setmaxnreg_inc<80>();
     // ============================================================ compute warps
@@ -1108,7 +1112,8 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         // valid queries for this key row: q_lo <= q < q_hi (empty when the key row is padding)
         const int q_lo = p.causal ? kv : 0;
         const int q_hi = row_ok ? Lq : 0;
-        // warp-uniform on purpose: the two instantiations contain warp-collective TMEM accesses
+        // warp-uniform on purpose: the two instantiations contain warp-collective TMEM accesses.  True for every tile with rows that the producer
+        // clears (clear_k implies ragged_kv, clear_q reaches columns from Lq on only): those rows may change while S^T and dP^T are computed from them.
         const bool need_mask = it.ragged_kv || (q0 + 32 > Lq) || (p.causal && q0 < kv0 + kBwdTileKV - 1);
         float2 pv[16];  // D = 128 only: the probabilities of this tile
         ok = mbar_wait_warp(bar(L::kSFull + sbuf(gt)), spar(gt), abort_flag, kSiteBase + 12);
@@ -1155,8 +1160,8 @@ sigattn_bwd_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       if (!ok) break;
 
       // ------------------------------------------------------------ epilogue of the item
-      // (before the drain of the last dQ tile, whose product is still running); short items' at D = 64 is the
-      // drain warps' (kDrainEpilogueMaxTiles<D>): nothing of the accumulators is needed here then
+      // (before the drain of the last dQ tile; at D = 128 its product may still be running while the accumulators are read, but not while rows
+      // are turned through dS); short items' at D = 64 is the drain warps' (kDrainEpilogueMaxTiles<D>): nothing of the accumulators is needed here then
       // column groups 0,1 store dV, groups 2,3 store dK (each half of the head dimension)
       if (n_q <= kDrainEpilogueMaxTiles<D>) {
         // (no arrival either: each of the two hand-back barriers is arrived on only by the warps that read the

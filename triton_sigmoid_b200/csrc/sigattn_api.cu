@@ -543,6 +543,12 @@ int launch_fwd(const SigAttnParams* p, const CUtensorMap& qm, const CUtensorMap&
 //    average of 0.3 of it; the general form's passes only cover the rows there are).  Some of 768 tokens among many of 128
 //    1.12 - 1.21, of 192 1.02 - 1.05, of 256 0.92 - 1.07; of 512 tokens 1.01 - 1.13, 0.95 - 1.09, 0.91 - 0.98.  This also covers that
 //    the accumulator must have room for a region per CTA.  (Padded, 768 among 96: 0.71 - 0.89.)
+// Both forms have become faster since, the general one more so at D = 64.  Forced again (bf16, by head over general; 640 to 4800 pairs, equal lengths or packed):
+//  - Tq, D = 64: 0.82 - 0.89 up to 256, 0.88 - 0.99 up to 512, 0.91 at 700, 1.03 at 768, 0.99 - 1.04 at 900 and 1000, 1.10 - 1.15 at 1024; causal 0.87 - 0.97 up to
+//    1200, 1.01 at 1500.  D = 128: 0.60 - 0.87 up to 256, 0.98 at 384, 1.06 - 1.10 at 448 to 512, causal 0.88 at 512, 1.13 at 1000.
+//  - Tk, D = 64: 64 queries 0.97 / 1.03 / 1.06 - 1.07 / 1.08 - 1.10 with 2 / 4 / 8 / 16 key tiles, 256 queries 0.94 / 1.01 - 1.02 / 1.07 - 1.09 with 4 / 8 / 16; the rule still takes
+//    some of the slower ones.  D = 128: 0.88 / 0.95 / 1.00 - 1.03 / 1.04 - 1.06 and 0.93 / 1.00 / 1.03 - 1.04.  Causal, 128 queries on 512 keys 0.96 and 0.77.
+//  - packed, D = 64 0.83 - 0.92; D = 128 0.81 - 0.93 up to 384, causal 0.83 - 0.88 at 512; at 512 and 700 (not taken) 1.01 - 1.06.
 // The accurate sigmoid, an option for comparisons, has the general form only.
 bool bwd_by_head(const SigAttnParams* p, int n_sm) {
   const bool causal = (p->flags & SIGATTN_CAUSAL) != 0, wide = p->D == 128;
